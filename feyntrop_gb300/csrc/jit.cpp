@@ -26,46 +26,59 @@ namespace ft {
 
 static const char* kArch = "--gpu-architecture=sm_103a";
 
+unsigned scratch_slots(const kernel_key& k)
+{
+    const unsigned E = (unsigned)k.E;
+    if (k.mode == 0) return 4u * E;   // two samples
+    return 2u * E + (k.scratch >= 1 ? 2u * E : 0u) + (k.scratch >= 2 ? E * (E + 1u) / 2u : 0u);
+}
+
 unsigned table_smem_bytes(const kernel_key& k)
 {
-    // staged table (unless read from global memory), then the per-thread accumulators:
-    // FP64 form two doubles per slot; mixed form two doubles and two floats per slot and
-    // four sample counters (a double and a float each)
+    // staged table (unless read from global memory): 1/r (FP64, or two floats), a word per
+    // subgraph and the cut thresholds (E 2^(E-1)); then the sums: FP64 form two doubles per
+    // slot and thread, mixed form two floats per slot and thread, two doubles per slot and
+    // warp, and the threads' scratch
     const unsigned entries = 1u << k.E;
-    const unsigned tab = k.table_global ? 0u : (k.prec == 0 ? 25u * entries : 17u * entries);
-    const unsigned parts = k.mode == 1 ? 4u : 2u;
-    const unsigned acc = (unsigned)k.block * (parts * (unsigned)k.K * (k.prec == 0 ? 16u : 24u) + (k.prec == 0 ? 0u : 48u));
-    return ((tab + 15u) & ~15u) + acc;
+    const unsigned tab = k.table_global ? 0u : (12u + 2u * (unsigned)k.E) * entries;
+    const unsigned slots = (k.mode == 1 ? 4u : 2u) * (unsigned)k.K, block = (unsigned)k.block;
+    const unsigned acc = k.prec == 0 ? 16u * slots * block
+                                     : 8u * slots * block + 16u * slots * (block / 32u) + 4u * block * scratch_slots(k);
+    return ((tab + 15u) & ~15u) + acc + 16u;
 }
 
 // Tables of the two-float logarithm, exponential and sine / cosine of the mixed kernels
 // (FP32 values written exactly as hexadecimal literals):
-//   FT_LOGTAB[3i .. 3i+2] = r_i = fl(1 / (1 + (i + 1/2)/64)), -log(r_i) as hi, lo (i < 64)
-//   FT_EXPTAB[2j .. 2j+1] = 2^(j/32) as hi, lo (j < 32)
-//   FT_SCTAB[4j .. 4j+3]  = sin(j pi/64) as hi, lo, cos(j pi/64) as hi, lo (j < 128)
+//   FT_LOGTAB[i] = r_i = fl(1 / (1 + (i + 1/2)/64)), -log(r_i) as hi, lo, 0 (i < 64)
+//   FT_EXPTAB[j] = 2^(j/32) as hi, lo (j < 32)
+//   FT_SCTAB[j] = sin(j pi/64) as hi, lo, cos(j pi/64) as hi, lo (j < 128)
 static std::string tables_source()
 {
     static const std::string text = [] {
         std::ostringstream s;
         char buf[64];
-        s << "__device__ const float FT_LOGTAB[192] = {";
+        s << "__device__ const float4 FT_LOGTAB[64] = {";
         for (int i = 0; i < 64; i++) {
             const float r = (float)(1.0 / (1.0 + (i + 0.5) / 64.0));
             const double nl = -std::log((double)r);
             const float hi = (float)nl, lo = (float)(nl - (double)hi);
-            for (float v : {r, hi, lo}) {
+            s << "{";
+            for (float v : {r, hi, lo, 0.0f}) {
                 std::snprintf(buf, sizeof buf, "%af,", (double)v);
                 s << buf;
             }
+            s << "},";
         }
-        s << "};\n__device__ const float FT_EXPTAB[64] = {";
+        s << "};\n__device__ const float2 FT_EXPTAB[32] = {";
         for (int j = 0; j < 32; j++) {
             const double t = std::exp2(j / 32.0);
             const float hi = (float)t, lo = (float)(t - (double)hi);
+            s << "{";
             for (float v : {hi, lo}) {
                 std::snprintf(buf, sizeof buf, "%af,", (double)v);
                 s << buf;
             }
+            s << "},";
         }
         s << "};\n__device__ const float4 FT_SCTAB[128] = {";
         const double pi = 3.14159265358979323846;
@@ -131,6 +144,7 @@ std::string kernel_source(const kernel_key& k)
     s << "#define FT_BLOCK " << k.block << "\n#define FT_TABLE_GLOBAL " << k.table_global << "\n";
     s << "#define FT_MINB " << k.minb << "\n#define FT_VARIANT " << k.variant << "\n";
     s << "#define FT_BATCH " << k.batch << "\n#define FT_XA_DIGITS " << kExactDigits << "\n";
+    s << "#define FT_SCRATCH " << k.scratch << "\n";
     s << "#define FT_Q0 " << k.q0 << "\n";
     s << "__device__ constexpr int FT_EK[" << k.E << "] = {";
     for (int e = 0; e < k.E; e++) s << (e ? "," : "") << k.ek[e];
@@ -142,7 +156,7 @@ std::string kernel_source(const kernel_key& k)
         elimination_pattern(k, nz, nzg, nzm);
         const int n = k.V - 1;
         auto matrix = [&](const char* name, const std::vector<int>& m) {
-            s << "__device__ constexpr unsigned char " << name << "[" << n << "][" << n << "] = {";
+            s << "__device__ constexpr signed char " << name << "[" << n << "][" << n << "] = {";
             for (int i = 0; i < n; i++) {
                 s << "{";
                 for (int j = 0; j < n; j++) s << (j ? "," : "") << m[i * n + j];
@@ -150,11 +164,40 @@ std::string kernel_source(const kernel_key& k)
             }
             s << "};\n";
         };
+        // contributions to each conductance (edges, then fill by eliminated vertices)
+        std::vector<int> cf((size_t)n * n, n), cs((size_t)n * n, 0), gf(n, n), gs(n, 0);
+        for (int e = 0; e < k.E; e++) {
+            const int a = k.ek[e], b = k.el[e];
+            (a == k.V - 1 ? gf[b] : cf[b * n + a]) = -1;
+            (a == k.V - 1 ? gs[b] : cs[b * n + a])++;
+        }
+        for (int m = 0; m < n; m++)
+            for (int i = m + 1; i < n; i++) {
+                if (!nz[m * n + i]) continue;
+                if (nzg[m]) {
+                    gf[i] = std::min(gf[i], m);
+                    gs[i]++;
+                }
+                for (int j = i + 1; j < n; j++)
+                    if (nz[m * n + j]) {
+                        cf[i * n + j] = std::min(cf[i * n + j], m);
+                        cs[i * n + j]++;
+                    }
+            }
+        for (int& x : cs) x = x > 1;
+        for (int& x : gs) x = x > 1;
+        auto row = [&](const char* name, const std::vector<int>& m) {
+            s << "__device__ constexpr signed char " << name << "[" << n << "] = {";
+            for (int i = 0; i < n; i++) s << (i ? "," : "") << m[i];
+            s << "};\n";
+        };
+        matrix("FT_CF", cf);
+        matrix("FT_CS", cs);
+        row("FT_GF", gf);
+        row("FT_GS", gs);
         matrix("FT_NZC", nz);
         matrix("FT_NZM", nzm);
-        s << "__device__ constexpr unsigned char FT_NZG[" << n << "] = {";
-        for (int i = 0; i < n; i++) s << (i ? "," : "") << nzg[i];
-        s << "};\n#define FT_HAVE_PATTERN 1\n";
+        row("FT_NZG", nzg);
     }
     s << tables_source();
     s << ft_sample_body_source;
@@ -324,7 +367,7 @@ static std::string key_string(const kernel_key& k)
     std::ostringstream s;
     s << k.E << "," << k.V << "," << k.K << "," << k.loops << "," << k.rank << "," << k.prec << "," << k.mode << ","
       << k.only_psi << "," << k.record << "," << k.block << "," << k.table_global << "," << k.minb << "," << k.variant
-      << "," << k.batch << "," << k.q0;
+      << "," << k.batch << "," << k.q0 << "," << k.scratch;
     for (int e = 0; e < k.E; e++) s << ";" << k.ek[e] << "-" << k.el[e];
     return s.str();
 }

@@ -25,9 +25,15 @@ struct kernel_key {
     int minb = 1;           // minimum resident blocks per SM asked of the register allocator
     int variant = 0;        // code-size options of the kernel body (FT_VARIANT)
     int batch = 0;          // 1: the batch kernels (many integrals of the topology per launch)
+    int scratch = 0;        // mixed: what the threads' shared-memory scratch holds (FT_SCRATCH of the kernel body)
     int q0 = 0;             // reduced vertices [0, q0) carry no external momentum (zero rows of P~)
     std::vector<int> ek, el;   // endpoints in the kernel's vertex labels, ek > el
 };
+
+// Graphs of up to 12 edges stage their table in shared memory, with the cut thresholds (E
+// 2^(E-1) words: 98 KB of 147 at E = 12, beside the sums); larger ones read it from global
+// memory and find cuts by a running-sum scan over Jr/r, 12 times smaller.
+inline bool staged_table(int E) { return E <= 12; }
 
 struct kernel_set {
     CUmodule module = nullptr;
@@ -48,7 +54,10 @@ std::string kernel_source(const kernel_key& key);
 // directory of the compiled-kernel cache (and of the launch-shape tuning table)
 std::string cache_dir();
 
-// shared memory the kernel stages the table into (0 when read from global memory)
+// floats per thread in the shared-memory scratch of the mixed form
+unsigned scratch_slots(const kernel_key& key);
+
+// dynamic shared memory of a block: the staged table, the sums, the scratch
 unsigned table_smem_bytes(const kernel_key& key);
 
 struct driver_api {

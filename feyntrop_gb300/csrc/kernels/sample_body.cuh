@@ -78,22 +78,17 @@ typedef unsigned int u32;
 #ifndef FT_VARIANT
 #define FT_VARIANT 0
 #endif
-#if (FT_VARIANT & 1) && !defined(FT_HOST_SIM)
+#if (FT_VARIANT & 1)
 #define FT_MATHFN __noinline__
 #else
 #define FT_MATHFN __forceinline__
 #endif
-#if (FT_VARIANT & 2) && !defined(FT_HOST_SIM)
-#define FT_DFFN __noinline__
-#else
-#define FT_DFFN __forceinline__
-#endif
-#if (FT_VARIANT & 8) && !defined(FT_HOST_SIM)
+#if (FT_VARIANT & 8)
 #define FT_BIGFN __noinline__
 #else
 #define FT_BIGFN __forceinline__
 #endif
-#if (FT_VARIANT & 16) && !defined(FT_HOST_SIM)
+#if (FT_VARIANT & 16)
 #define FT_CXFN __noinline__
 #else
 #define FT_CXFN __forceinline__
@@ -117,16 +112,18 @@ static __device__ FT_MATHFN float m_atan(float x) { return atanf(x); }
 // Structural pattern of the eliminations, generated per topology: NZC(i, j) (i < j) a
 // conductance between i and j that can be non-zero when i is eliminated (an edge or
 // fill), NZG(i) a conductance to ground, NZM(i, j) an entry of M^-1 that can be
-// non-zero.  Updates on structural zeros are left out (without the tables: dense).
-#ifdef FT_HAVE_PATTERN
+// non-zero.  Updates on structural zeros are left out.
 #define NZC(i, j) (FT_NZC[i][j] != 0)
 #define NZG(i) (FT_NZG[i] != 0)
 #define NZM(i, j) (FT_NZM[i][j] != 0)
-#else
-#define NZC(i, j) true
-#define NZG(i) true
-#define NZM(i, j) true
-#endif
+// Contributions to a conductance come from edges, then from eliminated vertices: FT_CF[i][j]
+// (FT_GF[i] for the ground) is the first of those vertices, -1 with an edge before; the
+// first contribution is assigned, not added to zero.  FT_CS, FT_GS: more than one
+// contribution (a sum, which the two-float forms renormalise before it is used).
+#define ADDS_C(k, i, j) (FT_CF[i][j] < (k))
+#define ADDS_G(k, i) (FT_GF[i] < (k))
+#define SUMS_C(i, j) (FT_CS[i][j] != 0)
+#define SUMS_G(i) (FT_GS[i] != 0)
 // edge e is the first to contribute to its conductance slot (the pair of endpoints, or
 // the ground slot of its lower endpoint): its conductance is assigned, not added to zero
 static __device__ constexpr bool first_in_slot(int e)
@@ -157,21 +154,36 @@ static __device__ constexpr bool first_in_slot(int e)
 #define P_SIZE (P_PT + FT_NE * (FT_NE + 1) / 2)
 // entry (j, k), j <= k, of the external block of P~ (indices from Q0)
 #define PT_AT(j, k) (P_PT + (j) * FT_NE - (j) * ((j) - 1) / 2 + ((k) - (j)))
-// the same block as floats follows at prm + P_SIZE, then as two-float (hi, lo) pairs at
-// prm + P_SIZE + (P_SIZE + 1) / 2 (the mixed form reads only those two)
+// the same block as floats follows at prm + P_SIZE, then in two-float as (hi, hi, lo, lo)
+// float4s at prm + P_PAIR (the mixed form reads only those two)
+#define P_PAIR ((P_SIZE + (P_SIZE + 1) / 2 + 1) & ~1)
 
 // ------------------------------------------------------------------ table layout
-// [w64 | Jr64 | rinv64 : 8 bytes each][meta : 1 byte][pad to 16][w32 | Jr32 : 4 bytes each]
-// [rinv32 : (hi, lo) float pairs]
+// [w64 | Jr64 | rinv64 : 8 bytes each][pad to 16][rinv32 hi | rinv32 lo | meta : 4 bytes each]
+// then the cut thresholds (FT_CUT: one u32 per edge of every subgraph, see find_cut) or,
+// for tables read from global memory, [w32 | Jr32 : 4 bytes each] for the running-sum
+// scan.  meta: offset of the subgraph's thresholds << 16 | mass-momentum spanning << 7 |
+// loop number.
 #define T_ENTRIES (1u << FT_E)
 #define T_W64 0
 #define T_JR64 (8u * T_ENTRIES)
 #define T_RI64 (16u * T_ENTRIES)
-#define T_META (24u * T_ENTRIES)
-#define T_F32 ((25u * T_ENTRIES + 15u) & ~15u)
-#define T_W32 (T_F32)
-#define T_JR32 (T_F32 + 4u * T_ENTRIES)
-#define T_RI32 (T_F32 + 8u * T_ENTRIES)   // (hi, lo) float pairs: 1/r in two-float
+#define T_F32 ((24u * T_ENTRIES + 15u) & ~15u)
+#define T_RH32 (T_F32)                    // 1/r in two-float: high parts, low parts
+#define T_RL32 (T_F32 + 4u * T_ENTRIES)
+#define T_META (T_F32 + 8u * T_ENTRIES)
+#define T_Q (T_F32 + 12u * T_ENTRIES)
+#define T_W32 (T_F32 + 12u * T_ENTRIES)
+#define T_JR32 (T_F32 + 16u * T_ENTRIES)
+#define FT_CUT (!FT_TABLE_GLOBAL)
+#if FT_CUT
+#define T_QBYTES (2u * FT_E * T_ENTRIES)  // E 2^(E-1) thresholds
+#else
+#define T_QBYTES 0u
+#endif
+#define META_OFF(m) ((m) >> 16)
+#define META_MM(m) (((m) >> 7) & 1u)
+#define META_L(m) ((m) & 127u)
 
 // ------------------------------------------------------------------ accumulator slots
 // per eps order j: [8j + 0..7] = re S1 (hi, lo), re S2 (hi, lo), im S1 (hi, lo), im S2 (hi, lo)
@@ -237,11 +249,7 @@ static __device__ __forceinline__ cx<T> operator*(T s, cx<T> a) { return cmk(s *
 // reciprocals: IEEE division in FP64; the correctly rounded reciprocal instruction
 // sequence in FP32 (a division there expands to a long inline sequence)
 static __device__ __forceinline__ double rcp_(double x) { return 1.0 / x; }
-#ifdef FT_HOST_SIM
-static __device__ __forceinline__ float rcp_(float x) { return 1.0f / x; }
-#else
 static __device__ __forceinline__ float rcp_(float x) { return __frcp_rn(x); }
-#endif
 template <class T>
 static __device__ __forceinline__ cx<T> crecip(cx<T> z)
 {
@@ -648,10 +656,11 @@ static __device__ __noinline__ void robust_derivatives(const double* X, const do
 
 // ------------------------------------------------------------------ sector draw, FP64
 struct table_ref {
-    const void* w;              // staged copies (shared memory): w, Jr, 1/r in the working precision
-    const void* Jr;
-    const void* ri;
-    const unsigned char* meta;  // mm << 7 | loop number
+    const void* q;              // cut thresholds (w in the working precision where FT_CUT is 0)
+    const void* Jr;             // Jr in the working precision (FT_CUT 0 only)
+    const void* ri;             // 1/r in FP64, or its two-float high parts
+    const float* rl;            // two-float low parts of 1/r (mixed)
+    const u32* meta;
     const unsigned char* gm;    // global copy (FP64 sections for exact re-checks)
 };
 
@@ -662,6 +671,7 @@ struct table_ref {
 __shared__ unsigned long long s_batch_item;
 __shared__ const unsigned char* s_batch_tab;
 #define TABLE_GM(t) s_batch_tab
+#define FT_EXACT_TABLE(t) ((t).gm ? (t).gm : s_batch_tab)
 // first word of an FP64-pass queue entry: item << 28 | lane << 18 | offset of the
 // sample in the lane's chunk (the other four hold the sample's stream state)
 #define BQ_ITEM_SHIFT 28
@@ -670,189 +680,13 @@ __shared__ const unsigned char* s_batch_tab;
 #define BQ_LANE_MASK 1023ull
 #else
 #define TABLE_GM(t) ((t).gm)
+#define FT_EXACT_TABLE(t) ((t).gm)
 #endif
 
-static __device__ __forceinline__ void draw_sector64(xo& g, const table_ref& t, double Jr_full, double* X, double& F,
-                                                     double& Gv, unsigned char* ord)
-{
-    const double* w = (const double*)t.w;
-    const double* Jr = (const double*)t.Jr;
-    const double* ri = (const double*)t.ri;
-    const unsigned char* meta = t.meta;
-    u32 sub = FT_FULL;
-    double JJr = Jr_full, XX = 1.0;
-    bool MM = true;
-    int oL = FT_LOOPS;
-    F = 1.0;
-    Gv = 0.0;
-#pragma unroll
-    for (int j = 0; j < FT_E; j++) {
-        const double R = u01(g.next()) * JJr;
-        double T = 0.0;
-        int e = 0;
-        // the subgraph's edges in ascending order (its set bits) until the running sum
-        // passes R, else the last one
-        for (u32 left = sub; left != 0u; left &= left - 1u) {
-            e = __ffs(left) - 1;
-            T += w[sub ^ (1u << e)];
-            if (T > R) break;
-        }
-        sub ^= 1u << e;
-        JJr = Jr[sub];
-        const double rinv = ri[sub];
-        const unsigned m = meta[sub];
-        const bool mm = (m >> 7) != 0;
-        const int L = (int)(m & 127u);
-        if (MM && !mm) Gv = XX;
-        MM = mm;
-#pragma unroll
-        for (int k = 0; k < FT_E; k++)
-            if (k == e) X[k] = XX;
-        if (L < oL) {
-            F *= XX;
-            oL = L;
-        }
-        if (FT_RECORD) ord[j] = (unsigned char)e;
-        if (j < FT_E - 1) XX *= pow(1.0 - u01(g.next()), rinv);
-    }
-}
-
-// ------------------------------------------------------------------ sector draw, mixed
-// two-float value hi + lo
-struct f2 {
-    float hi, lo;
-};
-static __device__ __forceinline__ f2 f2_add(f2 a, float b)
-{
-    float s = a.hi + b;
-    float bb = s - a.hi;
-    float err = (a.hi - (s - bb)) + (b - bb);
-    float lo = a.lo + err;
-    float h = s + lo;
-    f2 r;
-    r.hi = h;
-    r.lo = lo - (h - s);
-    return r;
-}
-static __device__ __forceinline__ f2 f2_add2(f2 a, f2 b)
-{
-    f2 r = f2_add(a, b.hi);
-    return f2_add(r, b.lo);
-}
-
-// log(1 - u) for u = (x >> 11) 2^-53, to about 1e-7 absolute (undeformed integrands), with integer and FP32
-// instructions only (64-bit integer to float conversions would run on the FP64 pipe).
-// A positive integer v is turned into the float bits of 2^k (1 + f) directly: k from
-// the leading-zero count, f from the next 23 bits rounded (a carry bumps k).
-static __device__ __forceinline__ int float_bits_of(u64 v, int scale_exp)
-{
-    const int lz = __clzll(v);
-    const u64 frac = ((((v << lz) << 1) >> 40) + 1ull) >> 1;   // 23 bits after the leading 1, rounded
-    return ((63 - lz + scale_exp + 127) << 23) + (int)frac;
-}
-
-static __device__ __forceinline__ f2 log1m_u32(u64 x)
-{
-    const u64 m = x >> 11;
-    f2 r;
-    r.lo = 0.0f;
-    if (m < (1ull << 52)) {
-        // u < 1/2: log1p(-u)
-        r.hi = m ? m_log1p(-__int_as_float(float_bits_of(m, -53))) : 0.0f;
-        return r;
-    }
-    // 1 - u = q 2^-53 exactly (q < 2^52); q = 2^k (1 + f): log(1 - u) = (k - 53) ln2 + log1p(f)
-    const int bits = float_bits_of((1ull << 53) - m, 0);
-    const int k = (bits >> 23) - 127;
-    const float f = __int_as_float((bits & 0x007fffff) | 0x3f800000) - 1.0f;
-    const float kk = (float)(k - 53);
-    // ln2 split so that kk * LN2_HI is exact
-    const float LN2_HI = 0.693145751953125f, LN2_LO = 1.42860682030941723212e-6f;
-    f2 a;
-    a.hi = kk * LN2_HI;
-    a.lo = kk * LN2_LO;
-    return f2_add(a, m_log1p(f));
-}
-
-static __device__ __forceinline__ f2 f2_two_sum(float a, float b)
-{
-    const float s = a + b;
-    const float bb = s - a;
-    f2 r;
-    r.hi = s;
-    r.lo = (a - (s - bb)) + (b - bb);
-    return r;
-}
-
-// log(1 - u) for u = (x >> 11) 2^-53 in two-float, to about 1e-12 absolute, with integer
-// and FP32 instructions only (64-bit conversions and FP64 would run on the FP64 pipe).
-// Table-driven reduction after Tang (ACM TOMS 16, 1990): 1 - u = q 2^-53 with the
-// integer q = 2^53 - (x >> 11) exactly, q = 2^k M with M in [1, 2) held as two floats
-// (47 fraction bits); c_i = 1 + (i + 1/2)/64 for the top 6 fraction bits i,
-// r_i = fl(1/c_i) and -log r_i (two-float) from FT_LOGTAB; z = M r_i - 1 (|z| < 1/100)
-// from exact products, log M = -log r_i + log1p(z) with log1p(z) = z - z^2/2 + z^3/3 -
-// z^4/4 + z^5/5, the terms past z in FP32.
-static __device__ FT_BIGFN f2 log1m_u2(u64 x)
-{
-    const u64 q = (1ull << 53) - (x >> 11);   // 1 .. 2^53
-    const int lz = __clzll(q);
-    const u64 mb = q << lz;                    // M = mb / 2^63, leading 1 at bit 63
-    const u32 top = (u32)(mb >> 40);           // 1 + 23 fraction bits
-    const float m_hi = __int_as_float(0x3f800000 | (int)(top & 0x7fffffu));
-    const float m_lo = (float)(u32)((mb >> 16) & 0xffffffull) * 0x1.0p-47f;
-    const int i = (int)((top >> 17) & 63u);
-    const float r = FT_LOGTAB[3 * i], nl_hi = FT_LOGTAB[3 * i + 1], nl_lo = FT_LOGTAB[3 * i + 2];
-    // z = M r - 1: m_hi r = p + e exactly, p - 1 exact (p within 1% of 1)
-    const float p = m_hi * r;
-    const float e = fmaf(m_hi, r, -p);
-    const f2 z = f2_two_sum(p - 1.0f, fmaf(m_lo, r, e));
-    const float zh = z.hi;
-    const float tail = zh * zh * fmaf(zh, fmaf(zh, fmaf(zh, 0.2f, -0.25f), 0.333333343f), -0.5f);
-    // (k - 53) ln2 with ln2 in three parts (LN2_HI has 16 bits: the products are exact)
-    const float kk = (float)(10 - lz);          // k - 53 with k = 63 - lz
-    const float LN2_HI = 0.693145751953125f, LN2_LO = 1.428606765330187e-06f, LN2_LO2 = 5.497923e-14f;
-    f2 acc = f2_two_sum(kk * LN2_HI, nl_hi);
-    acc = f2_add(acc, fmaf(kk, LN2_LO, nl_lo));
-    acc = f2_add(acc, fmaf(kk, LN2_LO2, z.lo + tail));
-    return f2_add(acc, zh);
-}
-
-// e^a for a two-float a (|a| < 80) in two-float, about 1e-12 relative; table-driven
-// after Tang (ACM TOMS 15, 1989): a = (32 m + j) ln2/32 + s with |s| <= ln2/64,
-// e^a = 2^m 2^(j/32) e^s, 2^(j/32) as two floats from FT_EXPTAB, e^s = 1 + s + s^2/2 +
-// s^3/6 + s^4/24 with the terms past s in FP32.  ln2/32 = C1 + C2 + C3, C1 with 11
-// significant bits so that k C1 is exact for |k| < 2^13.
-static __device__ FT_BIGFN f2 exp_f2(f2 a)
-{
-    const float C1 = 0x1.62cp-6f, C2 = 0x1.217f7ep-17f, C3 = -0x1.c610cap-42f;
-    const float kf = rintf(a.hi * 46.1662407f);
-    const int k = (int)kf;
-    // a - k C1 is exact; k C2 = p2 + e2 exactly
-    const float p2 = kf * C2;
-    const float e2 = fmaf(kf, C2, -p2);
-    f2 sv = f2_two_sum(fmaf(-kf, C1, a.hi), -p2);
-    sv = f2_add(sv, fmaf(-kf, C3, a.lo - e2));
-    const float sh = sv.hi;
-    const float tail = sh * sh * fmaf(sh, fmaf(sh, 0.0416666679f, 0.166666672f), 0.5f);
-    // e^s = 1 + es
-    f2 es = f2_two_sum(sh, sv.lo + tail);
-    es = f2_add(f2_two_sum(1.0f, es.hi), es.lo);
-    const int j = k & 31, m = k >> 5;
-    const float t_hi = FT_EXPTAB[2 * j], t_lo = FT_EXPTAB[2 * j + 1];
-    // (t_hi + t_lo)(es.hi + es.lo) with the product error of the leading term
-    const float ph = t_hi * es.hi;
-    const float pl = fmaf(t_hi, es.hi, -ph) + fmaf(t_hi, es.lo, t_lo * es.hi);
-    const f2 pr = f2_two_sum(ph, pl);
-    const float sc = __int_as_float((127 + m) << 23);   // 2^m, |m| < 126
-    f2 out;
-    out.hi = pr.hi * sc;
-    out.lo = pr.lo * sc;
-    return out;
-}
-
-// The reference's comparison, exactly (FP64, ascending edges, first running sum above
-// u * Jr(gamma), else the last edge): used when an FP32 comparison is within its
-// error margin.  Out of line: it runs for a few steps per 1e4 samples.
+// The reference's comparison, exactly (srcs/tropical_sampling.hpp:468-501: FP64 running
+// sums of Jr/r in ascending edge order, the first above u * Jr(gamma), else the last
+// edge): used when a threshold comparison cannot decide.  Out of line: it runs for a
+// few steps per 1e4 samples at most.
 static __device__ __noinline__ int exact_cut(u64 x, u32 sub, const unsigned char* __restrict__ gm)
 {
     const double* w64 = (const double*)(gm + T_W64);
@@ -870,84 +704,100 @@ static __device__ __noinline__ int exact_cut(u64 x, u32 sub, const unsigned char
     return cut;
 }
 
-static __device__ __forceinline__ int draw_sector32(xo& g, const table_ref& t, const float* pf, f2* lx, f2& lF,
-                                                    f2& lG, unsigned char* ord)
+#if FT_CUT
+// The cut of a subgraph of n edges for the draw x, h = x >> 32: the first edge whose running
+// sum T_k = sum_{k' <= k} Jr/r (its edges in ascending order) exceeds u Jr.  The host
+// stores per edge floor(2^28 T_k / Jr) << 4 | edge number, so the answer is the first
+// entry above h, found by a binary search of ceil(log2 n) dependent shared-memory reads,
+// the same for every lane (all lanes have subgraphs of n edges), instead of a scan whose
+// trips are those of the warp's slowest lane (up to n of them).  Thresholds and h are
+// exact to one unit of 2^-28: a probe within 18 of h does not decide, `unsure` is set and
+// the caller repeats the step in FP64 (exact_cut).  The two thresholds that bound the
+// answer are always among the probes.
+static __device__ __forceinline__ int find_cut(u32 h, u32 sub, u32 meta, const table_ref& t, int n, bool& unsure)
 {
-    const float* w = (const float*)t.w;
-    const float* Jr = (const float*)t.Jr;
-    const float* ri = (const float*)t.ri;
-    const unsigned char* meta = t.meta;
-    u32 sub = FT_FULL;
-    float JJr = pf[P_JRFULL];
-    bool MM = true;
-    int oL = FT_LOOPS, exact = 0;
-    f2 lxx;
-    lxx.hi = lxx.lo = 0.0f;
-    lF = lxx;
-    lG = lxx;
+    if (n == 1) return __ffs(sub) - 1;
+    const u32* q = (const u32*)t.q + META_OFF(meta);
+    int lo = 0;
+#pragma unroll
+    for (int m = n; m > 1;) {   // the answer is among entries lo .. lo + m - 1
+        const int half = m / 2;
+        const u32 e = q[lo + half - 1];
+        unsure |= h - e + 18u <= 36u;
+        lo += h >= e ? half : 0;
+        m -= half;
+    }
+    return (int)(q[lo] & 15u);
+}
+#elif FT_PREC == 1
+// Tables in global memory: the running sums in FP32 with a rigorous margin (|T32 - T64| <=
+// (2E) 2^-24 Jr, |R32 - R64| <= 4 2^-24 Jr), up to the first sure decision.
+static __device__ __forceinline__ int scan_cut(u64 x, u32 sub, const table_ref& t, bool& unsure)
+{
+    const float* w = (const float*)t.q;
+    const float JJr = ((const float*)t.Jr)[sub];
+    const float Rf = (float)(u32)(x >> 40) * 0x1.0p-24f * JJr;
+    const float margin = (float)(2 * FT_E + 8) * 0x1.0p-24f * JJr;
+    float T = 0.0f;
+    int cut = 0;
+    for (u32 left = sub; left != 0u; left &= left - 1u) {
+        cut = __ffs(left) - 1;
+        T += w[sub ^ (1u << cut)];
+        const float d = T - Rf;
+        if (d > margin) break;
+        if (d >= -margin) unsure = true;
+    }
+    return cut;
+}
+#endif
+
+static __device__ __forceinline__ void draw_sector64(xo& g, const table_ref& t, const unsigned char* gm,
+                                                     double Jr_full, double* X, double& F, double& Gv,
+                                                     unsigned char* ord)
+{
+    const double* ri = (const double*)t.ri;
+    u32 sub = FT_FULL, meta = t.meta[FT_FULL];
+    double XX = 1.0;
+    F = 1.0;
+    Gv = 0.0;
+#if !FT_CUT
+    const double* w = (const double*)t.q;
+    const double* Jr = (const double*)t.Jr;
+    double JJr = Jr_full;
+#endif
 #pragma unroll
     for (int j = 0; j < FT_E; j++) {
         const u64 x = g.next();
-        // FP32 decision with margin: |T32 - T64| <= (2E) 2^-24 Jr, |R32 - R64| <= 4 2^-24 Jr
-        const float uf = (float)(u32)(x >> 40) * 0x1.0p-24f;
-        const float Rf = uf * JJr;
-        const float margin = (float)(2 * FT_E + 8) * 0x1.0p-24f * JJr;
-        float T = 0.0f;
-        int e = 0, sure = -1;
+#if FT_CUT
         bool unsure = false;
-        // the edges of the current subgraph in ascending order (its set bits), up to the
-        // first sure decision: the same comparisons as a scan over all E edges, without
-        // the trips over edges already cut
+        int e = find_cut((u32)(x >> 32), sub, meta, t, FT_E - j, unsure);
+        if (unsure) e = exact_cut(x, sub, gm);
+        sub ^= 1u << e;
+#else
+        const double R = u01(x) * JJr;
+        double T = 0.0;
+        int e = 0;
+        // the subgraph's edges in ascending order (its set bits) until the running sum
+        // passes R, else the last one
         for (u32 left = sub; left != 0u; left &= left - 1u) {
-            const int c = __ffs(left) - 1;
-            T += w[sub ^ (1u << c)];
-            e = c;
-            const float d = T - Rf;
-            if (d > margin) {
-                sure = c;
-                break;
-            }
-            if (d >= -margin) unsure = true;
+            e = __ffs(left) - 1;
+            T += w[sub ^ (1u << e)];
+            if (T > R) break;
         }
-        int cut = sure >= 0 ? sure : e;
-        if (unsure) {
-            cut = exact_cut(x, sub, TABLE_GM(t));
-            exact++;
-        }
-        sub ^= 1u << cut;
+        sub ^= 1u << e;
         JJr = Jr[sub];
-        const float2 rinv = ((const float2*)ri)[sub];   // 1/r as two floats
-        const unsigned m = meta[sub];
-        const bool mm = (m >> 7) != 0;
-        const int L = (int)(m & 127u);
-        if (MM && !mm) lG = lxx;
-        MM = mm;
+#endif
+        const double rinv = ri[sub];
+        const u32 m = t.meta[sub];
+        if (META_MM(meta) && !META_MM(m)) Gv = XX;
 #pragma unroll
         for (int k = 0; k < FT_E; k++)
-            if (k == cut) lx[k] = lxx;
-        if (L < oL) {
-            lF = f2_add2(lF, lxx);
-            oL = L;
-        }
-        if (FT_RECORD) ord[j] = (unsigned char)cut;
-        if (j < FT_E - 1) {
-#if FT_MODE == 1
-            // deformed integrands: the phase moves by |theta| per unit of log X, so the
-            // sector point is carried to ~1e-12 (two-float logarithm)
-            f2 l = log1m_u2(g.next());
-#else
-            f2 l = log1m_u32(g.next());
-#endif
-            // (hi + lo) * (rinv.x + rinv.y) with the product error kept
-            float p = l.hi * rinv.x;
-            float pe = fmaf(l.hi, rinv.x, -p) + fmaf(l.hi, rinv.y, l.lo * rinv.x);
-            f2 inc;
-            inc.hi = p;
-            inc.lo = pe;
-            lxx = f2_add2(lxx, inc);
-        }
+            if (k == e) X[k] = XX;
+        if (META_L(m) < META_L(meta)) F *= XX;
+        meta = m;
+        if (FT_RECORD) ord[j] = (unsigned char)e;
+        if (j < FT_E - 1) XX *= pow(1.0 - u01(g.next()), rinv);
     }
-    return exact;
 }
 
 // ------------------------------------------------------------------ integrand, FP64
@@ -1172,179 +1022,735 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
 }
 
 
-// ------------------------------------------------------------------ integrand, mixed
 #if FT_PREC == 1
-#if FT_MODE == 1
-// ------------------------------------------------------------------ two-float arithmetic
-// Values hi + lo with |lo| <= ulp(hi)/2 (about 48 significant bits) from error-free
-// transformations of FP32 operations (Knuth's two-sum, the FMA two-product); they run
-// on the FP32 pipe, which is ~60x wider than the FP64 pipe on this GPU.
-struct df {
-    float hi, lo;
-};
-static __device__ __forceinline__ df df_mk(float x)
+// ------------------------------------------------------------------ mixed form: FP32 values and pairs
+// Pairs of FP32 values use the paired instructions (add, mul, fma .f32x2, each component
+// rounded as the scalar operation): the same rate per result, half the issue slots and
+// half the instruction fetches, which bound the mixed kernels.  The undeformed form
+// evaluates two consecutive samples of a thread's range side by side (one component per
+// sample); the deformed form, whose live state would not fit the registers twice, one
+// sample, with its exponentials, logarithms and phases for two edges at a time.
+typedef float2 fv;
+
+static __device__ __forceinline__ fv fv_of(float a) { return make_float2(a, a); }
+static __device__ __forceinline__ fv operator+(fv a, fv b) { return __fadd2_rn(a, b); }
+static __device__ __forceinline__ fv operator*(fv a, fv b) { return __fmul2_rn(a, b); }
+static __device__ __forceinline__ fv fma_(fv a, fv b, fv c) { return __ffma2_rn(a, b, c); }
+static __device__ __forceinline__ float fma_(float a, float b, float c) { return fmaf(a, b, c); }
+static __device__ __forceinline__ fv operator-(fv a, fv b) { return __ffma2_rn(b, fv_of(-1.0f), a); }
+static __device__ __forceinline__ fv operator-(fv a) { return __fmul2_rn(a, fv_of(-1.0f)); }
+static __device__ __forceinline__ fv mul_(fv a, fv b) { return a * b; }
+static __device__ __forceinline__ float mul_(float a, float b) { return __fmul_rn(a, b); }   // never contracted
+static __device__ __forceinline__ fv abs_(fv a) { return make_float2(fabsf(a.x), fabsf(a.y)); }
+static __device__ __forceinline__ float abs_(float a) { return fabsf(a); }
+static __device__ __forceinline__ void set_all(fv& r, float a) { r = fv_of(a); }
+static __device__ __forceinline__ void set_all(float& r, float a) { r = a; }
+template <class V>
+static __device__ __forceinline__ V all_of(float a)
 {
-    df r;
-    r.hi = x;
-    r.lo = 0.0f;
+    V r;
+    set_all(r, a);
     return r;
 }
-static __device__ __forceinline__ df df_norm(float s, float e)
+// reciprocal to an ulp (the approximate instruction), for values that a Newton step or the
+// two-float reciprocal refines
+static __device__ __forceinline__ float rcp_fast(float x)
 {
-    df r;
-    r.hi = s + e;
-    r.lo = e - (r.hi - s);
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-static __device__ FT_DFFN df df_add(df x, df y)
+static __device__ __forceinline__ fv rcp_fast(fv x) { return make_float2(rcp_fast(x.x), rcp_fast(x.y)); }
+template <class V>
+static __device__ __forceinline__ V rcp_newton(V x)
 {
-    const float s = x.hi + y.hi;
-    const float bb = s - x.hi;
-    float e = (x.hi - (s - bb)) + (y.hi - bb);
-    e += x.lo + y.lo;
-    return df_norm(s, e);
+    const V r = rcp_fast(x);
+    return fma_(r, fma_(x, -r, all_of<V>(1.0f)), r);
 }
-static __device__ __forceinline__ df df_neg(df x)
+// x^(-1/2): the approximate instruction and one Newton step
+static __device__ __forceinline__ float rsqrt_newton(float x)
 {
-    x.hi = -x.hi;
-    x.lo = -x.lo;
-    return x;
-}
-static __device__ __forceinline__ df df_sub(df x, df y) { return df_add(x, df_neg(y)); }
-// A product cannot cancel: its low part e stays within ~1.5 ulp of p, which every
-// consumer (sums, products, the reciprocal, conversions) handles, so it is returned
-// without renormalisation.
-static __device__ FT_DFFN df df_mul(df x, df y)
-{
-    const float p = x.hi * y.hi;
-    float e = fmaf(x.hi, y.hi, -p);
-    e = fmaf(x.hi, y.lo, e);
-    e = fmaf(x.lo, y.hi, e);
-    df r;
-    r.hi = p;
-    r.lo = e;
-    return r;
-}
-// x y + z: the leading product exact (FMA residual), one two-sum with z.hi, the small
-// terms added once
-static __device__ FT_DFFN df df_fma(df x, df y, df z)
-{
-    const float p = x.hi * y.hi;
-    const float pe = fmaf(x.hi, y.hi, -p);
-    const float s = p + z.hi;
-    const float bb = s - p;
-    float e = (p - (s - bb)) + (z.hi - bb);
-    e += pe + fmaf(x.hi, y.lo, fmaf(x.lo, y.hi, z.lo));
-    return df_norm(s, e);
-}
-static __device__ FT_DFFN df df_inv(df x)
-{
-    // one Newton step from the FP32 reciprocal r: 1/x = r (1 + e) with e = 1 - x r;
-    // 1 - x.hi r (about 2^-23) is exact to 2^-47 by the FMA, then x.lo r is removed.
-    // |r e| stays within about an ulp of r, so the pair needs no renormalisation.
-    const float r = rcp_(x.hi);
-    const float e = fmaf(-x.lo, r, fmaf(-x.hi, r, 1.0f));
-    df o;
-    o.hi = r;
-    o.lo = r * e;
-    return o;
-}
-static __device__ __forceinline__ float df_f(df x) { return x.hi + x.lo; }
-static __device__ __forceinline__ df df_of(f2 x)
-{
-    df r;
-    r.hi = x.hi;
-    r.lo = x.lo;
-    return r;
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return fmaf(0.5f * r, fmaf(x * r, -r, 1.0f), r);
 }
 
-// ------------------------------------------------------------------ complex two-float
-// Complex two-float numbers, and sin / cos of a two-float angle to ~1e-13, table-driven
-// after Tang: x = k pi/64 + r with |r| <= pi/128 (pi/64 as three FP32 parts, each
-// k * part formed exactly with an FMA); sin(k pi/64), cos(k pi/64) as float pairs from
-// FT_SCTAB (k mod 128); sin r = r - r^3/6 + r^5/120 and cos r = 1 - r^2/2 + r^4/24 -
-// r^6/720 with r and r^2 in two-float and the terms below 3e-6 in FP32; then
-// sin x = sin a cos r + cos a sin r, cos x = cos a cos r - sin a sin r in two-float.
-struct cdf {
-    df re, im;
+// Two-float numbers hi + lo (about 48 significant bits) from error-free transformations
+// (Knuth's two-sum, Dekker's fast two-sum, the FMA two-product).  They run on the FP32
+// pipe, which is 64x wider than the FP64 pipe on this GPU.
+template <class V>
+struct tf {
+    V hi, lo;
 };
-static __device__ __forceinline__ cdf cdf_mk(df r, df i)
+typedef tf<float> sf;
+typedef tf<fv> df;
+template <class V>
+static __device__ __forceinline__ tf<V> tf_mk(V h, V l)
+{
+    tf<V> r;
+    r.hi = h;
+    r.lo = l;
+    return r;
+}
+template <class V>
+static __device__ __forceinline__ tf<V> tf_zero()
+{
+    return tf_mk(all_of<V>(0.0f), all_of<V>(0.0f));
+}
+template <class V>
+static __device__ __forceinline__ tf<V> two_sum(V a, V b)
+{
+    const V s = a + b, bb = s - a;
+    return tf_mk(s, (a - (s - bb)) + (b - bb));
+}
+// |a| >= |b| or a = 0
+template <class V>
+static __device__ __forceinline__ tf<V> fast_two_sum(V a, V b)
+{
+    const V s = a + b;
+    return tf_mk(s, b - (s - a));
+}
+template <class V>
+static __device__ __forceinline__ tf<V> tf_norm(tf<V> x)
+{
+    return fast_two_sum(x.hi, x.lo);
+}
+// Sums whose low part is not renormalised (`_n`): it stays within a few ulps of the
+// terms' high parts, so further sums lose nothing; chains renormalise once, at their
+// end, before the value is multiplied or inverted.
+template <class V>
+static __device__ __forceinline__ tf<V> tf_add_n(tf<V> x, tf<V> y)
+{
+    const tf<V> s = two_sum(x.hi, y.hi);
+    return tf_mk(s.hi, s.lo + (x.lo + y.lo));
+}
+template <class V>
+static __device__ __forceinline__ tf<V> tf_sub_n(tf<V> x, tf<V> y)
+{
+    const V s = x.hi - y.hi, bb = s - x.hi;
+    const V e = (x.hi - (s - bb)) - (y.hi + bb);
+    return tf_mk(s, e + (x.lo - y.lo));
+}
+template <class V>
+static __device__ __forceinline__ tf<V> tf_add(tf<V> x, tf<V> y)
+{
+    return tf_norm(tf_add_n(x, y));
+}
+template <class V>
+static __device__ __forceinline__ tf<V> tf_sub(tf<V> x, tf<V> y)
+{
+    return tf_norm(tf_sub_n(x, y));
+}
+template <class V>
+static __device__ __forceinline__ tf<V> tf_neg(tf<V> x)
+{
+    return tf_mk(-x.hi, -x.lo);
+}
+// A product cannot cancel: its low part stays within ~1.5 ulp of the high one, which
+// every consumer handles, so it is returned without renormalisation.
+template <class V>
+static __device__ __forceinline__ tf<V> tf_mul(tf<V> x, tf<V> y)
+{
+    const V p = mul_(x.hi, y.hi);
+    V e = fma_(x.hi, y.hi, -p);
+    e = fma_(x.hi, y.lo, e);
+    return tf_mk(p, fma_(x.lo, y.hi, e));
+}
+template <class V>
+static __device__ __forceinline__ tf<V> tf_fma_n(tf<V> x, tf<V> y, tf<V> z)
+{
+    const tf<V> p = tf_mul(x, y);
+    const tf<V> s = two_sum(p.hi, z.hi);
+    return tf_mk(s.hi, s.lo + (p.lo + z.lo));
+}
+// x s, s a float
+template <class V>
+static __device__ __forceinline__ tf<V> tf_mulf(tf<V> x, V s)
+{
+    const V p = mul_(x.hi, s);
+    return tf_mk(p, fma_(x.lo, s, fma_(x.hi, s, -p)));
+}
+template <class V>
+static __device__ __forceinline__ tf<V> tf_addf_n(tf<V> x, V y)
+{
+    const tf<V> s = two_sum(x.hi, y);
+    return tf_mk(s.hi, s.lo + x.lo);
+}
+template <class V>
+static __device__ __forceinline__ tf<V> tf_inv(tf<V> x)
+{
+    // one Newton step from the FP32 reciprocal r: 1/x = r (1 + e), e = 1 - x r exact to
+    // 2^-47 by the FMA; |r e| stays within an ulp or two of r
+    const V r = rcp_fast(x.hi), nr = -r;
+    const V e = fma_(x.lo, nr, fma_(x.hi, nr, all_of<V>(1.0f)));
+    return tf_mk(r, r * e);
+}
+template <class V>
+static __device__ __forceinline__ V tf_f(tf<V> x)
+{
+    return x.hi + x.lo;
+}
+static __device__ __forceinline__ df pair_of(sf a, sf b) { return tf_mk(make_float2(a.hi, b.hi), make_float2(a.lo, b.lo)); }
+static __device__ __forceinline__ sf first_of(df a) { return tf_mk(a.hi.x, a.lo.x); }
+static __device__ __forceinline__ sf second_of(df a) { return tf_mk(a.hi.y, a.lo.y); }
+// parameter i, stored as (hi, hi, lo, lo)
+static __device__ __forceinline__ sf prm_sf(const float4* pp, int i)
+{
+    const float4 v = pp[i];
+    return tf_mk(v.x, v.z);
+}
+static __device__ __forceinline__ fv prm_fv(const float4* pp, int i) { return *(const float2*)(pp + i); }
+
+// log(1 - u), u = (x >> 11) 2^-53, of two draws, to about 1e-12 absolute, with integer and FP32
+// instructions only (64-bit conversions and FP64 would run on the FP64 pipe).
+// Table-driven reduction after Tang (ACM TOMS 16, 1990): 1 - u = 2^kk M with M in [1, 2)
+// held as two floats (46 fraction bits); c_i = 1 + (i + 1/2)/64 for the top 6 fraction
+// bits i, r_i = fl(1/c_i) and -log r_i (two-float) from FT_LOGTAB; z = M r_i - 1 (|z| <
+// 1/100) from exact products, log M = -log r_i + log1p(z) with log1p(z) = z - z^2/2 +
+// z^3/3 - z^4/4 + z^5/5, the terms past z in FP32.
+struct log_arg {
+    float m, l, r, nh, nl, k;
+};
+static __device__ __forceinline__ log_arg log_split(u64 x)
+{
+    const u64 q = (~x & ~0x7ffull) + 0x800ull;   // (1 - u) 2^64, 0 for u = 0
+    const int lz = __clzll((long long)q);
+    const u64 mb = q << (lz & 63);
+    const u32 hi = (u32)(mb >> 32) | 0x80000000u;
+    log_arg a;
+    a.m = __int_as_float((int)((hi >> 8) + 0x3f000000u));
+    a.l = __int_as_float((int)((__funnelshift_r((u32)mb, hi, 17) & 0x7fffffu) | 0x4b000000u));
+    const float4 t = FT_LOGTAB[(hi >> 25) & 63u];
+    a.r = t.x;
+    a.nh = t.y;
+    a.nl = t.z;
+    a.k = lz == 64 ? 0.0f : 8388608.0f - __int_as_float(0x4b000001 + lz);   // -1 - lz
+    return a;
+}
+static __device__ FT_BIGFN df log1m_pair(u64 xa, u64 xb)
+{
+    const log_arg a = log_split(xa), b = log_split(xb);
+    const fv m = make_float2(a.m, b.m), r = make_float2(a.r, b.r), kk = make_float2(a.k, b.k);
+    const fv ml = (make_float2(a.l, b.l) - fv_of(8388608.0f)) * fv_of(0x1.0p-46f);
+    // z = M r - 1: m r = p + e exactly, p - 1 exact (p within 1 % of 1)
+    const fv p = m * r;
+    const df z = fast_two_sum(p - fv_of(1.0f), fma_(ml, r, fma_(m, r, -p)));
+    const fv zh = z.hi;
+    const fv tail = zh * zh *
+                    fma_(zh, fma_(zh, fma_(zh, fv_of(0.2f), fv_of(-0.25f)), fv_of(0.333333343f)), fv_of(-0.5f));
+    // kk ln2 with ln2 in three parts (the first has 16 bits: the product is exact)
+    const df s = fast_two_sum(kk * fv_of(0.693145751953125f), make_float2(a.nh, b.nh));
+    const df t = two_sum(s.hi, zh);
+    const fv lo = fma_(kk, fv_of(1.428606765330187e-06f), make_float2(a.nl, b.nl)) +
+                  fma_(kk, fv_of(5.497923e-14f), z.lo + tail);
+    return fast_two_sum(t.hi, (t.lo + s.lo) + lo);
+}
+
+static __device__ __forceinline__ void rewind(xo& g, int n)
+{
+    // n steps back: b = y ^ (b << 17) with y = b' ^ c' solved by substitution
+#pragma unroll 1
+    for (int i = 0; i < n; i++) {
+        const u64 d1 = rotl64(g.d, 19);
+        const u64 y = g.b ^ g.c;
+        const u64 b = y ^ (y << 17) ^ (y << 34) ^ (y << 51);
+        const u64 c1 = g.c ^ (b << 17);
+        g.a ^= d1;
+        g.b = b;
+        g.c = c1 ^ g.a;
+        g.d = d1 ^ b;
+    }
+}
+
+// the draw of the step undecided by the thresholds, in FP64; g stands `back` draws behind it
+static __device__ __noinline__ int exact_step(xo g, int back, u32 sub, const unsigned char* gm)
+{
+    rewind(g, back);
+    return exact_cut(g.next(), sub, gm);
+}
+
+// The thread's scratch in shared memory, [slot][thread]: log X of edge e (part 0 hi, 1 lo),
+// later overwritten by 1/X; with FT_SCRATCH 1 also the deformation angles, with 2 the
+// upper triangle of X^1/2 H X^1/2: values that live across the long blocks of the
+// deformed integrand and would otherwise be spilled to local memory, whose frames (256
+// threads of 2 KB on every SM) are read back from L2.
+#if FT_MODE == 0
+typedef fv scr;
+#else
+typedef float scr;
+#endif
+#define SCR(slot) (((scr*)lxs)[(slot) * FT_BLOCK + threadIdx.x])
+#define LX(e, p) SCR((e) * 2 + (p))
+#define SCR_TH(e, p) SCR(2 * FT_E + (e) * 2 + (p))
+#define SCR_H(a, b) SCR(4 * FT_E + (a) * FT_E - (a) * ((a) - 1) / 2 + ((b) - (a)))
+
+#if FT_MODE == 0
+// Sectors of two consecutive samples: log X per edge into the scratch (X in the order of
+// removal, srcs/tropical_sampling.hpp:503-564), log psi_tr and log(xi_tr / psi_tr).  The
+// first sample's draws are taken ahead, so that both walk their steps together.
+static __device__ __forceinline__ void draw_pair(xo& g, const table_ref& t, unsigned char* lxs, df& lF, df& lG,
+                                                 u32& exA, u32& exB, unsigned char* ordA, unsigned char* ordB)
+{
+    const float* ri = (const float*)t.ri;
+    u32 hA[FT_E];
+    u64 yA[FT_E];
+#if !FT_CUT
+    u32 lA[FT_E];
+#endif
+#pragma unroll
+    for (int j = 0; j < FT_E; j++) {
+        const u64 x = g.next();
+        hA[j] = (u32)(x >> 32);
+#if !FT_CUT
+        lA[j] = (u32)x;
+#endif
+        yA[j] = j < FT_E - 1 ? g.next() : 0ull;
+    }
+    u32 sA = FT_FULL, sB = FT_FULL, mA = t.meta[FT_FULL], mB = mA;
+    df lxx = tf_zero<fv>();
+    lF = lG = lxx;
+    exA = exB = 0;
+#pragma unroll
+    for (int j = 0; j < FT_E; j++) {
+        const u64 xB = g.next();
+        bool uA = false, uB = false;
+#if FT_CUT
+        int cA = find_cut(hA[j], sA, mA, t, FT_E - j, uA), cB = find_cut((u32)(xB >> 32), sB, mB, t, FT_E - j, uB);
+#else
+        int cA = scan_cut(((u64)hA[j] << 32) | lA[j], sA, t, uA), cB = scan_cut(xB, sB, t, uB);
+#endif
+        if (uA) {
+            cA = exact_step(g, 2 * FT_E, sA, TABLE_GM(t));
+            exA++;
+        }
+        if (uB) {
+            cB = exact_step(g, 1, sB, TABLE_GM(t));
+            exB++;
+        }
+        sA ^= 1u << cA;
+        sB ^= 1u << cB;
+        const u32 nA = t.meta[sA], nB = t.meta[sB];
+        // the subgraph stops being mass-momentum spanning: xi_tr / psi_tr
+        if (META_MM(mA) && !META_MM(nA)) {
+            lG.hi.x = lxx.hi.x;
+            lG.lo.x = lxx.lo.x;
+        }
+        if (META_MM(mB) && !META_MM(nB)) {
+            lG.hi.y = lxx.hi.y;
+            lG.lo.y = lxx.lo.y;
+        }
+        LX(cA, 0).x = lxx.hi.x;
+        LX(cA, 1).x = lxx.lo.x;
+        LX(cB, 0).y = lxx.hi.y;
+        LX(cB, 1).y = lxx.lo.y;
+        // it loses a loop: psi_tr
+        if (j > 0) {
+            const bool dA = META_L(nA) < META_L(mA), dB = META_L(nB) < META_L(mB);
+            lF = tf_add_n(lF, tf_mk(make_float2(dA ? lxx.hi.x : 0.0f, dB ? lxx.hi.y : 0.0f),
+                                    make_float2(dA ? lxx.lo.x : 0.0f, dB ? lxx.lo.y : 0.0f)));
+        }
+        mA = nA;
+        mB = nB;
+        if (FT_RECORD) {
+            ordA[j] = (unsigned char)cA;
+            ordB[j] = (unsigned char)cB;
+        }
+        if (j < FT_E - 1) {
+            const df r = tf_mk(make_float2(ri[sA], ri[sB]), make_float2(t.rl[sA], t.rl[sB]));
+            const df inc = tf_mul(log1m_pair(yA[j], g.next()), r);
+            lxx = j == 0 ? inc : tf_norm(tf_add_n(lxx, inc));
+        }
+    }
+    lF = tf_norm(lF);
+}
+
+#else
+// Sector of one sample: log X per edge into the scratch (X in the order of removal,
+// srcs/tropical_sampling.hpp:503-564), log psi_tr and log(xi_tr / psi_tr) in two-float.
+// The phase of a deformed integrand moves by |theta| per unit of log X, so log X is
+// carried to ~1e-12.  The logarithms are taken two draws at a time.
+static __device__ __forceinline__ void draw_one(xo& g, const table_ref& t, unsigned char* lxs, sf& lF, sf& lG, u32& ex,
+                                                unsigned char* ord)
+{
+    const float* ri = (const float*)t.ri;
+    u32 sub = FT_FULL, meta = t.meta[FT_FULL];
+    sf lxx = tf_zero<float>();
+    lF = lG = lxx;
+    ex = 0;
+    u64 x = g.next();   // the draw of the next cut
+    df l;
+#pragma unroll
+    for (int j = 0; j < FT_E; j++) {
+        u64 x1 = 0;
+        if (j < FT_E - 1 && !(j & 1)) {
+            const u64 y0 = g.next();
+            x1 = g.next();
+            const u64 y1 = j < FT_E - 2 ? g.next() : y0;
+            l = log1m_pair(y0, y1);
+        }
+        // draws taken from this cut's one on: x y0 x1 y1 at an even step (x y0 x1 and x at the
+        // last two), x y1 at an odd one (x at the last)
+        const int back = j & 1 ? (j < FT_E - 1 ? 2 : 1) : (j < FT_E - 2 ? 4 : (j < FT_E - 1 ? 3 : 1));
+        bool unsure = false;
+#if FT_CUT
+        int c = find_cut((u32)(x >> 32), sub, meta, t, FT_E - j, unsure);
+#else
+        int c = scan_cut(x, sub, t, unsure);
+#endif
+        if (unsure) {
+            c = exact_step(g, back, sub, TABLE_GM(t));
+            ex++;
+        }
+        sub ^= 1u << c;
+        const u32 m = t.meta[sub];
+        if (META_MM(meta) && !META_MM(m)) lG = lxx;   // it stops being mass-momentum spanning: xi_tr / psi_tr
+        LX(c, 0) = lxx.hi;
+        LX(c, 1) = lxx.lo;
+        if (j > 0 && META_L(m) < META_L(meta)) lF = tf_add_n(lF, lxx);   // it loses a loop: psi_tr
+        meta = m;
+        if (FT_RECORD) ord[j] = (unsigned char)c;
+        if (j < FT_E - 1) {
+            const sf inc = tf_mul(j & 1 ? second_of(l) : first_of(l), tf_mk(ri[sub], t.rl[sub]));
+            lxx = j == 0 ? inc : tf_norm(tf_add_n(lxx, inc));
+            x = j & 1 ? g.next() : x1;
+        }
+    }
+    lF = tf_norm(lF);
+}
+
+#endif
+
+// positive value m * 2^e with m in [1, 2) per sample: products without overflow
+struct mexp {
+    fv m;
+    int ea, eb;
+    bool ba, bb;
+};
+static __device__ __forceinline__ void mx_lane(float& m, int& e, bool& bad)
+{
+    const int b = __float_as_int(m);
+    const int be = (b >> 23) & 0xff;
+    bad |= (be == 0) | (be == 255) | (b < 0);
+    e += be - 127;
+    m = __int_as_float((b & 0x007fffff) | 0x3f800000);
+}
+static __device__ __forceinline__ void mx_mul(mexp& a, fv x)
+{
+    a.m = a.m * x;
+    mx_lane(a.m.x, a.ea, a.ba);
+    mx_lane(a.m.y, a.eb, a.bb);
+}
+static __device__ __forceinline__ mexp mx_one()
+{
+    mexp r;
+    r.m = fv_of(1.0f);
+    r.ea = r.eb = 0;
+    r.ba = r.bb = false;
+    return r;
+}
+static __device__ __forceinline__ fv fv_log2(fv x) { return make_float2(m_log2(x.x), m_log2(x.y)); }
+static __device__ __forceinline__ fv fv_ints(int a, int b) { return make_float2((float)a, (float)b); }
+#define RLN2_HI 1.44269502162933349609375f
+#define RLN2_LO 1.925963033500011e-8f
+#define LN2_F 0.69314718055994531f
+// a natural logarithm in base 2
+template <class V>
+static __device__ __forceinline__ tf<V> tf_log2e(tf<V> x)
+{
+    return tf_mul(x, tf_mk(all_of<V>(RLN2_HI), all_of<V>(RLN2_LO)));
+}
+static __device__ __forceinline__ bool finite_(float x) { return isfinite(x); }
+
+// undeformed integrand: relative size of V below which the FP32 evaluation hands the
+// sample to FP64
+#ifndef V_CANCEL
+#define V_CANCEL 0.05f
+#endif
+// smallest pivot-to-row ratio accepted in the FP32 elimination of the Jacobian
+#ifndef PIVOT_GROWTH
+#define PIVOT_GROWTH 0.02f
+#endif
+
+#if FT_MODE == 0
+// Undeformed integrand (srcs/feynman_integral.hpp:218-276) of two samples in FP32, in the
+// frame X_e = exp(lx_e - sh).  Components of `bad`: the FP32 evaluation cannot be trusted
+// (the sample then goes to the FP64 pass).
+static __device__ __forceinline__ void integrand_pair(const float4* pp, const float* pf, unsigned char* lxs, df lF,
+                                                      df lG, fv* out, bool& badA, bool& badB)
+{
+    const float D2 = 0.5f * pf[P_D], W = pf[P_W], IGtr = pf[P_IGTR];
+    fv lmin = fv_of(0.0f);
+#pragma unroll
+    for (int e = 0; e < FT_E; e++) lmin = make_float2(fminf(lmin.x, LX(e, 0).x), fminf(lmin.y, LX(e, 0).y));
+    // sh an integer near the middle of the range; R and the eps factor are ratios to the
+    // tropical approximants and do not depend on it
+    const fv sh = make_float2(rintf(0.5f * lmin.x), rintf(0.5f * lmin.y));
+    fv X[FT_E], Xi[FT_E];
+    mexp det = mx_one();
+    df sumlx = tf_zero<fv>();   // log prod X
+    badA = badB = false;
+#pragma unroll
+    for (int e = 0; e < FT_E; e++) {
+        const df a = tf_norm(tf_addf_n(tf_mk(LX(e, 0), LX(e, 1)), -sh));
+        sumlx = e == 0 ? a : tf_add_n(sumlx, a);
+        const fv ep = make_float2(m_exp(a.hi.x), m_exp(a.hi.y));
+        X[e] = fma_(ep, a.lo, ep);
+        Xi[e] = rcp_newton(X[e]);
+        badA |= !(fabsf(a.hi.x) < 80.0f);   // beyond FP32's exponential
+        badB |= !(fabsf(a.hi.y) < 80.0f);
+    }
+    sumlx = tf_norm(sumlx);
+    const df lFs = tf_norm(tf_addf_n(lF, fv_of(-(float)FT_LOOPS) * sh));   // log psi_tr in the frame
+    const df lGs = tf_norm(tf_addf_n(lG, -sh));                            // log V_tr = log(xi_tr / psi_tr)
+    // conductance-form elimination (all values positive)
+    fv c[FT_N][FT_N], g[FT_N], d[FT_N], id[FT_N], a[FT_N][FT_N];
+#pragma unroll
+    for (int e = 0; e < FT_E; e++) {
+        const int k = FT_EK[e], l = FT_EL[e];
+        fv& slot = (k == FT_V - 1) ? g[l] : c[l][k];
+        slot = first_in_slot(e) ? Xi[e] : slot + Xi[e];
+    }
+#pragma unroll
+    for (int k = 0; k < FT_N; k++) {
+        fv dk = g[k];
+        bool any = NZG(k);
+#pragma unroll
+        for (int j = k + 1; j < FT_N; j++)
+            if (NZC(k, j)) {
+                dk = any ? dk + c[k][j] : c[k][j];
+                any = true;
+            }
+        d[k] = dk;
+        id[k] = rcp_newton(dk);
+        mx_mul(det, dk);
+#pragma unroll
+        for (int i = k + 1; i < FT_N; i++)
+            if (NZC(k, i)) a[k][i] = c[k][i] * id[k];
+#pragma unroll
+        for (int i = k + 1; i < FT_N; i++) {
+            if (!NZC(k, i)) continue;
+            if (NZG(k)) g[i] = ADDS_G(k, i) ? fma_(a[k][i], g[k], g[i]) : a[k][i] * g[k];
+#pragma unroll
+            for (int j = i + 1; j < FT_N; j++)
+                if (NZC(k, j)) c[i][j] = ADDS_C(k, i, j) ? fma_(a[k][i], c[k][j], c[i][j]) : a[k][i] * c[k][j];
+        }
+    }
+    badA |= det.ba;
+    badB |= det.bb;
+    // log2 psi (exponents and prod X exact, the rest in FP32), log2(psi / psi_tr)
+    const df l2psi = tf_norm(tf_addf_n(tf_addf_n(tf_log2e(sumlx), fv_ints(det.ea, det.eb)), fv_log2(det.m)));
+    const df lpsi = tf_sub(l2psi, tf_log2e(lFs));
+#if FT_ONLY_PSI
+    const df t = tf_norm(tf_mulf(lpsi, fv_of(-D2)));
+    const fv R = make_float2(m_exp2(t.hi.x) * (1.0f + t.lo.x * LN2_F), m_exp2(t.hi.y) * (1.0f + t.lo.y * LN2_F));
+    out[0] = fv_of(IGtr) * R;
+#else
+    // V = -sum_r sigma_r q_r^T L^-1 q_r + sum_e m2_e X_e
+    fv v = fv_of(0.0f), mag = fv_of(0.0f);
+#pragma unroll
+    for (int r = 0; r < FT_RANK; r++) {
+        fv y[FT_N], s = fv_of(0.0f);
+#pragma unroll
+        for (int i = FT_Q0; i < FT_N; i++) {
+            fv yi = prm_fv(pp, P_Q + r * FT_N + i);
+#pragma unroll
+            for (int k = FT_Q0; k < i; k++)
+                if (NZC(k, i)) yi = fma_(a[k][i], y[k], yi);
+            y[i] = yi;
+            s = i == FT_Q0 ? yi * yi * id[i] : fma_(yi * yi, id[i], s);
+        }
+        const fv w = prm_fv(pp, P_SIG + r) * s;
+        v = v - w;
+        mag = mag + abs_(w);
+    }
+#pragma unroll
+    for (int e = 0; e < FT_E; e++) {
+        const fv w = prm_fv(pp, P_M2 + e) * X[e];
+        v = v + w;
+        mag = mag + abs_(w);
+    }
+    // cancellation, or a sign the FP64 pass must decide
+    badA |= !(v.x > V_CANCEL * mag.x);
+    badB |= !(v.y > V_CANCEL * mag.y);
+    mexp V = mx_one();
+    mx_mul(V, v);
+    const df l2v = fast_two_sum(fv_ints(V.ea, V.eb), fv_log2(V.m));
+    const df lv = tf_sub(l2v, tf_log2e(lGs));   // log2(V / V_tr)
+    const df t = tf_norm(tf_add_n(tf_mulf(lpsi, fv_of(-D2)), tf_mulf(lv, fv_of(-W))));
+    fv R = make_float2(m_exp2(t.hi.x) * (1.0f + t.lo.x * LN2_F), m_exp2(t.hi.y) * (1.0f + t.lo.y * LN2_F));
+    badA |= !finite_(R.x) || V.ba;
+    badB |= !finite_(R.y) || V.bb;
+    R = fv_of(IGtr) * R;
+    out[0] = R;
+    if (FT_K > 1) {
+        const fv ef = fv_of(LN2_F) * tf_f(tf_add(l2psi, tf_mulf(l2v, fv_of(-(float)FT_LOOPS))));
+#pragma unroll
+        for (int j = 1; j < FT_K; j++) {
+            R = R * (ef * fv_of(1.0f / (float)j));
+            out[j] = R;
+        }
+    }
+#endif
+}
+#else
+// ------------------------------------------------------------------ deformed integrand
+struct cdf {
+    sf re, im;
+};
+static __device__ __forceinline__ cdf cdf_mk(sf r, sf i)
 {
     cdf z;
     z.re = r;
     z.im = i;
     return z;
 }
-static __device__ __forceinline__ cdf cdf_zero() { return cdf_mk(df_mk(0.0f), df_mk(0.0f)); }
-static __device__ __forceinline__ cdf operator+(cdf a, cdf b) { return cdf_mk(df_add(a.re, b.re), df_add(a.im, b.im)); }
-static __device__ __forceinline__ cdf operator-(cdf a, cdf b) { return cdf_mk(df_sub(a.re, b.re), df_sub(a.im, b.im)); }
+static __device__ __forceinline__ cdf cdf_add_n(cdf a, cdf b) { return cdf_mk(tf_add_n(a.re, b.re), tf_add_n(a.im, b.im)); }
+static __device__ __forceinline__ cdf cdf_norm(cdf a) { return cdf_mk(tf_norm(a.re), tf_norm(a.im)); }
+static __device__ __forceinline__ cdf cdf_scale(sf s, cdf a) { return cdf_mk(tf_mul(s, a.re), tf_mul(s, a.im)); }
+// x1 y1 - x2 y2 and x1 y1 + x2 y2, the low parts not renormalised
+template <class V>
+static __device__ __forceinline__ tf<V> dot_sub_n(tf<V> x1, tf<V> y1, tf<V> x2, tf<V> y2)
+{
+    const tf<V> p = tf_mul(x1, y1);
+    const V n = mul_(-x2.hi, y2.hi);
+    V l = fma_(x2.hi, y2.hi, n);   // x2 y2 + n, exactly
+    l = fma_(x2.hi, y2.lo, l);
+    l = fma_(x2.lo, y2.hi, l);
+    const tf<V> s = two_sum(p.hi, n);
+    return tf_mk(s.hi, s.lo + (p.lo - l));
+}
+template <class V>
+static __device__ __forceinline__ tf<V> dot_add_n(tf<V> x1, tf<V> y1, tf<V> x2, tf<V> y2)
+{
+    const tf<V> p = tf_mul(x1, y1), q = tf_mul(x2, y2);
+    const tf<V> s = two_sum(p.hi, q.hi);
+    return tf_mk(s.hi, s.lo + (p.lo + q.lo));
+}
 static __device__ FT_CXFN cdf operator*(cdf a, cdf b)
 {
-    return cdf_mk(df_fma(a.re, b.re, df_neg(df_mul(a.im, b.im))), df_fma(a.re, b.im, df_mul(a.im, b.re)));
+    return cdf_norm(cdf_mk(dot_sub_n(a.re, b.re, a.im, b.im), dot_add_n(a.re, b.im, a.im, b.re)));
 }
-static __device__ __forceinline__ cdf operator*(df s, cdf a) { return cdf_mk(df_mul(s, a.re), df_mul(s, a.im)); }
+// a b + c, the sums' low parts left as they are (renormalised where the value is used)
+static __device__ FT_CXFN cdf cdf_fma_n(cdf a, cdf b, cdf c)
+{
+    return cdf_add_n(cdf_mk(dot_sub_n(a.re, b.re, a.im, b.im), dot_add_n(a.re, b.im, a.im, b.re)), c);
+}
 static __device__ FT_BIGFN cdf cdf_inv(cdf a)
 {
-    const df m = df_inv(df_fma(a.re, a.re, df_mul(a.im, a.im)));
-    return cdf_mk(df_mul(a.re, m), df_neg(df_mul(a.im, m)));
+    const sf m = tf_inv(tf_norm(dot_add_n(a.re, a.re, a.im, a.im)));
+    return cdf_mk(tf_mul(a.re, m), tf_mul(tf_neg(a.im), m));
 }
-// a b + c with four two-float FMAs
-static __device__ FT_CXFN cdf cdf_fma(cdf a, cdf b, cdf c)
+// z 2^-k for the exponent k of z's larger part (exact), the exponent added to k;
+// ok false where z is zero or not finite
+static __device__ __forceinline__ float exp_scale(float re, float im, int& k, bool& ok)
 {
-    return cdf_mk(df_fma(a.re, b.re, df_fma(df_neg(a.im), b.im, c.re)), df_fma(a.re, b.im, df_fma(a.im, b.re, c.im)));
-}
-// z 2^-k for the exponent k of z's larger part (exact), the exponent added to k_acc;
-// false when z is zero or not finite
-static __device__ __forceinline__ bool cdf_renorm(cdf& z, int& k_acc)
-{
-    const float mx = fmaxf(fabsf(z.re.hi), fabsf(z.im.hi));
+    const float mx = fmaxf(fabsf(re), fabsf(im));
     const int be = (__float_as_int(mx) >> 23) & 0xff;
-    const bool ok = be > 0 && be < 255;
-    const int k = ok ? be - 127 : 0;
-    const float sc = __int_as_float((127 - k) << 23);
+    const bool fine = be > 0 && be < 254;
+    ok &= fine;
+    k += fine ? be - 127 : 0;
+    return __int_as_float((fine ? 254 - be : 127) << 23);
+}
+static __device__ __forceinline__ void cdf_renorm(cdf& z, int& k, bool& ok)
+{
+    const float sc = exp_scale(z.re.hi, z.im.hi, k, ok);
     z.re.hi *= sc;
     z.re.lo *= sc;
     z.im.hi *= sc;
     z.im.lo *= sc;
-    k_acc += k;
-    return ok;
 }
 
-// e^(ix) = cos x + i sin x
-static __device__ FT_BIGFN cdf expi_df(df x)
+// e^a for two two-floats a (|a| < 80) in two-float, about 1e-12 relative; table-driven
+// after Tang (ACM TOMS 15, 1989): a = (32 m + j) ln2/32 + s with |s| <= ln2/64,
+// e^a = 2^m 2^(j/32) e^s, 2^(j/32) as two floats from FT_EXPTAB, e^s = 1 + s + s^2/2 +
+// s^3/6 + s^4/24 with the terms past s in FP32.  ln2/32 = C1 + C2 + C3, C1 with 11
+// significant bits so that k C1 is exact for |k| < 2^13.
+static __device__ FT_BIGFN df exp_pair(df a)
 {
-    const float P1 = 0x1.921fb6p-5f, P2 = -0x1.777a5cp-30f, P3 = -0x1.ee59dap-55f;
-    const float k = rintf((x.hi + x.lo) * 0x1.45f306p+4f);
-    const float p1 = k * P1, e1 = fmaf(k, P1, -p1);
-    const float p2 = k * P2, e2 = fmaf(k, P2, -p2);
-    df r = df_add(x, df_norm(-p1, -e1));
-    r = df_add(r, df_norm(-p2, -e2));
-    r = df_add(r, df_mk(-k * P3));
-    const float rh = r.hi, r2 = rh * rh;
-    // sin r = r + rh^3 (-1/6 + rh^2/120)
-    const df sr = df_add(r, df_mk(rh * r2 * fmaf(r2, 0x1.111112p-7f, -0x1.555556p-3f)));
-    // cos r = 1 - (rh^2 + 2 rh r.lo)/2 + rh^4/24 - rh^6/720, with rh^2 = r2 + qe exactly
-    const float qe = fmaf(rh, rh, -r2);
-    const df cr = df_add(df_norm(1.0f, -0.5f * r2),
-                         df_mk(fmaf(-rh, r.lo, -0.5f * qe) + r2 * r2 * fmaf(r2, -0x1.6c16c2p-10f, 0x1.555556p-5f)));
-    const float4 t = FT_SCTAB[((int)k) & 127];
-    df sa, ca;
-    sa.hi = t.x;
-    sa.lo = t.y;
-    ca.hi = t.z;
-    ca.lo = t.w;
-    return cdf_mk(df_fma(ca, cr, df_neg(df_mul(sa, sr))), df_fma(sa, cr, df_mul(ca, sr)));
+    const float C1 = 0x1.62cp-6f, C2 = 0x1.217f7ep-17f, C3 = -0x1.c610cap-42f, MAGIC = 12582912.0f;
+    // k = rint(32 a / ln2) by the rounding of the addition; its integer in the low bits
+    const fv kb = fma_(a.hi, fv_of(46.1662407f), fv_of(MAGIC));
+    const fv kf = kb - fv_of(MAGIC);
+    const int kx = __float_as_int(kb.x) - 0x4b400000, ky = __float_as_int(kb.y) - 0x4b400000;
+    // a - k C1 is exact; k C2 = p2 + e2 exactly
+    const fv p2 = kf * fv_of(-C2);
+    const fv e2 = fma_(kf, fv_of(C2), p2);
+    df s = two_sum(fma_(kf, fv_of(-C1), a.hi), p2);
+    s = fast_two_sum(s.hi, s.lo + fma_(kf, fv_of(-C3), a.lo - e2));
+    const fv sh = s.hi;
+    const fv tail = sh * sh * fma_(sh, fma_(sh, fv_of(0.0416666679f), fv_of(0.166666672f)), fv_of(0.5f));
+    // e^s = 1 + es
+    const df es = fast_two_sum(sh, s.lo + tail);
+    df E = fast_two_sum(fv_of(1.0f), es.hi);
+    E.lo = E.lo + es.lo;
+    const float2 tx = FT_EXPTAB[kx & 31], ty = FT_EXPTAB[ky & 31];
+    const df pr = tf_norm(tf_mul(tf_mk(make_float2(tx.x, ty.x), make_float2(tx.y, ty.y)), E));
+    const fv sc = make_float2(__int_as_float((127 + (kx >> 5)) << 23), __int_as_float((127 + (ky >> 5)) << 23));
+    return tf_mk(pr.hi * sc, pr.lo * sc);
 }
 
-// The deformed Laplacian at the sample (srcs/feynman_integral.hpp:293-310) and V there
-// (:322-336) in two-float complex arithmetic, for every deformed sample: in FP32 both
-// suffer cancellation (the spanning-tree sum with phases, the quadratic forms against
-// the mass terms), and their errors enter the integrand as D/2 arg psi and W arg V.
-// Conductances y_e = e^(-i theta_e) / X_e from the two-float contour and sector point,
-// the conductance-form elimination of `elim`, the product of its pivots (rescaled by
-// powers of two as it goes: det L(y) = det * 2^det_e) and
-// V = -sum_jk P~_jk (L(y)^-1)_jk + sum_e m2_e X_e e^(i theta_e) (the reference's
-// -sum_r sigma_r q_r^T L^-1 q_r, contracted with P~ itself here).
+// e^(ix) = cos x + i sin x of two angles to ~1e-13 (|x| < 1e5), table-driven after Tang: x = k pi/64 + r with
+// |r| <= pi/128, pi/64 in three FP32 parts (x.hi - k P1 is exact: both are multiples of
+// the same power of two and the difference is small); sin(k pi/64), cos(k pi/64) as float
+// pairs from FT_SCTAB (k mod 128); sin r = r - r^3/6 + r^5/120 and cos r = 1 - r^2/2 +
+// r^4/24 - r^6/720 with r and r^2 in two-float and the terms below 3e-6 in FP32; then
+// the product of the two.
+static __device__ __forceinline__ void expi_pair(df x, cdf* out)
+{
+    const float P1 = 0x1.921fb6p-5f, P2 = -0x1.777a5cp-30f, P3 = -0x1.ee59dap-55f, MAGIC = 12582912.0f;
+    const fv kb = fma_(x.hi, fv_of(0x1.45f306p+4f), fv_of(MAGIC));
+    const fv k = kb - fv_of(MAGIC);
+    const df r = fast_two_sum(fma_(k, fv_of(-P1), x.hi), fma_(k, fv_of(-P3), fma_(k, fv_of(-P2), x.lo)));
+    const fv rh = r.hi, r2 = rh * rh;
+    // sin r = r + rh^3 (-1/6 + rh^2/120)
+    const df sr = fast_two_sum(rh, fma_(rh * r2, fma_(r2, fv_of(0x1.111112p-7f), fv_of(-0x1.555556p-3f)), r.lo));
+    // cos r = 1 - (rh^2 + 2 rh r.lo)/2 + rh^4/24 - rh^6/720, with rh^2 = r2 + qe exactly
+    const fv qe = fma_(rh, rh, -r2);
+    df cr = fast_two_sum(fv_of(1.0f), fv_of(-0.5f) * r2);
+    cr.lo = cr.lo + fma_(r2 * r2, fma_(r2, fv_of(-0x1.6c16c2p-10f), fv_of(0x1.555556p-5f)),
+                           fma_(-rh, r.lo, fv_of(-0.5f) * qe));
+    const float4 tx = FT_SCTAB[__float_as_int(kb.x) & 127], ty = FT_SCTAB[__float_as_int(kb.y) & 127];
+    const df sa = tf_mk(make_float2(tx.x, ty.x), make_float2(tx.y, ty.y));
+    const df ca = tf_mk(make_float2(tx.z, ty.z), make_float2(tx.w, ty.w));
+        const df re = tf_norm(dot_sub_n(ca, cr, sa, sr)), im = tf_norm(dot_add_n(ca, sr, sa, cr));
+    out[0] = cdf_mk(first_of(re), first_of(im));
+    out[1] = cdf_mk(second_of(re), second_of(im));
+}
+
+// |theta| beyond which expi_pair's reduction is not used (the FP64 pass takes the sample)
+#define THETA_MAX 1e5f
+
+// Principal argument of x + i y in two-float to about 1.5e-7 absolute: atanf of the
+// ratio of the smaller to the larger part (a result in [0, pi/4], where an ulp is
+// 6e-8), the octant restored with multiples of pi/2 in two-float, plus the first-order
+// effect of the low parts, (x dy - y dx) / |z|^2.  Zero gives 0.
+static __device__ FT_BIGFN sf arg_f2(float x, float y, float xl, float yl)
+{
+    const float PIO2_HI = 1.57079637f, PIO2_LO = -4.37113883e-8f;
+    const float ax = fabsf(x), ay = fabsf(y);
+    const bool sw = ay > ax;
+    const float num = sw ? ax : ay, den = sw ? ay : ax;
+    // the ratio through the correctly rounded reciprocal (within 1.5 ulp of num / den)
+    const float a = den > 0.0f ? m_atan(num * rcp_(den)) : 0.0f;
+    sf r = sw ? tf_add(tf_mk(PIO2_HI, PIO2_LO), tf_mk(-a, 0.0f)) : tf_mk(a, 0.0f);
+    if (x < 0.0f) r = tf_add(tf_mk(2.0f * PIO2_HI, 2.0f * PIO2_LO), tf_neg(r));
+    if (y < 0.0f) r = tf_neg(r);
+    const float n2 = fmaf(x, x, y * y);
+    return n2 > 0.0f ? tf_add(r, tf_mk((x * yl - y * xl) * rcp_(n2), 0.0f)) : r;
+}
+static __device__ __forceinline__ sf arg_of(cdf z) { return arg_f2(z.re.hi, z.im.hi, z.re.lo, z.im.lo); }
+// principal argument reduced to (-pi, pi] in two-float
+static __device__ __forceinline__ sf wrap_pi(sf x)
+{
+    const float TWO_PI_HI = 6.28318548202514648f, TWO_PI_LO = -1.7484555e-7f;
+    const float f = tf_f(x);
+    const float k = rintf(f * 0.159154943091895336f);
+    // k 2 pi as an exact two-float product
+    const float p = mul_(k, -TWO_PI_HI);
+    const float e = fma_(k, (TWO_PI_HI), p);
+    return tf_norm(tf_addf_n(tf_norm(tf_addf_n(x, p)), -fma_(k, (TWO_PI_LO), e)));
+}
+
 // deformed integrand, the two-float complex block (det L(y) and V): smallest accepted
 // pivot-to-row ratio, smallest |V| relative to the sum of its terms' magnitudes, and
 // largest W qmag / |V| (qmag: the magnitudes of every term summed into V, through the
@@ -1363,63 +1769,93 @@ static __device__ FT_BIGFN cdf expi_df(df x)
 struct cblock {
     cdf V;
     cdf det;
-    int det_e;
-    bool ok;       // pivots and the determinant finite and non-zero
-    bool growth_ok;  // every pivot above ACC_GROWTH of its row's size
-    float mag;     // sum of the magnitudes of V's terms: masses, and one term per external row
-    float qmag;    // the same through the row quadratic forms: sum_i |1/d_i| sum_jk |P~_jk| |U_ij| |U_ik| + mag
+    int e;       // det L(y) = det 2^e
+    bool ok;     // pivots above ACC_GROWTH of their rows, the determinant finite and non-zero
+    float mag;   // sum of the magnitudes of V's terms: masses, and one term per external row
+    float qmag;  // the same through the row quadratic forms: sum_i |1/d_i| sum_jk |P~_jk| |U_ij| |U_ik| + mag
 };
-static __device__ __forceinline__ float cmag_hi(const cdf& z) { return fabsf(z.re.hi) + fabsf(z.im.hi); }
+static __device__ __forceinline__ float cmag_hi(const cdf& z) { return abs_(z.re.hi) + abs_(z.im.hi); }
 
-static __device__ __forceinline__ void complex_block(const df* theta, const f2* Xi2, const float* pd, cblock& o)
-{
-    auto pdf = [&](int i) -> df {
-        df v;
-        v.hi = pd[2 * i];
-        v.lo = pd[2 * i + 1];
-        return v;
-    };
-    cdf c[FT_N][FT_N], g[FT_N];
-#pragma unroll
-    for (int i = 0; i < FT_N; i++) {
-        g[i] = cdf_zero();
-#pragma unroll
-        for (int j = 0; j < FT_N; j++) c[i][j] = cdf_zero();
+// the deformation angles and the upper triangle of X^1/2 H X^1/2, in the scratch or not
+struct angles {
+#if FT_SCRATCH >= 1
+    __device__ __forceinline__ void set(unsigned char* lxs, int e, sf v)
+    {
+        SCR_TH(e, 0) = v.hi;
+        SCR_TH(e, 1) = v.lo;
     }
-    cdf v = cdf_zero();
+    __device__ __forceinline__ sf get(unsigned char* lxs, int e) const { return tf_mk(SCR_TH(e, 0), SCR_TH(e, 1)); }
+#else
+    sf v[FT_E];
+    __device__ __forceinline__ void set(unsigned char*, int e, sf x) { v[e] = x; }
+    __device__ __forceinline__ sf get(unsigned char*, int e) const { return v[e]; }
+#endif
+};
+struct hessian {
+#if FT_SCRATCH >= 2
+    __device__ __forceinline__ void set(unsigned char* lxs, int a, int b, float v) { SCR_H(a, b) = v; }
+    __device__ __forceinline__ float get(unsigned char* lxs, int a, int b) const { return SCR_H(a, b); }
+#else
+    float v[FT_E][FT_E];
+    __device__ __forceinline__ void set(unsigned char*, int a, int b, float x) { v[a][b] = x; }
+    __device__ __forceinline__ float get(unsigned char*, int a, int b) const { return v[a][b]; }
+#endif
+};
+#define XI(e) tf_mk(LX(e, 0), LX(e, 1))
+
+// The deformed Laplacian at the sample (srcs/feynman_integral.hpp:293-310) and V there
+// (:322-336) in two-float complex arithmetic, for every deformed sample: in FP32 both
+// suffer cancellation (the spanning-tree sum with phases, the quadratic forms against
+// the mass terms), and their errors enter the integrand as D/2 arg psi and W arg V.
+// Conductances y_e = e^(-i theta_e) / X_e from the two-float contour and sector point,
+// the conductance-form elimination of `elim`, the product of its pivots (rescaled by
+// powers of two as it goes: det L(y) = det 2^e) and
+// V = -sum_jk P~_jk (L(y)^-1)_jk + sum_e m2_e X_e e^(i theta_e) (the reference's
+// -sum_r sigma_r q_r^T L^-1 q_r, contracted with P~ itself here).
+static __device__ __forceinline__ void complex_block(unsigned char* lxs, const angles& th, const float4* pp, cblock& o)
+{
+    cdf c[FT_N][FT_N], g[FT_N];
+    cdf v, ei[2];
     float mag = 0.0f;
 #pragma unroll
     for (int e = 0; e < FT_E; e++) {
-        const cdf eix = expi_df(theta[e]);
-        const df cs = eix.re, sn = eix.im;
-        const df xi = df_of(Xi2[e]);
-        const cdf y = cdf_mk(df_mul(xi, cs), df_neg(df_mul(xi, sn)));
+        if (!(e & 1)) expi_pair(pair_of(th.get(lxs, e), th.get(lxs, e + 1 < FT_E ? e + 1 : e)), ei);
+        const cdf eix = ei[e & 1];
+        const sf xi = XI(e);
+        const cdf y = cdf_mk(tf_mul(xi, eix.re), tf_mul(tf_neg(xi), eix.im));
         const int k = FT_EK[e], l = FT_EL[e];
         cdf& slot = (k == FT_V - 1) ? g[l] : c[l][k];
-        slot = first_in_slot(e) ? y : slot + y;
-        const df m2x = df_mul(pdf(P_M2 + e), df_inv(xi));
-        const cdf mt = cdf_mk(df_mul(m2x, cs), df_mul(m2x, sn));
-        v = e == 0 ? mt : v + mt;
-        mag += fabsf(m2x.hi);
+        slot = first_in_slot(e) ? y : cdf_add_n(slot, y);
+        const sf m2x = tf_mul(prm_sf(pp, P_M2 + e), tf_inv(xi));
+        const cdf mt = cdf_scale(m2x, eix);
+        v = e == 0 ? mt : cdf_add_n(v, mt);
+        mag = mag + abs_(m2x.hi);
     }
-    cdf a[FT_N][FT_N], dinv[FT_N];
-    cdf det = cdf_mk(df_mk(1.0f), df_mk(0.0f));
-    int det_e = 0;
-    bool ok = true;
-    bool growth_ok = true;
+    cdf a[FT_N][FT_N], dinv[FT_N], det;
+    o.e = 0;
+    o.ok = true;
 #pragma unroll
     for (int k = 0; k < FT_N; k++) {
-        cdf dk = g[k];
-        float row = cmag_hi(g[k]);
+        if (NZG(k) && SUMS_G(k)) g[k] = cdf_norm(g[k]);
+        cdf dk;
+        float row;
+        bool any = NZG(k);
+        if (any) {
+            dk = g[k];
+            row = cmag_hi(g[k]);
+        }
 #pragma unroll
         for (int j = k + 1; j < FT_N; j++) {
             if (!NZC(k, j)) continue;
-            dk = dk + c[k][j];
-            row += cmag_hi(c[k][j]);
+            if (SUMS_C(k, j)) c[k][j] = cdf_norm(c[k][j]);
+            dk = any ? cdf_add_n(dk, c[k][j]) : c[k][j];
+            row = any ? row + cmag_hi(c[k][j]) : cmag_hi(c[k][j]);
+            any = true;
         }
-        growth_ok &= cmag_hi(dk) > ACC_GROWTH * row;
-        det = det * dk;
-        ok &= cdf_renorm(det, det_e);
+        dk = cdf_norm(dk);
+        o.ok &= cmag_hi(dk) > ACC_GROWTH * row;
+        det = k == 0 ? dk : det * dk;
+        cdf_renorm(det, o.e, o.ok);
         dinv[k] = cdf_inv(dk);
 #pragma unroll
         for (int i = k + 1; i < FT_N; i++)
@@ -1427,10 +1863,10 @@ static __device__ __forceinline__ void complex_block(const df* theta, const f2* 
 #pragma unroll
         for (int i = k + 1; i < FT_N; i++) {
             if (!NZC(k, i)) continue;
-            if (NZG(k)) g[i] = cdf_fma(a[k][i], g[k], g[i]);
+            if (NZG(k)) g[i] = ADDS_G(k, i) ? cdf_fma_n(a[k][i], g[k], g[i]) : a[k][i] * g[k];
 #pragma unroll
             for (int j = i + 1; j < FT_N; j++)
-                if (NZC(k, j)) c[i][j] = cdf_fma(a[k][i], c[k][j], c[i][j]);
+                if (NZC(k, j)) c[i][j] = ADDS_C(k, i, j) ? cdf_fma_n(a[k][i], c[k][j], c[i][j]) : a[k][i] * c[k][j];
         }
     }
     // The momentum part, sum_jk P~_jk (L(y)^-1)_jk over the external rows [Q0, N) (P~
@@ -1441,61 +1877,65 @@ static __device__ __forceinline__ void complex_block(const df* theta, const f2* 
     float qmag = 0.0f;
 #if FT_NE > 0
     {
-        auto ptd = [&](int j, int k) -> df { return pdf(PT_AT(j, k)); };
+        auto ptd = [&](int j, int k) -> sf { return prm_sf(pp, PT_AT(j, k)); };
         cdf U[FT_NE][FT_NE];   // U[i][j], j < i (indices from Q0)
-        cdf vq = cdf_zero();
+        cdf vq;
 #pragma unroll
         for (int ii = 0; ii < FT_NE; ii++) {
             const int i = FT_Q0 + ii;
 #pragma unroll
             for (int jj = 0; jj < ii; jj++) {
                 const int j = FT_Q0 + jj;
-                cdf u = cdf_zero();
-                bool any = false;
+                cdf u;
+                int terms = 0;
                 if (NZC(j, i)) {
                     u = a[j][i];
-                    any = true;
+                    terms = 1;
                 }
 #pragma unroll
                 for (int kk = jj + 1; kk < ii; kk++) {
                     const int k = FT_Q0 + kk;
-                    if (!NZC(k, i)) continue;
-                    u = any ? cdf_fma(a[k][i], U[kk][jj], u) : a[k][i] * U[kk][jj];
-                    any = true;
+                    if (!NZC(k, i) || !NZM(j, k)) continue;
+                    u = terms ? cdf_fma_n(a[k][i], U[kk][jj], u) : a[k][i] * U[kk][jj];
+                    terms++;
                 }
-                U[ii][jj] = u;
+                if (terms) U[ii][jj] = terms > 1 ? cdf_norm(u) : u;
             }
             // Q = u^T P~ u with u = (U_i0 .. U_i,i-1, 1): Q = P_ii + sum_j u_j w_j,
             // w_j = sum_{j <= k < i} P_jk u_k + P_ji (off-diagonal P doubled)
-            cdf Q = cdf_mk(ptd(ii, ii), df_mk(0.0f));
-            float qm = fabsf(ptd(ii, ii).hi);
+            const sf pii = ptd(ii, ii);
+            cdf Q = cdf_mk(pii, tf_zero<float>());
+            float qm = abs_(pii.hi);
+            bool one = true;
 #pragma unroll
             for (int jj = 0; jj < ii; jj++) {
-                cdf w = ptd(jj, jj) * U[ii][jj];
-                float wm = fabsf(ptd(jj, jj).hi) * cmag_hi(U[ii][jj]);
+                if (!NZM(FT_Q0 + jj, i)) continue;
+                const sf pj = ptd(jj, ii);
+                cdf w = cdf_scale(ptd(jj, jj), U[ii][jj]);
+                float wm = abs_(ptd(jj, jj).hi) * cmag_hi(U[ii][jj]);
 #pragma unroll
                 for (int kk = jj + 1; kk < ii; kk++) {
-                    w = w + ptd(jj, kk) * U[ii][kk];
-                    wm += fabsf(ptd(jj, kk).hi) * cmag_hi(U[ii][kk]);
+                    if (!NZM(FT_Q0 + kk, i)) continue;
+                    w = cdf_add_n(w, cdf_scale(ptd(jj, kk), U[ii][kk]));
+                    wm = fma_(abs_(ptd(jj, kk).hi), cmag_hi(U[ii][kk]), wm);
                 }
-                w.re = df_add(w.re, ptd(jj, ii));
-                wm += fabsf(ptd(jj, ii).hi);
-                Q = cdf_fma(U[ii][jj], w, Q);
-                qm += cmag_hi(U[ii][jj]) * wm;
+                w.re = tf_add_n(w.re, pj);
+                w = cdf_norm(w);
+                wm = wm + abs_(pj.hi);
+                Q = cdf_fma_n(U[ii][jj], w, Q);
+                qm = fma_(cmag_hi(U[ii][jj]), wm, qm);
+                one = false;
             }
-            const cdf t = Q * dinv[i];
-            vq = ii == 0 ? t : vq + t;
-            mag += cmag_hi(t);
-            qmag += qm * cmag_hi(dinv[i]);
+            const cdf t = one ? cdf_scale(pii, dinv[i]) : cdf_norm(Q) * dinv[i];
+            vq = ii == 0 ? t : cdf_add_n(vq, t);
+            mag = mag + cmag_hi(t);
+            qmag = fma_(qm, cmag_hi(dinv[i]), qmag);
         }
-        v = v - vq;
+        v = cdf_mk(tf_sub_n(v.re, vq.re), tf_sub_n(v.im, vq.im));
     }
 #endif
-    o.V = v;
+    o.V = cdf_norm(v);
     o.det = det;
-    o.det_e = det_e;
-    o.ok = ok;
-    o.growth_ok = growth_ok;
     o.mag = mag;
     o.qmag = qmag + mag;
 }
@@ -1506,108 +1946,115 @@ static __device__ __forceinline__ void complex_block(const df* theta, const f2* 
 // sizeable fraction of sectors, so the block runs in two-float arithmetic: the
 // conductance-form elimination (all operations on positive values), G = L^-1, the
 // potentials h_r = G q_r and their drops across the edges, the effective-resistance
-// combinations t, and the Minkowski products s.  Outputs theta and the upper
-// triangle of H in FP32.  pd: the parameter block as two-float pairs.
-static __device__ __forceinline__ void derivatives_df(const float* Xi32, const f2* XiT, const float* pd, df* theta_out,
-                                                      float (*H_out)[FT_E], bool& cancel)
+// combinations t, and the Minkowski products s.  Reads 1/X from the scratch; outputs theta
+// and the upper triangle of X^1/2 H X^1/2 in FP32.
+static __device__ __forceinline__ void derivatives(unsigned char* lxs, const float4* pp, angles& th, hessian& H,
+                                                        bool& cancel)
 {
-    df c[FT_N][FT_N], g[FT_N];
-#pragma unroll
-    for (int i = 0; i < FT_N; i++) {
-        g[i] = df_mk(0.0f);
-#pragma unroll
-        for (int j = 0; j < FT_N; j++) c[i][j] = df_mk(0.0f);
-    }
+    sf c[FT_N][FT_N], g[FT_N];
 #pragma unroll
     for (int e = 0; e < FT_E; e++) {
         const int k = FT_EK[e], l = FT_EL[e];
-        df& slot = (k == FT_V - 1) ? g[l] : c[l][k];
-        slot = first_in_slot(e) ? df_of(XiT[e]) : df_add(slot, df_of(XiT[e]));
+        sf& slot = (k == FT_V - 1) ? g[l] : c[l][k];
+        slot = first_in_slot(e) ? XI(e) : tf_add_n(slot, XI(e));
     }
-    df a[FT_N][FT_N], id[FT_N];
+    sf a[FT_N][FT_N], id[FT_N];
 #pragma unroll
     for (int k = 0; k < FT_N; k++) {
-        df dk = g[k];
+        if (NZG(k) && SUMS_G(k)) g[k] = tf_norm(g[k]);
+        sf dk;
+        bool any = NZG(k);
+        if (any) dk = g[k];
 #pragma unroll
         for (int j = k + 1; j < FT_N; j++)
-            if (NZC(k, j)) dk = df_add(dk, c[k][j]);
-        id[k] = df_inv(dk);
+            if (NZC(k, j)) {
+                if (SUMS_C(k, j)) c[k][j] = tf_norm(c[k][j]);
+                dk = any ? tf_add_n(dk, c[k][j]) : c[k][j];
+                any = true;
+            }
+        id[k] = tf_inv(tf_norm(dk));
 #pragma unroll
         for (int i = k + 1; i < FT_N; i++)
-            if (NZC(k, i)) a[k][i] = df_mul(c[k][i], id[k]);
+            if (NZC(k, i)) a[k][i] = tf_mul(c[k][i], id[k]);
 #pragma unroll
         for (int i = k + 1; i < FT_N; i++) {
             if (!NZC(k, i)) continue;
-            if (NZG(k)) g[i] = df_fma(a[k][i], g[k], g[i]);
+            if (NZG(k)) g[i] = ADDS_G(k, i) ? tf_fma_n(a[k][i], g[k], g[i]) : tf_mul(a[k][i], g[k]);
 #pragma unroll
             for (int j = i + 1; j < FT_N; j++)
-                if (NZC(k, j)) c[i][j] = df_fma(a[k][i], c[k][j], c[i][j]);
+                if (NZC(k, j)) c[i][j] = ADDS_C(k, i, j) ? tf_fma_n(a[k][i], c[k][j], c[i][j]) : tf_mul(a[k][i], c[k][j]);
         }
     }
     // N = M^-1 (unit upper triangular, non-negative), G = N diag(1/d) N^T
-    df Nm[FT_N][FT_N];
+    sf Nm[FT_N][FT_N];
 #pragma unroll
     for (int i = FT_N - 1; i >= 0; i--) {
 #pragma unroll
         for (int j = i + 1; j < FT_N; j++) {
             if (!NZM(i, j)) continue;
-            df s = NZC(i, j) ? a[i][j] : df_mk(0.0f);
-            bool any = NZC(i, j);
+            sf s;
+            int terms = 0;
+            if (NZC(i, j)) {
+                s = a[i][j];
+                terms = 1;
+            }
 #pragma unroll
             for (int k = i + 1; k < j; k++)
                 if (NZC(i, k) && NZM(k, j)) {
-                    s = any ? df_fma(a[i][k], Nm[k][j], s) : df_mul(a[i][k], Nm[k][j]);
-                    any = true;
+                    s = terms ? tf_fma_n(a[i][k], Nm[k][j], s) : tf_mul(a[i][k], Nm[k][j]);
+                    terms++;
                 }
-            Nm[i][j] = s;
+            Nm[i][j] = terms > 1 ? tf_norm(s) : s;
         }
     }
     // Nd[j][k] = N[j][k] / d_k, so that each term of G is one two-float multiply-add
-    df Nd[FT_N][FT_N];
+    sf Nd[FT_N][FT_N];
 #pragma unroll
     for (int j = 0; j < FT_N; j++)
 #pragma unroll
         for (int k = j + 1; k < FT_N; k++)
-            if (NZM(j, k)) Nd[j][k] = df_mul(Nm[j][k], id[k]);
-    df G[FT_N][FT_N];
+            if (NZM(j, k)) Nd[j][k] = tf_mul(Nm[j][k], id[k]);
+    sf G[FT_N][FT_N];
 #pragma unroll
     for (int i = 0; i < FT_N; i++)
 #pragma unroll
         for (int j = i; j < FT_N; j++) {
             // k = j term has N[j][j] = 1
-            df s = (i == j) ? id[j] : (NZM(i, j) ? Nd[i][j] : df_mk(0.0f));
+            sf s = tf_zero<float>();
+            int terms = 0;
+            if (i == j || NZM(i, j)) {
+                s = (i == j) ? id[j] : Nd[i][j];
+                terms = 1;
+            }
 #pragma unroll
             for (int k = j + 1; k < FT_N; k++)
-                if (NZM(i, k) && NZM(j, k)) s = df_fma(Nm[i][k], Nd[j][k], s);
-            G[i][j] = s;
-            G[j][i] = s;
+                if (NZM(i, k) && NZM(j, k)) {
+                    s = terms ? tf_fma_n(Nm[i][k], Nd[j][k], s) : tf_mul(Nm[i][k], Nd[j][k]);
+                    terms++;
+                }
+            G[i][j] = G[j][i] = terms > 1 ? tf_norm(s) : s;
         }
-    df hb[FT_RANK][FT_E];
+    sf hb[FT_RANK][FT_E];
 #pragma unroll
     for (int r = 0; r < FT_RANK; r++) {
-        df h[FT_N];
+        sf h[FT_N];
 #pragma unroll
         for (int i = 0; i < FT_N; i++) {
-            df s = df_mk(0.0f);
+            sf s = tf_zero<float>();
 #pragma unroll
             for (int j = FT_Q0; j < FT_N; j++) {
-                df q;
-                q.hi = pd[2 * (P_Q + r * FT_N + j)];
-                q.lo = pd[2 * (P_Q + r * FT_N + j) + 1];
-                s = j == FT_Q0 ? df_mul(G[i][j], q) : df_fma(G[i][j], q, s);
+                const sf q = prm_sf(pp, P_Q + r * FT_N + j);
+                s = j == FT_Q0 ? tf_mul(G[i][j], q) : tf_fma_n(G[i][j], q, s);
             }
             h[i] = s;
         }
 #pragma unroll
         for (int e = 0; e < FT_E; e++) {
             const int k = FT_EK[e], l = FT_EL[e];
-            hb[r][e] = (k == FT_V - 1) ? df_neg(h[l]) : df_sub(h[k], h[l]);
+            hb[r][e] = (k == FT_V - 1) ? tf_norm(tf_neg(h[l])) : tf_sub(h[k], h[l]);
         }
     }
-    auto Gx = [&](int i, int j) -> df { return (i == FT_V - 1 || j == FT_V - 1) ? df_mk(0.0f) : G[i][j]; };
-    df kappa;
-    kappa.hi = pd[2 * P_DEF];
-    kappa.lo = pd[2 * P_DEF + 1];
+    const sf kappa = prm_sf(pp, P_DEF);
 #pragma unroll
     for (int a2 = 0; a2 < FT_E; a2++) {
         const int ka = FT_EK[a2], la = FT_EL[a2];
@@ -1615,295 +2062,101 @@ static __device__ __forceinline__ void derivatives_df(const float* Xi32, const f
         // L^-1 is zero): edge a2's resistance combination with any edge (k, l),
         // G_ka,k + G_la,l - G_ka,l - G_la,k, is then w_k - w_l.  The entries no edge
         // pair reads are dropped at compile time.
-        df w[FT_N];
+        sf w[FT_N];
 #pragma unroll
         for (int v = 0; v < FT_N; v++)
-            w[v] = ka == FT_V - 1 ? df_neg(G[la][v]) : (la == FT_V - 1 ? G[ka][v] : df_sub(G[ka][v], G[la][v]));
-        auto wd = [&](int k, int l) -> df {
-            return k == FT_V - 1 ? df_neg(w[l]) : (l == FT_V - 1 ? w[k] : df_sub(w[k], w[l]));
+            w[v] = ka == FT_V - 1 ? tf_neg(G[la][v]) : (la == FT_V - 1 ? G[ka][v] : tf_sub_n(G[ka][v], G[la][v]));
+        auto wd = [&](int k, int l) -> sf {
+            return k == FT_V - 1 ? tf_neg(w[l]) : (l == FT_V - 1 ? w[k] : tf_sub_n(w[k], w[l]));
         };
-        df sig_hb[FT_RANK];
-        df s = df_mk(0.0f);
+        sf sig_hb[FT_RANK];
+        sf s = tf_zero<float>();
 #pragma unroll
         for (int r = 0; r < FT_RANK; r++) {
-            df sg;
-            sg.hi = pd[2 * (P_SIG + r)];
-            sg.lo = pd[2 * (P_SIG + r) + 1];
-            sig_hb[r] = df_mul(sg, hb[r][a2]);
-            s = r == 0 ? df_mul(sig_hb[r], hb[r][a2]) : df_fma(sig_hb[r], hb[r][a2], s);
+            sig_hb[r] = tf_mul(prm_sf(pp, P_SIG + r), hb[r][a2]);
+            s = r == 0 ? tf_mul(sig_hb[r], hb[r][a2]) : tf_fma_n(sig_hb[r], hb[r][a2], s);
         }
-        const df t = wd(ka, la);
+        if (FT_RANK > 1) s = tf_norm(s);
+        const sf t = tf_norm(wd(ka, la));
         // an edge whose ends float together: the FP64 pass takes the sample
-        cancel |= ka != FT_V - 1 && !(df_f(t) > 1e-7f * (df_f(Gx(ka, ka)) + df_f(Gx(la, la))));
-        const df xi = df_of(XiT[a2]);
-        const df xa = df_mul(xi, xi);
-        const df xas = df_mul(xa, s);
-        df m2;
-        m2.hi = pd[2 * (P_M2 + a2)];
-        m2.lo = pd[2 * (P_M2 + a2) + 1];
-        theta_out[a2] = df_mul(df_sub(m2, xas), kappa);
-        // 2 xa s (1/x - xa t)
-        H_out[a2][a2] = 2.0f * df_f(df_mul(xas, df_sub(xi, df_mul(xa, t))));
-        // the off-diagonal entries are FP32 products of their (two-float) factors
-        const float xaf = df_f(xa);
+        if (ka != FT_V - 1) {
+            cancel |= !(t.hi > 1e-7f * (G[ka][ka].hi + G[la][la].hi));
+        }
+        const sf xi = XI(a2);
+        const sf xa = tf_mul(xi, xi);
+        const sf xas = tf_mul(xa, s);
+        th.set(lxs, a2, tf_mul(tf_sub(prm_sf(pp, P_M2 + a2), xas), kappa));
+        const float sxa = rsqrt_newton(xi.hi);   // X^1/2
+        // 2 xa s (1/x - xa t), times x
+        H.set(lxs, a2, a2, 2.0f * tf_f(tf_mul(xas, tf_sub(xi, tf_mul(xa, t)))) * (sxa * sxa));
+        // the off-diagonal entries are FP32 products of their (two-float) factors;
+        // X^-3/2 of an edge scales its row and column
+        const float xaf = -2.0f * tf_f(xa) * sxa;
 #pragma unroll
         for (int b = a2 + 1; b < FT_E; b++) {
             const int kb = FT_EK[b], lb = FT_EL[b];
-            df s2 = df_mk(0.0f);
+            sf s2 = tf_zero<float>();
 #pragma unroll
-            for (int r = 0; r < FT_RANK; r++) s2 = r == 0 ? df_mul(sig_hb[r], hb[r][b]) : df_fma(sig_hb[r], hb[r][b], s2);
-            const df t2 = wd(kb, lb);
-            const float xb = Xi32[b];
-            H_out[a2][b] = -2.0f * (xaf * (xb * xb)) * df_f(s2) * df_f(t2);
+            for (int r = 0; r < FT_RANK; r++)
+                s2 = r == 0 ? tf_mul(sig_hb[r], hb[r][b]) : tf_fma_n(sig_hb[r], hb[r][b], s2);
+            const float xb = LX(b, 0);
+            H.set(lxs, a2, b, xaf * (xb * xb * rsqrt_newton(xb)) * tf_f(s2) * tf_f(wd(kb, lb)));
         }
     }
 }
-#endif
 
-// positive value m * 2^e with m in [1, 2): products of many pivots and X values
-// without overflow, and logarithms split into an exact integer and a small part
-struct mexp {
-    float m;
-    int e;
-    bool bad;
-};
-static __device__ __forceinline__ void mx_mul(mexp& a, float x)
+// Deformed integrand (srcs/feynman_integral.hpp:278-362) of a sample, in the frame X_e =
+// exp(lx_e - sh).  False: the evaluation cannot be trusted (the sample then goes to the
+// FP64 pass).
+static __device__ __forceinline__ bool integrand_one(const float4* pp, const float* pf, unsigned char* lxs, sf lF,
+                                                     sf lG, cx<float>* out)
 {
-    const float p = a.m * x;
-    const int b = __float_as_int(p);
-    const int be = (b >> 23) & 0xff;
-    a.bad |= (be == 0) | (be == 255) | (b < 0);
-    a.e += be - 127;
-    a.m = __int_as_float((b & 0x007fffff) | 0x3f800000);
-}
-static __device__ __forceinline__ mexp mx_one()
-{
-    mexp r;
-    r.m = 1.0f;
-    r.e = 0;
-    r.bad = false;
-    return r;
-}
-static __device__ __forceinline__ f2 f2_make(float h, float l)
-{
-    f2 r;
-    r.hi = h;
-    r.lo = l;
-    return r;
-}
-static __device__ __forceinline__ f2 f2_mulf(f2 a, float b)
-{
-    const float p = a.hi * b;
-    const float e = fmaf(a.hi, b, -p) + a.lo * b;
-    const float h = p + e;
-    return f2_make(h, e - (h - p));
-}
-static __device__ __forceinline__ f2 f2_mul2(f2 a, f2 b)
-{
-    const float p = a.hi * b.hi;
-    const float e = fmaf(a.hi, b.hi, -p) + (a.hi * b.lo + a.lo * b.hi);
-    const float h = p + e;
-    return f2_make(h, e - (h - p));
-}
-static __device__ __forceinline__ f2 f2_neg(f2 a) { return f2_make(-a.hi, -a.lo); }
-// undeformed integrand: relative size of V below which the FP32 evaluation hands the
-// sample to FP64
-#ifndef V_CANCEL
-#define V_CANCEL 0.05f
-#endif
-// smallest pivot-to-row ratio accepted in the FP32 elimination of the Jacobian
-#ifndef PIVOT_GROWTH
-#define PIVOT_GROWTH 0.02f
-#endif
-#define RLN2_HI 1.44269502162933349609375f
-#define RLN2_LO 1.925963033500011e-8f
-#define LN2_F 0.69314718055994531f
-
-// log2(value / exp(lref)) for value = mx and a natural-log reference lref (two-float)
-static __device__ __forceinline__ f2 log2_ratio(const mexp& mx, f2 lref)
-{
-    f2 r = f2_mul2(lref, f2_make(RLN2_HI, RLN2_LO));
-    r = f2_add(f2_neg(r), (float)mx.e);
-    return f2_add(r, m_log2(mx.m));
-}
-
-// principal argument reduced to (-pi, pi]; `edge` reports a value within 1e-5 of
-// the branch cut, where FP32 cannot decide the branch the way the reference does
-static __device__ __forceinline__ float wrap_pi(float x, bool& edge)
-{
-    const float TWO_PI_HI = 6.28318548202514648f, TWO_PI_LO = -1.7484555e-7f;
-    const float k = rintf(x * 0.159154943091895336f);
-    float r = fmaf(-k, TWO_PI_HI, x);
-    r = fmaf(-k, TWO_PI_LO, r);
-    edge |= fabsf(r) > 3.14158265f;
-    return r;
-}
-
-// two-float variant of wrap_pi
-static __device__ __forceinline__ f2 wrap_pi2(f2 x, bool& edge)
-{
-    const float TWO_PI_HI = 6.28318548202514648f, TWO_PI_LO = -1.7484555e-7f;
-    const float k = rintf((x.hi + x.lo) * 0.159154943091895336f);
-    // k * 2pi as an exact two-float product (k * TWO_PI_HI alone is rounded once |k| > 1)
-    const float p = k * TWO_PI_HI;
-    f2 r = f2_add(x, -p);
-    r = f2_add(r, -fmaf(k, TWO_PI_HI, -p));
-    r = f2_add(r, -k * TWO_PI_LO);
-    edge |= fabsf(r.hi + r.lo) > 3.14158265f;
-    return r;
-}
-
-// Principal argument of x + i y in two-float to about 1.5e-7 absolute: atanf of the
-// ratio of the smaller to the larger part (a result in [0, pi/4], where an ulp is
-// 6e-8), the octant restored with multiples of pi/2 in two-float, plus the first-order
-// effect of the low parts, (x dy - y dx) / |z|^2.  Zero gives 0.
-static __device__ FT_BIGFN f2 arg_f2(float x, float y, float xl, float yl)
-{
-    const float PIO2_HI = 1.57079637f, PIO2_LO = -4.37113883e-8f;
-    const float ax = fabsf(x), ay = fabsf(y);
-    const bool sw = ay > ax;
-    const float num = sw ? ax : ay, den = sw ? ay : ax;
-    // the ratio through the correctly rounded reciprocal (within 1.5 ulp of num / den)
-    const float a = den > 0.0f ? m_atan(num * rcp_(den)) : 0.0f;
-    f2 r = sw ? f2_add(f2_make(PIO2_HI, PIO2_LO), -a) : f2_make(a, 0.0f);
-    if (x < 0.0f) r = f2_add2(f2_make(2.0f * PIO2_HI, 2.0f * PIO2_LO), f2_neg(r));
-    if (y < 0.0f) r = f2_neg(r);
-    const float n2 = fmaf(x, x, y * y);
-    return n2 > 0.0f ? f2_add(r, (x * yl - y * xl) * rcp_(n2)) : r;
-}
-
-// Sets need64 when the FP32 / two-float evaluation cannot be trusted (the sample then
-// goes to the FP64 pass); returns false for a dropped (non-finite) sample.
-static __device__ __forceinline__ bool integrand32(const float* pd, const float* pf, const f2* lx, f2 lF, f2 lG,
-                                                   cx<float>* out, bool& need64)
-{
-    need64 = false;
-    const float D2 = 0.5f * pf[P_D], W = pf[P_W];
-    // working frame X_e = exp(lx_e - sh), sh an integer near the middle of the range;
-    // R and the eps factor are ratios to the tropical approximants and do not depend on it
+    const float D2 = 0.5f * pf[P_D], W = pf[P_W], IGtr = pf[P_IGTR];
     float lmin = 0.0f;
 #pragma unroll
-    for (int e = 0; e < FT_E; e++) lmin = fminf(lmin, lx[e].hi);
+    for (int e = 0; e < FT_E; e++) lmin = fminf(lmin, LX(e, 0));
+    // sh an integer near the middle of the range; R and the eps factor are ratios to the
+    // tropical approximants and do not depend on it
     const float sh = rintf(0.5f * lmin);
-    float X[FT_E], Xi[FT_E];
-#if FT_MODE == 1
     // 1/X in two-float for the derivative block and the complex Laplacian (theta is a
-    // function of X whose phase effect grows with |theta|); X and 1/X in FP32 from it;
-    // log prod X (in the frame) in two-float
-    f2 Xi2[FT_E];
-    f2 sumlx = f2_make(0.0f, 0.0f);
-    bool xbad = false;
+    // function of X whose phase effect grows with |theta|), over log X in the scratch;
+    // log prod X in the frame
+    bool bad = false;
+    df sums = tf_zero<fv>();
 #pragma unroll
-    for (int e = 0; e < FT_E; e++) {
-        const f2 a = f2_add(lx[e], -sh);
-        sumlx = f2_add2(sumlx, a);
-        Xi2[e] = exp_f2(f2_make(-a.hi, -a.lo));
-        Xi[e] = Xi2[e].hi;
-        X[e] = rcp_(Xi[e]);
-        xbad |= !(Xi[e] > 1e-30f && Xi[e] < 1e30f);
+    for (int e = 0; e < FT_E; e += 2) {
+        const int f = e + 1 < FT_E ? e + 1 : e;
+        const df na = tf_norm(tf_sub_n(tf_mk(fv_of(sh), fv_of(0.0f)), pair_of(XI(e), XI(f))));
+        const df xi = exp_pair(na);
+        const sf na1 = f == e ? tf_zero<float>() : second_of(na);
+        sums = e == 0 ? na : tf_add_n(sums, f == e ? pair_of(first_of(na), na1) : na);
+        LX(e, 0) = xi.hi.x;
+        LX(e, 1) = xi.lo.x;
+        LX(f, 0) = xi.hi.y;
+        LX(f, 1) = xi.lo.y;
+        // outside the two-float exponential's range: the FP64 pass takes it
+        bad |= !(fabsf(na.hi.x) < 69.0f) || !(fabsf(na.hi.y) < 69.0f);
     }
-    if (xbad) {   // outside the two-float exponential's range: the FP64 pass takes it
-        need64 = true;
-        return false;
-    }
-#else
-#pragma unroll
-    for (int e = 0; e < FT_E; e++) {
-        const f2 a = f2_add(lx[e], -sh);
-        const float ep = m_exp(a.hi), em = m_exp(-a.hi);
-        X[e] = fmaf(ep, a.lo, ep);
-        Xi[e] = fmaf(em, -a.lo, em);
-    }
-#endif
-    const f2 lFs = f2_add(lF, -(float)FT_LOOPS * sh);   // log psi_tr in the frame
-    const f2 lGs = f2_add(lG, -sh);                      // log V_tr = log(xi_tr / psi_tr)
-    const float IGtr = pf[P_IGTR];
-#if FT_MODE == 0
-    elim<float, float> L;
-    L.factor(Xi);
-    mexp psi = mx_one();
-#pragma unroll
-    for (int k = 0; k < FT_N; k++) mx_mul(psi, L.d[k]);
-#pragma unroll
-    for (int e = 0; e < FT_E; e++) mx_mul(psi, X[e]);
-    if (psi.bad) {
-        need64 = true;
-        return false;
-    }
-    const f2 lpsi = log2_ratio(psi, lFs);   // log2(psi / psi_tr)
-#if FT_ONLY_PSI
-    const f2 t = f2_mulf(lpsi, -D2);
-    const float R = m_exp2(t.hi) * (1.0f + t.lo * LN2_F);
-    out[0] = cmk(IGtr * R, 0.0f);
-    return true;
-#else
-    float pphi = 0.0f, mag = 0.0f;
-#pragma unroll
-    for (int r = 0; r < FT_RANK; r++) {
-        const float v = pf[P_SIG + r] * L.quad(pf + P_Q + r * FT_N);
-        pphi -= v;
-        mag += fabsf(v);
-    }
-    float pxi = pphi;
-#pragma unroll
-    for (int e = 0; e < FT_E; e++) {
-        const float v = pf[P_M2 + e] * X[e];
-        pxi += v;
-        mag += fabsf(v);
-    }
-    if (!(pxi > V_CANCEL * mag)) {   // cancellation, or a sign the FP64 pass must decide
-        need64 = true;
-        return false;
-    }
-    mexp V = mx_one();
-    mx_mul(V, pxi);
-    const f2 lv = log2_ratio(V, lGs);   // log2(V / V_tr)
-    const f2 t = f2_add2(f2_mulf(lpsi, -D2), f2_mulf(lv, -W));
-    const float Rf = m_exp2(t.hi) * (1.0f + t.lo * LN2_F);
-    if (!isfinite(Rf) || V.bad) {
-        need64 = true;
-        return false;
-    }
-    float R = IGtr * Rf;
-    out[0] = cmk(R, 0.0f);
-    if (FT_K > 1) {
-        const float ef = LN2_F * ((float)(psi.e - FT_LOOPS * V.e) + (m_log2(psi.m) - (float)FT_LOOPS * m_log2(V.m)));
-#pragma unroll
-        for (int j = 1; j < FT_K; j++) {
-            R *= ef * (1.0f / (float)j);
-            out[j] = cmk(R, 0.0f);
-        }
-    }
-    return true;
-#endif
-#else
-    const float kappa = pf[P_DEF];
-    // The contour (theta) and its Jacobian come from differences of entries of L^-1,
-    // which cancel in FP32 for a sizeable fraction of sectors; this block runs in two-float.
-    df theta[FT_E];
-    float H[FT_E][FT_E];
-    bool cancel = false;
-    derivatives_df(Xi, Xi2, pd, theta, H, cancel);
-    if (cancel) {
-        need64 = true;
-        return false;
-    }
-    // det(I + i kappa X^1/2 H X^1/2) (similar to I + i kappa H X, srcs/feynman_integral.hpp:312-320):
-    // the real part is the identity, so the symmetric elimination needs no pivoting; FP32,
-    // the pivots' product rescaled by powers of two (det J = pj 2^pj_e).  Before the complex
-    // block, so that H is no longer live there.
-    cx<float> pj = cmk(1.0f, 0.0f);
-    int pj_e = 0;
-    bool jok = true;   // pivots above PIVOT_GROWTH of their rows, scaled product finite
+    const sf sumlx = tf_neg(FT_E > 1 ? tf_add(first_of(sums), second_of(sums)) : first_of(sums));
+    const sf lFs = tf_norm(tf_addf_n(lF, -(float)FT_LOOPS * sh));   // log psi_tr in the frame
+    const sf lGs = tf_norm(tf_addf_n(lG, -sh));                     // log V_tr = log(xi_tr / psi_tr)
+    angles th;
+    cx<float> pj;
+    int pe = 0;
     {
+        hessian H;
+        derivatives(lxs, pp, th, H, bad);
+        // det(I + i kappa X^1/2 H X^1/2) (similar to I + i kappa H X, srcs/feynman_integral.hpp:312-320):
+        // the real part is the identity, so the symmetric elimination needs no pivoting (every
+        // pivot's real part is at least 1); FP32, the pivots' product rescaled by powers of two
+        // (det J = pj 2^pe).  Before the complex block, so that H is no longer live there.
+        const float kappa = pf[P_DEF];
         cx<float> J[FT_E][FT_E];
-        float sx[FT_E];
-#pragma unroll
-        for (int e = 0; e < FT_E; e++) sx[e] = sqrtf(X[e]);
 #pragma unroll
         for (int a = 0; a < FT_E; a++)
 #pragma unroll
-            for (int b = a; b < FT_E; b++) J[a][b] = cmk(a == b ? 1.0f : 0.0f, kappa * H[a][b] * sx[a] * sx[b]);
+            for (int b = a; b < FT_E; b++) J[a][b] = cmk(a == b ? 1.0f : 0.0f, kappa * H.get(lxs, a, b));
+        bool ok = true;
 #pragma unroll
         for (int k = 0; k < FT_E; k++) {
             const cx<float> piv = J[k][k];
@@ -1911,18 +2164,15 @@ static __device__ __forceinline__ bool integrand32(const float* pd, const float*
             float row = m;
 #pragma unroll
             for (int j = k + 1; j < FT_E; j++) row += fabsf(J[k][j].re) + fabsf(J[k][j].im);
-            jok &= m > PIVOT_GROWTH * row;
-            pj = pj * piv;
-            {
-                const float mx = fmaxf(fabsf(pj.re), fabsf(pj.im));
-                const int be = (__float_as_int(mx) >> 23) & 0xff;
-                jok &= be > 0 && be < 255;
-                const int kk = (be > 0 && be < 255) ? be - 127 : 0;
-                const float sc = __int_as_float((127 - kk) << 23);
+            const float n2 = fmaf(piv.re, piv.re, piv.im * piv.im);
+            ok &= m > PIVOT_GROWTH * row && n2 < 1e36f;
+            pj = k == 0 ? piv : pj * piv;
+            if ((k & 1) || k == FT_E - 1) {   // |piv| < 1e18: two of them stay in range
+                const float sc = exp_scale(pj.re, pj.im, pe, ok);
                 pj = cmk(pj.re * sc, pj.im * sc);
-                pj_e += kk;
             }
-            const cx<float> inv = crecip(piv);
+            const float id = rcp_newton(n2);
+            const cx<float> inv = cmk(piv.re * id, -piv.im * id);
 #pragma unroll
             for (int i = k + 1; i < FT_E; i++) {
                 const cx<float> f = J[k][i] * inv;
@@ -1930,94 +2180,66 @@ static __device__ __forceinline__ bool integrand32(const float* pd, const float*
                 for (int j = i; j < FT_E; j++) J[i][j] = J[i][j] - f * J[k][j];
             }
         }
-    }
-    if (!jok) {
-        need64 = true;
-        return false;
+        bad |= !ok;
     }
     // phase sums in two-float: sum theta and nu . theta
-    f2 xnu = f2_make(0.0f, 0.0f), thsum = f2_make(0.0f, 0.0f);
+    sf xnu = tf_zero<float>(), thsum = xnu;
 #pragma unroll
     for (int e = 0; e < FT_E; e++) {
-        FT_DBG(e, theta[e].hi + theta[e].lo);
-        thsum = f2_add2(thsum, f2_make(theta[e].hi, theta[e].lo));
-        xnu = f2_add2(xnu, f2_mulf(f2_make(theta[e].hi, theta[e].lo), pf[P_NU + e]));
+        const sf t = th.get(lxs, e), tn = tf_mulf(t, pp[P_NU + e].x);
+        thsum = e == 0 ? t : tf_add_n(thsum, t);
+        xnu = e == 0 ? tn : tf_add_n(xnu, tn);
+        bad |= !(fabsf(t.hi) < THETA_MAX);
     }
+    thsum = tf_norm(thsum);
+    xnu = tf_norm(xnu);
+    if (bad) return false;
     cblock cb;
-    complex_block(theta, Xi2, pd, cb);
+    complex_block(lxs, th, pp, cb);
     // two-float pivots lose ~1e-14 / growth
-    if (!cb.ok || !cb.growth_ok) {
-        need64 = true;
-        return false;
-    }
-    // V = Vn 2^v_e, |Vn| in [1, 2 sqrt 2)
+    if (!cb.ok) return false;
+    // V = Vn 2^ve, |Vn| in [1, 2 sqrt 2)
     cdf Vn = cb.V;
-    int v_e = 0;
-    if (!cdf_renorm(Vn, v_e) || v_e > 126) {
-        need64 = true;
-        return false;
-    }
-    const float vsc = __int_as_float((127 - v_e) << 23);   // 2^-v_e
+    int ve = 0;
+    bool ok = true;
+    cdf_renorm(Vn, ve, ok);
+    if (!ok || ve > 126) return false;
+    const float vsc = __int_as_float((127 - ve) << 23);   // 2^-ve
     const float vn2 = fmaf(Vn.re.hi, Vn.re.hi, Vn.im.hi * Vn.im.hi);
     const float vm = sqrtf(vn2);
-    FT_DBG(20, Vn.re.hi);
-    FT_DBG(21, Vn.im.hi);
-    FT_DBG(34, W * cb.qmag * vsc / vm);
     // V in two-float keeps ~1e-14 of its terms' magnitudes (and ~1e-12 from the sector
     // point and contour it is built from): samples where V cancels to below 1e-6 of its
     // terms, or where W qmag / |V| exceeds 1e5, go to the FP64 pass
-    if (!(vm > ACC_V_CANCEL * (cb.mag * vsc)) || !(W * (cb.qmag * vsc) < ACC_V_AMPLIFY * vm)) {
-        need64 = true;
-        return false;
-    }
-    bool edge = false;
-    const f2 av2 = arg_f2(Vn.re.hi, Vn.im.hi, Vn.re.lo, Vn.im.lo);
-    const float av = av2.hi + av2.lo;
-    edge |= fabsf(av) > 3.14158265f;
-    FT_DBG(32, av);
-    FT_DBG(33, xnu.hi + xnu.lo);
+    if (!(vm > ACC_V_CANCEL * (cb.mag * vsc)) || !(W * (cb.qmag * vsc) < ACC_V_AMPLIFY * vm)) return false;
+    // an argument within 1e-5 of the branch cut: the FP64 pass decides the branch
+    const sf av2 = arg_of(Vn);
+    const float av = tf_f(av2);
     // arg cPsi = sum theta + arg det L(y), reduced to the principal branch in two-float
     const float dn2 = fmaf(cb.det.re.hi, cb.det.re.hi, cb.det.im.hi * cb.det.im.hi);
-    const f2 apsi2 = wrap_pi2(f2_add2(thsum, arg_f2(cb.det.re.hi, cb.det.im.hi, cb.det.re.lo, cb.det.im.lo)), edge);
-    const float apsi = apsi2.hi + apsi2.lo;
-    FT_DBG(26, apsi);
-    if (edge) {
-        need64 = true;
-        return false;
-    }
+    const sf apsi2 = wrap_pi(tf_add(thsum, arg_of(cb.det)));
+    const float apsi = tf_f(apsi2);
+    if (fabsf(av) > 3.14158265f || fabsf(apsi) > 3.14158265f) return false;
     // log2 |cPsi| and log2 |V| (exponents exact, small parts in FP32), then
     // log2 |cR / IGtr| = -D/2 log2(|cPsi| / psi_tr) - W log2(|V| / V_tr) + log2 |det J|
-    const float l2dm = 0.5f * m_log2(dn2), l2vm = 0.5f * m_log2(vn2);
-    const f2 l2psi_abs = f2_add(f2_add(f2_mul2(sumlx, f2_make(RLN2_HI, RLN2_LO)), (float)cb.det_e), l2dm);
-    const f2 lpsi = f2_add2(l2psi_abs, f2_neg(f2_mul2(lFs, f2_make(RLN2_HI, RLN2_LO))));
-    const f2 l2v_abs = f2_add(f2_make((float)v_e, 0.0f), l2vm);
-    const f2 lv = f2_add2(l2v_abs, f2_neg(f2_mul2(lGs, f2_make(RLN2_HI, RLN2_LO))));
-    f2 t = f2_add2(f2_mulf(lpsi, -D2), f2_mulf(lv, -W));
-    t = f2_add(t, (float)pj_e);
-    t = f2_add(t, 0.5f * m_log2(fmaf(pj.re, pj.re, pj.im * pj.im)));
+    const sf l2psi = tf_norm(tf_addf_n(tf_addf_n(tf_log2e(sumlx), (float)cb.e), 0.5f * m_log2(dn2)));
+    const sf l2v = fast_two_sum((float)ve, 0.5f * m_log2(vn2));
+    const sf lpsi = tf_sub(l2psi, tf_log2e(lFs));
+    const sf lv = tf_sub(l2v, tf_log2e(lGs));
+    sf t = tf_add_n(tf_mulf(lpsi, -D2), tf_mulf(lv, -W));
+    t = tf_norm(tf_addf_n(tf_addf_n(t, (float)pe), 0.5f * m_log2(fmaf(pj.re, pj.re, pj.im * pj.im))));
     // arg cR = -D/2 arg cPsi + arg det J + nu . theta - W arg V (two-float sum)
-    f2 angf = f2_add2(f2_mulf(apsi2, -D2), xnu);
-    angf = f2_add2(angf, arg_f2(pj.re, pj.im, 0.0f, 0.0f));
-    angf = f2_add2(angf, f2_mulf(av2, -W));
-    const float ang = angf.hi;
-    const float mod = m_exp2(t.hi) * (1.0f + t.lo * LN2_F);
+    const sf aj = arg_f2(pj.re, pj.im, 0.0f, 0.0f);
+    const sf ang = tf_norm(tf_add_n(tf_add_n(tf_mulf(apsi2, -D2), xnu), tf_add_n(aj, tf_mulf(av2, -W))));
     float sn, cs;
-    m_sincos(ang, &sn, &cs);
-    {
-        const float c2 = fmaf(-angf.lo, sn, cs), s2 = fmaf(angf.lo, cs, sn);
-        cs = c2;
-        sn = s2;
-    }
-    if (!isfinite(mod)) {
-        need64 = true;
-        return false;
-    }
-    cx<float> c = cmk(IGtr * mod * cs, IGtr * mod * sn);
+    m_sincos(ang.hi, &sn, &cs);
+    const float c2 = fmaf(-ang.lo, sn, cs), s2 = fmaf(ang.lo, cs, sn);
+    const float mod = m_exp2(t.hi) * (1.0f + t.lo * LN2_F);
+    if (!isfinite(mod)) return false;
+    cx<float> c = cmk(IGtr * mod * c2, IGtr * mod * s2);
     out[0] = c;
     if (FT_K > 1) {
         // log cPsi - L log V (srcs/feynman_integral.hpp:336-341): the large parts in two-float
-        const f2 dl = f2_add2(l2psi_abs, f2_mulf(l2v_abs, -(float)FT_LOOPS));
-        const float er = LN2_F * (dl.hi + dl.lo);
+        const float er = LN2_F * tf_f(tf_add(l2psi, tf_mulf(l2v, -(float)FT_LOOPS)));
         const float ei = apsi - (float)FT_LOOPS * av;
 #pragma unroll
         for (int j = 1; j < FT_K; j++) {
@@ -2026,23 +2248,11 @@ static __device__ __forceinline__ bool integrand32(const float* pd, const float*
         }
     }
     return true;
-#endif
 }
 #endif
+#endif
 
-#ifndef FT_HOST_SIM
 // ------------------------------------------------------------------ accumulation
-// Neumaier-compensated running sums per thread
-struct nsum {
-    double s, c;
-    __device__ __forceinline__ void add(double v)
-    {
-        double t = s + v;
-        c += (fabs(s) >= fabs(v)) ? ((s - t) + v) : ((v - t) + s);
-        s = t;
-    }
-};
-
 // double-double sum of two (hi, lo) pairs
 static __device__ __forceinline__ void dd_add(double& ah, double& al, double bh, double bl)
 {
@@ -2052,53 +2262,6 @@ static __device__ __forceinline__ void dd_add(double& ah, double& al, double bh,
     err += al + bl;
     ah = s + err;
     al = err - (ah - s);
-}
-
-// Block reduction of per-thread (hi, lo) accumulators into o[0 .. ACC_SLOTS)
-static __device__ __noinline__ void block_reduce(double* vals /* ACC_SLOTS per thread, (hi,lo) pairs for the first 8K */,
-                                                 double* o)
-{
-    // runs once per thread at the end: kept as loops (small code), not unrolled
-    __shared__ double red[FT_BLOCK / 32][ACC_SLOTS];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll 1
-    for (int s = 0; s < 8 * FT_K; s += 2) {
-        double h = vals[s], l = vals[s + 1];
-#pragma unroll 1
-        for (int off = 16; off; off >>= 1) {
-            double oh = __shfl_down_sync(0xffffffffu, h, off), ol = __shfl_down_sync(0xffffffffu, l, off);
-            dd_add(h, l, oh, ol);
-        }
-        if (lane == 0) {
-            red[wid][s] = h;
-            red[wid][s + 1] = l;
-        }
-    }
-#pragma unroll 1
-    for (int s = 8 * FT_K; s < ACC_SLOTS; s++) {
-        double v = vals[s];
-#pragma unroll 1
-        for (int off = 16; off; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-        if (lane == 0) red[wid][s] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll 1
-        for (int s = 0; s < 8 * FT_K; s += 2) {
-            double h = red[0][s], l = red[0][s + 1];
-#pragma unroll 1
-            for (int w = 1; w < FT_BLOCK / 32; w++) dd_add(h, l, red[w][s], red[w][s + 1]);
-            o[s] = h;
-            o[s + 1] = l;
-        }
-#pragma unroll 1
-        for (int s = 8 * FT_K; s < ACC_SLOTS; s++) {
-            double v = 0.0;
-#pragma unroll 1
-            for (int w = 0; w < FT_BLOCK / 32; w++) v += red[w][s];
-            o[s] = v;
-        }
-    }
 }
 
 // stream state from 4 words (16-byte aligned)
@@ -2144,14 +2307,12 @@ static __device__ __forceinline__ void skip_lanes(xo& g, u32 lane, const u64* __
 }
 
 // ------------------------------------------------------------------ table staging
-// FP64 form: shared = [w64 | Jr64 | 1/r64 | meta] (25 bytes per entry, the global
-// layout's first sections).  Mixed form: shared = [w32 | Jr32 | 1/r32 | meta].
+// FP64 form: shared = [1/r64 | meta | thresholds].  Mixed form: shared = [1/r32 hi |
+// 1/r32 lo | meta | thresholds].
 #if FT_TABLE_GLOBAL
 #define SM_USED 0u
-#elif FT_PREC == 0
-#define SM_USED (25u * T_ENTRIES)
 #else
-#define SM_USED (17u * T_ENTRIES)
+#define SM_USED (12u * T_ENTRIES + T_QBYTES)
 #endif
 static __device__ __forceinline__ void copy_bytes(unsigned char* dst, const unsigned char* __restrict__ src, u32 bytes)
 {
@@ -2160,36 +2321,43 @@ static __device__ __forceinline__ void copy_bytes(unsigned char* dst, const unsi
     for (u32 i = n16 * 16u + threadIdx.x; i < bytes; i += blockDim.x) dst[i] = src[i];
 }
 
-// the table's sections: in global memory (large tables, L2 / L1 cached) or the staged
-// copy in shared memory
-static __device__ __forceinline__ table_ref table_at(unsigned char* sm, const unsigned char* __restrict__ tab)
+// the table's sections: in global memory (large tables, L2 / L1 cached)
+static __device__ __forceinline__ table_ref global_table(const unsigned char* __restrict__ tab)
 {
     table_ref t;
     t.gm = tab;
+#if FT_CUT
+    t.q = tab + T_Q;
+    t.Jr = nullptr;
+#elif FT_PREC == 0
+    t.q = tab + T_W64;
+    t.Jr = tab + T_JR64;
+#else
+    t.q = tab + T_W32;
+    t.Jr = tab + T_JR32;
+#endif
+    t.ri = tab + (FT_PREC == 0 ? T_RI64 : T_RH32);
+    t.rl = (const float*)(tab + T_RL32);
+    t.meta = (const u32*)(tab + T_META);
+    return t;
+}
+
+// the same in global memory or the staged copy in shared memory
+static __device__ __forceinline__ table_ref table_at(unsigned char* sm, const unsigned char* __restrict__ tab)
+{
 #if FT_TABLE_GLOBAL
     (void)sm;
-#if FT_PREC == 0
-    t.w = tab + T_W64;
-    t.Jr = tab + T_JR64;
-    t.ri = tab + T_RI64;
+    return global_table(tab);
 #else
-    t.w = tab + T_W32;
-    t.Jr = tab + T_JR32;
-    t.ri = tab + T_RI32;
-#endif
-    t.meta = tab + T_META;
-#elif FT_PREC == 0
-    t.w = sm + T_W64;
-    t.Jr = sm + T_JR64;
-    t.ri = sm + T_RI64;
-    t.meta = sm + T_META;
-#else
-    t.w = sm;
-    t.Jr = sm + 4u * T_ENTRIES;
-    t.ri = sm + 8u * T_ENTRIES;
-    t.meta = sm + 16u * T_ENTRIES;
-#endif
+    table_ref t;
+    t.gm = tab;
+    t.Jr = nullptr;
+    t.ri = sm;
+    t.rl = (const float*)(sm + 4u * T_ENTRIES);
+    t.meta = (const u32*)(sm + 8u * T_ENTRIES);
+    t.q = sm + 12u * T_ENTRIES;
     return t;
+#endif
 }
 
 // the block's copy of a staged table (no barrier)
@@ -2198,11 +2366,13 @@ static __device__ __forceinline__ void copy_table(unsigned char* sm, const unsig
 #if FT_TABLE_GLOBAL
     (void)sm;
     (void)tab;
-#elif FT_PREC == 0
-    copy_bytes(sm, tab, 25u * T_ENTRIES);
 #else
-    copy_bytes(sm, tab + T_F32, 16u * T_ENTRIES);
-    copy_bytes(sm + 16u * T_ENTRIES, tab + T_META, T_ENTRIES);
+#if FT_PREC == 0
+    copy_bytes(sm, tab + T_RI64, 8u * T_ENTRIES);
+    copy_bytes(sm + 8u * T_ENTRIES, tab + T_META, 4u * T_ENTRIES + T_QBYTES);   // adjacent
+#else
+    copy_bytes(sm, tab + T_RH32, 12u * T_ENTRIES + T_QBYTES);
+#endif
 #endif
 }
 
@@ -2215,15 +2385,18 @@ static __device__ __forceinline__ table_ref stage_table(unsigned char* sm, const
     return table_at(sm, tab);
 }
 
-// ------------------------------------------------------------------ per-thread accumulators
+// ------------------------------------------------------------------ accumulators
 // Per-thread sums live in shared memory (slot-major, so a warp touches consecutive
 // words), which keeps them out of the register budget of the sampling code:
 //   FP64 form: Neumaier-compensated FP64 sums per sample.
-//   mixed form: Kahan-compensated FP32 sums per sample, folded into the FP64
-//   Neumaier sums every 256 kept samples; the sample counters too (FP32 counts since
-//   the last fold, FP64 totals), so that no accumulator state is held in registers
-//   across the per-sample code.
+//   mixed form: Kahan-compensated FP32 sums per sample, folded every FT_FOLD samples
+//   (and at the end) into one double-double sum per warp.  A Kahan sum's error does not
+//   grow with the number of terms, so the fold only has to be rare enough to cost
+//   nothing; one FP64 sum per warp instead of two FP64 words per thread leaves the
+//   shared memory to the cut thresholds (the cube's block: 40 KB of sums instead of 123).
 // Slots: 4 per eps order (re f, re f^2, im f, im f^2).
+// Dropped, queued, exact and robust samples are rare and counted per block; kept is what
+// remains of the samples the block owns.
 #if FT_MODE == 0
 #define ACC_PARTS 2   // undeformed integrand: real parts only
 #else
@@ -2231,39 +2404,83 @@ static __device__ __forceinline__ table_ref stage_table(unsigned char* sm, const
 #endif
 #define ACC_NS (ACC_PARTS * FT_K)
 #define ACC_SMEM_OFFSET ((SM_USED + 15u) & ~15u)
-// mixed form, counters: kept, dropped, queued, exact
-#define ACC_NC 4
+#define FT_WARPS (FT_BLOCK / 32)
+#define FT_FOLD 1024
+#if FT_PREC == 1
+// after the sums: the threads' log X (draw_pair), two floats per edge and sample
+#define LX_SMEM_OFFSET ((ACC_SMEM_OFFSET + 16u * ACC_NS * FT_WARPS + 8u * ACC_NS * FT_BLOCK + 15u) & ~15u)
+#else
+#define LX_SMEM_OFFSET 0u
+#endif
+
+enum { CNT_OWNED, CNT_DROPPED, CNT_QUEUED, CNT_EXACT, CNT_ROBUST, CNT_N };
+__shared__ u64 s_count[CNT_N];
+
+// slot s = (order j, part q) -> output pair 4 j + q
+static __device__ __forceinline__ int out_pair(int s) { return 4 * (s / ACC_PARTS) + (s % ACC_PARTS); }
+
+// the block's counters and the output slots no sum is kept for (the first threads)
+static __device__ __forceinline__ void write_counts(double* dst)
+{
+    for (int s = threadIdx.x; s < ACC_SLOTS; s += FT_BLOCK) {
+        if (s < 8 * FT_K) {
+            if (ACC_PARTS == 2 && (s & 4)) dst[s] = 0.0;
+            continue;
+        }
+        double v = 0.0;
+        if (s == ACC_KEPT) v = (double)(s_count[CNT_OWNED] - s_count[CNT_DROPPED] - s_count[CNT_QUEUED]);
+        if (s == ACC_DROPPED) v = (double)s_count[CNT_DROPPED];
+        if (s == ACC_QUEUED) v = (double)s_count[CNT_QUEUED];
+        if (s == ACC_EXACT) v = (double)s_count[CNT_EXACT];
+        if (s == ACC_ROBUST) v = (double)s_count[CNT_ROBUST];
+        dst[s] = v;
+    }
+}
+
+static __device__ __forceinline__ void warp_dd_sum(double& h, double& l)
+{
+#pragma unroll 1
+    for (int off = 16; off; off >>= 1) {
+        const double oh = __shfl_down_sync(0xffffffffu, h, off), ol = __shfl_down_sync(0xffffffffu, l, off);
+        dd_add(h, l, oh, ol);
+    }
+}
+
+struct accum {
+    unsigned char* base;
+
+    __device__ __forceinline__ void count(int c, u32 n)
+    {
+        if (n) atomicAdd(&s_count[c], (u64)n);
+    }
 
 #if FT_PREC == 0
-struct accum {
-    double* S;   // [slot][thread] sums
-    double* C;   // [slot][thread] Neumaier compensations
-    double kept, dropped, queued, exact, robust;
+    __device__ __forceinline__ double& S(int s) { return ((double*)base)[s * FT_BLOCK + threadIdx.x]; }
+    __device__ __forceinline__ double& C(int s) { return ((double*)base)[(ACC_NS + s) * FT_BLOCK + threadIdx.x]; }
 
+    // block-wide (ends with a barrier)
     __device__ __forceinline__ void init(unsigned char* smem_acc)
     {
-        const int t = threadIdx.x;
-        S = (double*)smem_acc + t;
-        C = S + ACC_NS * FT_BLOCK;
+        base = smem_acc;
 #pragma unroll
         for (int s = 0; s < ACC_NS; s++) {
-            S[s * FT_BLOCK] = 0.0;
-            C[s * FT_BLOCK] = 0.0;
+            S(s) = 0.0;
+            C(s) = 0.0;
         }
-        kept = dropped = queued = exact = robust = 0.0;
+        if (threadIdx.x < CNT_N) s_count[threadIdx.x] = 0;
+        __syncthreads();
     }
 
     __device__ __forceinline__ void nadd(int slot, double v)
     {
-        const double s = S[slot * FT_BLOCK];
+        const double s = S(slot);
         const double t = s + v;
-        C[slot * FT_BLOCK] += (fabs(s) >= fabs(v)) ? ((s - t) + v) : ((v - t) + s);
-        S[slot * FT_BLOCK] = t;
+        C(slot) += (fabs(s) >= fabs(v)) ? ((s - t) + v) : ((v - t) + s);
+        S(slot) = t;
     }
 
     __device__ __forceinline__ void add64(const cx<double>* R)
     {
-        kept += 1;
 #pragma unroll
         for (int j = 0; j < FT_K; j++) {
             if (FT_ONLY_PSI && j > 0) break;
@@ -2276,71 +2493,57 @@ struct accum {
         }
     }
 
-    // block-wide: every thread of the block calls it; the block's sums go to dst[0 .. ACC_SLOTS)
-    __device__ __forceinline__ void finish(double* dst)
+    // block-wide: every thread of the block calls it with the samples it owned; the
+    // block's sums go to dst[0 .. ACC_SLOTS).  A warp takes whole slots: its lanes add
+    // the threads' sums in turn, then a tree over the lanes (a tree over every warp's
+    // own threads took three times the FP64 additions).
+    __device__ __forceinline__ void finish(double* dst, u64 owned)
     {
-        double vals[ACC_SLOTS];
-#pragma unroll
-        for (int s = 0; s < 8 * FT_K; s++) vals[s] = 0.0;
-#pragma unroll
-        for (int s = 0; s < ACC_NS; s++) {
-            const double sv = S[s * FT_BLOCK], cv = C[s * FT_BLOCK];
-            const double h = sv + cv;
-            // slot s = (order j, part q) -> output pair 4 j + q
-            const int o = 4 * (s / ACC_PARTS) + (s % ACC_PARTS);
-            vals[2 * o] = h;
-            vals[2 * o + 1] = cv - (h - sv);
+        if (owned) atomicAdd(&s_count[CNT_OWNED], owned);
+        __syncthreads();
+        const int lane = threadIdx.x & 31;
+#pragma unroll 1
+        for (int s = threadIdx.x >> 5; s < ACC_NS; s += FT_WARPS) {
+            double h = 0.0, l = 0.0;
+#pragma unroll 1
+            for (int t = lane; t < FT_BLOCK; t += 32) {
+                const double sv = ((const double*)base)[s * FT_BLOCK + t];
+                const double cv = ((const double*)base)[(ACC_NS + s) * FT_BLOCK + t];
+                dd_add(h, l, sv, cv);
+            }
+            warp_dd_sum(h, l);
+            if (lane == 0) {
+                dst[2 * out_pair(s)] = h;
+                dst[2 * out_pair(s) + 1] = l;
+            }
         }
-        vals[ACC_KEPT] = kept;
-        vals[ACC_DROPPED] = dropped;
-        vals[ACC_QUEUED] = queued;
-        vals[ACC_EXACT] = exact;
-        vals[ACC_ROBUST] = robust;
-#pragma unroll
-        for (int s = ACC_ROBUST + 1; s < ACC_SLOTS; s++) vals[s] = 0.0;
-        block_reduce(vals, dst);
+        write_counts(dst);
     }
-};
 #else
-// Shared-memory layout from ACC_SMEM_OFFSET, [slot][thread]: S, C (ACC_NS doubles
-// each), N (ACC_NC doubles), then Sf, Cf (ACC_NS floats each), Nf (ACC_NC floats).
-// Every address is the block's fixed offset plus the thread index, so the struct holds
-// nothing but the base.
-#define ACC_D(k) (((double*)base)[(k) * FT_BLOCK + threadIdx.x])
-#define ACC_F(k) (((float*)((double*)base + (2 * ACC_NS + ACC_NC) * FT_BLOCK))[(k) * FT_BLOCK + threadIdx.x])
-struct accum {
-    unsigned char* base;
+    // from base: the warps' double-double sums [slot][warp] (hi, lo), then Sf, Cf
+    // [slot][thread]
+    __device__ __forceinline__ double2& W(int s, int w) { return ((double2*)base)[s * FT_WARPS + w]; }
+    __device__ __forceinline__ float& Sf(int s)
+    {
+        return ((float*)(base + 16 * ACC_NS * FT_WARPS))[s * FT_BLOCK + threadIdx.x];
+    }
+    __device__ __forceinline__ float& Cf(int s)
+    {
+        return ((float*)(base + 16 * ACC_NS * FT_WARPS))[(ACC_NS + s) * FT_BLOCK + threadIdx.x];
+    }
 
-    __device__ __forceinline__ double& S(int s) { return ACC_D(s); }
-    __device__ __forceinline__ double& C(int s) { return ACC_D(ACC_NS + s); }
-    __device__ __forceinline__ double& N(int c) { return ACC_D(2 * ACC_NS + c); }
-    __device__ __forceinline__ float& Sf(int s) { return ACC_F(s); }
-    __device__ __forceinline__ float& Cf(int s) { return ACC_F(ACC_NS + s); }
-    __device__ __forceinline__ float& Nf(int c) { return ACC_F(2 * ACC_NS + c); }
-
+    // block-wide (ends with a barrier)
     __device__ __forceinline__ void init(unsigned char* smem_acc)
     {
         base = smem_acc;
 #pragma unroll
         for (int s = 0; s < ACC_NS; s++) {
-            S(s) = 0.0;
-            C(s) = 0.0;
             Sf(s) = 0.0f;
             Cf(s) = 0.0f;
+            if ((threadIdx.x & 31) == 0) W(s, threadIdx.x >> 5) = make_double2(0.0, 0.0);
         }
-#pragma unroll
-        for (int c = 0; c < ACC_NC; c++) {
-            N(c) = 0.0;
-            Nf(c) = 0.0f;
-        }
-    }
-
-    __device__ __forceinline__ void nadd(int slot, double v)
-    {
-        const double s = S(slot);
-        const double t = s + v;
-        C(slot) += (fabs(s) >= fabs(v)) ? ((s - t) + v) : ((v - t) + s);
-        S(slot) = t;
+        if (threadIdx.x < CNT_N) s_count[threadIdx.x] = 0;
+        __syncthreads();
     }
 
     __device__ __forceinline__ void add32(const cx<float>* R)
@@ -2360,61 +2563,46 @@ struct accum {
                 Sf(o) = tt;
             }
         }
-        const float k = Nf(0) + 1.0f;
-        Nf(0) = k;
-        if (k == 256.0f) fold();
     }
-    // every sample: dropped d, queued q (constants 0 or 1 at the call sites), exact steps e
-    __device__ __forceinline__ void note32(float d, float q, float e)
+
+    // warp-wide
+    __device__ __noinline__ void fold()
     {
-        if (d != 0.0f) Nf(1) += d;
-        if (q != 0.0f) Nf(2) += q;
-        if (e != 0.0f) Nf(3) += e;
-    }
-    __device__ __forceinline__ void fold()
-    {
-#pragma unroll
+#pragma unroll 1
         for (int s = 0; s < ACC_NS; s++) {
-            nadd(s, (double)Sf(s) - (double)Cf(s));
+            double h = (double)Sf(s) - (double)Cf(s), l = 0.0;
             Sf(s) = 0.0f;
             Cf(s) = 0.0f;
-        }
-#pragma unroll
-        for (int c = 0; c < ACC_NC; c++) {
-            N(c) += (double)Nf(c);
-            Nf(c) = 0.0f;
+            warp_dd_sum(h, l);
+            if ((threadIdx.x & 31) == 0) {
+                double2 w = W(s, threadIdx.x >> 5);
+                dd_add(w.x, w.y, h, l);
+                W(s, threadIdx.x >> 5) = w;
+            }
         }
     }
 
-    // block-wide: every thread of the block calls it; the block's sums go to dst[0 .. ACC_SLOTS)
-    __device__ __forceinline__ void finish(double* dst)
+    // block-wide: every thread of the block calls it with the samples it owned; the
+    // block's sums go to dst[0 .. ACC_SLOTS)
+    __device__ __forceinline__ void finish(double* dst, u64 owned)
     {
+        if (owned) atomicAdd(&s_count[CNT_OWNED], owned);
         fold();
-        double vals[ACC_SLOTS];
-#pragma unroll
-        for (int s = 0; s < 8 * FT_K; s++) vals[s] = 0.0;
-#pragma unroll
-        for (int s = 0; s < ACC_NS; s++) {
-            const double sv = S(s), cv = C(s);
-            const double h = sv + cv;
-            // slot s = (order j, part q) -> output pair 4 j + q
-            const int o = 4 * (s / ACC_PARTS) + (s % ACC_PARTS);
-            vals[2 * o] = h;
-            vals[2 * o + 1] = cv - (h - sv);
+        __syncthreads();
+        for (int s = threadIdx.x; s < ACC_NS; s += FT_BLOCK) {
+            double2 w = W(s, 0);
+#pragma unroll 1
+            for (int k = 1; k < FT_WARPS; k++) {
+                const double2 v = W(s, k);
+                dd_add(w.x, w.y, v.x, v.y);
+            }
+            dst[2 * out_pair(s)] = w.x;
+            dst[2 * out_pair(s) + 1] = w.y;
         }
-        vals[ACC_KEPT] = N(0);
-        vals[ACC_DROPPED] = N(1);
-        vals[ACC_QUEUED] = N(2);
-        vals[ACC_EXACT] = N(3);
-        vals[ACC_ROBUST] = 0.0;
-#pragma unroll
-        for (int s = ACC_ROBUST + 1; s < ACC_SLOTS; s++) vals[s] = 0.0;
-        block_reduce(vals, dst);
+        write_counts(dst);
     }
-};
-#undef ACC_D
-#undef ACC_F
 #endif
+};
 
 template <class T>
 static __device__ __forceinline__ void write_record(u64 i, const unsigned char* ord, const cx<T>* R, bool ok,
@@ -2441,17 +2629,17 @@ static __device__ __forceinline__ void sample64(xo& g, const table_ref& tr, cons
     for (int j = 0; j < FT_K; j++) R[j] = cmk(0.0, 0.0);
     double X[FT_E];
     double F, Gv;
-    draw_sector64(g, tr, prm[P_JRFULL], X, F, Gv, ord);
+    draw_sector64(g, tr, FT_EXACT_TABLE(tr), prm[P_JRFULL], X, F, Gv, ord);
     if (FT_RECORD)
         for (int e = 0; e < FT_E; e++) rec_X[i * FT_E + e] = X[e];
     bool rob = false;
     const bool ok = integrand64(prm, X, F, Gv * F, R, rob);
     if (rob) {
-        A.robust += 1;
+        A.count(CNT_ROBUST, 1);
         flags |= REC_ROBUST;
     }
     if (!ok) {
-        A.dropped += 1;
+        A.count(CNT_DROPPED, 1);
         flags |= REC_DROPPED;
     } else {
         A.add64(R);
@@ -2466,73 +2654,112 @@ static __device__ __forceinline__ void sample64(xo& g, const table_ref& tr, cons
 // pass and left out of the sums here: 5 words, the sample (its index in the
 // single-integral kernels; item << BQ_ITEM_SHIFT | lane << BQ_LANE_SHIFT | (i - first)
 // naming the block's work item in the batch kernels) and its stream state.
-static __device__ __forceinline__ void sample_range(xo& g, const table_ref& tr, const double* __restrict__ prm,
-                                                    u64 first, u64 last, u64 chunk, accum& A, u64* __restrict__ queue,
-                                                    unsigned int* __restrict__ qcount, unsigned int qcap,
-                                                    unsigned char* __restrict__ rec_order, double* __restrict__ rec_X,
-                                                    double* __restrict__ rec_R, unsigned char* __restrict__ rec_flags)
-{
+// Every thread of the block makes `chunk` trips (two samples a trip in the
+// undeformed mixed form).  With the barrier (FT_VARIANT bit 2) the block starts each trip together: the
+// warps then run the same stretch of the (long, straight-line) per-sample code at the
+// same time and share its instruction fetches.
 #if FT_PREC == 1
-    const float* pf = (const float*)(prm + P_SIZE);
-    const float* pd = (const float*)(prm + P_SIZE + (P_SIZE + 1) / 2);   // two-float pairs
+static __device__ __noinline__ void queue_sample(xo g, u64 i, u64 offset, u64* __restrict__ queue,
+                                                 unsigned int* __restrict__ qcount, unsigned int qcap, int back)
+{
+    const unsigned int slot = atomicAdd(qcount, 1u);
+    if (slot >= qcap) return;
+    rewind(g, back);   // to the sample's first draw
+    u64* q = queue + (size_t)slot * 5;
+#if FT_BATCH
+    q[0] = (s_batch_item << BQ_ITEM_SHIFT) | ((u64)threadIdx.x << BQ_LANE_SHIFT) | offset;
+#else
+    q[0] = i;
 #endif
-    (void)chunk;
-#if FT_VARIANT & 4
-    // Every thread of the block makes `chunk` trips and the block starts each sample
-    // together: the warps then run the same stretch of the (long, straight-line)
-    // per-sample code at the same time and share its instruction fetches.
+    q[1] = g.a;
+    q[2] = g.b;
+    q[3] = g.c;
+    q[4] = g.d;
+}
+#endif
+
+static __device__ __forceinline__ void sample_range(xo& g, const table_ref& tr, const double* __restrict__ prm,
+                                                    u64 first, u64 last, u64 chunk, accum& A, unsigned char* lxs,
+                                                    u64* __restrict__ queue, unsigned int* __restrict__ qcount,
+                                                    unsigned int qcap, unsigned char* __restrict__ rec_order,
+                                                    double* __restrict__ rec_X, double* __restrict__ rec_R,
+                                                    unsigned char* __restrict__ rec_flags)
+{
+#if FT_PREC == 0
+    (void)lxs;
     for (u64 k = 0; k < chunk; k++) {
+#if FT_VARIANT & 4
         __syncthreads();
+#endif
         const u64 i = first + k;
         if (i >= last) continue;
-#else
-    for (u64 i = first; i < last; i++) {
-#endif
-#if FT_PREC == 0
         sample64(g, tr, prm, i, A, 0, rec_order, rec_X, rec_R, rec_flags);
-#else
-        unsigned char ord[FT_E];
-        unsigned char flags = 0;
-        cx<float> R[FT_K];
-#pragma unroll
-        for (int j = 0; j < FT_K; j++) R[j] = cmk(0.0f, 0.0f);
-        const xo g0 = g;
-        f2 lx[FT_E], lF, lG;
-        const int ex = draw_sector32(g, tr, pf, lx, lF, lG, ord);
-        if (ex) flags |= REC_EXACT;
-        if (FT_RECORD)
-            for (int e = 0; e < FT_E; e++) rec_X[i * FT_E + e] = exp((double)lx[e].hi + (double)lx[e].lo);
-        bool need64 = false;
-        const bool ok = integrand32(pd, pf, lx, lF, lG, R, need64);
-        if (need64) {
-            flags |= REC_QUEUED;
-            A.note32(0.0f, 1.0f, (float)ex);
-            const unsigned int slot = atomicAdd(qcount, 1u);
-            if (slot < qcap) {
-                u64* q = queue + (size_t)slot * 5;
-#if FT_BATCH
-                q[0] = (s_batch_item << BQ_ITEM_SHIFT) | ((u64)threadIdx.x << BQ_LANE_SHIFT) | (i - first);
-#else
-                q[0] = i;
-#endif
-                q[1] = g0.a;
-                q[2] = g0.b;
-                q[3] = g0.c;
-                q[4] = g0.d;
-            }
-            if (FT_RECORD) write_record(i, ord, R, false, flags, rec_order, rec_R, rec_flags);
-            continue;
-        }
-        if (!ok) {
-            A.note32(1.0f, 0.0f, (float)ex);
-            flags |= REC_DROPPED;
-        } else {
-            A.note32(0.0f, 0.0f, (float)ex);
-            A.add32(R);
-        }
-        if (FT_RECORD) write_record(i, ord, R, ok, flags, rec_order, rec_R, rec_flags);
-#endif
     }
+#else
+    const float* pf = (const float*)(prm + P_SIZE);
+    const float4* pp = (const float4*)(prm + P_PAIR);
+    const int per = FT_MODE == 0 ? 2 : 1;   // samples of a trip
+    for (u64 k = 0; k < chunk; k += per) {
+#if FT_VARIANT & 4
+        __syncthreads();
+#endif
+        if ((k & (FT_FOLD - 1)) == FT_FOLD - per) A.fold();
+        const u64 i = first + k;
+        if (i >= last) continue;
+        unsigned char ord[2][FT_E];
+        cx<float> r[2][FT_K];
+        u32 ex[2] = {0, 0};
+        bool bad[2] = {true, true};
+#pragma unroll
+        for (int j = 0; j < FT_K; j++) r[0][j] = r[1][j] = cmk(0.0f, 0.0f);
+#if FT_MODE == 0
+        const int n = i + 1 < last ? 2 : 1;   // the second half of an odd last sample's pair is left out
+        df lF, lG;
+        fv R[FT_K];
+#pragma unroll
+        for (int j = 0; j < FT_K; j++) R[j] = fv_of(0.0f);
+        draw_pair(g, tr, lxs, lF, lG, ex[0], ex[1], ord[0], ord[1]);
+#else
+        const int n = 1;
+        sf lF, lG;
+        draw_one(g, tr, lxs, lF, lG, ex[0], ord[0]);
+#endif
+        if (FT_RECORD)
+            for (int e = 0; e < FT_E; e++) {
+#if FT_MODE == 0
+                rec_X[i * FT_E + e] = exp((double)LX(e, 0).x + (double)LX(e, 1).x);
+                if (n > 1) rec_X[(i + 1) * FT_E + e] = exp((double)LX(e, 0).y + (double)LX(e, 1).y);
+#else
+                rec_X[i * FT_E + e] = exp((double)LX(e, 0) + (double)LX(e, 1));
+#endif
+            }
+#if FT_MODE == 0
+        integrand_pair(pp, pf, lxs, lF, lG, R, bad[0], bad[1]);
+#pragma unroll
+        for (int j = 0; j < FT_K; j++) {
+            r[0][j].re = R[j].x;
+            r[1][j].re = R[j].y;
+        }
+#else
+        bad[0] = !integrand_one(pp, pf, lxs, lF, lG, r[0]);
+#endif
+#pragma unroll
+        for (int h = 0; h < per; h++) {
+            if (h >= n) break;
+            A.count(CNT_EXACT, ex[h]);
+            if (bad[h]) {
+                A.count(CNT_QUEUED, 1);
+                queue_sample(g, i + h, k + h, queue, qcount, qcap, (per - h) * (2 * FT_E - 1));
+            } else {
+                A.add32(r[h]);
+            }
+            if (FT_RECORD)
+                write_record(i + h, ord[h], r[h], !bad[h],
+                             (unsigned char)((bad[h] ? REC_QUEUED : 0) | (ex[h] ? REC_EXACT : 0)), rec_order, rec_R,
+                             rec_flags);
+        }
+    }
+#endif
 }
 
 #if !FT_BATCH
@@ -2561,8 +2788,8 @@ extern "C" __global__ void __launch_bounds__(FT_BLOCK, FT_MINB) ft_sample(
 
     accum A;
     A.init(smem + ACC_SMEM_OFFSET);
-    sample_range(g, tr, prm, first, last, chunk, A, queue, qcount, qcap, rec_order, rec_X, rec_R, rec_flags);
-    A.finish(acc_out + (size_t)blockIdx.x * ACC_SLOTS);
+    sample_range(g, tr, prm, first, last, chunk, A, smem + LX_SMEM_OFFSET, queue, qcount, qcap, rec_order, rec_X, rec_R, rec_flags);
+    A.finish(acc_out + (size_t)blockIdx.x * ACC_SLOTS, first < last ? last - first : 0);
 }
 
 #if FT_PREC == 0
@@ -2584,8 +2811,10 @@ extern "C" __global__ void __launch_bounds__(FT_BLOCK) ft_sample_queue(
     const table_ref tr = stage_table(smem, tab);
     accum A;
     A.init(smem + ACC_SMEM_OFFSET);
+    u64 owned = 0;
     for (unsigned int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const u64* q = queue + (size_t)k * 5;
+        owned++;
         xo g;
         g.a = q[1];
         g.b = q[2];
@@ -2593,7 +2822,7 @@ extern "C" __global__ void __launch_bounds__(FT_BLOCK) ft_sample_queue(
         g.d = q[4];
         sample64(g, tr, prm, q[0], A, REC_QUEUED, rec_order, rec_X, rec_R, rec_flags);
     }
-    A.finish(acc_out + (size_t)blockIdx.x * ACC_SLOTS);
+    A.finish(acc_out + (size_t)blockIdx.x * ACC_SLOTS, owned);
 }
 #endif
 
@@ -2632,8 +2861,8 @@ static __device__ __forceinline__ int find_instance(const batch_inst* __restrict
 }
 
 // parameter block of the current instance, staged beside its table (P_SIZE doubles,
-// the same as floats, then as two-float pairs)
-#define PRM_WORDS (P_SIZE + (P_SIZE + 1) / 2 + P_SIZE)
+// the same as floats, then the two-float quadruples)
+#define PRM_WORDS (P_PAIR + 2 * P_SIZE)
 
 extern "C" __global__ void __launch_bounds__(FT_BLOCK, FT_MINB) ft_sample_batch(
     const batch_inst* __restrict__ inst, int ninst, const u64* __restrict__ total_items,
@@ -2679,11 +2908,12 @@ extern "C" __global__ void __launch_bounds__(FT_BLOCK, FT_MINB) ft_sample_batch(
         skip_lanes(g, threadIdx.x, lanepw, lanebits);
         accum A;
         A.init(smem + ACC_SMEM_OFFSET);
-        sample_range(g, tr, s_prm, first, last, chunk, A, queue, qcount, qcap, nullptr, nullptr, nullptr, nullptr);
+        sample_range(g, tr, s_prm, first, last, chunk, A, smem + LX_SMEM_OFFSET, queue, qcount, qcap, nullptr, nullptr,
+                     nullptr, nullptr);
         // read before the reduction's barriers, after which the first thread may take
         // the next item
         double* dst = acc_out + s_batch_item * ACC_SLOTS;
-        A.finish(dst);
+        A.finish(dst, first < last ? last - first : 0);
     }
 }
 
@@ -2737,19 +2967,14 @@ extern "C" __global__ void __launch_bounds__(FT_BLOCK) ft_sample_queue_batch(
         const int id = find_instance(inst, ninst, item);
         const double* prm = inst[id].prm;
         const unsigned char* tab = inst[id].tab;
-        table_ref tr;
-        tr.w = tab + T_W64;
-        tr.Jr = tab + T_JR64;
-        tr.ri = tab + T_RI64;
-        tr.meta = tab + T_META;
-        tr.gm = tab;
+        const table_ref tr = global_table(tab);
         cx<double> R[FT_K];
 #pragma unroll
         for (int j = 0; j < FT_K; j++) R[j] = cmk(0.0, 0.0);
         double X[FT_E];
         double F, Gv;
         unsigned char ord[FT_E];
-        draw_sector64(g, tr, prm[P_JRFULL], X, F, Gv, ord);
+        draw_sector64(g, tr, FT_EXACT_TABLE(tr), prm[P_JRFULL], X, F, Gv, ord);
         bool rob = false;
         const bool ok = integrand64(prm, X, F, Gv * F, R, rob);
         u64* qa = qacc + (size_t)id * (4 * FT_K * FT_XA_DIGITS + 4);
@@ -2774,4 +2999,4 @@ extern "C" __global__ void __launch_bounds__(FT_BLOCK) ft_sample_queue_batch(
 }
 #endif
 #endif  // FT_BATCH
-#endif  // FT_HOST_SIM
+

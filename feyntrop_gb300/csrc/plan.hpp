@@ -43,7 +43,7 @@ struct device_state {
 device_state& dev_state();
 
 // the device parameter block of a plan: the FP64 values, then the same as floats,
-// then as two-float (hi, lo) pairs (the layout the kernel body reads)
+// then in two-float as (hi, hi, lo, lo) quadruples (the layout the kernel body reads)
 std::vector<double> param_block(const std::vector<double>& prm);
 
 // sums of one integration (8K+8 slots) into the caller's result
@@ -108,10 +108,10 @@ struct ft_plan {
         k.ek = kek;
         k.el = kel;
         k.q0 = q0;
-        // tables are staged per block in shared memory up to E = 12 (102 KB FP64, 70 KB
-        // mixed, beside one block's per-thread sums: the cube's mixed kernel ran 8 % faster
-        // than reading its table through L1); from E = 13 on they are read through L1
-        k.table_global = P.E >= 13 ? 1 : 0;
+        // tables are staged per block in shared memory up to E = 12 (147 KB, beside one
+        // block's sums: the cube's mixed kernel ran 8 % faster than reading its table through
+        // L1); from E = 13 on they are read through L1
+        k.table_global = ft::staged_table(P.E) ? 0 : 1;
         // launch shape: a shape being measured by the autotuner, else the tuning table's
         // (or the default) for this kernel class
         ft::apply_shape(k, (forced && forced_prec == prec) ? forced_shape : ft::choose_shape(k));

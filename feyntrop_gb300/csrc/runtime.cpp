@@ -91,14 +91,15 @@ device_state& dev_state()
 std::vector<double> param_block(const std::vector<double>& prm)
 {
     const size_t n = prm.size();
-    std::vector<double> blk(n + (n + 1) / 2 + n, 0.0);
+    const size_t pair = (n + (n + 1) / 2 + 1) & ~(size_t)1;   // 16-byte aligned
+    std::vector<double> blk(pair + 2 * n, 0.0);
     std::memcpy(blk.data(), prm.data(), n * 8);
     float* f = (float*)(blk.data() + n);
     for (size_t i = 0; i < n; i++) f[i] = (float)prm[i];
-    float* pd = (float*)(blk.data() + n + (n + 1) / 2);
+    float* pd = (float*)(blk.data() + pair);
     for (size_t i = 0; i < n; i++) {
-        pd[2 * i] = (float)prm[i];
-        pd[2 * i + 1] = (float)(prm[i] - (double)pd[2 * i]);
+        pd[4 * i] = pd[4 * i + 1] = (float)prm[i];
+        pd[4 * i + 2] = pd[4 * i + 3] = (float)(prm[i] - (double)pd[4 * i]);
     }
     return blk;
 }
@@ -224,25 +225,44 @@ void build_blocks(ft_plan& pl)
     for (int j = 0, o = 8 + 2 * E + R + R * n; j < ne; j++)
         for (int k = j; k < ne; k++) pl.prm[o++] = (j == k ? 1.0 : 2.0) * pl.kP[(size_t)(pl.q0 + j) * p.V + pl.q0 + k];
     const size_t N = 1ULL << E;
-    const size_t f32 = (25 * N + 15) & ~(size_t)15;
-    pl.tab.assign(f32 + 16 * N, 0);
+    const size_t f32 = (24 * N + 15) & ~(size_t)15;
+    const bool cut = ft::staged_table(E);
+    pl.tab.assign(f32 + (cut ? 12 + 2 * (size_t)E : 20) * N, 0);
     double* w64 = (double*)pl.tab.data();
     double* Jr64 = w64 + N;
     double* ri64 = w64 + 2 * N;
-    unsigned char* meta = pl.tab.data() + 24 * N;
-    float* w32 = (float*)(pl.tab.data() + f32);
+    float* rh = (float*)(pl.tab.data() + f32);
+    float* rl = rh + N;
+    unsigned* meta = (unsigned*)(rl + N);
+    unsigned* q = meta + N;
+    float* w32 = (float*)(meta + N);
     float* Jr32 = w32 + N;
-    float* ri32 = w32 + 2 * N;
+    unsigned off = 0;
     for (size_t s = 0; s < N; s++) {
         // the scan adds Jr/r and the X update raises to 1./r (srcs/tropical_sampling.hpp:487,558)
         w64[s] = p.Jr[s] / p.r[s];
         Jr64[s] = p.Jr[s];
         ri64[s] = 1. / p.r[s];
-        meta[s] = (unsigned char)((p.mm[s] ? 0x80 : 0) | (p.L[s] & 0x7f));
-        w32[s] = (float)w64[s];
-        Jr32[s] = (float)Jr64[s];
-        ri32[2 * s] = (float)ri64[s];   // 1/r as two floats (hi, lo)
-        ri32[2 * s + 1] = (float)(ri64[s] - (double)ri32[2 * s]);
+        rh[s] = (float)ri64[s];   // 1/r as two floats (hi, lo)
+        rl[s] = (float)(ri64[s] - (double)rh[s]);
+        meta[s] = (p.mm[s] ? 0x80u : 0u) | (unsigned)(p.L[s] & 0x7f);
+        if (!cut) {
+            w32[s] = (float)w64[s];
+            Jr32[s] = (float)Jr64[s];
+            continue;
+        }
+        // cut thresholds: floor(2^28 T_k / Jr(s)) << 4 | edge, T_k the running sum of Jr/r over
+        // the subgraph's edges in the reference's order (srcs/tropical_sampling.hpp:482-490);
+        // smaller subgraphs (those with an edge less) have smaller masks, so w64 is complete
+        meta[s] |= off << 16;
+        const double scale = 268435456.0 / Jr64[s];
+        double T = 0.0;
+        for (size_t left = s; left; left &= left - 1) {
+            const int c = __builtin_ctzll(left);
+            T += w64[s ^ ((size_t)1 << c)];
+            const double v = T * scale;
+            q[off++] = (v < 268435455.0 ? (unsigned)v : 268435455u) << 4 | (unsigned)c;
+        }
     }
 }
 
@@ -846,19 +866,22 @@ int ft_autotune(ft_plan* pl, int32_t precision, uint64_t samples, ft_tune_result
             cands.push_back(s);
         };
         if (prec == 1 && deformed) {
-            // two-float determinant and V: out-of-line two-float routines (bits 3, 4) and
-            // shapes from 128 registers (16 warps per SM) to 255 (8 warps, no spills)
+            // out-of-line two-float routines (bits 3, 4) and shapes from 128 registers (16 warps
+            // per SM) to 255 (8 warps, no spills)
             // (four 128-thread blocks won one-integral trials by noise and ran the
             // persistent batch kernel 9 % slower: not a candidate)
             add(256, 2, 29);
             add(512, 1, 29);
             add(384, 1, 29);
+            add(384, 1, 21);
+            add(256, 2, 5);
             add(256, 1, 29);
-            add(512, 1, 13);
-            add(256, 1, 13);
         } else if (prec == 1) {
-            for (int var : {4, 0})
-                for (int bm : {512, 256, 128}) add(bm, 512 / bm, var);
+            for (int var : {4, 0}) {
+                add(256, 1, var);
+                add(256, 2, var);
+                add(512, 1, var);
+            }
         } else {
             const int v = deformed ? 1 : 0;
             for (int var : {v | 4, v})

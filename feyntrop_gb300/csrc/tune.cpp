@@ -82,21 +82,18 @@ std::string tune_class(const kernel_key& k)
 
 launch_shape default_shape(const kernel_key& k)
 {
-    // GB300 sweeps (double box, box-pentagon, 3-loop ladder, K4, cube): the mixed form is
-    // bound by instruction fetch and gains 15-25 % from blocks whose warps start each
-    // sample together (variant bit 2).  Deformed integrands, whose determinant and V run
-    // in two-float, gain most from a smaller code: one out-of-line copy of the FP32
-    // transcendentals (bit 0), of the larger two-float routines (bit 3) and of the
-    // complex two-float product and multiply-add (bit 4: +37 % on the double box, +82 %
-    // on the box-pentagon).  With it they run best as two 256-thread blocks per SM
-    // (128 registers; double box 1.59e9 samples/s, 3-loop ladder 7.2e8; the box-pentagon
-    // 0.94e9 against 1.01e9 for 512 x 1).  Out-of-line two-float add and multiply (bit 1)
-    // cost 45 %.  Undeformed integrands keep one 512-thread block.  The FP64 form is
-    // FP64-pipe bound (256 x 1); the per-sample barrier keeps its warps from drifting
-    // apart too (cube +10 %, double box +1 %).
+    // GB300 sweeps.  Mixed form: the per-sample barrier (variant bit 2) makes the warps of a
+    // block share their instruction fetches.  Undeformed (two samples per thread) 256 threads
+    // with up to 255 registers (five-loop cube, N = 5e7: 5.3 ms; 512 x 128 registers 5.4,
+    // 384 7.1).  Deformed: 16 warps of 128 registers per SM, with one out-of-line copy of the
+    // FP32 transcendentals, of the larger two-float routines and of the complex two-float
+    // product (bits 0, 3, 4): 3-loop ladder 1.35e9 samples/s (inlined 0.86e9), box-pentagon
+    // 1.73e9 (inlined 1.72e9, 12 warps of 168 registers 1.48e9), double box 2.62e9 (12 warps
+    // 2.77e9), one-loop box 5.8e9.  The FP64 form is FP64-pipe bound (256 x 1); the barrier
+    // keeps its warps from drifting apart too (cube +10 %, double box +1 %).
     launch_shape s;
     if (k.prec == 1) {
-        s.block = k.mode == 1 ? 256 : 512;
+        s.block = 256;
         s.minb = k.mode == 1 ? 2 : 1;
     } else {
         s.block = 256;
@@ -106,21 +103,18 @@ launch_shape default_shape(const kernel_key& k)
     return s;
 }
 
-// Shared memory of one block: the dynamic part (staged table, per-thread sums) plus the
-// kernel body's static arrays, the block reduction's per-warp slots and, in the batch
-// kernels, the staged parameter block (its doubles, floats and two-float pairs) and the
-// work-item variables.
+// Shared memory of one block: the dynamic part (staged table, sums) plus the kernel
+// body's static variables, in the batch kernels with the staged parameter block (its
+// doubles, floats and two-float quadruples) and the work item.
 static unsigned block_smem_bytes(const kernel_key& k)
 {
-    const unsigned slots = 8u * (unsigned)k.K + 8u;
-    const unsigned red = (unsigned)(k.block / 32) * slots * 8u;
     unsigned prm = 0;
     if (k.batch) {
         const unsigned n = (unsigned)(k.V - 1), ne = n - (unsigned)k.q0, r = (unsigned)k.rank;
         const unsigned p = 8u + 2u * (unsigned)k.E + r + r * n + ne * (ne + 1u) / 2u;
-        prm = (p + (p + 1u) / 2u + p) * 8u + 64u;
+        prm = (p + (p + 1u) / 2u + 1u + 2u * p) * 8u + 64u;
     }
-    return table_smem_bytes(k) + red + prm;
+    return table_smem_bytes(k) + 64u + prm;
 }
 
 void apply_shape(kernel_key& k, const launch_shape& s)
@@ -128,6 +122,9 @@ void apply_shape(kernel_key& k, const launch_shape& s)
     k.block = s.block;
     k.minb = s.minb;
     k.variant = s.variant;
+    // as much of the deformed integrand's scratch in shared memory as fits
+    k.scratch = k.prec == 1 && k.mode == 1 ? 2 : 0;
+    while (k.scratch > 0 && block_smem_bytes(k) * (unsigned)k.minb > kSmemLimit) k.scratch--;
     // keep the warps per SM while halving the block until the shared memory fits
     while (k.block > 64 && block_smem_bytes(k) > kSmemLimit) {
         k.block /= 2;
