@@ -7,7 +7,7 @@
 // side by side on forked streams.  One run is
 //   1. one host-to-device copy of the per-run descriptors (N, seed state, first item of
 //      every integral, and each class's item total with its counters zeroed),
-//   2. per class: the item stream states (one warp per integral, GF(2) skip-ahead),
+//   2. per class: the integrals' start states (one warp per integral, GF(2) skip-ahead),
 //      the persistent sampling launch, in mixed precision the FP64 pass over the
 //      handed-off samples, and the per-integral reduction,
 //   3. one device-to-host copy of every integral's sums and the classes' counters,
@@ -41,7 +41,7 @@ struct batch_inst {
 struct item_prep {
     unsigned long long s[4];
     unsigned long long skip;
-    unsigned long long first_item, nitems, pad;
+    unsigned long long pad[3];
 };
 static_assert(sizeof(batch_inst) == 64 && sizeof(item_prep) == 64, "descriptor layout");
 
@@ -65,16 +65,16 @@ struct ft_batch {
         std::vector<int> members;               // indices into plans
         int K = 1, rank = 1, draws = 1;
         unsigned long long chunk = 64;
-        int lanebits = 8;
         unsigned grid = 0, qgrid = 0;
         size_t prm_stride = 0, tab_stride = 0;  // bytes
         // offsets of this class's records in the run descriptors
         size_t off_hdr = 0, off_inst = 0, off_prep = 0, off_out = 0, off_qacc = 0;
         unsigned char* d_prm = nullptr;
         unsigned char* d_tab = nullptr;
-        unsigned long long* d_lanepw = nullptr;
-        unsigned long long* d_itemM = nullptr;
-        unsigned long long* d_item_state = nullptr;
+        unsigned long long* d_mats = nullptr;        // stride matrices of the chunk
+        unsigned long long* d_item_mats = nullptr;   // powers of the item stride, item_digits octal digits
+        int item_digits = 0, want_digits = 0;
+        unsigned long long* d_state = nullptr;       // the integrals' start states
         size_t item_cap = 0;
         double* d_parts = nullptr;
         unsigned long long* d_queue = nullptr;
@@ -111,9 +111,9 @@ struct ft_batch {
         for (group& g : groups) {
             cudaFree(g.d_prm);
             cudaFree(g.d_tab);
-            cudaFree(g.d_lanepw);
-            cudaFree(g.d_itemM);
-            cudaFree(g.d_item_state);
+            cudaFree(g.d_mats);
+            cudaFree(g.d_item_mats);
+            cudaFree(g.d_state);
             cudaFree(g.d_parts);
             cudaFree(g.d_queue);
             if (g.stream) cudaStreamDestroy(g.stream);
@@ -219,8 +219,6 @@ void build(ft_batch& b)
                       ? ft::chunk_override()
                       : env_u64("FEYNTROP_GB300_BATCH_CHUNK", tuned.chunk ? tuned.chunk : (prec ? 128 : 16));
         if (g.chunk < 1 || g.chunk >= (1ull << 18)) throw std::invalid_argument("batch chunk out of range");
-        g.lanebits = 1;
-        while ((1 << g.lanebits) < g.ks->block) g.lanebits++;
         g.grid = (unsigned)(ds.sms * g.ks->blocks_per_sm);
         g.qgrid = prec ? (unsigned)(ds.sms * 2) : 0;
         // parameter blocks and tables of the class's integrals
@@ -239,12 +237,10 @@ void build(ft_batch& b)
         cu(cudaMalloc(&g.d_tab, ht.size()), "cudaMalloc(batch tables)");
         cu(cudaMemcpy(g.d_prm, hp.data(), hp.size(), cudaMemcpyHostToDevice), "cudaMemcpy(batch parameters)");
         cu(cudaMemcpy(g.d_tab, ht.data(), ht.size(), cudaMemcpyHostToDevice), "cudaMemcpy(batch tables)");
-        // lane skip matrices (T^(chunk draws))^(2^b) and the item step T^(block chunk draws)
-        cu(cudaMalloc(&g.d_lanepw, (size_t)g.lanebits * 1024 * 8), "cudaMalloc(lane skip matrices)");
-        cu(cudaMalloc(&g.d_itemM, 1024 * 8), "cudaMalloc(item skip matrix)");
-        cu(ft::launch_lane_powers(ds.tpow, g.chunk * g.draws, g.lanebits, g.d_lanepw, 0), "lane skip matrices");
-        cu(ft::launch_lane_powers(ds.tpow, (unsigned long long)g.ks->block * g.chunk * g.draws, 1, g.d_itemM, 0),
-           "item skip matrix");
+        // stride matrices of the chunk for a block's threads (two octal digits of warps)
+        cu(cudaMalloc(&g.d_mats, ft::stride_words(2) * 8), "cudaMalloc(stride matrices)");
+        cu(cudaMalloc(&g.d_state, nm * 32), "cudaMalloc(batch start states)");
+        cu(ft::launch_stride_matrices(ds.tpow, g.chunk * g.draws, 2, g.d_mats, 0), "stride matrices");
         cu(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking), "cudaStreamCreate");
         cu(cudaEventCreateWithFlags(&g.done, cudaEventDisableTiming), "cudaEventCreate");
         g.off_hdr = hdr;
@@ -295,9 +291,8 @@ void record(ft_batch& b)
     const device_state& ds = dev_state();
     b.launches = 0;
     for (ft_batch::group& g : b.groups) {
-        cu(ft::launch_batch_item_states(b.d_desc + g.off_prep, (int)g.members.size(), ds.tpow, g.d_itemM,
-                                        g.d_item_state, s),
-           "batch item states");
+        cu(ft::launch_batch_start_states(b.d_desc + g.off_prep, (int)g.members.size(), ds.tpow, g.d_state, s),
+           "batch start states");
         b.launches++;
     }
     cu(cudaEventRecord(b.fork, s), "cudaEventRecord");
@@ -309,14 +304,14 @@ void record(ft_batch& b)
         const unsigned long long* total = &hd->total_items;
         unsigned long long* counter = &hd->counter;
         unsigned int* qcount = (unsigned int*)&hd->qcount;
-        const unsigned long long* item_state = g.d_item_state;
-        const unsigned long long* lanepw = g.d_lanepw;
-        int lanebits = g.lanebits;
+        const unsigned long long* state = g.d_state;
+        const unsigned long long* item_mats = g.d_item_mats;
+        const unsigned long long* mats = g.d_mats;
         unsigned long long chunk = g.chunk;
         double* parts = g.d_parts;
         unsigned long long* queue = g.d_queue;
         unsigned int qcap = (unsigned int)g.qcap;
-        void* args[] = {&inst, &ninst, &total, &item_state, &lanepw, &lanebits, &chunk, &counter, &parts, &queue,
+        void* args[] = {&inst, &ninst, &total, &state, &item_mats, &mats, &chunk, &counter, &parts, &queue,
                         &qcount, &qcap};
         ft::check(ft::drv().LaunchKernel(g.ks->sample, g.grid, 1, 1, g.ks->block, 1, 1, g.ks->smem,
                                          (CUstream)g.stream, args, nullptr),
@@ -374,14 +369,24 @@ bool ensure_capacity(ft_batch& b, const std::vector<size_t>& qwant)
         const size_t items = std::max<size_t>(g.total_items, 1);
         if (items > g.item_cap) {
             const size_t cap = std::max(items, g.item_cap + g.item_cap / 4);
-            cudaFree(g.d_item_state);
             cudaFree(g.d_parts);
-            g.d_item_state = nullptr;
             g.d_parts = nullptr;
             g.item_cap = 0;
-            cu(cudaMalloc(&g.d_item_state, cap * 32), "cudaMalloc(batch item states)");
             cu(cudaMalloc(&g.d_parts, cap * (8 * g.K + 8) * 8), "cudaMalloc(batch item sums)");
             g.item_cap = cap;
+            grew = true;
+        }
+        if (g.want_digits > g.item_digits) {
+            cudaFree(g.d_item_mats);
+            g.d_item_mats = nullptr;
+            g.item_digits = 0;
+            const size_t bytes = (size_t)g.want_digits * 7 * 1024 * 8;
+            cu(cudaMalloc(&g.d_item_mats, bytes), "cudaMalloc(item stride matrices)");
+            cu(ft::launch_digit_matrices(dev_state().tpow, (unsigned long long)g.ks->block * g.chunk * g.draws,
+                                         g.want_digits, g.d_item_mats, b.stream),
+               "item stride matrices");
+            cu(cudaStreamSynchronize(b.stream), "item stride matrices");   // the graph may run on another stream
+            g.item_digits = g.want_digits;
             grew = true;
         }
         if (b.precision && qwant[gi] > g.qcap) {
@@ -435,7 +440,7 @@ int ft_batch_run(ft_batch* b, const ft_run_options* opts, ft_result* results)
         for (size_t gi = 0; gi < b->groups.size(); gi++) {
             ft_batch::group& g = b->groups[gi];
             const unsigned long long per_item = (unsigned long long)g.ks->block * g.chunk;
-            unsigned long long next = 0;
+            unsigned long long next = 0, most = 0;
             size_t q = 0;
             for (size_t m = 0; m < g.members.size(); m++) {
                 const ft_run_options& o = opts[g.members[m]];
@@ -451,15 +456,17 @@ int ft_batch_run(ft_batch* b, const ft_run_options* opts, ft_result* results)
                 const ft::xstate s = ft::seed_state(o.seed);
                 for (int w = 0; w < 4; w++) p->s[w] = s.s[w];
                 p->skip = o.first_sample * (unsigned long long)g.draws;
-                p->first_item = next;
-                p->nitems = items;
                 next += items;
+                most = std::max(most, items);
                 // hand-offs run at ~1e-5 of the samples; a larger share overflows the
                 // queue, which then grows and the run repeats once
                 q += (size_t)std::min<unsigned long long>(N, N / 1024 + 1024);
             }
             if (next >= (1ull << 36)) throw std::invalid_argument("ft_batch_run: too many work items");
             g.total_items = next;
+            // octal digits of an item's number within its integral
+            g.want_digits = 0;
+            while (most > 1 && ((most - 1) >> (3 * g.want_digits))) g.want_digits++;
             class_header* h = (class_header*)(b->h_desc + g.off_hdr);
             h->total_items = next;
             h->counter = 0;

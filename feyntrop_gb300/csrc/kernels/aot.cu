@@ -1,17 +1,11 @@
 // Topology-independent kernels, compiled ahead of time with nvcc for sm_103a.
 //
-//  ft_gf2_lane_powers  the skip matrices a sampling launch needs: P_b = (T^S)^(2^b)
-//                      for b < nbits, where T is one xoshiro256+ step and S the number
-//                      of draws per lane; one CTA of 256 threads, thread c owns
-//                      column c of the 256x256 GF(2) matrices.
-//  ft_finalize_parts   sums the per-block partial moments of one integration into a
-//                      single vector: double-double for the moment slots, plain for
-//                      the counters.
-//  ft_batch_item_states  stream states of the work items of a batch (one warp per
-//                      integral, GF(2) skip-ahead).
+//  ft_stride_matrices  powers of a stride's skip matrix (T^S)^n over GF(2), T the xoshiro256+
+//                      step: the matrices the sampling kernels reach their threads' start
+//                      states with.
+//  ft_batch_start_states  stream state of each of a batch's integrals' first samples (one
+//                      warp per integral, GF(2) skip-ahead).
 //  ft_batch_finalize   per-integral sums of a batch's work items and FP64 pass.
-//  ft_warp_states      stream states of the warps of a sampling launch (one warp per
-//                      warp, GF(2) skip-ahead), so each thread skips only its lane.
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -22,59 +16,72 @@ typedef unsigned long long u64;
 
 namespace {
 
-// column c of A * B, A in shared memory by columns
-__device__ __forceinline__ void gf2_col(const u64* A, const u64* bcol, u64* out)
+// Block b < 32 writes the images under (T^S)^b of every nibble n of the state and value v of
+// it at out[((16 n + v) * 32 + b) * 4 ..] (with `lanes`), the next
+// ones (T^S)^(f 8^d v), v = 1 .. 7, f = 32 with `lanes`, else 1, 1024 words each.  Every
+// matrix is the product of the T^(2^j) of its exponent's set bits, so the blocks are
+// independent (a chain of squarings in one block took 190 us).  A product M <- A M by 1024
+// threads: thread (w, c) adds the columns of A in rows' word w for column c of M, all lanes
+// of a warp reading the same column of A (broadcasts), then the four words' parts meet.
+__global__ void __launch_bounds__(1024) ft_stride_matrices(const u64* __restrict__ tpow, u64 S, int lanes,
+                                                           u64* __restrict__ out)
 {
-    u64 r0 = 0, r1 = 0, r2 = 0, r3 = 0;
-#pragma unroll
-    for (int w = 0; w < 4; w++) {
-        u64 bits = bcol[w];
-        while (bits) {
-            const int b = __ffsll((long long)bits) - 1;
-            bits &= bits - 1;
-            const u64* col = A + (w * 64 + b) * 4;
-            r0 ^= col[0];
-            r1 ^= col[1];
-            r2 ^= col[2];
-            r3 ^= col[3];
+    __shared__ u64 A[1024], M[1024];
+    __shared__ ulonglong2 part[4][256][2];
+    const int w = threadIdx.x >> 8, c = threadIdx.x & 255;
+    int b = (int)blockIdx.x;
+    u64 n, *dst;
+    const bool nibbles = lanes && b < 32;
+    if (nibbles) {
+        n = S * (u64)b;
+        dst = out + b * 4;
+    } else {
+        if (lanes) b -= 32;
+        n = (lanes ? 32ull : 1ull) * S * (u64)(b % 7 + 1) << (3 * (b / 7));
+        dst = out + (lanes ? 131072 : 0) + (size_t)b * 1024;
+    }
+    M[c * 4 + w] = (w == (c >> 6)) ? (1ull << (c & 63)) : 0ull;
+    bool first = true;
+    for (; n; n &= n - 1) {
+        const u64* P = tpow + (size_t)(__ffsll((long long)n) - 1) * 1024;
+        if (first) {
+            M[threadIdx.x] = P[threadIdx.x];
+            first = false;
+            continue;
         }
+        A[threadIdx.x] = P[threadIdx.x];
+        __syncthreads();
+        const u64 bits = M[c * 4 + w];
+        const ulonglong2* col = (const ulonglong2*)(A + w * 256);
+        u64 r0 = 0, r1 = 0, r2 = 0, r3 = 0;
+#pragma unroll 8
+        for (int k = 0; k < 64; k++) {
+            const u64 mask = 0ull - ((bits >> k) & 1ull);
+            const ulonglong2 lo = col[2 * k], hi = col[2 * k + 1];
+            r0 ^= lo.x & mask;
+            r1 ^= lo.y & mask;
+            r2 ^= hi.x & mask;
+            r3 ^= hi.y & mask;
+        }
+        part[w][c][0] = make_ulonglong2(r0, r1);
+        part[w][c][1] = make_ulonglong2(r2, r3);
+        __syncthreads();
+        const u64* p = (const u64*)part;
+        M[threadIdx.x] = p[threadIdx.x] ^ p[1024 + threadIdx.x] ^ p[2048 + threadIdx.x] ^ p[3072 + threadIdx.x];
+        __syncthreads();
     }
-    out[0] = r0;
-    out[1] = r1;
-    out[2] = r2;
-    out[3] = r3;
-}
-
-__global__ void __launch_bounds__(256) ft_gf2_lane_powers(const u64* __restrict__ tpow, u64 S, int nbits,
-                                                          u64* __restrict__ out)
-{
-    __shared__ u64 A[1024];
-    __shared__ u64 M[1024];
-    const int c = threadIdx.x;
-    for (int w = 0; w < 4; w++) M[c * 4 + w] = (w == (c >> 6)) ? (1ull << (c & 63)) : 0ull;
     __syncthreads();
-    // M = T^S = product of T^(2^j) over the set bits j of S (powers of T commute)
-    for (int j = 0; j < 64; j++) {
-        if (!((S >> j) & 1ull)) continue;
-        for (int w = 0; w < 4; w++) A[c * 4 + w] = tpow[(size_t)j * 1024 + c * 4 + w];
-        __syncthreads();
-        u64 r[4];
-        gf2_col(A, M + c * 4, r);
-        __syncthreads();
-        for (int w = 0; w < 4; w++) M[c * 4 + w] = r[w];
-        __syncthreads();
+    if (!nibbles) {
+        dst[threadIdx.x] = M[threadIdx.x];
+        return;
     }
-    for (int b = 0; b < nbits; b++) {
-        for (int w = 0; w < 4; w++) out[(size_t)b * 1024 + c * 4 + w] = M[c * 4 + w];
-        if (b + 1 == nbits) break;
-        for (int w = 0; w < 4; w++) A[c * 4 + w] = M[c * 4 + w];
-        __syncthreads();
-        u64 r[4];
-        gf2_col(A, A + c * 4, r);
-        __syncthreads();
-        for (int w = 0; w < 4; w++) M[c * 4 + w] = r[w];
-        __syncthreads();
-    }
+    const int nib = threadIdx.x >> 4, v = threadIdx.x & 15;
+    u64 r[4] = {0, 0, 0, 0};
+    for (int k = 0; k < 4; k++)
+        for (int i = 0; i < 4; i++) r[i] ^= (v >> k) & 1 ? M[(nib * 4 + k) * 4 + i] : 0ull;
+    ulonglong2* q = (ulonglong2*)(dst + (size_t)threadIdx.x * 128);
+    q[0] = make_ulonglong2(r[0], r[1]);
+    q[1] = make_ulonglong2(r[2], r[3]);
 }
 
 __device__ __forceinline__ void dd_add(double& ah, double& al, double bh, double bl)
@@ -85,49 +92,6 @@ __device__ __forceinline__ void dd_add(double& ah, double& al, double bh, double
     err += al + bl;
     ah = s + err;
     al = err - (ah - s);
-}
-
-// one block per slot pair (moments) or slot (counters): the block's threads take the
-// parts in turn, then a double-double (or plain) tree across the block
-__global__ void __launch_bounds__(256) ft_finalize_parts(const double* __restrict__ parts, int nparts, int slots,
-                                                         int ndd, double* __restrict__ out)
-{
-    __shared__ double sh[8], sl[8];
-    const int u = blockIdx.x;
-    const int npairs = ndd / 2;
-    const bool pair = u < npairs;
-    const int s = pair ? 2 * u : ndd + (u - npairs);
-    double h = 0.0, l = 0.0;
-    for (int p = threadIdx.x; p < nparts; p += blockDim.x) {
-        if (pair)
-            dd_add(h, l, parts[(size_t)p * slots + s], parts[(size_t)p * slots + s + 1]);
-        else
-            h += parts[(size_t)p * slots + s];
-    }
-    for (int off = 16; off; off >>= 1) {
-        const double oh = __shfl_down_sync(0xffffffffu, h, off), ol = __shfl_down_sync(0xffffffffu, l, off);
-        if (pair)
-            dd_add(h, l, oh, ol);
-        else
-            h += oh;
-    }
-    const int w = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) {
-        sh[w] = h;
-        sl[w] = l;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double H = sh[0], L = sl[0];
-        for (int i = 1; i < (int)(blockDim.x >> 5); i++) {
-            if (pair)
-                dd_add(H, L, sh[i], sl[i]);
-            else
-                H += sh[i];
-        }
-        out[s] = H;
-        if (pair) out[s + 1] = L;
-    }
 }
 
 // ------------------------------------------------------------------ batches
@@ -141,7 +105,7 @@ struct batch_inst_view {
 struct item_prep {
     u64 s[4];         // seed state of the instance's stream
     u64 skip;         // draws before its first sample
-    u64 first_item, nitems, pad;
+    u64 pad[3];
 };
 
 __device__ __forceinline__ u64 word_of(const u64 (&g)[4], int w)
@@ -178,10 +142,9 @@ __device__ __forceinline__ void warp_gf2_apply(const u64* __restrict__ M, u64 (&
     g[3] = r3;
 }
 
-// one warp per instance: the stream state of each of its work items' first samples
-__global__ void __launch_bounds__(128) ft_batch_item_states(const item_prep* __restrict__ d, int n,
-                                                            const u64* __restrict__ tpow,
-                                                            const u64* __restrict__ itemM, u64* __restrict__ out)
+// one warp per instance: the stream state of its first sample
+__global__ void __launch_bounds__(128) ft_batch_start_states(const item_prep* __restrict__ d, int n,
+                                                            const u64* __restrict__ tpow, u64* __restrict__ out)
 {
     const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = (int)(threadIdx.x & 31u);
     if (w >= n) return;   // the whole warp
@@ -189,24 +152,6 @@ __global__ void __launch_bounds__(128) ft_batch_item_states(const item_prep* __r
     const u64 skip = d[w].skip;
     for (int b = 0; b < 64; b++)
         if ((skip >> b) & 1ull) warp_gf2_apply(tpow + (size_t)b * 1024, g, lane);
-    const u64 f = d[w].first_item, m = d[w].nitems;
-    for (u64 k = 0; k < m; k++) {
-        if (lane < 4) out[(f + k) * 4 + lane] = word_of(g, lane);
-        if (k + 1 < m) warp_gf2_apply(itemM, g, lane);
-    }
-}
-
-// one warp per output warp: the first lane's state of warp w of a sampling launch is
-// (T^S)^(32 w) base, i.e. the lane skip matrices of the bits of w shifted by 5
-__global__ void __launch_bounds__(128) ft_warp_states(const u64* __restrict__ lanepw, int lanebits, u64 s0, u64 s1,
-                                                      u64 s2, u64 s3, unsigned nwarps, u64* __restrict__ out)
-{
-    const unsigned w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = (int)(threadIdx.x & 31u);
-    if (w >= nwarps) return;   // the whole warp
-    u64 g[4] = {s0, s1, s2, s3};
-    for (int j = 0; j + 5 < lanebits; j++)
-        if ((w >> j) & 1u) warp_gf2_apply(lanepw + (size_t)(j + 5) * 1024, g, lane);
     if (lane < 4) out[(size_t)w * 4 + lane] = word_of(g, lane);
 }
 
@@ -341,24 +286,20 @@ double fma_peak_tflops(bool fp64)
 // Scratch of ft_integrate_noalloc, for callers that must not allocate device memory
 // during an integration.  It is one file-scope device array per GPU that loads this
 // library, held until the process exits:
-//   [2 words] FP64 hand-off queue count, [NOALLOC_PART_DOUBLES] per-block partial
-//   moments, [5 * NOALLOC_QUEUE_ENTRIES] hand-off queue, [NOALLOC_LANE_WORDS] lane
-//   skip matrices, [NOALLOC_WARP_WORDS] warp start states.
+//   [2 words] FP64 hand-off queue count and the finished blocks' ticket,
+//   [NOALLOC_PART_DOUBLES] per-block partial moments, [5 * NOALLOC_QUEUE_ENTRIES]
+//   hand-off queue, [NOALLOC_MAT_WORDS] stride matrices.
 // Every call shares it (and it keeps the last call's contents), so calls that overlap
 // on the GPU race; the queue count is cleared at the start of each call.
 constexpr unsigned long long kNoallocParts = 2, kNoallocQueue = kNoallocParts + NOALLOC_PART_DOUBLES,
-                             kNoallocLanes = kNoallocQueue + 5ull * NOALLOC_QUEUE_ENTRIES,
-                             kNoallocWarps = kNoallocLanes + NOALLOC_LANE_WORDS;
+                             kNoallocMats = kNoallocQueue + 5ull * NOALLOC_QUEUE_ENTRIES;
 // the regions end inside the array, and each holds what the host-side checks of
 // ft_integrate_noalloc let a call use: 2048 blocks of up to 8K+8 = 136 slots (16 eps
-// orders), the stream states of every warp of 2048 blocks of up to 1024 threads, the
-// 1024-word skip matrices of up to 24 lane bits
-static_assert(kNoallocWarps + NOALLOC_WARP_WORDS <= NOALLOC_TOTAL_WORDS, "no-allocation layout overruns");
-static_assert(NOALLOC_PART_DOUBLES >= NOALLOC_MAX_BLOCKS * (8 * 16 + 8), "partial sums of 16 eps orders");
-static_assert(NOALLOC_WARP_WORDS >= NOALLOC_MAX_BLOCKS * (1024 / 32) * 4, "warp states of 1024-thread blocks");
-static_assert(NOALLOC_LANE_WORDS >= NOALLOC_MAX_LANE_BITS * 1024, "lane skip matrices");
-static_assert(kNoallocQueue % 2 == 0 && kNoallocLanes % 2 == 0 && kNoallocWarps % 2 == 0,
-              "16-byte aligned regions (ulonglong2 loads)");
+// orders), the matrices of up to 2^24 threads
+static_assert(kNoallocMats + NOALLOC_MAT_WORDS <= NOALLOC_TOTAL_WORDS, "no-allocation layout overruns");
+static_assert(NOALLOC_PART_DOUBLES >= (NOALLOC_MAX_BLOCKS + 1) * (8 * 16 + 8), "partial sums of 16 eps orders");
+static_assert(NOALLOC_MAT_WORDS >= (128 + 7 * ((NOALLOC_MAX_LANE_BITS - 5 + 2) / 3)) * 1024, "stride matrices");
+static_assert(kNoallocQueue % 2 == 0 && kNoallocMats % 2 == 0, "16-byte aligned regions (ulonglong2 loads)");
 static __device__ __align__(256) u64 g_noalloc_scratch[NOALLOC_TOTAL_WORDS];
 
 cudaError_t noalloc_scratch(noalloc_layout* out)
@@ -385,24 +326,30 @@ cudaError_t noalloc_scratch(noalloc_layout* out)
     }
     u64* w = (u64*)base;
     out->qcount = (unsigned int*)w;
+    out->ticket = (unsigned int*)w + 1;
     out->parts = (double*)(w + kNoallocParts);
     out->queue = w + kNoallocQueue;
-    out->lanepw = w + kNoallocLanes;
-    out->warpst = w + kNoallocWarps;
+    out->mats = w + kNoallocMats;
     return cudaSuccess;
 }
 
-cudaError_t launch_lane_powers(const u64* tpow, u64 S, int nbits, u64* out, cudaStream_t st)
+cudaError_t launch_stride_matrices(const u64* tpow, u64 S, int digits, u64* out, cudaStream_t st)
 {
-    ft_gf2_lane_powers<<<1, 256, 0, st>>>(tpow, S, nbits, out);
+    ft_stride_matrices<<<32 + 7 * digits, 1024, 0, st>>>(tpow, S, 1, out);
     return cudaGetLastError();
 }
 
-cudaError_t launch_batch_item_states(const void* prep, int n, const u64* tpow, const u64* itemM, u64* out,
-                                     cudaStream_t st)
+cudaError_t launch_digit_matrices(const u64* tpow, u64 S, int digits, u64* out, cudaStream_t st)
+{
+    if (digits <= 0) return cudaSuccess;
+    ft_stride_matrices<<<7 * digits, 1024, 0, st>>>(tpow, S, 0, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_batch_start_states(const void* prep, int n, const u64* tpow, u64* out, cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
-    ft_batch_item_states<<<(n + 3) / 4, 128, 0, st>>>((const item_prep*)prep, n, tpow, itemM, out);
+    ft_batch_start_states<<<(n + 3) / 4, 128, 0, st>>>((const item_prep*)prep, n, tpow, out);
     return cudaGetLastError();
 }
 
@@ -413,21 +360,6 @@ cudaError_t launch_batch_finalize(const void* inst, int n, const double* parts, 
     const long long threads = (long long)n * (4 * K + 8);
     ft_batch_finalize<<<(unsigned)((threads + 127) / 128), 128, 0, st>>>((const batch_inst_view*)inst, n, parts, K,
                                                                          qacc, out);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_warp_states(const u64* lanepw, int lanebits, const u64* base, unsigned nwarps, u64* out,
-                               cudaStream_t st)
-{
-    if (nwarps == 0) return cudaSuccess;
-    ft_warp_states<<<(nwarps + 3) / 4, 128, 0, st>>>(lanepw, lanebits, base[0], base[1], base[2], base[3], nwarps, out);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_finalize(const double* parts, int nparts, int slots, int ndd, double* out, cudaStream_t st)
-{
-    const int units = ndd / 2 + (slots - ndd);
-    ft_finalize_parts<<<units, 256, 0, st>>>(parts, nparts, slots, ndd, out);
     return cudaGetLastError();
 }
 

@@ -5,15 +5,23 @@
 
 namespace ft {
 
-// out[b] = (T^S)^(2^b), b < nbits; tpow = T^(2^j), j < 64 (1024 words per matrix)
-cudaError_t launch_lane_powers(const unsigned long long* tpow, unsigned long long S, int nbits,
-                               unsigned long long* out, cudaStream_t st);
+// The matrices that take a sampling kernel's threads to their start states (layout in
+// sample_body.cuh): nibble images under (T^S)^l, l < 32, then (T^S)^(32 8^d v), v = 1 .. 7, d <
+// digits; tpow = T^(2^j), j < 64 (1024 words per matrix).  stride_words(digits) words.
+inline unsigned long long stride_words(int digits) { return (128ull + 7ull * (unsigned long long)digits) * 1024ull; }
+// octal digits of a warp index in a launch of 2^bits threads
+inline int stride_digits(int bits) { return bits <= 5 ? 0 : (bits - 5 + 2) / 3; }
+cudaError_t launch_stride_matrices(const unsigned long long* tpow, unsigned long long S, int digits,
+                                   unsigned long long* out, cudaStream_t st);
+// (T^S)^(8^d v), v = 1 .. 7, d < digits
+cudaError_t launch_digit_matrices(const unsigned long long* tpow, unsigned long long S, int digits,
+                                  unsigned long long* out, cudaStream_t st);
 
-// Batches (layouts in aot.cu): item stream states from per-instance item_prep records
-// (one warp per instance), and the per-instance sums of the work items plus the FP64
-// pass (qacc may be NULL).
-cudaError_t launch_batch_item_states(const void* prep, int n, const unsigned long long* tpow,
-                                     const unsigned long long* itemM, unsigned long long* out, cudaStream_t st);
+// Batches (layouts in aot.cu): the integrals' start states from item_prep records (one warp
+// per integral), and the per-instance sums of the work items plus the FP64 pass (qacc may
+// be NULL).
+cudaError_t launch_batch_start_states(const void* prep, int n, const unsigned long long* tpow,
+                                      unsigned long long* out, cudaStream_t st);
 cudaError_t launch_batch_finalize(const void* inst, int n, const double* parts, int K,
                                   const unsigned long long* qacc, double* out, cudaStream_t st);
 
@@ -26,35 +34,24 @@ cudaError_t launch_batch_finalize(const void* inst, int n, const double* parts, 
 constexpr int kExactDigits = 68;
 inline unsigned long long exact_words(int K) { return 4ull * (unsigned long long)K * kExactDigits + 4ull; }
 
-// out[s] = sum over parts of parts[p * slots + s]; slots [0, ndd) are (hi, lo) pairs
-cudaError_t launch_finalize(const double* parts, int nparts, int slots, int ndd, double* out, cudaStream_t st);
-
 // Limits of the no-allocation path (ft_integrate_noalloc): per-block partial moments
 // for up to 2048 blocks of up to 136 slots (16 eps orders), 65536 FP64 hand-off
-// entries, lane skip matrices for up to 2^24 lanes, the stream states of up to 32
-// warps per block.  About 7 MB per device.
+// entries, stride matrices for up to 2^24 threads.  About 7 MB per device.
 #define NOALLOC_MAX_BLOCKS 2048
 #define NOALLOC_MAX_SLOTS 136
-#define NOALLOC_PART_DOUBLES (NOALLOC_MAX_BLOCKS * NOALLOC_MAX_SLOTS)
+#define NOALLOC_PART_DOUBLES ((NOALLOC_MAX_BLOCKS + 1) * NOALLOC_MAX_SLOTS)   // one for the sampling launch's sum
 #define NOALLOC_QUEUE_ENTRIES 65536
 #define NOALLOC_MAX_LANE_BITS 24
-#define NOALLOC_LANE_WORDS (NOALLOC_MAX_LANE_BITS * 1024)
-#define NOALLOC_WARP_WORDS (NOALLOC_MAX_BLOCKS * 32 * 4)
-#define NOALLOC_TOTAL_WORDS \
-    (2 + NOALLOC_PART_DOUBLES + 5 * NOALLOC_QUEUE_ENTRIES + NOALLOC_LANE_WORDS + NOALLOC_WARP_WORDS)
+#define NOALLOC_MAT_WORDS (177 * 1024)
+#define NOALLOC_TOTAL_WORDS (2 + NOALLOC_PART_DOUBLES + 5 * NOALLOC_QUEUE_ENTRIES + NOALLOC_MAT_WORDS)
 
 struct noalloc_layout {
     unsigned int* qcount;
     double* parts;
     unsigned long long* queue;
-    unsigned long long* lanepw;
-    unsigned long long* warpst;
+    unsigned long long* mats;
+    unsigned int* ticket;
 };
-
-// stream states of the first lane of every warp of a launch: warp w starts at
-// (T^S)^(32 w) base, from the lane skip matrices lanepw[b] = (T^S)^(2^b), b < lanebits
-cudaError_t launch_warp_states(const unsigned long long* lanepw, int lanebits, const unsigned long long* base,
-                               unsigned nwarps, unsigned long long* out, cudaStream_t st);
 
 // device addresses inside the static scratch of the current device (first call per
 // device looks the symbol up)

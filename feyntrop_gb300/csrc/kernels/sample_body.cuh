@@ -2276,34 +2276,78 @@ static __device__ __forceinline__ xo load_state(const u64* __restrict__ s)
     return g;
 }
 
-// ------------------------------------------------------------------ lane start states
-// state <- P_b state for every set bit b of `lane`, with P_b = (T^S)^(2^b) supplied by
-// the host (S = draws per lane).  The loop is uniform across the warp so that the
-// matrix columns are broadcast loads.
-static __device__ __forceinline__ void skip_lanes(xo& g, u32 lane, const u64* __restrict__ pw, int nbits)
+// ------------------------------------------------------------------ start states
+// The state of a stream after t strides, from the stride's matrices A^n over GF(2) (T the
+// generator's step, A = T^S; written by ft_stride_matrices): first, for every nibble n of
+// the state and value v of it, its image under A^l, l < 32, as [16 n + v][l] (4 words
+// each), then A^(32 8^d v), v = 1 .. 7, for the octal digits d of t / 32 (1024 words each).
+#define MAT_LANES 131072u
+// g <- M g by the whole warp: lane l owns input bits 8l .. 8l+7 (column c of M is the four
+// words M[4c .. 4c+3]); the partial results are XOR-reduced across the warp
+static __device__ __forceinline__ u64 warp_xor(u64 x)
 {
-    for (int b = 0; b < nbits; b++) {
-        const bool mine = (lane >> b) & 1u;
-        if (!__any_sync(0xffffffffu, mine)) continue;
-        const ulonglong2* M = (const ulonglong2*)(pw + (size_t)b * 1024);
-        u64 r0 = 0, r1 = 0, r2 = 0, r3 = 0;
-        const u64 sv[4] = {g.a, g.b, g.c, g.d};
-#pragma unroll 4
-        for (int c = 0; c < 256; c++) {
-            const u64 mask = 0ull - ((sv[c >> 6] >> (c & 63)) & 1ull);
-            const ulonglong2 lo = __ldg(M + 2 * c), hi = __ldg(M + 2 * c + 1);
-            r0 ^= lo.x & mask;
-            r1 ^= lo.y & mask;
-            r2 ^= hi.x & mask;
-            r3 ^= hi.y & mask;
+    return ((u64)__reduce_xor_sync(0xffffffffu, (u32)(x >> 32)) << 32) | __reduce_xor_sync(0xffffffffu, (u32)x);
+}
+static __device__ __noinline__ xo warp_apply(const u64* __restrict__ M, xo g)
+{
+    const u32 lane = threadIdx.x & 31u;
+    const u64 word = lane < 8u ? g.a : lane < 16u ? g.b : lane < 24u ? g.c : g.d;
+    const u32 bits = (u32)(word >> ((lane & 7u) * 8u)) & 255u;
+    u64 r0 = 0, r1 = 0, r2 = 0, r3 = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const u64 mask = 0ull - (u64)((bits >> k) & 1u);
+        const ulonglong2* col = (const ulonglong2*)(M + 4u * (lane * 8u + k));
+        const ulonglong2 lo = __ldg(col), hi = __ldg(col + 1);
+        r0 ^= lo.x & mask;
+        r1 ^= lo.y & mask;
+        r2 ^= hi.x & mask;
+        r3 ^= hi.y & mask;
+    }
+    g.a = warp_xor(r0);
+    g.b = warp_xor(r1);
+    g.c = warp_xor(r2);
+    g.d = warp_xor(r3);
+    return g;
+}
+// g, the same in all lanes, to t strides on in the lane of thread t (t / 32 the same in all
+// lanes): one product per octal digit by the warp together, then every lane its own A^lane
+// g, whose nibbles are the same in all lanes: 64 reads of a kilobyte, eight in flight (a
+// thread's five products of 256 masked columns, one after the other, took 300 us of a call
+// with 1e5 one-loop samples and a third of its batch; the columns of the set bits, twice the
+// bytes, 20 us).
+static __device__ __noinline__ xo start_state(xo g, const u64* __restrict__ mats, u32 t, int digits)
+{
+    u32 w = t >> 5;
+#pragma unroll 1
+    for (int d = 0; d < digits; d++, w >>= 3)
+        if (w & 7u) g = warp_apply(mats + MAT_LANES + (size_t)(d * 7u + (w & 7u) - 1u) * 1024u, g);
+    u64 r0 = 0, r1 = 0, r2 = 0, r3 = 0;
+    const ulonglong2* p = (const ulonglong2*)mats + (t & 31u) * 2u;
+#pragma unroll 1
+    for (int k = 0; k < 8; k++) {
+        const u64 word = k < 2 ? g.a : k < 4 ? g.b : k < 6 ? g.c : g.d;
+        const u32 half = (u32)(k & 1 ? word >> 32 : word);
+        ulonglong2 lo[8], hi[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const ulonglong2* e = p + ((k * 8 + i) * 16 + ((half >> (4 * i)) & 15u)) * 64u;
+            lo[i] = __ldg(e);
+            hi[i] = __ldg(e + 1);
         }
-        if (mine) {
-            g.a = r0;
-            g.b = r1;
-            g.c = r2;
-            g.d = r3;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            r0 ^= lo[i].x;
+            r1 ^= lo[i].y;
+            r2 ^= hi[i].x;
+            r3 ^= hi[i].y;
         }
     }
+    g.a = r0;
+    g.b = r1;
+    g.c = r2;
+    g.d = r3;
+    return g;
 }
 
 // ------------------------------------------------------------------ table staging
@@ -2437,13 +2481,29 @@ static __device__ __forceinline__ void write_counts(double* dst)
     }
 }
 
+// (h, l) += (bh, bl): h the rounded sum, the errors collected in l and not renormalised, so
+// that a chain of additions waits for one FP64 addition per term (the FP64 pipe takes 16
+// cycles per warp instruction)
+static __device__ __forceinline__ void dd_acc(double& h, double& l, double bh, double bl)
+{
+    const double s = h + bh, bb = s - h;
+    l += ((h - (s - bb)) + (bh - bb)) + bl;
+    h = s;
+}
+static __device__ __forceinline__ void dd_norm(double& h, double& l)
+{
+    const double s = h + l;
+    l = l - (s - h);
+    h = s;
+}
 static __device__ __forceinline__ void warp_dd_sum(double& h, double& l)
 {
 #pragma unroll 1
     for (int off = 16; off; off >>= 1) {
         const double oh = __shfl_down_sync(0xffffffffu, h, off), ol = __shfl_down_sync(0xffffffffu, l, off);
-        dd_add(h, l, oh, ol);
+        dd_acc(h, l, oh, ol);
     }
+    dd_norm(h, l);
 }
 
 struct accum {
@@ -2509,7 +2569,7 @@ struct accum {
             for (int t = lane; t < FT_BLOCK; t += 32) {
                 const double sv = ((const double*)base)[s * FT_BLOCK + t];
                 const double cv = ((const double*)base)[(ACC_NS + s) * FT_BLOCK + t];
-                dd_add(h, l, sv, cv);
+                dd_acc(h, l, sv, cv);
             }
             warp_dd_sum(h, l);
             if (lane == 0) {
@@ -2565,20 +2625,70 @@ struct accum {
         }
     }
 
-    // warp-wide
+    // the FP32 value x in units of 2^(emax - 184) (24 bits of significand, 34 below the largest)
+    static __device__ __forceinline__ long long fixed_of(float x, int emax)
+    {
+        const int b = __float_as_int(x), e = (b >> 23) & 255;
+        const long long m = (b & 0x7fffff) | (e ? 0x800000 : 0);
+        const int sh = 34 - emax + (e ? e : 1);
+        const long long v = sh >= 0 ? m << sh : (sh > -32 ? m >> -sh : 0);
+        return b < 0 ? -v : v;
+    }
+    // warp-wide: the warp's FP32 sums into its double-double ones.  The lanes' values are added
+    // as integers, 58 bits below the largest: the FP64 pipe takes 16 cycles of the whole SM
+    // per warp instruction, and a double-double tree over the lanes kept a small launch's
+    // 16 warps at its end for 130 us (11 now).
     __device__ __noinline__ void fold()
     {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll 1
+        for (int s0 = 0; s0 < ACC_NS; s0 += 32) {
+            long long mine = 0;
+            int emine = 0;
+            bool slow = false;
+#pragma unroll 1
+            for (int i = 0; i < 32 && s0 + i < ACC_NS; i++) {
+                const float a = Sf(s0 + i), c = Cf(s0 + i);
+                const u32 ea = ((u32)__float_as_int(a) >> 23) & 255u, ec = ((u32)__float_as_int(c) >> 23) & 255u;
+                const int emax = (int)__reduce_max_sync(0xffffffffu, ea > ec ? ea : ec);
+                if (emax == 255) {
+                    slow = true;   // infinite or NaN sums: below
+                    continue;
+                }
+                long long v = fixed_of(a, emax) - fixed_of(c, emax);
+#pragma unroll
+                for (int off = 16; off; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+                if (lane == i) {
+                    mine = v;
+                    emine = emax;
+                }
+            }
+            if (s0 + lane < ACC_NS) {
+                const double unit = __longlong_as_double((long long)(emine - 184 + 1023) << 52);
+                const double h = (double)mine, l = (double)(mine - (long long)h);
+                double2 w = W(s0 + lane, warp);
+                dd_acc(w.x, w.y, h * unit, l * unit);
+                W(s0 + lane, warp) = w;
+            }
+            __syncwarp();
+#pragma unroll 1
+            for (int i = 0; slow && i < 32 && s0 + i < ACC_NS; i++) {
+                const float a = Sf(s0 + i), c = Cf(s0 + i);
+                if (__any_sync(0xffffffffu, !isfinite(a) || !isfinite(c))) {
+                    double h = (double)a - (double)c, l = 0.0;
+                    warp_dd_sum(h, l);
+                    if (lane == 0) {
+                        double2 w = W(s0 + i, warp);
+                        dd_acc(w.x, w.y, h, l);
+                        W(s0 + i, warp) = w;
+                    }
+                }
+            }
+        }
 #pragma unroll 1
         for (int s = 0; s < ACC_NS; s++) {
-            double h = (double)Sf(s) - (double)Cf(s), l = 0.0;
             Sf(s) = 0.0f;
             Cf(s) = 0.0f;
-            warp_dd_sum(h, l);
-            if ((threadIdx.x & 31) == 0) {
-                double2 w = W(s, threadIdx.x >> 5);
-                dd_add(w.x, w.y, h, l);
-                W(s, threadIdx.x >> 5) = w;
-            }
         }
     }
 
@@ -2594,8 +2704,9 @@ struct accum {
 #pragma unroll 1
             for (int k = 1; k < FT_WARPS; k++) {
                 const double2 v = W(s, k);
-                dd_add(w.x, w.y, v.x, v.y);
+                dd_acc(w.x, w.y, v.x, v.y);
             }
+            dd_norm(w.x, w.y);
             dst[2 * out_pair(s)] = w.x;
             dst[2 * out_pair(s) + 1] = w.y;
         }
@@ -2603,6 +2714,64 @@ struct accum {
     }
 #endif
 };
+
+#if !FT_BATCH
+// The launch's sums, by the block that finishes last: parts [p0, p1) added into out, a warp
+// per slot (the moments in double-double).  `ticket` counts the finished blocks and wraps
+// to zero for the next launch.
+static __device__ __forceinline__ bool last_block(unsigned int* ticket)
+{
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(ticket, gridDim.x - 1u) == gridDim.x - 1u;
+    __syncthreads();
+    __threadfence();
+    return last;
+}
+// unit u of the sums (a moment's pair, or a counter) over n parts, by a warp; in lane 0
+#define FT_UNITS (4 * FT_K + 5)
+static __device__ __noinline__ void sum_unit(int u, const double* parts, unsigned int n, double& h, double& l)
+{
+    const unsigned int lane = threadIdx.x & 31u;
+    const bool pair = u < 4 * FT_K;
+    const double* v = parts + (pair ? 2 * u : 4 * FT_K + u);
+    h = l = 0.0;
+    if (ACC_PARTS == 2 && pair && (u & 2)) return;   // no imaginary parts
+    if (pair) {
+#pragma unroll 4
+        for (unsigned int k = lane; k < n; k += 32u)
+            dd_acc(h, l, __ldcg(v + (size_t)k * ACC_SLOTS), __ldcg(v + (size_t)k * ACC_SLOTS + 1));
+        warp_dd_sum(h, l);
+    } else {   // whole numbers below 2^52: their integers from the bits
+        u64 c = 0;
+        for (unsigned int k = lane; k < n; k += 32u)
+            c += (u64)__double_as_longlong(__ldcg(v + (size_t)k * ACC_SLOTS) + 0x1p52) & 0xfffffffffffffull;
+#pragma unroll
+        for (int off = 16; off; off >>= 1) c += __shfl_down_sync(0xffffffffu, c, off);
+        h = (double)c;
+    }
+}
+static __device__ __forceinline__ void write_unit(int u, double h, double l, double* out)
+{
+    if (u < 4 * FT_K) {
+        out[2 * u] = h;
+        out[2 * u + 1] = l;
+    } else {
+        out[4 * FT_K + u] = h;
+    }
+}
+static __device__ __forceinline__ void sum_parts(const double* parts, unsigned int n, double* out)
+{
+#pragma unroll 1
+    for (int u = threadIdx.x >> 5; u < FT_UNITS; u += FT_WARPS) {
+        double h, l;
+        sum_unit(u, parts, n, h, l);
+        if ((threadIdx.x & 31u) == 0) write_unit(u, h, l, out);
+    }
+    if (threadIdx.x < 3) out[8 * FT_K + 5 + threadIdx.x] = 0.0;
+}
+#endif
 
 template <class T>
 static __device__ __forceinline__ void write_record(u64 i, const unsigned char* ord, const cx<T>* R, bool ok,
@@ -2765,13 +2934,13 @@ static __device__ __forceinline__ void sample_range(xo& g, const table_ref& tr, 
 #if !FT_BATCH
 // ------------------------------------------------------------------ single-integral kernels
 // Thread t of the launch owns samples [t*chunk, min(nsamples, (t+1)*chunk)) counted
-// from the launch's first sample.  warp_states[4w ..] is the stream state of the first
-// sample of warp w's lane 0 (computed by a preparation kernel), so a thread skips only
-// over its lane's offset.  Block b writes its partial sums to acc_out[b * ACC_SLOTS ...].
+// from the launch's first sample, whose stream state is (s0 .. s3).  Block b writes its
+// partial sums to acc_out[b * ACC_SLOTS ...]; the last one to finish adds them into
+// final_out (NULL in the mixed form, whose FP64 pass does it).
 extern "C" __global__ void __launch_bounds__(FT_BLOCK, FT_MINB) ft_sample(
-    const double* __restrict__ prm, const unsigned char* __restrict__ tab, const u64* __restrict__ lanepw,
-    int lanebits, const u64* __restrict__ warp_states, u64 nsamples, u64 chunk, double* __restrict__ acc_out,
-    u64* __restrict__ queue, unsigned int* __restrict__ qcount, unsigned int qcap,
+    const double* __restrict__ prm, const unsigned char* __restrict__ tab, const u64* __restrict__ mats, int digits,
+    u64 s0, u64 s1, u64 s2, u64 s3, u64 nsamples, u64 chunk, double* acc_out, u64* __restrict__ queue,
+    unsigned int* __restrict__ qcount, unsigned int qcap, unsigned int* __restrict__ ticket, double* final_out,
     unsigned char* __restrict__ rec_order, double* __restrict__ rec_X, double* __restrict__ rec_R,
     unsigned char* __restrict__ rec_flags)
 {
@@ -2779,8 +2948,12 @@ extern "C" __global__ void __launch_bounds__(FT_BLOCK, FT_MINB) ft_sample(
     const table_ref tr = stage_table(smem, tab);
 
     const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
-    xo g = load_state(warp_states + (size_t)(t >> 5) * 4);
-    skip_lanes(g, t & 31u, lanepw, lanebits < 5 ? lanebits : 5);
+    xo g;
+    g.a = s0;
+    g.b = s1;
+    g.c = s2;
+    g.d = s3;
+    g = start_state(g, mats, t, digits);
 
     u64 first = (u64)t * chunk;
     u64 last = first + chunk;
@@ -2788,41 +2961,64 @@ extern "C" __global__ void __launch_bounds__(FT_BLOCK, FT_MINB) ft_sample(
 
     accum A;
     A.init(smem + ACC_SMEM_OFFSET);
-    sample_range(g, tr, prm, first, last, chunk, A, smem + LX_SMEM_OFFSET, queue, qcount, qcap, rec_order, rec_X, rec_R, rec_flags);
+    sample_range(g, tr, prm, first, last, chunk, A, smem + LX_SMEM_OFFSET, queue, qcount, qcap, rec_order, rec_X,
+                 rec_R, rec_flags);
     A.finish(acc_out + (size_t)blockIdx.x * ACC_SLOTS, first < last ? last - first : 0);
+    if (final_out && last_block(ticket)) sum_parts(acc_out, gridDim.x, final_out);
 }
 
 #if FT_PREC == 0
-// FP64 pass over the samples a mixed launch queued (grid-stride over the entries).
+// FP64 pass over the samples a mixed launch queued (grid-stride over the entries).  The
+// blocks with entries add their sums after the nparts of the sampling launch in acc_out.
+// Meanwhile the last blocks add those parts (a unit of the sums each, one warp: the FP64
+// pipe is the bound) into the part after all of them, so that the block that finishes last
+// has only this one and the few with entries to add into final_out; it clears the count.
 extern "C" __global__ void __launch_bounds__(FT_BLOCK) ft_sample_queue(
     const double* __restrict__ prm, const unsigned char* __restrict__ tab, const u64* __restrict__ queue,
-    const unsigned int* __restrict__ qcount, unsigned int qcap, double* __restrict__ acc_out,
-    unsigned char* __restrict__ rec_order, double* __restrict__ rec_X, double* __restrict__ rec_R,
-    unsigned char* __restrict__ rec_flags)
+    unsigned int* __restrict__ qcount, unsigned int qcap, double* acc_out, unsigned int nparts,
+    unsigned int* __restrict__ ticket, double* final_out, unsigned char* __restrict__ rec_order,
+    double* __restrict__ rec_X, double* __restrict__ rec_R, unsigned char* __restrict__ rec_flags)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned int n = *qcount;
     if (n > qcap) n = qcap;
-    if ((size_t)blockIdx.x * blockDim.x >= n) {
-        // no entry for this block (the whole block leaves together): zero sums
-        for (int s = threadIdx.x; s < ACC_SLOTS; s += blockDim.x) acc_out[(size_t)blockIdx.x * ACC_SLOTS + s] = 0.0;
-        return;
+    const unsigned int busy = min((n + FT_BLOCK - 1u) / FT_BLOCK, gridDim.x);   // blocks with entries
+    if (blockIdx.x < busy) {
+        const table_ref tr = stage_table(smem, tab);
+        accum A;
+        A.init(smem + ACC_SMEM_OFFSET);
+        u64 owned = 0;
+        for (unsigned int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+            const u64* q = queue + (size_t)k * 5;
+            owned++;
+            xo g;
+            g.a = q[1];
+            g.b = q[2];
+            g.c = q[3];
+            g.d = q[4];
+            sample64(g, tr, prm, q[0], A, REC_QUEUED, rec_order, rec_X, rec_R, rec_flags);
+        }
+        A.finish(acc_out + (size_t)(nparts + 1u + blockIdx.x) * ACC_SLOTS, owned);
     }
-    const table_ref tr = stage_table(smem, tab);
-    accum A;
-    A.init(smem + ACC_SMEM_OFFSET);
-    u64 owned = 0;
-    for (unsigned int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const u64* q = queue + (size_t)k * 5;
-        owned++;
-        xo g;
-        g.a = q[1];
-        g.b = q[2];
-        g.c = q[3];
-        g.d = q[4];
-        sample64(g, tr, prm, q[0], A, REC_QUEUED, rec_order, rec_X, rec_R, rec_flags);
+    // acc_out: [sampling launch's parts][their sum][the busy blocks' parts]
+    if (threadIdx.x < 32) {
+#pragma unroll 1
+        for (int u = gridDim.x - 1u - blockIdx.x; u < FT_UNITS; u += gridDim.x) {
+            double h, l;
+            sum_unit(u, acc_out, nparts, h, l);
+            if (threadIdx.x == 0) write_unit(u, h, l, acc_out + (size_t)nparts * ACC_SLOTS);
+        }
     }
-    A.finish(acc_out + (size_t)blockIdx.x * ACC_SLOTS, owned);
+    if (last_block(ticket)) {
+        const double* rest = acc_out + (size_t)nparts * ACC_SLOTS;
+        if (busy == 0) {
+            for (int s = threadIdx.x; s < ACC_SLOTS; s += FT_BLOCK)
+                final_out[s] = s < 8 * FT_K + 5 ? __ldcg(rest + s) : 0.0;
+        } else {
+            sum_parts(rest, busy + 1u, final_out);
+        }
+        if (threadIdx.x == 0) *qcount = 0u;
+    }
 }
 #endif
 
@@ -2834,9 +3030,11 @@ extern "C" __global__ void __launch_bounds__(FT_BLOCK) ft_sample_queue(
 // (instance i owns items [first_item, first_item + nitems)).  A block takes the next
 // item from a device counter, thread t of the block owns samples
 // [item_base + t*chunk, item_base + (t+1)*chunk) of the instance, and the block writes
-// the item's sums to acc_out[item * ACC_SLOTS ...].  item_state[item] is the stream
-// state of the item's first sample (computed by a preparation kernel); thread t
-// reaches its own first sample with the lane skip matrices (T^(chunk * (2E-1)))^(2^b).
+// the item's sums to acc_out[item * ACC_SLOTS ...].  inst_state[4 i ..] is the stream state
+// of instance i's first sample (computed by a preparation kernel); a warp reaches its item
+// with the powers B^(8^d v) of the item stride B = T^(FT_BLOCK chunk (2E-1)) (1024 words
+// each, v = 1 .. 7 per octal digit d), then its threads with the chunk's matrices
+// (start_state).
 struct batch_inst {
     const double* prm;          // parameter block of the instance (P_SIZE doubles, floats, two-floats)
     const unsigned char* tab;   // J(gamma) table of the instance (global layout)
@@ -2866,7 +3064,7 @@ static __device__ __forceinline__ int find_instance(const batch_inst* __restrict
 
 extern "C" __global__ void __launch_bounds__(FT_BLOCK, FT_MINB) ft_sample_batch(
     const batch_inst* __restrict__ inst, int ninst, const u64* __restrict__ total_items,
-    const u64* __restrict__ item_state, const u64* __restrict__ lanepw, int lanebits, u64 chunk,
+    const u64* __restrict__ inst_state, const u64* __restrict__ item_mats, const u64* __restrict__ mats, u64 chunk,
     unsigned long long* __restrict__ counter, double* __restrict__ acc_out, u64* __restrict__ queue,
     unsigned int* __restrict__ qcount, unsigned int qcap)
 {
@@ -2904,8 +3102,14 @@ extern "C" __global__ void __launch_bounds__(FT_BLOCK, FT_MINB) ft_sample_batch(
         const u64 first = (it - inst[id].first_item) * (u64)FT_BLOCK * chunk + (u64)threadIdx.x * chunk;
         u64 last = first + chunk;
         if (last > n) last = n;
-        xo g = load_state(item_state + it * 4);
-        skip_lanes(g, threadIdx.x, lanepw, lanebits);
+        xo g = load_state(inst_state + (size_t)id * 4);
+        {
+            const u64* M = item_mats;
+#pragma unroll 1
+            for (u64 k = it - inst[id].first_item; k; k >>= 3, M += 7u * 1024u)
+                if (k & 7u) g = warp_apply(M + (size_t)((k & 7u) - 1u) * 1024u, g);
+        }
+        g = start_state(g, mats, threadIdx.x, 2);
         accum A;
         A.init(smem + ACC_SMEM_OFFSET);
         sample_range(g, tr, s_prm, first, last, chunk, A, smem + LX_SMEM_OFFSET, queue, qcount, qcap, nullptr, nullptr,

@@ -67,24 +67,20 @@ struct ft_plan {
     // scratch reused by launches
     double* d_parts = nullptr;
     size_t parts_cap = 0;
-    double* d_final = nullptr;
-    double* h_final = nullptr;
+    double* h_final = nullptr;   // pinned, written by the last block of a launch
     unsigned long long* d_queue = nullptr;
-    unsigned int* d_qcount = nullptr;
+    unsigned int* d_qcount = nullptr;   // hand-offs, finished blocks: both zero between launches
     size_t qcap = 0;
-    // lane skip matrices for the last few per-thread strides S (alternating precisions
-    // or sample counts reuse them): 64 matrices of 8 KB each per entry
-    struct lane_entry {
+    // stride matrices for the last few per-thread strides S (alternating precisions or sample
+    // counts reuse them): 1.3 MB per entry
+    struct stride_entry {
         unsigned long long* d = nullptr;
         unsigned long long S = 0;
-        int bits = 0;
+        int digits = -1, cap = -1;
         unsigned long long used = 0;
     };
-    lane_entry lanes[4];
-    unsigned long long lane_clock = 0;
-    unsigned long long* d_lanepw = nullptr;   // the entry of the current launch
-    unsigned long long* d_warpst = nullptr;   // stream states of the warps of the last launch
-    size_t warpst_cap = 0;
+    stride_entry strides[4];
+    unsigned long long stride_clock = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::mutex mu;
@@ -125,13 +121,11 @@ struct ft_plan {
         if (d_prm) cudaFree(d_prm);
         if (d_tab) cudaFree(d_tab);
         if (d_parts) cudaFree(d_parts);
-        if (d_final) cudaFree(d_final);
         if (h_final) cudaFreeHost(h_final);
         if (d_queue) cudaFree(d_queue);
         if (d_qcount) cudaFree(d_qcount);
-        for (lane_entry& e : lanes)
+        for (stride_entry& e : strides)
             if (e.d) cudaFree(e.d);
-        if (d_warpst) cudaFree(d_warpst);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
         if (stream) cudaStreamDestroy(stream);

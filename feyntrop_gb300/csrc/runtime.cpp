@@ -3,11 +3,11 @@
 // A plan holds one integral: the host preprocessing result, its parameter block
 // and J(gamma) table in device memory, and the scratch its launches reuse.  An
 // integration is
-//   1. skip matrices for the launch's lane stride (cached per stride),
+//   1. skip matrices for the launch's stride (cached per stride),
 //   2. the sampling kernel (one thread per contiguous block of samples),
 //   3. in mixed precision, the FP64 pass over the samples the FP32 kernel queued,
-//   4. the reduction of the per-block partial moments and one 512-byte copy back,
-// all on one stream.
+// all on one stream; the last launch's last block adds the blocks' sums into pinned host
+// memory.
 #include <cuda_runtime.h>
 
 #include <chrono>
@@ -279,9 +279,9 @@ void upload(ft_plan& pl)
     cu(cudaStreamCreateWithFlags(&pl.stream, cudaStreamNonBlocking), "cudaStreamCreate");
     cu(cudaEventCreate(&pl.ev0), "cudaEventCreate");
     cu(cudaEventCreate(&pl.ev1), "cudaEventCreate");
-    cu(cudaMalloc(&pl.d_final, pl.slots() * 8), "cudaMalloc(final)");
     cu(cudaMallocHost(&pl.h_final, pl.slots() * 8), "cudaMallocHost(final)");
     cu(cudaMalloc(&pl.d_qcount, 16), "cudaMalloc(queue count)");
+    cu(cudaMemset(pl.d_qcount, 0, 16), "cudaMemset(queue count)");
 }
 
 void ensure_parts(ft_plan& pl, size_t nparts)
@@ -303,37 +303,33 @@ void ensure_queue(ft_plan& pl, size_t entries)
     pl.qcap = entries;
 }
 
-void ensure_warpst(ft_plan& pl, size_t nwarps)
+// the stride's matrices; *made is set when they had to be computed (one launch)
+const unsigned long long* stride_matrices(ft_plan& pl, unsigned long long S, int digits, cudaStream_t st, bool* made)
 {
-    if (nwarps <= pl.warpst_cap) return;
-    if (pl.d_warpst) cudaFree(pl.d_warpst);
-    pl.d_warpst = nullptr;
-    pl.warpst_cap = 0;
-    cu(cudaMalloc(&pl.d_warpst, nwarps * 32), "cudaMalloc(warp stream states)");
-    pl.warpst_cap = nwarps;
-}
-
-// points pl.d_lanepw at the lane skip matrices (T^S)^(2^b), b < bits; returns true when
-// it had to compute them (one launch), false when a cached entry served
-bool ensure_lanepw(ft_plan& pl, unsigned long long S, int bits, cudaStream_t st)
-{
-    pl.lane_clock++;
-    ft_plan::lane_entry* victim = &pl.lanes[0];
-    for (ft_plan::lane_entry& e : pl.lanes) {
-        if (e.d && e.S == S && e.bits >= bits) {
-            e.used = pl.lane_clock;
-            pl.d_lanepw = e.d;
-            return false;
+    pl.stride_clock++;
+    ft_plan::stride_entry* victim = &pl.strides[0];
+    for (ft_plan::stride_entry& e : pl.strides) {
+        if (e.d && e.S == S && e.digits >= digits) {
+            e.used = pl.stride_clock;
+            *made = false;
+            return e.d;
         }
         if (e.used < victim->used) victim = &e;
     }
-    if (!victim->d) cu(cudaMalloc(&victim->d, (size_t)64 * 1024 * 8), "cudaMalloc(lane skip matrices)");
-    cu(ft::launch_lane_powers(dev_state().tpow, S, bits, victim->d, st), "lane skip matrices");
+    victim->digits = -1;
+    if (victim->cap < digits) {
+        if (victim->d) cudaFree(victim->d);
+        victim->d = nullptr;
+        victim->cap = -1;
+        cu(cudaMalloc(&victim->d, ft::stride_words(digits) * 8), "cudaMalloc(stride matrices)");
+        victim->cap = digits;
+    }
+    cu(ft::launch_stride_matrices(dev_state().tpow, S, digits, victim->d, st), "stride matrices");
     victim->S = S;
-    victim->bits = bits;
-    victim->used = pl.lane_clock;
-    pl.d_lanepw = victim->d;
-    return true;
+    victim->digits = digits;
+    victim->used = pl.stride_clock;
+    *made = true;
+    return victim->d;
 }
 
 struct launch_geometry {
@@ -402,32 +398,25 @@ run_out run(ft_plan& pl, const ft_run_options& o, cudaStream_t st, const records
     out.acc.assign(pl.slots(), 0.0);
     if (N == 0) return out;
 
-    if (ensure_lanepw(pl, g.chunk * draws, g.lanebits, st)) out.launches++;
+    bool made = false;
+    int digits = ft::stride_digits(g.lanebits);
+    const unsigned long long* mats = stride_matrices(pl, g.chunk * draws, digits, st, &made);
+    if (made) out.launches++;
     const unsigned qblocks = prec ? (unsigned)(dev_state().sms * std::max(1, k64->queue_blocks_per_sm)) : 0;
-    ensure_parts(pl, g.blocks + qblocks);
+    ensure_parts(pl, g.blocks + qblocks + 1);
     if (prec) {
         size_t want = (size_t)std::min<unsigned long long>(N, N / 16 + 65536);
         ensure_queue(pl, want);
     }
-    cu(cudaMemsetAsync(pl.d_qcount, 0, 16, st), "cudaMemsetAsync");
-    const ft::xstate base = ft::advance(ft::seed_state(o.seed), o.first_sample * draws);
-
-    const unsigned nwarps = (unsigned)(((unsigned long long)g.blocks * ks.block + 31) / 32);
-    ensure_warpst(pl, nwarps);
+    ft::xstate base = ft::advance(ft::seed_state(o.seed), o.first_sample * draws);
     cu(cudaEventRecord(pl.ev0, st), "cudaEventRecord");
-    cu(ft::launch_warp_states(pl.d_lanepw, g.lanebits, (const unsigned long long*)base.s, nwarps, pl.d_warpst, st),
-       "warp stream states");
-    out.launches++;
-    const unsigned long long* warpst = pl.d_warpst;
     unsigned long long nsamples = N, chunk = g.chunk;
-    int lanebits = g.lanebits;
     unsigned int qcap = (unsigned int)pl.qcap;
     unsigned long long* queue = pl.d_queue;
-    unsigned int* qcount = pl.d_qcount;
-    double* parts = pl.d_parts;
+    unsigned int *qcount = pl.d_qcount, *ticket = pl.d_qcount + 1;
+    double *parts = pl.d_parts, *final_out = pl.h_final, *none = nullptr;
     const double* prm = pl.d_prm;
     const unsigned char* tab = pl.d_tab;
-    const unsigned long long* lanepw = pl.d_lanepw;
     uint8_t* r_order = nullptr;
     double* r_X = nullptr;
     double* r_R = nullptr;
@@ -438,39 +427,33 @@ run_out run(ft_plan& pl, const ft_run_options& o, cudaStream_t st, const records
         r_R = rec->R;
         r_flags = rec->flags;
     }
-    void* args[] = {&prm, &tab, &lanepw, &lanebits, &warpst, &nsamples, &chunk, &parts, &queue, &qcount,
-                    &qcap, &r_order, &r_X, &r_R, &r_flags};
+    void* args[] = {&prm, &tab, &mats, &digits, &base.s[0], &base.s[1], &base.s[2], &base.s[3], &nsamples, &chunk,
+                    &parts, &queue, &qcount, &qcap, &ticket, prec ? &none : &final_out, &r_order, &r_X, &r_R, &r_flags};
     ft::check(ft::drv().LaunchKernel(ks.sample, g.blocks, 1, 1, ks.block, 1, 1, ks.smem, (CUstream)st, args, nullptr),
               "launch ft_sample");
     out.launches++;
     if (prec) {
-        double* qparts = pl.d_parts + (size_t)g.blocks * pl.slots();
-        const unsigned long long* cq = pl.d_queue;
-        const unsigned int* cqc = pl.d_qcount;
-        void* qargs[] = {&prm, &tab, &cq, &cqc, &qcap, &qparts, &r_order, &r_X, &r_R, &r_flags};
+        unsigned int nparts = g.blocks;
+        void* qargs[] = {&prm, &tab, &queue, &qcount, &qcap, &parts, &nparts, &ticket, &final_out,
+                         &r_order, &r_X, &r_R, &r_flags};
         ft::check(ft::drv().LaunchKernel(k64->queue, qblocks, 1, 1, k64->block, 1, 1, k64->smem, (CUstream)st, qargs,
                                          nullptr),
                   "launch ft_sample_queue");
         out.launches++;
     }
     cu(cudaEventRecord(pl.ev1, st), "cudaEventRecord");
-    cu(ft::launch_finalize(pl.d_parts, (int)(g.blocks + qblocks), pl.slots(), 8 * pl.P.K, pl.d_final, st),
-       "finalize");
-    out.launches++;
-    cu(cudaMemcpyAsync(pl.h_final, pl.d_final, pl.slots() * 8, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
-    unsigned int qc_host = 0;
-    if (prec) cu(cudaMemcpyAsync(&qc_host, pl.d_qcount, 4, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
     cu(cudaStreamSynchronize(st), "sampling");
     float ms = 0;
     cu(cudaEventElapsedTime(&ms, pl.ev0, pl.ev1), "cudaEventElapsedTime");
     out.kernel_ms = ms;
     out.acc.assign(pl.h_final, pl.h_final + pl.slots());
-    if (prec && qc_host > pl.qcap) {
+    const unsigned long long queued = (unsigned long long)out.acc[8 * pl.P.K + 2];
+    if (prec && queued > pl.qcap) {
         // more samples needed FP64 than the queue holds: redo the whole range in FP64
         ft_run_options o64 = o;
         o64.precision = FT_PRECISION_FP64;
         run_out r = run(pl, o64, st, rec);
-        r.acc[8 * pl.P.K + 2] = qc_host;
+        r.acc[8 * pl.P.K + 2] = (double)queued;
         r.launches += out.launches;
         r.kernel_ms += out.kernel_ms;
         return r;
@@ -797,49 +780,44 @@ int ft_integrate_noalloc(ft_plan* pl, const ft_run_options* o, double* d_slots)
         const unsigned qblocks = prec ? (unsigned)(dev_state().sms * std::max(1, k64->queue_blocks_per_sm)) : 0;
         // ft_integrate's launch shape, its waves capped to the blocks the scratch holds
         const launch_geometry g =
-            geometry(*ks, N, qblocks < NOALLOC_MAX_BLOCKS ? (unsigned long long)(NOALLOC_MAX_BLOCKS - qblocks) : 1ull);
+            geometry(*ks, N,
+                     qblocks < NOALLOC_MAX_BLOCKS ? (unsigned long long)(NOALLOC_MAX_BLOCKS - qblocks) : 1ull);
         if (g.blocks + qblocks > NOALLOC_MAX_BLOCKS || g.lanebits > NOALLOC_MAX_LANE_BITS)
             throw std::invalid_argument("ft_integrate_noalloc: launch exceeds the static scratch (2048 blocks)");
         ft::noalloc_layout sc;
         cu(ft::noalloc_scratch(&sc), "cudaGetSymbolAddress(no-allocation scratch)");
         cudaStream_t st = o->stream ? (cudaStream_t)o->stream : pl->stream;
         const unsigned long long draws = 2ULL * pl->P.E - 1;
-        cu(ft::launch_lane_powers(dev_state().tpow, g.chunk * draws, g.lanebits, sc.lanepw, st), "lane skip matrices");
-        cu(cudaMemsetAsync(sc.qcount, 0, 8, st), "cudaMemsetAsync");
-        const ft::xstate base = ft::advance(ft::seed_state(o->seed), o->first_sample * draws);
-        const unsigned nwarps = (unsigned)(((unsigned long long)g.blocks * ks->block + 31) / 32);
-        cu(ft::launch_warp_states(sc.lanepw, g.lanebits, (const unsigned long long*)base.s, nwarps, sc.warpst, st),
-           "warp stream states");
-        const unsigned long long* warpst = sc.warpst;
+        int digits = ft::stride_digits(g.lanebits);
+        cu(ft::launch_stride_matrices(dev_state().tpow, g.chunk * draws, digits, sc.mats, st), "stride matrices");
+        cu(cudaMemsetAsync(sc.qcount, 0, 8, st), "cudaMemsetAsync");   // hand-offs and ticket
+        ft::xstate base = ft::advance(ft::seed_state(o->seed), o->first_sample * draws);
         unsigned long long nsamples = N, chunk = g.chunk;
-        int lanebits = g.lanebits;
         unsigned int qcap = NOALLOC_QUEUE_ENTRIES;
         unsigned long long* queue = sc.queue;
-        unsigned int* qcount = sc.qcount;
-        double* parts = sc.parts;
+        unsigned int *qcount = sc.qcount, *ticket = sc.ticket;
+        double *parts = sc.parts, *none = nullptr;
         const double* prm = pl->d_prm;
         const unsigned char* tab = pl->d_tab;
-        const unsigned long long* lanepw = sc.lanepw;
+        const unsigned long long* mats = sc.mats;
         uint8_t* r_order = nullptr;
         double* r_X = nullptr;
         double* r_R = nullptr;
         uint8_t* r_flags = nullptr;
-        void* args[] = {&prm, &tab, &lanepw, &lanebits, &warpst, &nsamples, &chunk, &parts, &queue, &qcount,
-                        &qcap, &r_order, &r_X, &r_R, &r_flags};
+        void* args[] = {&prm, &tab, &mats, &digits, &base.s[0], &base.s[1], &base.s[2], &base.s[3], &nsamples,
+                        &chunk, &parts, &queue, &qcount, &qcap, &ticket, prec ? &none : &d_slots, &r_order, &r_X,
+                        &r_R, &r_flags};
         ft::check(ft::drv().LaunchKernel(ks->sample, g.blocks, 1, 1, ks->block, 1, 1, ks->smem, (CUstream)st, args,
                                          nullptr),
                   "launch ft_sample");
         if (prec) {
-            double* qparts = sc.parts + (size_t)g.blocks * pl->slots();
-            const unsigned long long* cq = sc.queue;
-            const unsigned int* cqc = sc.qcount;
-            void* qargs[] = {&prm, &tab, &cq, &cqc, &qcap, &qparts, &r_order, &r_X, &r_R, &r_flags};
+            unsigned int nparts = g.blocks;
+            void* qargs[] = {&prm, &tab, &queue, &qcount, &qcap, &parts, &nparts, &ticket, &d_slots,
+                             &r_order, &r_X, &r_R, &r_flags};
             ft::check(ft::drv().LaunchKernel(k64->queue, qblocks, 1, 1, k64->block, 1, 1, k64->smem, (CUstream)st,
                                              qargs, nullptr),
                       "launch ft_sample_queue");
         }
-        cu(ft::launch_finalize(sc.parts, (int)(g.blocks + qblocks), pl->slots(), 8 * pl->P.K, d_slots, st),
-           "finalize");
         return FT_OK;
     } catch (...) {
         return status_of(std::current_exception());
