@@ -51,6 +51,7 @@ unsigned table_smem_bytes(const kernel_key& k)
 // (FP32 values written exactly as hexadecimal literals):
 //   FT_LOGTAB[i] = r_i = fl(1 / (1 + (i + 1/2)/64)), -log(r_i) as hi, lo, 0 (i < 64)
 //   FT_EXPTAB[j] = 2^(j/32) as hi, lo (j < 32)
+//   FT_ATANTAB[i] = atan(i/64) as hi, lo (i <= 64; 128 entries, as its index is masked)
 //   FT_SCTAB[j] = sin(j pi/64) as hi, lo, cos(j pi/64) as hi, lo (j < 128)
 static std::string tables_source()
 {
@@ -72,6 +73,17 @@ static std::string tables_source()
         s << "};\n__device__ const float2 FT_EXPTAB[32] = {";
         for (int j = 0; j < 32; j++) {
             const double t = std::exp2(j / 32.0);
+            const float hi = (float)t, lo = (float)(t - (double)hi);
+            s << "{";
+            for (float v : {hi, lo}) {
+                std::snprintf(buf, sizeof buf, "%af,", (double)v);
+                s << buf;
+            }
+            s << "},";
+        }
+        s << "};\n__device__ const float2 FT_ATANTAB[128] = {";
+        for (int i = 0; i < 128; i++) {
+            const double t = std::atan(i / 64.0);
             const float hi = (float)t, lo = (float)(t - (double)hi);
             s << "{";
             for (float v : {hi, lo}) {

@@ -1271,7 +1271,7 @@ static __device__ __noinline__ int exact_step(xo g, int back, u32 sub, const uns
 
 // The thread's scratch in shared memory, [slot][thread]: log X of edge e (part 0 hi, 1 lo),
 // later overwritten by 1/X; with FT_SCRATCH 1 also the deformation angles, with 2 the
-// upper triangle of X^1/2 H X^1/2: values that live across the long blocks of the
+// upper triangle of kappa D H D: values that live across the long blocks of the
 // deformed integrand and would otherwise be spilled to local memory, whose frames (256
 // threads of 2 KB on every SM) are read back from L2.
 #if FT_MODE == 0
@@ -1720,24 +1720,52 @@ static __device__ __forceinline__ void expi_pair(df x, cdf* out)
 // |theta| beyond which expi_pair's reduction is not used (the FP64 pass takes the sample)
 #define THETA_MAX 1e5f
 
-// Principal argument of x + i y in two-float to about 1.5e-7 absolute: atanf of the
-// ratio of the smaller to the larger part (a result in [0, pi/4], where an ulp is
-// 6e-8), the octant restored with multiples of pi/2 in two-float, plus the first-order
-// effect of the low parts, (x dy - y dx) / |z|^2.  Zero gives 0.
+// Principal argument of (x + xl) + i (y + yl) to about 1e-9: with a, b the larger and smaller
+// modulus and c = i/64 their rounded ratio, atan(b/a) = atan c + atan z, z = (b - c a) /
+// (a + c b) below 1/128, the first from FT_ATANTAB as two floats; then the octant.  (atanf of
+// the rounded ratio kept 1.5e-7, which D/2 and W multiply.)  Zero gives 0.
 static __device__ FT_BIGFN sf arg_f2(float x, float y, float xl, float yl)
 {
-    const float PIO2_HI = 1.57079637f, PIO2_LO = -4.37113883e-8f;
     const float ax = fabsf(x), ay = fabsf(y);
-    const bool sw = ay > ax;
-    const float num = sw ? ax : ay, den = sw ? ay : ax;
-    // the ratio through the correctly rounded reciprocal (within 1.5 ulp of num / den)
-    const float a = den > 0.0f ? m_atan(num * rcp_(den)) : 0.0f;
-    sf r = sw ? tf_add(tf_mk(PIO2_HI, PIO2_LO), tf_mk(-a, 0.0f)) : tf_mk(a, 0.0f);
-    if (x < 0.0f) r = tf_add(tf_mk(2.0f * PIO2_HI, 2.0f * PIO2_LO), tf_neg(r));
-    if (y < 0.0f) r = tf_neg(r);
-    const float n2 = fmaf(x, x, y * y);
-    return n2 > 0.0f ? tf_add(r, tf_mk((x * yl - y * xl) * rcp_(n2), 0.0f)) : r;
+    const float bxl = x < 0.0f ? -xl : xl, byl = y < 0.0f ? -yl : yl;
+    const bool sw = ay > ax, left = x < 0.0f;
+    const float a = sw ? ay : ax, b = sw ? ax : ay, al = sw ? byl : bxl, bl = sw ? bxl : byl;
+    const float ib = fmaf(b * rcp_fast(a), 64.0f, 12582912.0f);   // i in the low bits
+    const float c = (ib - 12582912.0f) * 0.015625f;
+    const float num = fmaf(-c, a, b) + fmaf(-c, al, bl);
+    const float z = num * rcp_newton(fmaf(c, b, a));
+    const float2 T = FT_ATANTAB[__float_as_int(ib) & 127];
+    sf v = fast_two_sum(T.x, z);
+    v.lo += fmaf(z * z * z, -0.333333343f, T.y);
+    // K +- v, K = 0, pi/2 or pi
+    if (sw != left) v = tf_neg(v);
+    const float K = sw ? 1.57079637f : (left ? 3.14159274f : 0.0f);
+    const float Kl = sw ? -4.37113883e-8f : (left ? -8.74227766e-8f : 0.0f);
+    v = tf_add(tf_mk(K, Kl), v);
+    if (!(a > 0.0f)) v = tf_zero<float>();
+    return y < 0.0f ? tf_neg(v) : v;
 }
+// log of a positive two-float x in two-float, to about 1e-9 (tables and steps of log1m_pair)
+static __device__ FT_BIGFN sf log_tf(sf x)
+{
+    const int bits = __float_as_int(x.hi);
+    const int e = (bits >> 23) - 127;
+    const float sc = __int_as_float((127 - e) << 23);   // 2^-e
+    const float4 T = FT_LOGTAB[(bits >> 17) & 63];
+    const float z = fmaf(x.hi * sc, T.x, -1.0f) + x.lo * sc * T.x;
+    const float kk = (float)e;
+    const sf s = two_sum(kk * 0.693145751953125f, T.y);
+    const sf t = two_sum(s.hi, z);
+    const float tail = z * z * fmaf(z, fmaf(z, fmaf(z, 0.2f, -0.25f), 0.333333343f), -0.5f);
+    return fast_two_sum(t.hi, (t.lo + s.lo) + (fmaf(kk, 1.428606765330187e-06f, T.z) + tail));
+}
+static __device__ __forceinline__ sf times_ln2(int k)
+{
+    const float f = (float)k;
+    return fast_two_sum(f * 0.693145751953125f, f * 1.428606765330187e-06f);
+}
+// |z|^2 in two-float
+static __device__ __forceinline__ sf norm2(cdf z) { return tf_norm(dot_add_n(z.re, z.re, z.im, z.im)); }
 static __device__ __forceinline__ sf arg_of(cdf z) { return arg_f2(z.re.hi, z.im.hi, z.re.lo, z.im.lo); }
 // principal argument reduced to (-pi, pi] in two-float
 static __device__ __forceinline__ sf wrap_pi(sf x)
@@ -1776,7 +1804,7 @@ struct cblock {
 };
 static __device__ __forceinline__ float cmag_hi(const cdf& z) { return abs_(z.re.hi) + abs_(z.im.hi); }
 
-// the deformation angles and the upper triangle of X^1/2 H X^1/2, in the scratch or not
+// the deformation angles and the upper triangle of kappa D H D, in the scratch or not
 struct angles {
 #if FT_SCRATCH >= 1
     __device__ __forceinline__ void set(unsigned char* lxs, int e, sf v)
@@ -1802,6 +1830,9 @@ struct hessian {
 #endif
 };
 #define XI(e) tf_mk(LX(e, 0), LX(e, 1))
+// D, a power of two with D^2 / X in [1, 4), from 1/X
+static __device__ __forceinline__ int edge_exp(float xi) { return -((((__float_as_int(xi) >> 23) & 255) - 127) >> 1); }
+static __device__ __forceinline__ float edge_scale(float xi) { return __int_as_float((edge_exp(xi) + 127) << 23); }
 
 // The deformed Laplacian at the sample (srcs/feynman_integral.hpp:293-310) and V there
 // (:322-336) in two-float complex arithmetic, for every deformed sample: in FP32 both
@@ -1947,7 +1978,10 @@ static __device__ __forceinline__ void complex_block(unsigned char* lxs, const a
 // conductance-form elimination (all operations on positive values), G = L^-1, the
 // potentials h_r = G q_r and their drops across the edges, the effective-resistance
 // combinations t, and the Minkowski products s.  Reads 1/X from the scratch; outputs theta
-// and the upper triangle of X^1/2 H X^1/2 in FP32.
+// and the upper triangle of kappa D H D in FP32, D ~ X^1/2 a power of two per edge: with
+// hb = D / X^2 h . b_e and s_ab = -2 kappa sum_r sigma_r hb_a hb_b its entries are s_ab t_ab
+// (the diagonal s_aa (t_aa - X_a)), two roundings each, and theta_a = kappa m2_a + s_aa X_a^2 /
+// (2 D_a^2).
 static __device__ __forceinline__ void derivatives(unsigned char* lxs, const float4* pp, angles& th, hessian& H,
                                                         bool& cancel)
 {
@@ -2051,10 +2085,18 @@ static __device__ __forceinline__ void derivatives(unsigned char* lxs, const flo
 #pragma unroll
         for (int e = 0; e < FT_E; e++) {
             const int k = FT_EK[e], l = FT_EL[e];
-            hb[r][e] = (k == FT_V - 1) ? tf_norm(tf_neg(h[l])) : tf_sub(h[k], h[l]);
+            const sf xi = XI(e), xa = tf_mul(xi, xi);
+            const float D = edge_scale(xi.hi);
+            hb[r][e] = tf_mul((k == FT_V - 1) ? tf_norm(tf_neg(h[l])) : tf_sub(h[k], h[l]), tf_mk(xa.hi * D, xa.lo * D));
         }
     }
     const sf kappa = prm_sf(pp, P_DEF);
+    sf ks[FT_RANK];   // -2 kappa sigma
+#pragma unroll
+    for (int r = 0; r < FT_RANK; r++) {
+        ks[r] = tf_mul(prm_sf(pp, P_SIG + r), kappa);
+        ks[r] = tf_mk(-2.0f * ks[r].hi, -2.0f * ks[r].lo);
+    }
 #pragma unroll
     for (int a2 = 0; a2 < FT_E; a2++) {
         const int ka = FT_EK[a2], la = FT_EL[a2];
@@ -2073,7 +2115,7 @@ static __device__ __forceinline__ void derivatives(unsigned char* lxs, const flo
         sf s = tf_zero<float>();
 #pragma unroll
         for (int r = 0; r < FT_RANK; r++) {
-            sig_hb[r] = tf_mul(prm_sf(pp, P_SIG + r), hb[r][a2]);
+            sig_hb[r] = tf_mul(ks[r], hb[r][a2]);
             s = r == 0 ? tf_mul(sig_hb[r], hb[r][a2]) : tf_fma_n(sig_hb[r], hb[r][a2], s);
         }
         if (FT_RANK > 1) s = tf_norm(s);
@@ -2082,16 +2124,11 @@ static __device__ __forceinline__ void derivatives(unsigned char* lxs, const flo
         if (ka != FT_V - 1) {
             cancel |= !(t.hi > 1e-7f * (G[ka][ka].hi + G[la][la].hi));
         }
-        const sf xi = XI(a2);
-        const sf xa = tf_mul(xi, xi);
-        const sf xas = tf_mul(xa, s);
-        th.set(lxs, a2, tf_mul(tf_sub(prm_sf(pp, P_M2 + a2), xas), kappa));
-        const float sxa = rsqrt_newton(xi.hi);   // X^1/2
-        // 2 xa s (1/x - xa t), times x
-        H.set(lxs, a2, a2, 2.0f * tf_f(tf_mul(xas, tf_sub(xi, tf_mul(xa, t)))) * (sxa * sxa));
-        // the off-diagonal entries are FP32 products of their (two-float) factors;
-        // X^-3/2 of an edge scales its row and column
-        const float xaf = -2.0f * tf_f(xa) * sxa;
+        const sf xi = XI(a2), x = tf_inv(xi);
+        const float D = edge_scale(xi.hi), iD2 = 0.5f / (D * D);   // powers of two
+        const sf q = tf_mul(s, tf_mul(x, x));
+        th.set(lxs, a2, tf_add(tf_mul(kappa, prm_sf(pp, P_M2 + a2)), tf_mk(q.hi * iD2, q.lo * iD2)));
+        H.set(lxs, a2, a2, tf_f(tf_mul(s, tf_sub(t, x))));
 #pragma unroll
         for (int b = a2 + 1; b < FT_E; b++) {
             const int kb = FT_EK[b], lb = FT_EL[b];
@@ -2099,8 +2136,7 @@ static __device__ __forceinline__ void derivatives(unsigned char* lxs, const flo
 #pragma unroll
             for (int r = 0; r < FT_RANK; r++)
                 s2 = r == 0 ? tf_mul(sig_hb[r], hb[r][b]) : tf_fma_n(sig_hb[r], hb[r][b], s2);
-            const float xb = LX(b, 0);
-            H.set(lxs, a2, b, xaf * (xb * xb * rsqrt_newton(xb)) * tf_f(s2) * tf_f(wd(kb, lb)));
+            H.set(lxs, a2, b, tf_f(s2) * tf_f(wd(kb, lb)));
         }
     }
 }
@@ -2146,17 +2182,23 @@ static __device__ __forceinline__ bool integrand_one(const float4* pp, const flo
     {
         hessian H;
         derivatives(lxs, pp, th, H, bad);
-        // det(I + i kappa X^1/2 H X^1/2) (similar to I + i kappa H X, srcs/feynman_integral.hpp:312-320):
-        // the real part is the identity, so the symmetric elimination needs no pivoting (every
-        // pivot's real part is at least 1); FP32, the pivots' product rescaled by powers of two
-        // (det J = pj 2^pe).  Before the complex block, so that H is no longer live there.
-        const float kappa = pf[P_DEF];
+        // det(I + i kappa H X) = det(D^2/X + i kappa D H D) prod X/D^2 (srcs/feynman_integral.hpp:312-320):
+        // the real part is diagonal and at least 1, so the symmetric elimination needs no
+        // pivoting (no pivot's real part falls below); FP32, the pivots' product rescaled by powers
+        // of two (pj 2^pe).  Before the complex block, so that H is no longer live there.
         cx<float> J[FT_E][FT_E];
 #pragma unroll
         for (int a = 0; a < FT_E; a++)
 #pragma unroll
-            for (int b = a; b < FT_E; b++) J[a][b] = cmk(a == b ? 1.0f : 0.0f, kappa * H.get(lxs, a, b));
+            for (int b = a; b < FT_E; b++) J[a][b] = cmk(0.0f, H.get(lxs, a, b));
         bool ok = true;
+#pragma unroll
+        for (int e = 0; e < FT_E; e++) {
+            const sf xi = XI(e);
+            const int ex = edge_exp(xi.hi);
+            J[e][e].re = tf_f(xi) * __int_as_float((2 * ex + 127) << 23);
+            pe -= 2 * ex;   // prod X is taken with its logarithm
+        }
 #pragma unroll
         for (int k = 0; k < FT_E; k++) {
             const cx<float> piv = J[k][k];
@@ -2205,8 +2247,8 @@ static __device__ __forceinline__ bool integrand_one(const float4* pp, const flo
     cdf_renorm(Vn, ve, ok);
     if (!ok || ve > 126) return false;
     const float vsc = __int_as_float((127 - ve) << 23);   // 2^-ve
-    const float vn2 = fmaf(Vn.re.hi, Vn.re.hi, Vn.im.hi * Vn.im.hi);
-    const float vm = sqrtf(vn2);
+    const sf vn2 = norm2(Vn);
+    const float vm = sqrtf(vn2.hi);
     // V in two-float keeps ~1e-14 of its terms' magnitudes (and ~1e-12 from the sector
     // point and contour it is built from): samples where V cancels to below 1e-6 of its
     // terms, or where W qmag / |V| exceeds 1e5, go to the FP64 pass
@@ -2215,36 +2257,42 @@ static __device__ __forceinline__ bool integrand_one(const float4* pp, const flo
     const sf av2 = arg_of(Vn);
     const float av = tf_f(av2);
     // arg cPsi = sum theta + arg det L(y), reduced to the principal branch in two-float
-    const float dn2 = fmaf(cb.det.re.hi, cb.det.re.hi, cb.det.im.hi * cb.det.im.hi);
     const sf apsi2 = wrap_pi(tf_add(thsum, arg_of(cb.det)));
     const float apsi = tf_f(apsi2);
     if (fabsf(av) > 3.14158265f || fabsf(apsi) > 3.14158265f) return false;
-    // log2 |cPsi| and log2 |V| (exponents exact, small parts in FP32), then
-    // log2 |cR / IGtr| = -D/2 log2(|cPsi| / psi_tr) - W log2(|V| / V_tr) + log2 |det J|
-    const sf l2psi = tf_norm(tf_addf_n(tf_addf_n(tf_log2e(sumlx), (float)cb.e), 0.5f * m_log2(dn2)));
-    const sf l2v = fast_two_sum((float)ve, 0.5f * m_log2(vn2));
-    const sf lpsi = tf_sub(l2psi, tf_log2e(lFs));
-    const sf lv = tf_sub(l2v, tf_log2e(lGs));
-    sf t = tf_add_n(tf_mulf(lpsi, -D2), tf_mulf(lv, -W));
-    t = tf_norm(tf_addf_n(tf_addf_n(t, (float)pe), 0.5f * m_log2(fmaf(pj.re, pj.re, pj.im * pj.im))));
+    // log |cPsi| and log |V|, then
+    // log |cR / IGtr| = -D/2 log(|cPsi| / psi_tr) - W log(|V| / V_tr) + log |det J|
+    auto half = [](sf a) -> sf { return tf_mk(0.5f * a.hi, 0.5f * a.lo); };
+    const sf lpsi = tf_add(tf_add_n(sumlx, times_ln2(cb.e)), half(log_tf(norm2(cb.det))));
+    const sf lv = tf_add(times_ln2(ve), half(log_tf(vn2)));
+    const float pn = pj.re * pj.re;
+    const sf pn2 = tf_mk(fmaf(pj.im, pj.im, pn), fmaf(pj.re, pj.re, -pn));
+    sf t = tf_add_n(tf_mulf(tf_sub(lpsi, lFs), -D2), tf_mulf(tf_sub(lv, lGs), -W));
+    t = tf_add_n(t, tf_add_n(tf_add_n(sumlx, times_ln2(pe)), half(log_tf(tf_norm(pn2)))));
+    t = tf_norm(t);
     // arg cR = -D/2 arg cPsi + arg det J + nu . theta - W arg V (two-float sum)
     const sf aj = arg_f2(pj.re, pj.im, 0.0f, 0.0f);
     const sf ang = tf_norm(tf_add_n(tf_add_n(tf_mulf(apsi2, -D2), xnu), tf_add_n(aj, tf_mulf(av2, -W))));
     float sn, cs;
     m_sincos(ang.hi, &sn, &cs);
     const float c2 = fmaf(-ang.lo, sn, cs), s2 = fmaf(ang.lo, cs, sn);
-    const float mod = m_exp2(t.hi) * (1.0f + t.lo * LN2_F);
+    const float mod = m_exp(t.hi) * (1.0f + t.lo);
     if (!isfinite(mod)) return false;
-    cx<float> c = cmk(IGtr * mod * c2, IGtr * mod * s2);
+    const sf ig = prm_sf(pp, P_IGTR);
+    const float im = fmaf(mod, ig.hi, mod * ig.lo);
+    const cx<float> c = cmk(im * c2, im * s2);
     out[0] = c;
     if (FT_K > 1) {
-        // log cPsi - L log V (srcs/feynman_integral.hpp:336-341): the large parts in two-float
-        const float er = LN2_F * tf_f(tf_add(l2psi, tf_mulf(l2v, -(float)FT_LOOPS)));
-        const float ei = apsi - (float)FT_LOOPS * av;
+        // orders j: c ef^j / j!, ef = log cPsi - L log V (srcs/feynman_integral.hpp:336-341)
+        const float nl = -(float)FT_LOOPS;
+        const cdf ef = cdf_mk(tf_add(lpsi, tf_mulf(lv, nl)), tf_add(apsi2, tf_mulf(av2, nl)));
+        cdf z = cdf_mk(tf_mk(c.re, 0.0f), tf_mk(c.im, 0.0f));
+        float fact = 1.0f;
 #pragma unroll
         for (int j = 1; j < FT_K; j++) {
-            c = c * cmk(er * (1.0f / (float)j), ei * (1.0f / (float)j));
-            out[j] = c;
+            z = z * ef;
+            fact *= 1.0f / (float)j;
+            out[j] = cmk(z.re.hi * fact, z.im.hi * fact);
         }
     }
     return true;
