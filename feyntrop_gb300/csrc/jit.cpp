@@ -110,6 +110,72 @@ static std::string tables_source()
     return text;
 }
 
+// Tables and constants of the FP64 form's functions (exact hexadecimal literals; second
+// parts from the host's long double):
+//   FT_LOG64[2i], [2i+1] = {r, hi}, {lo, 0}, r = 1 / (1 + (i + 1/2)/128) to 9 bits, -log r = hi +
+//   lo with hi a multiple of 2^-41 (i < 128); ln 2 likewise
+//   FT_EXP64[j] = 2^(j/128) as hi, lo (j < 128); ln2/128 = L1 + L2, L1 a multiple of 2^-40
+//   FT_SC64[k] = sin(k pi/128), cos(k pi/128) (k < 256); pi/128 = P1 + P2, P1 a multiple of 2^-38
+//   FT_ATAN64[2i], [2i+1] = {i/128, hi}, {lo, 0}, atan(i/128) = hi + lo (i <= 128)
+static std::string tables64_source()
+{
+    static const std::string text = [] {
+        std::ostringstream s;
+        char buf[64];
+        auto num = [&](double v) {
+            std::snprintf(buf, sizeof buf, "%a", v);
+            s << buf;
+        };
+        auto pair = [&](double a, double b) {
+            s << "{";
+            num(a);
+            s << ",";
+            num(b);
+            s << "},";
+        };
+        auto define = [&](const char* name, double v) {
+            s << "#define " << name << " ";
+            num(v);
+            s << "\n";
+        };
+        auto split = [](long double v, int bits) { return (double)(std::nearbyint(std::ldexp(v, bits)) / std::ldexp(1.0L, bits)); };
+        const long double ln2 = std::log(2.0L), pi = std::acos(-1.0L);
+        s << "__device__ const double2 FT_LOG64[256] = {";
+        for (int i = 0; i < 128; i++) {
+            const double r = std::nearbyint(512.0 / (1.0 + (i + 0.5) / 128.0)) / 512.0;
+            const long double nl = -std::log((long double)r);
+            const double hi = split(nl, 41);
+            pair(r, hi);
+            pair((double)(nl - hi), 0.0);
+        }
+        s << "};\n__device__ const double2 FT_EXP64[128] = {";
+        for (int j = 0; j < 128; j++) {
+            const long double t = std::exp2(j / 128.0L);
+            pair((double)t, (double)(t - (double)t));
+        }
+        s << "};\n__device__ const double2 FT_SC64[256] = {";
+        for (int k = 0; k < 256; k++) pair((double)std::sin(k * pi / 128.0L), (double)std::cos(k * pi / 128.0L));
+        s << "};\n__device__ const double2 FT_ATAN64[258] = {";
+        for (int i = 0; i <= 128; i++) {
+            const long double t = std::atan(i / 128.0L);
+            pair(i / 128.0, (double)t);
+            pair((double)(t - (double)t), 0.0);
+        }
+        s << "};\n";
+        const double lh = split(ln2, 41), l1 = split(ln2 / 128.0L, 40), p1 = split(pi / 128.0L, 38);
+        define("FT_LN2_HI", lh);
+        define("FT_LN2_LO", (double)(ln2 - lh));
+        define("FT_EXP_C", (double)(128.0L / ln2));
+        define("FT_EXP_L1", l1);
+        define("FT_EXP_L2", (double)(ln2 / 128.0L - l1));
+        define("FT_SC_C", (double)(128.0L / pi));
+        define("FT_SC_P1", p1);
+        define("FT_SC_P2", (double)(pi / 128.0L - p1));
+        return s.str();
+    }();
+    return text;
+}
+
 // Structural pattern of the conductance-form elimination of the reduced Laplacian (the
 // deleted vertex is V-1): nz[i*n+j] (i < j) marks a conductance between i and j that is
 // non-zero when vertex i is eliminated (an edge, or fill from an earlier elimination),
@@ -211,7 +277,7 @@ std::string kernel_source(const kernel_key& k)
         matrix("FT_NZM", nzm);
         row("FT_NZG", nzg);
     }
-    s << tables_source();
+    s << (k.prec == 0 ? tables64_source() : tables_source());
     s << ft_sample_body_source;
     return s.str();
 }

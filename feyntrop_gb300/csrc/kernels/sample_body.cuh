@@ -61,11 +61,6 @@
 typedef unsigned long long u64;
 typedef unsigned int u32;
 
-// intermediate values for host-side numerical studies (compiled out on the device)
-#ifndef FT_DBG
-#define FT_DBG(slot, value)
-#endif
-
 // Code size: the per-topology kernel is straight-line code (every loop unrolled so
 // that the small matrices stay in registers), and the FP32 library functions carry
 // large slow paths.  FT_VARIANT bit 0 keeps one out-of-line copy of each FP32
@@ -93,14 +88,10 @@ typedef unsigned int u32;
 #else
 #define FT_CXFN __forceinline__
 #endif
-static __device__ FT_MATHFN float m_log1p(float x) { return log1pf(x); }
 static __device__ FT_MATHFN float m_exp(float x) { return expf(x); }
 static __device__ FT_MATHFN float m_exp2(float x) { return exp2f(x); }
 static __device__ FT_MATHFN float m_log2(float x) { return log2f(x); }
-static __device__ FT_MATHFN float m_atan2(float y, float x) { return atan2f(y, x); }
-static __device__ FT_MATHFN float m_hypot(float x, float y) { return hypotf(x, y); }
 static __device__ FT_MATHFN void m_sincos(float x, float* s, float* c) { sincosf(x, s, c); }
-static __device__ FT_MATHFN float m_atan(float x) { return atanf(x); }
 
 #define FT_N (FT_V - 1)
 // reduced vertices [0, FT_Q0) carry no external momentum: the vectors q_r of P~ vanish
@@ -261,12 +252,6 @@ static __device__ __forceinline__ cx<T> crecip(cx<T> z)
     return cmk(r * id, -i * id);
 }
 static __device__ __forceinline__ double cabs_(cx<double> z) { return hypot(z.re, z.im); }
-// |z| for the pivots and determinants of the FP32 path (moduli far inside the
-// float range there: conductances 1/x of a sector stay below ~1e18)
-static __device__ __forceinline__ float cabs_(cx<float> z) { return sqrtf(fmaf(z.re, z.re, z.im * z.im)); }
-static __device__ __forceinline__ bool cfinite(cx<double> z) { return isfinite(z.re) && isfinite(z.im); }
-static __device__ __forceinline__ bool cfinite(cx<float> z) { return isfinite(z.re) && isfinite(z.im); }
-
 // principal logarithm, exp, real power (the reference's std::log / std::pow on
 // complex<double>, srcs/feynman_integral.hpp:310,327,354)
 static __device__ __forceinline__ cx<double> clog_(cx<double> z) { return cmk(log(hypot(z.re, z.im)), atan2(z.im, z.re)); }
@@ -284,114 +269,160 @@ static __device__ __forceinline__ cx<double> cpow_(cx<double> z, double y)
     return cmk(m * c, m * s);
 }
 
-// ------------------------------------------------------------------ conductance-form elimination
-// Reduced Laplacian of the graph with conductances y_e, ground = vertex V-1.
-// Fills the pivots d[k] and the elimination multipliers a[k][i] = c_ki / d_k
-// (i > k), which define L = M^T diag(d) M with M unit upper triangular and
-// M[k][i] = -a[k][i].  Returns the smallest pivot-to-row-size ratio (1 for
-// positive conductances).
-template <class F, class R>
-struct elim {
-    F d[FT_N];
-    F a[FT_N][FT_N];   // a[k][i], i > k
+#if FT_PREC == 0
+// ------------------------------------------------------------------ FP64 functions
+// The FP64 pipe takes 16 cycles of the whole SM per warp instruction (64x fewer lanes than
+// FP32), so the FP64 form costs what it issues there and integer work beside it is free.
+// Its functions are written for few FP64 instructions: table-driven after Tang (ACM TOMS
+// 15 (1989), 16 (1990); 18 (1992)) with the argument's exponent and table index taken by
+// integer operations, short polynomials (Taylor: the reduced arguments are below 0.013) and
+// textbook Newton steps from the approximate reciprocal.  Their results are within about an ulp
+// (log in two parts: 2^-62 absolute); arguments outside the stated ranges take the CUDA
+// library's function (out of line).  FP64 instructions: reciprocal 3, log 15, exp 12,
+// sincos 18, arg 17.  With them and the leaner algebra below the FP64 form issues half the
+// FP64 instructions per sample of the library's functions on the double box, a third on K4.
+static __device__ __forceinline__ int hi_word(double x) { return __double2hiint(x); }
+static __device__ __forceinline__ int exponent_of(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+static __device__ __forceinline__ bool finite_(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
+static __device__ __forceinline__ double pow2_of(int e) { return __hiloint2double((1023 + e) << 20, 0); }
 
-    __device__ __forceinline__ R factor(const F* y)
-    {
-        F c[FT_N][FT_N];   // c[i][j], i < j < N: conductance between i and j
-        F g[FT_N];         // conductance to ground
-#pragma unroll
-        for (int i = 0; i < FT_N; i++) {
-            g[i] = F{};
-#pragma unroll
-            for (int j = 0; j < FT_N; j++) c[i][j] = F{};
-        }
-#pragma unroll
-        for (int e = 0; e < FT_E; e++) {
-            const int k = FT_EK[e], l = FT_EL[e];
-            F& slot = (k == FT_V - 1) ? g[l] : c[l][k];
-            slot = first_in_slot(e) ? y[e] : slot + y[e];
-        }
-        R worst = R(1);
-#pragma unroll
-        for (int k = 0; k < FT_N; k++) {
-            F dk = g[k];
-            R mag = mag_of(g[k]);
-#pragma unroll
-            for (int j = k + 1; j < FT_N; j++) {
-                if (!NZC(k, j)) continue;
-                dk = dk + c[k][j];
-                mag += mag_of(c[k][j]);
-            }
-            d[k] = dk;
-            R ratio = mag_of(dk) * rcp_(mag);
-            worst = ratio < worst ? ratio : worst;
-            F inv = inv_of(dk);
-#pragma unroll
-            for (int i = k + 1; i < FT_N; i++) a[k][i] = NZC(k, i) ? c[k][i] * inv : F{};
-#pragma unroll
-            for (int i = k + 1; i < FT_N; i++) {
-                if (!NZC(k, i)) continue;
-                if (NZG(k)) g[i] = g[i] + a[k][i] * g[k];
-#pragma unroll
-                for (int j = i + 1; j < FT_N; j++)
-                    if (NZC(k, j)) c[i][j] = c[i][j] + a[k][i] * c[k][j];
-            }
-        }
-        return worst;
-    }
+static __device__ __noinline__ double rcp_slow(double x) { return 1.0 / x; }
+static __device__ __forceinline__ double rcp64(double x)
+{
+    if ((u32)(exponent_of(x) - 23) > 2000u) return rcp_slow(x);
+    // seed r with e = 1 - x r below 2^-19; r (1 + e + e^2) leaves e^3
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
 
-    // q^T L^{-1} q for a real vector q (forward substitution y = M^-T q, sum y^2/d;
-    // y vanishes on the rows before FT_Q0, where q does)
-    template <class Q>
-    __device__ __forceinline__ F quad(const Q* q) const
-    {
-        F y[FT_N];
-        F s = F{};
-#pragma unroll
-        for (int i = FT_Q0; i < FT_N; i++) {
-            F yi = from_real((R)q[i]);
-#pragma unroll
-            for (int k = FT_Q0; k < i; k++)
-                if (NZC(k, i)) yi = yi + a[k][i] * y[k];
-            y[i] = yi;
-            s = s + yi * yi * inv_of(d[i]);
-        }
-        return s;
-    }
-
-    // q^T L^{-1} q as quad(), adding sum_i |y_i|^2 / |d_i| (the magnitude of its terms) to mag
-    template <class Q>
-    __device__ __forceinline__ F quad_mag(const Q* q, R& mag) const
-    {
-        F y[FT_N];
-        F s = F{};
-#pragma unroll
-        for (int i = FT_Q0; i < FT_N; i++) {
-            F yi = from_real((R)q[i]);
-#pragma unroll
-            for (int k = FT_Q0; k < i; k++)
-                if (NZC(k, i)) yi = yi + a[k][i] * y[k];
-            y[i] = yi;
-            const F t = yi * yi * inv_of(d[i]);
-            s = s + t;
-            mag += mag_of(t);
-        }
-        return s;
-    }
-
-    static __device__ __forceinline__ R mag_of(R x) { return fabs(x); }
-    static __device__ __forceinline__ R mag_of(cx<R> x) { return fabs(x.re) + fabs(x.im); }
-    static __device__ __forceinline__ R inv_of(R x) { return rcp_(x); }
-    static __device__ __forceinline__ cx<R> inv_of(cx<R> x) { return crecip(x); }
-    static __device__ __forceinline__ F from_real(R x)
-    {
-        F f{};
-        set_real(f, x);
-        return f;
-    }
-    static __device__ __forceinline__ void set_real(R& f, R x) { f = x; }
-    static __device__ __forceinline__ void set_real(cx<R>& f, R x) { f = cmk(x, R(0)); }
+struct dd {
+    double hi, lo;
 };
+static __device__ __forceinline__ dd dd_mk(double h, double l)
+{
+    dd r;
+    r.hi = h;
+    r.lo = l;
+    return r;
+}
+// log(2^k M), M in [1, 2) with i its top 7 fraction bits: r_i a 9-bit approximation of 1/M
+// there, so that z = M r_i - 1 is exact, |z| < 0.006; -log r_i in two parts, the first a
+// multiple of 2^-41 like that of ln 2, so that k ln2 - log r_i is exact in the first.  The
+// result's low part is not below the high one's last place (up to 2e-5): add them where one
+// number is wanted.
+static __device__ __forceinline__ dd log_parts(double M, int i, int k)
+{
+    const double kd = __hiloint2double(0x43300000, k ^ 0x80000000) - 4503601774854144.0;   // k
+    const double2 a = FT_LOG64[2 * i], b = FT_LOG64[2 * i + 1];   // r, hi; lo, -
+    const double z = fma(M, a.x, -1.0);
+    const double H = fma(kd, FT_LN2_HI, a.y);
+    const double z2 = z * z;
+    const double P = fma(
+        z, fma(z, fma(z, fma(z, fma(z, 1.0 / 7.0, -1.0 / 6.0), 1.0 / 5.0), -1.0 / 4.0), 1.0 / 3.0), -1.0 / 2.0);
+    const double lo = fma(z2, P, fma(kd, FT_LN2_LO, b.x));
+    const double s = H + z;
+    return dd_mk(s, (z - (s - H)) + lo);
+}
+// log(1 - u), u = (x >> 11) 2^-53
+static __device__ __forceinline__ dd log1m_64(u64 x)
+{
+    const u64 q = (~x & ~0x7ffull) + 0x800ull;   // (1 - u) 2^64, 0 for u = 0
+    if (q == 0ull) return dd_mk(0.0, 0.0);
+    const int lz = __clzll((long long)q);
+    const u64 mb = q << lz;
+    const double M = __longlong_as_double((long long)(((mb >> 11) & 0xfffffffffffffull) | 0x3ff0000000000000ull));
+    return log_parts(M, (int)((mb >> 56) & 127ull), -1 - lz);
+}
+// log x of a positive normal x
+static __device__ __forceinline__ bool normal_positive(double x) { return (u32)(hi_word(x) - 0x00100000) < 0x7fe00000u; }
+static __device__ __forceinline__ dd log_64(double x)
+{
+    const int h = hi_word(x);
+    return log_parts(__hiloint2double((h & 0xfffff) | 0x3ff00000, __double2loint(x)), (h >> 13) & 127, (h >> 20) - 1023);
+}
+static __device__ __noinline__ double exp_slow(double x) { return exp(x); }
+// e^(hi + lo), |lo| far below 1: 128 steps per octave, |r| < 0.0028
+static __device__ __forceinline__ double exp_64(double hi, double lo)
+{
+    if ((u32)(hi_word(hi) & 0x7fffffff) > 0x40858000u) return exp_slow(hi + lo);   // |hi| > 691
+    const double MAGIC = 6755399441055744.0;
+    const double t = fma(hi, FT_EXP_C, MAGIC), kd = t - MAGIC;
+    const int k = __double2loint(t);
+    const double r = fma(kd, -FT_EXP_L2, fma(kd, -FT_EXP_L1, hi)) + lo;
+    const double q = fma(r * r, fma(r, fma(r, fma(r, 1.0 / 120.0, 1.0 / 24.0), 1.0 / 6.0), 0.5), r);
+    const double2 T = FT_EXP64[k & 127];
+    const double v = T.x + fma(T.x, q, T.y);
+    return __hiloint2double(hi_word(v) + ((k >> 7) << 20), __double2loint(v));
+}
+static __device__ __noinline__ void sincos_slow(double x, double* s, double* c) { sincos(x, s, c); }
+// 256 steps per turn, |r| <= pi/256
+static __device__ __forceinline__ void sincos_64(double x, double& sn, double& cs)
+{
+    if ((u32)(hi_word(x) & 0x7fffffff) > 0x40f86a00u) {   // |x| > 1e5
+        sincos_slow(x, &sn, &cs);
+        return;
+    }
+    const double MAGIC = 6755399441055744.0;
+    const double t = fma(x, FT_SC_C, MAGIC), kd = t - MAGIC;
+    const double2 T = FT_SC64[__double2loint(t) & 255];   // sin, cos
+    const double r = fma(kd, -FT_SC_P2, fma(kd, -FT_SC_P1, x));
+    const double r2 = r * r;
+    const double s = fma(r2 * r, fma(r2, fma(r2, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), r);
+    const double c = r2 * fma(r2, fma(r2, -1.0 / 720.0, 1.0 / 24.0), -0.5);
+    sn = T.x + fma(T.y, s, T.x * c);
+    cs = T.y + fma(-T.x, s, T.y * c);
+}
+static __device__ __noinline__ double arg_slow(double y, double x) { return atan2(y, x); }
+// principal argument of re + i im: with x, y the larger and smaller modulus, c = i/128 the
+// rounded ratio, atan(y/x) = atan c + atan((y - c x) / (x + c y)), the last below 1/256
+static __device__ __forceinline__ double arg_64(double re, double im)
+{
+    const double ar = fabs(re), ai = fabs(im);
+    const bool sw = hi_word(ai) > hi_word(ar);
+    const double x = sw ? ai : ar, y = sw ? ar : ai;
+    const int hx = hi_word(x), hy = hi_word(y);
+    if ((u32)((hx >> 20) - 23) > 2000u) return arg_slow(im, re);
+    const int d = (hy >> 20) - (hx >> 20);   // <= 0
+    const float fx = __int_as_float(0x3f800000 | ((hx & 0xfffff) << 3));
+    const float fy = d < -30 ? 0.0f : __int_as_float((0x3f800000 | ((hy & 0xfffff) << 3)) + d * 0x800000);
+    const int i = (int)(fy * __frcp_rn(fx) * 128.0f + 0.5f);
+    const double2 a = FT_ATAN64[2 * i], b = FT_ATAN64[2 * i + 1];   // c, hi; lo, -
+    const double num = fma(-a.x, x, y), den = fma(a.x, y, x);
+    const double r = rcp64(den);
+    double z = num * r;
+    z = fma(fma(-z, den, num), r, z);
+    const double z2 = z * z;
+    const double v = fma(z2 * z, fma(z2, fma(z2, -1.0 / 7.0, 1.0 / 5.0), -1.0 / 3.0), z) + b.x;
+    // the octant: K +- (hi + v), K = 0, pi/2 or pi
+    const bool left = hi_word(re) < 0;
+    const bool minus = sw != left;   // the angle from the axis counts backwards
+    const double K = sw ? 1.57079632679489655800 : (left ? 3.14159265358979311600 : 0.0);
+    const double Kl = sw ? 6.12323399573676603587e-17 : (left ? 1.22464679914735317720e-16 : 0.0);
+    const double A = (minus ? K - a.y : K + a.y) + (minus ? Kl - v : Kl + v);
+    return hi_word(im) < 0 ? -A : A;
+}
+// 1/z: |z|^2 within range (else the scaled form)
+static __device__ __noinline__ cx<double> cinv_slow(cx<double> z) { return crecip(z); }
+static __device__ __forceinline__ cx<double> cinv_64(cx<double> z)
+{
+    const int e = max(exponent_of(z.re), exponent_of(z.im)) - 1023;
+    if (e > 480 || e < -480) return cinv_slow(z);
+    const double m = rcp64(fma(z.re, z.re, z.im * z.im));
+    return cmk(z.re * m, -z.im * m);
+}
+// t (hi + lo) of a two-part logarithm and a factor
+static __device__ __forceinline__ dd dd_times(double t, dd l)
+{
+    const double p = t * l.hi;
+    return dd_mk(p, fma(t, l.lo, fma(t, l.hi, -p)));
+}
+static __device__ __forceinline__ dd dd_plus(dd a, dd b)
+{
+    const double s = a.hi + b.hi, bb = s - a.hi;
+    return dd_mk(s, ((a.hi - (s - bb)) + (b.hi - bb)) + (a.lo + b.lo));
+}
 
 // ------------------------------------------------------------------ robust complex LU
 // Complete-pivoting LU of the complex reduced Laplacian (largest modulus, first in
@@ -654,7 +685,9 @@ static __device__ __noinline__ void robust_derivatives(const double* X, const do
     }
 }
 
-// ------------------------------------------------------------------ sector draw, FP64
+#endif
+
+// ------------------------------------------------------------------ sector draw
 struct table_ref {
     const void* q;              // cut thresholds (w in the working precision where FT_CUT is 0)
     const void* Jr;             // Jr in the working precision (FT_CUT 0 only)
@@ -751,6 +784,7 @@ static __device__ __forceinline__ int scan_cut(u64 x, u32 sub, const table_ref& 
 }
 #endif
 
+#if FT_PREC == 0
 static __device__ __forceinline__ void draw_sector64(xo& g, const table_ref& t, const unsigned char* gm,
                                                      double Jr_full, double* X, double& F, double& Gv,
                                                      unsigned char* ord)
@@ -796,221 +830,463 @@ static __device__ __forceinline__ void draw_sector64(xo& g, const table_ref& t, 
         if (META_L(m) < META_L(meta)) F *= XX;
         meta = m;
         if (FT_RECORD) ord[j] = (unsigned char)e;
-        if (j < FT_E - 1) XX *= pow(1.0 - u01(g.next()), rinv);
+        if (j < FT_E - 1) {
+            const dd l = dd_times(rinv, log1m_64(g.next()));
+            XX *= exp_64(l.hi, l.lo);
+        }
     }
 }
 
 // ------------------------------------------------------------------ integrand, FP64
-// X: unnormalised sector point; returns R per eps order, false when dropped.
-// `robust` reports that the complete-pivoting LU was needed.
-static __device__ __forceinline__ bool integrand64(const double* prm, double* X, double psi_tr, double xi_tr,
+// powers of the undeformed integrand outside log_64's range, as the reference takes them
+// (srcs/feynman_integral.hpp:246-262): out = R per eps order, false when dropped
+static __device__ __noinline__ bool undeformed_slow(double psi, double pxi, double D, double W, double IGtr, double* out)
+{
+    double R = IGtr * pow(psi, -D / 2.);
+    if (!isfinite(R)) return false;
+#if !FT_ONLY_PSI
+    R *= pow(pxi, -W);
+    if (!isfinite(R)) return false;
+#endif
+    out[0] = R;
+    if (FT_K > 1) {
+        const double ef = log(psi) - FT_LOOPS * log(pxi);
+        for (int j = 1; j < FT_K; j++) {
+            R *= ef / (double)j;
+            out[j] = R;
+        }
+    }
+    return true;
+}
+static __device__ __noinline__ double scale_slow(double psi_tr, double Gv, double D, double W, double norm)
+{
+    return pow(pow(psi_tr, -D / 2.) * pow(1.0 / Gv, W), norm);
+}
+#if FT_MODE == 1
+static __device__ __noinline__ cx<double> powers_slow(cx<double> psi, cx<double> v, double D, double W, cx<double>& lp,
+                                                      cx<double>& lv)
+{
+    lp = clog_(psi);
+    lv = clog_(v);
+    return cpow_(psi, -D / 2.) * cpow_(v, -W);
+}
+#endif
+
+// X: unnormalised sector point, psi_tr and Gv = xi_tr / psi_tr there; returns R per eps
+// order, false when dropped.  `robust` reports that the complete-pivoting LU or the
+// reference's route to the derivatives was needed.
+static __device__ __forceinline__ bool integrand64(const double* prm, double* X, double psi_tr, double Gv,
                                                    cx<double>* out, bool& robust)
 {
     const double D = prm[P_D], W = prm[P_W], IGtr = prm[P_IGTR];
     // normalise so that psi_tr^(-D/2) (psi_tr/xi_tr)^W = 1 (srcs/feynman_integral.hpp:201-204)
-    const double tgt = pow(psi_tr, -D / 2.) * pow(psi_tr / xi_tr, W);
-    const double scale = pow(tgt, prm[P_NORM]);
+    double scale;
+    if (normal_positive(psi_tr) && normal_positive(Gv)) {
+        const dd l = dd_plus(dd_times(-0.5 * D, log_64(psi_tr)), dd_times(-W, log_64(Gv)));
+        const dd t = dd_times(prm[P_NORM], l);
+        scale = exp_64(t.hi, t.lo);
+    } else {
+        scale = scale_slow(psi_tr, Gv, D, W, prm[P_NORM]);
+    }
     double Xi[FT_E];
     double Xprod = 1.0;
 #pragma unroll
     for (int e = 0; e < FT_E; e++) {
         X[e] *= scale;
-        Xi[e] = 1.0 / X[e];
-        Xprod *= X[e];
+        Xi[e] = rcp64(X[e]);
+        Xprod = e == 0 ? X[e] : Xprod * X[e];
     }
-    elim<double, double> L;
-    L.factor(Xi);
-    double det = 1.0;
+    // the real reduced Laplacian in conductance form (every value positive)
+    double a[FT_N][FT_N], d[FT_N], id[FT_N];
+    {
+        double c[FT_N][FT_N], g[FT_N];
 #pragma unroll
-    for (int k = 0; k < FT_N; k++) det *= L.d[k];
-    robust = false;
-#if FT_MODE == 0
-    const double psi = det * Xprod;
-    double R = IGtr * pow(psi, -D / 2.);
-    if (!isfinite(R)) return false;
-#if FT_ONLY_PSI
-    out[0] = cmk(R, 0.0);
-    return true;
-#else
-    double tr = 0.0;
+        for (int e = 0; e < FT_E; e++) {
+            const int k = FT_EK[e], l = FT_EL[e];
+            double& slot = (k == FT_V - 1) ? g[l] : c[l][k];
+            slot = first_in_slot(e) ? Xi[e] : slot + Xi[e];
+        }
 #pragma unroll
-    for (int r = 0; r < FT_RANK; r++) tr += prm[P_SIG + r] * L.quad(prm + P_Q + r * FT_N);
-    double pxi = -tr;
+        for (int k = 0; k < FT_N; k++) {
+            double dk = 0.0;
+            bool any = NZG(k);
+            if (any) dk = g[k];
 #pragma unroll
-    for (int e = 0; e < FT_E; e++) pxi += prm[P_M2 + e] * X[e];
-    R *= pow(pxi, -W);
-    if (!isfinite(R)) return false;
-    out[0] = cmk(R, 0.0);
-    if (FT_K > 1) {
-        const double ef = log(psi) - FT_LOOPS * log(pxi);
+            for (int j = k + 1; j < FT_N; j++)
+                if (NZC(k, j)) {
+                    dk = any ? dk + c[k][j] : c[k][j];
+                    any = true;
+                }
+            d[k] = dk;
+            id[k] = rcp64(dk);
 #pragma unroll
-        for (int j = 1; j < FT_K; j++) {
-            R *= ef / (double)j;
-            out[j] = cmk(R, 0.0);
+            for (int i = k + 1; i < FT_N; i++)
+                if (NZC(k, i)) a[k][i] = c[k][i] * id[k];
+#pragma unroll
+            for (int i = k + 1; i < FT_N; i++) {
+                if (!NZC(k, i)) continue;
+                if (NZG(k)) g[i] = ADDS_G(k, i) ? fma(a[k][i], g[k], g[i]) : a[k][i] * g[k];
+#pragma unroll
+                for (int j = i + 1; j < FT_N; j++)
+                    if (NZC(k, j)) c[i][j] = ADDS_C(k, i, j) ? fma(a[k][i], c[k][j], c[i][j]) : a[k][i] * c[k][j];
+            }
         }
     }
-    return true;
+    robust = false;
+#if FT_MODE == 0
+    double det = d[0];
+#pragma unroll
+    for (int k = 1; k < FT_N; k++) det *= d[k];
+    const double psi = det * Xprod;
+    double pxi = 1.0;
+#if !FT_ONLY_PSI
+    // V = -sum_r sigma_r q_r^T L^-1 q_r + sum_e m2_e X_e
+    pxi = 0.0;
+#pragma unroll
+    for (int r = 0; r < FT_RANK; r++) {
+        double y[FT_N], s = 0.0;
+#pragma unroll
+        for (int i = FT_Q0; i < FT_N; i++) {
+            double yi = prm[P_Q + r * FT_N + i];
+#pragma unroll
+            for (int k = FT_Q0; k < i; k++)
+                if (NZC(k, i)) yi = fma(a[k][i], y[k], yi);
+            y[i] = yi;
+            s = i == FT_Q0 ? yi * yi * id[i] : fma(yi * yi, id[i], s);
+        }
+        pxi = r == 0 ? -(prm[P_SIG + r] * s) : fma(-prm[P_SIG + r], s, pxi);
+    }
+#pragma unroll
+    for (int e = 0; e < FT_E; e++) pxi = fma(prm[P_M2 + e], X[e], pxi);
 #endif
+    double R[FT_K];
+    if (!normal_positive(psi) || !normal_positive(pxi)) {
+        const bool ok = undeformed_slow(psi, pxi, D, W, IGtr, R);
+#pragma unroll
+        for (int j = 0; j < FT_K; j++) out[j] = cmk(R[j], 0.0);
+        return ok;
+    }
+    const dd lp = log_64(psi);
+#if FT_ONLY_PSI
+    const dd t = dd_times(-0.5 * D, lp);
+    const double v = IGtr * exp_64(t.hi, t.lo);
+    if (!finite_(v)) return false;
+    out[0] = cmk(v, 0.0);
+#else
+    const dd lv = log_64(pxi);
+    const dd t = dd_plus(dd_times(-0.5 * D, lp), dd_times(-W, lv));
+    double v = IGtr * exp_64(t.hi, t.lo);
+    if (!finite_(v)) return false;
+    out[0] = cmk(v, 0.0);
+    if (FT_K > 1) {
+        const double ef = fma(-(double)FT_LOOPS, lv.hi + lv.lo, lp.hi + lp.lo);
+#pragma unroll
+        for (int j = 1; j < FT_K; j++) {
+            v *= ef * (1.0 / (double)j);
+            out[j] = cmk(v, 0.0);
+        }
+    }
+#endif
+    return true;
 #else
     const double kappa = prm[P_DEF];
-    // G = L^-1 = N diag(1/d) N^T with N = M^-1 (entrywise non-negative)
-    double Nm[FT_N][FT_N];
+    // N = M^-1 (entrywise non-negative), G = L^-1 = N diag(1/d) N^T
+    double Nm[FT_N][FT_N], Nd[FT_N][FT_N];
 #pragma unroll
     for (int i = FT_N - 1; i >= 0; i--) {
-#pragma unroll
-        for (int j = 0; j < FT_N; j++) Nm[i][j] = 0.0;
-        Nm[i][i] = 1.0;
 #pragma unroll
         for (int j = i + 1; j < FT_N; j++) {
             if (!NZM(i, j)) continue;
             double s = 0.0;
+            bool any = false;
+            if (NZC(i, j)) {
+                s = a[i][j];
+                any = true;
+            }
 #pragma unroll
-            for (int k = i + 1; k <= j; k++)
-                if (NZC(i, k) && (k == j || NZM(k, j))) s += L.a[i][k] * Nm[k][j];
+            for (int k = i + 1; k < j; k++)
+                if (NZC(i, k) && NZM(k, j)) {
+                    s = any ? fma(a[i][k], Nm[k][j], s) : a[i][k] * Nm[k][j];
+                    any = true;
+                }
             Nm[i][j] = s;
+            Nd[i][j] = s * id[j];
         }
     }
-    double id[FT_N];
-#pragma unroll
-    for (int k = 0; k < FT_N; k++) id[k] = 1.0 / L.d[k];
     double G[FT_N][FT_N];
 #pragma unroll
     for (int i = 0; i < FT_N; i++)
 #pragma unroll
         for (int j = i; j < FT_N; j++) {
             double s = 0.0;
+            bool any = false;
+            if (i == j || NZM(i, j)) {
+                s = i == j ? id[j] : Nd[i][j];
+                any = true;
+            }
 #pragma unroll
-            for (int k = j; k < FT_N; k++)
-                if ((k == i || NZM(i, k)) && (k == j || NZM(j, k))) s += Nm[i][k] * Nm[j][k] * id[k];
+            for (int k = j + 1; k < FT_N; k++)
+                if (NZM(i, k) && NZM(j, k)) {
+                    s = any ? fma(Nm[i][k], Nd[j][k], s) : Nm[i][k] * Nd[j][k];
+                    any = true;
+                }
             G[i][j] = s;
             G[j][i] = s;
         }
-    // h_r = L^-1 q_r; per edge: hb[r][e] = h_r . b_e with b_e = e_k - e_l (ground row zero)
+    // Per edge its power of two D ~ X^1/2 and w = D / X^2; hb = w h_r . b_e with h_r = L^-1 q_r,
+    // b_e = e_k - e_l (ground row zero), so that
+    //   s_ab = -2 kappa sum_r sigma_r hb_a hb_b,  t_ab = b_a^T G b_b
+    // give kappa D_a D_b H_ab = s_ab t_ab (the diagonal s_aa (t_aa - X_a)) and
+    // theta_a = kappa m2_a + s_aa X_a^2 / (2 D_a^2) (srcs/laplacian.hpp:102-215)
+    int ex[FT_E];   // D = 2^ex
     double hb[FT_RANK][FT_E];
-#pragma unroll
-    for (int r = 0; r < FT_RANK; r++) {
-        double h[FT_N];
-#pragma unroll
-        for (int i = 0; i < FT_N; i++) {
-            double s = 0.0;
-#pragma unroll
-            for (int j = FT_Q0; j < FT_N; j++) s += G[i][j] * prm[P_Q + r * FT_N + j];
-            h[i] = s;
-        }
+    {
+        double w[FT_E];
 #pragma unroll
         for (int e = 0; e < FT_E; e++) {
-            const int k = FT_EK[e], l = FT_EL[e];
-            hb[r][e] = (k == FT_V - 1 ? 0.0 : h[k]) - h[l];
+            ex[e] = max(-500, min(500, (exponent_of(X[e]) - 1023) >> 1));
+            w[e] = Xi[e] * Xi[e] * pow2_of(ex[e]);
+        }
+#pragma unroll
+        for (int r = 0; r < FT_RANK; r++) {
+            double h[FT_N];
+#pragma unroll
+            for (int i = 0; i < FT_N; i++) {
+                double s = 0.0;
+#pragma unroll
+                for (int j = FT_Q0; j < FT_N; j++) {
+                    const double q = prm[P_Q + r * FT_N + j];
+                    s = j == FT_Q0 ? G[i][j] * q : fma(G[i][j], q, s);
+                }
+                h[i] = s;
+            }
+#pragma unroll
+            for (int e = 0; e < FT_E; e++) {
+                const int k = FT_EK[e], l = FT_EL[e];
+                hb[r][e] = ((k == FT_V - 1) ? -h[l] : h[k] - h[l]) * w[e];
+            }
         }
     }
-    // s_ab = sum_r sigma_r hb_a hb_b, t_ab = b_a^T G b_b
-    auto Gx = [&](int i, int j) -> double { return (i == FT_V - 1 || j == FT_V - 1) ? 0.0 : G[i][j]; };
-    double dphi[FT_E];
-    double H[FT_E][FT_E];
+    double A[FT_E][FT_E];   // kappa D H D, upper triangle
+    double theta[FT_E];
     bool cancel = false;
 #pragma unroll
-    for (int a = 0; a < FT_E; a++) {
-        const int ka = FT_EK[a], la = FT_EL[a];
+    for (int e = 0; e < FT_E; e++) {
+        const int ke = FT_EK[e], le = FT_EL[e];
+        double w[FT_N];   // row e of (edge incidence) L^-1
+#pragma unroll
+        for (int v = 0; v < FT_N; v++)
+            w[v] = ke == FT_V - 1 ? -G[le][v] : (le == FT_V - 1 ? G[ke][v] : G[ke][v] - G[le][v]);
+        auto wd = [&](int k, int l) -> double { return k == FT_V - 1 ? -w[l] : (l == FT_V - 1 ? w[k] : w[k] - w[l]); };
+        double sg[FT_RANK];
         double s = 0.0;
 #pragma unroll
-        for (int r = 0; r < FT_RANK; r++) s += prm[P_SIG + r] * hb[r][a] * hb[r][a];
-        const double t = Gx(ka, ka) + Gx(la, la) - 2.0 * Gx(ka, la);
-        // an edge whose ends float together: its resistance difference cancels
-        cancel |= ka != FT_V - 1 && !(t > 1e-7 * (Gx(ka, ka) + Gx(la, la)));
-        const double xa = Xi[a] * Xi[a];
-        const double xas = xa * s;
-        dphi[a] = -xas;
-        H[a][a] = 2.0 * xas * (Xi[a] - xa * t);
+        for (int r = 0; r < FT_RANK; r++) {
+            sg[r] = (-2.0 * kappa * prm[P_SIG + r]) * hb[r][e];
+            s = r == 0 ? sg[r] * hb[r][e] : fma(sg[r], hb[r][e], s);
+        }
+        const double t = wd(ke, le);
+        // an edge whose ends float together: its resistance difference cancels (t below about
+        // 1e-7 of the entries it comes from, by their exponents)
+        if (ke != FT_V - 1) {
+            const int big = max(exponent_of(G[ke][ke]), exponent_of(G[le][le]));
+            cancel |= hi_word(t) < 0 || exponent_of(t) < big - 23;
+        }
+        A[e][e] = s * (t - X[e]);
+        theta[e] = fma(s * (X[e] * X[e]), pow2_of(-2 * ex[e] - 1), kappa * prm[P_M2 + e]);
 #pragma unroll
-        for (int b = a + 1; b < FT_E; b++) {
-            const int kb = FT_EK[b], lb = FT_EL[b];
+        for (int f = e + 1; f < FT_E; f++) {
             double s2 = 0.0;
 #pragma unroll
-            for (int r = 0; r < FT_RANK; r++) s2 += prm[P_SIG + r] * hb[r][a] * hb[r][b];
-            const double t2 = Gx(ka, kb) + Gx(la, lb) - Gx(ka, lb) - Gx(la, kb);
-            H[a][b] = -2.0 * xa * (Xi[b] * Xi[b]) * s2 * t2;
+            for (int r = 0; r < FT_RANK; r++) s2 = r == 0 ? sg[r] * hb[r][f] : fma(sg[r], hb[r][f], s2);
+            A[e][f] = s2 * wd(FT_EK[f], FT_EL[f]);
         }
     }
     if (cancel) {
+        double dphi[FT_E], H[FT_E][FT_E];
         robust_derivatives(X, Xi, prm, dphi, H);
         robust = true;
-    }
-    // deformation x -> x exp(i theta), theta = -lambda (d(phi/psi)/dx + m^2)
-    double theta[FT_E];
-    cx<double> cX[FT_E], cy[FT_E];
-    double xnu = 0.0;
-    cx<double> cXprod = cmk(1.0, 0.0);
 #pragma unroll
-    for (int e = 0; e < FT_E; e++) {
-        theta[e] = (dphi[e] + prm[P_M2 + e]) * kappa;
-        FT_DBG(40 + e, theta[e]);
-        double sn, cs;
-        sincos(theta[e], &sn, &cs);
-        cX[e] = cmk(X[e] * cs, X[e] * sn);
-        cy[e] = cmk(Xi[e] * cs, -Xi[e] * sn);   // 1 / cX
-        xnu += prm[P_NU + e] * theta[e];
-        cXprod = cXprod * cX[e];
-    }
-    elim<cx<double>, double> CL;
-    const double growth = CL.factor(cy);
-    cx<double> cdet, cpphi;
-    if (growth > 1e-8) {
-        cdet = cmk(1.0, 0.0);
+        for (int e = 0; e < FT_E; e++) {
+            theta[e] = (dphi[e] + prm[P_M2 + e]) * kappa;
 #pragma unroll
-        for (int k = 0; k < FT_N; k++) cdet = cdet * CL.d[k];
-        cx<double> tr = cmk(0.0, 0.0);
-#pragma unroll
-        for (int r = 0; r < FT_RANK; r++) tr = tr + prm[P_SIG + r] * CL.quad(prm + P_Q + r * FT_N);
-        cpphi = cmk(-tr.re, -tr.im);
-    } else {
-        robust = true;
-        robust_complex(cy, prm, cdet, cpphi);
-    }
-    const cx<double> cPsi = cXprod * cdet;
-    cx<double> cR = IGtr * cpow_(cPsi, -D / 2.);
-    // det(I + i kappa X^1/2 H X^1/2), symmetric elimination without pivoting
-    cx<double> J[FT_E][FT_E];
-    double sx[FT_E];
-#pragma unroll
-    for (int e = 0; e < FT_E; e++) sx[e] = sqrt(X[e]);
-#pragma unroll
-    for (int a = 0; a < FT_E; a++)
-#pragma unroll
-        for (int b = a; b < FT_E; b++) J[a][b] = cmk(a == b ? 1.0 : 0.0, kappa * H[a][b] * sx[a] * sx[b]);
-    cx<double> detJ = cmk(1.0, 0.0);
-#pragma unroll
-    for (int k = 0; k < FT_E; k++) {
-        const cx<double> piv = J[k][k];
-        detJ = detJ * piv;
-        const cx<double> inv = crecip(piv);
-#pragma unroll
-        for (int i = k + 1; i < FT_E; i++) {
-            const cx<double> f = J[k][i] * inv;
-#pragma unroll
-            for (int j = i; j < FT_E; j++) J[i][j] = J[i][j] - f * J[k][j];
+            for (int f = e; f < FT_E; f++) A[e][f] = kappa * H[e][f] * pow2_of(ex[e]) * pow2_of(ex[f]);
         }
     }
-    double sn, cs;
-    sincos(xnu, &sn, &cs);
-    cR = cR * (detJ * cmk(cs, sn));
-    cx<double> cPXi = cpphi;
+    // deformation x -> x exp(i theta), theta = -lambda (d(phi/psi)/dx + m^2)
+    // (srcs/feynman_integral.hpp:290-310)
+    cx<double> cy[FT_E];
+    double xnu = 0.0;
+    cx<double> cXprod = cmk(1.0, 0.0), cV = cmk(0.0, 0.0);
 #pragma unroll
-    for (int e = 0; e < FT_E; e++) cPXi = cPXi + prm[P_M2 + e] * cX[e];
-    FT_DBG(50, log2(hypot(detJ.re, detJ.im)));
-    FT_DBG(51, atan2(detJ.im, detJ.re));
-    FT_DBG(52, atan2(cPsi.im, cPsi.re));
-    FT_DBG(54, atan2(cPXi.im, cPXi.re));
-    FT_DBG(55, xnu);
-    FT_DBG(56, cpphi.re);
-    FT_DBG(57, cpphi.im);
-    FT_DBG(58, cPXi.re);
-    FT_DBG(59, cPXi.im);
-    cR = cR * cpow_(cPXi, -W);
-    if (!cfinite(cR)) return false;
+    for (int e = 0; e < FT_E; e++) {
+        double sn, cs;
+        sincos_64(theta[e], sn, cs);
+        const cx<double> cX = cmk(X[e] * cs, X[e] * sn);
+        cy[e] = cmk(Xi[e] * cs, -Xi[e] * sn);   // 1 / cX
+        const double m2 = prm[P_M2 + e];
+        xnu = e == 0 ? prm[P_NU] * theta[0] : fma(prm[P_NU + e], theta[e], xnu);
+        cXprod = e == 0 ? cX : cXprod * cX;
+        cV = e == 0 ? m2 * cX : cmk(fma(m2, cX.re, cV.re), fma(m2, cX.im, cV.im));
+    }
+    // the deformed Laplacian, its determinant and -tr(L^-1 P~): U the unit lower triangular
+    // map of the forward substitution on the external rows, sum_i (u_i^T P~ u_i) / d_i
+    cx<double> cdet = cmk(1.0, 0.0), cphi = cmk(0.0, 0.0);
+    bool growth = true;
+    {
+        cx<double> c[FT_N][FT_N], g[FT_N], ca[FT_N][FT_N], ci[FT_N];
+#pragma unroll
+        for (int e = 0; e < FT_E; e++) {
+            const int k = FT_EK[e], l = FT_EL[e];
+            cx<double>& slot = (k == FT_V - 1) ? g[l] : c[l][k];
+            slot = first_in_slot(e) ? cy[e] : slot + cy[e];
+        }
+        auto expo = [](cx<double> z) -> int { return max(exponent_of(z.re), exponent_of(z.im)); };
+        auto cfma = [](cx<double> x, cx<double> y, cx<double> z) -> cx<double> {
+            return cmk(fma(x.re, y.re, fma(-x.im, y.im, z.re)), fma(x.re, y.im, fma(x.im, y.re, z.im)));
+        };
+#pragma unroll
+        for (int k = 0; k < FT_N; k++) {
+            cx<double> dk = cmk(0.0, 0.0);
+            int big = 0;
+            bool any = NZG(k);
+            if (any) {
+                dk = g[k];
+                big = expo(g[k]);
+            }
+#pragma unroll
+            for (int j = k + 1; j < FT_N; j++) {
+                if (!NZC(k, j)) continue;
+                dk = any ? dk + c[k][j] : c[k][j];
+                big = max(big, expo(c[k][j]));
+                any = true;
+            }
+            growth &= expo(dk) > big - 26;   // a pivot above about 1e-8 of its row, by the exponents
+            cdet = k == 0 ? dk : cdet * dk;
+            ci[k] = cinv_64(dk);
+#pragma unroll
+            for (int i = k + 1; i < FT_N; i++)
+                if (NZC(k, i)) ca[k][i] = c[k][i] * ci[k];
+#pragma unroll
+            for (int i = k + 1; i < FT_N; i++) {
+                if (!NZC(k, i)) continue;
+                if (NZG(k)) g[i] = ADDS_G(k, i) ? cfma(ca[k][i], g[k], g[i]) : ca[k][i] * g[k];
+#pragma unroll
+                for (int j = i + 1; j < FT_N; j++)
+                    if (NZC(k, j)) c[i][j] = ADDS_C(k, i, j) ? cfma(ca[k][i], c[k][j], c[i][j]) : ca[k][i] * c[k][j];
+            }
+        }
+#if FT_NE > 0
+        cx<double> U[FT_NE][FT_NE];
+#pragma unroll
+        for (int ii = 0; ii < FT_NE; ii++) {
+            const int i = FT_Q0 + ii;
+#pragma unroll
+            for (int jj = 0; jj < ii; jj++) {
+                const int j = FT_Q0 + jj;
+                if (!NZM(j, i)) continue;
+                cx<double> u = cmk(0.0, 0.0);
+                bool any = false;
+                if (NZC(j, i)) {
+                    u = ca[j][i];
+                    any = true;
+                }
+#pragma unroll
+                for (int kk = jj + 1; kk < ii; kk++) {
+                    const int k = FT_Q0 + kk;
+                    if (!NZC(k, i) || !NZM(j, k)) continue;
+                    u = any ? cfma(ca[k][i], U[kk][jj], u) : ca[k][i] * U[kk][jj];
+                    any = true;
+                }
+                U[ii][jj] = u;
+            }
+            cx<double> Q = cmk(prm[PT_AT(ii, ii)], 0.0);
+            bool real = true;
+#pragma unroll
+            for (int jj = 0; jj < ii; jj++) {
+                if (!NZM(FT_Q0 + jj, i)) continue;
+                cx<double> w = prm[PT_AT(jj, jj)] * U[ii][jj];
+#pragma unroll
+                for (int kk = jj + 1; kk < ii; kk++) {
+                    if (!NZM(FT_Q0 + kk, i)) continue;
+                    const double p = prm[PT_AT(jj, kk)];
+                    w = cmk(fma(p, U[ii][kk].re, w.re), fma(p, U[ii][kk].im, w.im));
+                }
+                w.re += prm[PT_AT(jj, ii)];
+                Q = cfma(U[ii][jj], w, Q);
+                real = false;
+            }
+            cphi = real ? cmk(fma(-Q.re, ci[i].re, cphi.re), fma(-Q.re, ci[i].im, cphi.im))
+                        : cfma(cmk(-Q.re, -Q.im), ci[i], cphi);
+        }
+#endif
+    }
+    if (!growth) {
+        robust = true;
+        robust_complex(cy, prm, cdet, cphi);
+    }
+    const cx<double> cPsi = cXprod * cdet;
+    cV = cV + cphi;
+    // det(I + i kappa H X) = det(D^2/X + i kappa D H D) prod X/D^2: the real part is positive
+    // and diagonal, so the symmetric elimination needs no pivoting (srcs/feynman_integral.hpp:312-320)
+    cx<double> detJ = cmk(1.0, 0.0);
+    {
+        cx<double> J[FT_E][FT_E];
+#pragma unroll
+        for (int e = 0; e < FT_E; e++)
+#pragma unroll
+            for (int f = e; f < FT_E; f++) J[e][f] = cmk(e == f ? pow2_of(2 * ex[e]) * Xi[e] : 0.0, A[e][f]);
+#pragma unroll
+        for (int k = 0; k < FT_E; k++) {
+            const cx<double> piv = J[k][k];
+            detJ = k == 0 ? piv : detJ * piv;
+            if (k == FT_E - 1) continue;
+            const cx<double> inv = cinv_64(piv);
+#pragma unroll
+            for (int i = k + 1; i < FT_E; i++) {
+                // the first row's entries have no real part
+                const cx<double> f = k == 0 ? cmk(-J[0][i].im * inv.im, J[0][i].im * inv.re) : J[k][i] * inv;
+#pragma unroll
+                for (int j = i; j < FT_E; j++) {
+                    const cx<double> q = J[k][j];
+                    if (k == 0)
+                        J[i][j] = cmk(fma(f.im, q.im, J[i][j].re), fma(-f.re, q.im, J[i][j].im));
+                    else
+                        J[i][j] = cmk(fma(-f.re, q.re, fma(f.im, q.im, J[i][j].re)),
+                                      fma(-f.re, q.im, fma(-f.im, q.re, J[i][j].im)));
+                }
+            }
+        }
+    }
+    {
+        int sum = 0;
+#pragma unroll
+        for (int e = 0; e < FT_E; e++) sum += ex[e];
+        sum = max(-1000, min(1000, sum));
+        detJ = (Xprod * pow2_of(-sum) * pow2_of(-sum)) * detJ;   // prod X / D^2
+    }
+    // cR = IGtr cPsi^(-D/2) cV^(-W) det J e^(i nu . theta)
+    cx<double> lp, lv, pw;
+    const double np = fma(cPsi.re, cPsi.re, cPsi.im * cPsi.im), nv = fma(cV.re, cV.re, cV.im * cV.im);
+    if (normal_positive(np) && normal_positive(nv)) {
+        const dd a2 = log_64(np), b2 = log_64(nv);
+        lp = cmk(0.5 * (a2.hi + a2.lo), arg_64(cPsi.re, cPsi.im));
+        lv = cmk(0.5 * (b2.hi + b2.lo), arg_64(cV.re, cV.im));
+        const dd t = dd_plus(dd_times(-0.25 * D, a2), dd_times(-0.5 * W, b2));
+        const double m = exp_64(t.hi, t.lo);
+        double sn, cs;
+        sincos_64(fma(-0.5 * D, lp.im, -W * lv.im), sn, cs);
+        pw = cmk(m * cs, m * sn);
+    } else {
+        pw = powers_slow(cPsi, cV, D, W, lp, lv);
+    }
+    double sn, cs;
+    sincos_64(xnu, sn, cs);
+    cx<double> cR = (IGtr * pw) * (detJ * cmk(cs, sn));
+    if (!finite_(cR.re) || !finite_(cR.im)) return false;
     out[0] = cR;
     if (FT_K > 1) {
-        const cx<double> lp = clog_(cPsi), lv = clog_(cPXi);
-        const cx<double> ef = cmk(lp.re - FT_LOOPS * lv.re, lp.im - FT_LOOPS * lv.im);
+        const cx<double> ef = cmk(fma(-(double)FT_LOOPS, lv.re, lp.re), fma(-(double)FT_LOOPS, lv.im, lp.im));
 #pragma unroll
         for (int j = 1; j < FT_K; j++) {
             cR = cR * ((1.0 / (double)j) * ef);
@@ -1021,8 +1297,7 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
 #endif
 }
 
-
-#if FT_PREC == 1
+#else
 // ------------------------------------------------------------------ mixed form: FP32 values and pairs
 // Pairs of FP32 values use the paired instructions (add, mul, fma .f32x2, each component
 // rounded as the scalar operation): the same rate per result, half the issue slots and
@@ -2583,7 +2858,9 @@ struct accum {
     {
         const double s = S(slot);
         const double t = s + v;
-        C(slot) += (fabs(s) >= fabs(v)) ? ((s - t) + v) : ((v - t) + s);
+        // the larger term first, by the exponents
+        const bool big = exponent_of(s) >= exponent_of(v);
+        C(slot) += ((big ? s : v) - t) + (big ? v : s);
         S(slot) = t;
     }
 
@@ -2850,7 +3127,7 @@ static __device__ __forceinline__ void sample64(xo& g, const table_ref& tr, cons
     if (FT_RECORD)
         for (int e = 0; e < FT_E; e++) rec_X[i * FT_E + e] = X[e];
     bool rob = false;
-    const bool ok = integrand64(prm, X, F, Gv * F, R, rob);
+    const bool ok = integrand64(prm, X, F, Gv, R, rob);
     if (rob) {
         A.count(CNT_ROBUST, 1);
         flags |= REC_ROBUST;
@@ -3228,7 +3505,7 @@ extern "C" __global__ void __launch_bounds__(FT_BLOCK) ft_sample_queue_batch(
         unsigned char ord[FT_E];
         draw_sector64(g, tr, FT_EXACT_TABLE(tr), prm[P_JRFULL], X, F, Gv, ord);
         bool rob = false;
-        const bool ok = integrand64(prm, X, F, Gv * F, R, rob);
+        const bool ok = integrand64(prm, X, F, Gv, R, rob);
         u64* qa = qacc + (size_t)id * (4 * FT_K * FT_XA_DIGITS + 4);
         u64* cnt = qa + 4 * FT_K * FT_XA_DIGITS;
         if (rob) atomicAdd(cnt + 2, 1ull);
