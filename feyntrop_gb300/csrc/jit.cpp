@@ -110,67 +110,50 @@ static std::string tables_source()
     return text;
 }
 
-// Tables and constants of the FP64 form's functions (exact hexadecimal literals; second
-// parts from the host's long double):
-//   FT_LOG64[2i], [2i+1] = {r, hi}, {lo, 0}, r = 1 / (1 + (i + 1/2)/128) to 9 bits, -log r = hi +
-//   lo with hi a multiple of 2^-41 (i < 128); ln 2 likewise
-//   FT_EXP64[j] = 2^(j/128) as hi, lo (j < 128); ln2/128 = L1 + L2, L1 a multiple of 2^-40
-//   FT_SC64[k] = sin(k pi/128), cos(k pi/128) (k < 256); pi/128 = P1 + P2, P1 a multiple of 2^-38
+// Tables and constants of the FP64 form's functions, in fixed point (Qn: units of 2^-n; from the
+// host's long double, to a unit or so) and as exact hexadecimal literals:
+//   FT_LOG64[i] = r, -log2(r / 1024) in Q62, r = ceil(1024 / (1 + i/256)) (i < 256)
+//   FT_EXP64[j] = 2^(j/256) in Q63 (j < 256)
+//   FT_SC64[k] = sin(k pi/128), cos(k pi/128) in Q63 (k < 64)
 //   FT_ATAN64[2i], [2i+1] = {i/128, hi}, {lo, 0}, atan(i/128) = hi + lo (i <= 128)
+//   log2 e in Q63, ln 2 in Q64, 128/pi in Q58 and the next 64 bits, pi/128 in Q69
 static std::string tables64_source()
 {
     static const std::string text = [] {
         std::ostringstream s;
         char buf[64];
-        auto num = [&](double v) {
-            std::snprintf(buf, sizeof buf, "%a", v);
+        auto fixed = [&](long double v, int q) {
+            std::snprintf(buf, sizeof buf, "0x%llxull,", (unsigned long long)(std::ldexp(v, q) + 0.5L));
             s << buf;
         };
-        auto pair = [&](double a, double b) {
-            s << "{";
-            num(a);
-            s << ",";
-            num(b);
+        const long double pi = std::acos(-1.0L);
+        s << "__device__ const ulonglong2 FT_LOG64[256] = {";
+        for (int i = 0; i < 256; i++) {
+            const int r = (1024 * 256 + 255 + i) / (256 + i);
+            s << "{" << r << "ull,";
+            fixed(-std::log2(r / 1024.0L), 62);
             s << "},";
-        };
-        auto define = [&](const char* name, double v) {
-            s << "#define " << name << " ";
-            num(v);
-            s << "\n";
-        };
-        auto split = [](long double v, int bits) { return (double)(std::nearbyint(std::ldexp(v, bits)) / std::ldexp(1.0L, bits)); };
-        const long double ln2 = std::log(2.0L), pi = std::acos(-1.0L);
-        s << "__device__ const double2 FT_LOG64[256] = {";
-        for (int i = 0; i < 128; i++) {
-            const double r = std::nearbyint(512.0 / (1.0 + (i + 0.5) / 128.0)) / 512.0;
-            const long double nl = -std::log((long double)r);
-            const double hi = split(nl, 41);
-            pair(r, hi);
-            pair((double)(nl - hi), 0.0);
         }
-        s << "};\n__device__ const double2 FT_EXP64[128] = {";
-        for (int j = 0; j < 128; j++) {
-            const long double t = std::exp2(j / 128.0L);
-            pair((double)t, (double)(t - (double)t));
+        s << "};\n__device__ const unsigned long long FT_EXP64[256] = {";
+        for (int j = 0; j < 256; j++) fixed(std::exp2(j / 256.0L), 63);
+        s << "};\n__device__ const ulonglong2 FT_SC64[64] = {";
+        for (int k = 0; k < 64; k++) {
+            s << "{";
+            fixed(std::sin(k * pi / 128.0L), 63);
+            fixed(std::cos(k * pi / 128.0L), 63);
+            s << "},";
         }
-        s << "};\n__device__ const double2 FT_SC64[256] = {";
-        for (int k = 0; k < 256; k++) pair((double)std::sin(k * pi / 128.0L), (double)std::cos(k * pi / 128.0L));
         s << "};\n__device__ const double2 FT_ATAN64[258] = {";
         for (int i = 0; i <= 128; i++) {
             const long double t = std::atan(i / 128.0L);
-            pair(i / 128.0, (double)t);
-            pair((double)(t - (double)t), 0.0);
+            std::snprintf(buf, sizeof buf, "{%a,%a},", i / 128.0, (double)t);
+            s << buf;
+            std::snprintf(buf, sizeof buf, "{%a,0.0},", (double)(t - (double)t));
+            s << buf;
         }
-        s << "};\n";
-        const double lh = split(ln2, 41), l1 = split(ln2 / 128.0L, 40), p1 = split(pi / 128.0L, 38);
-        define("FT_LN2_HI", lh);
-        define("FT_LN2_LO", (double)(ln2 - lh));
-        define("FT_EXP_C", (double)(128.0L / ln2));
-        define("FT_EXP_L1", l1);
-        define("FT_EXP_L2", (double)(ln2 / 128.0L - l1));
-        define("FT_SC_C", (double)(128.0L / pi));
-        define("FT_SC_P1", p1);
-        define("FT_SC_P2", (double)(pi / 128.0L - p1));
+        s << "};\n#define FT_LOG2E_Q63 0xb8aa3b295c17f0bcull\n#define FT_LN2_Q64 0xb17217f7d1cf79acull\n"
+             "#define FT_STEPS_Q58 0xa2f9836e4e441529ull\n#define FT_STEPS_LO 0xfc2757d1f534ddc0ull\n"
+             "#define FT_STEP_Q69 0xc90fdaa22168c235ull\n";
         return s.str();
     }();
     return text;

@@ -127,7 +127,7 @@ static __device__ constexpr bool first_in_slot(int e)
 #define FT_NPAIR (FT_E * (FT_E - 1) / 2)
 
 // ------------------------------------------------------------------ parameter block
-// doubles: 0 D, 1 W, 2 IGtr, 3 def_ref, 4 1/(D/2*L+W), 5 Jr(full), 6 unused, 7 unused,
+// doubles: 0 D, 1 W, 2 IGtr, 3 def_ref, 4 norm = 1/(D/2*L+W), 5 Jr(full), 6 -norm D/2, 7 -norm W,
 // then m2[E], nu[E], sigma[RANK], q[RANK][N], then P~ on the external rows [Q0, N)
 // (its upper triangle row by row, off-diagonal entries doubled)
 #define P_D 0
@@ -136,6 +136,9 @@ static __device__ constexpr bool first_in_slot(int e)
 #define P_DEF 3
 #define P_NORM 4
 #define P_JRFULL 5
+#define P_NORM_F 6
+#define P_NORM_G 7
+#define LN2_D 0.693147180559945309417
 #define P_M2 8
 #define P_NU (8 + FT_E)
 #define P_SIG (8 + 2 * FT_E)
@@ -272,19 +275,163 @@ static __device__ __forceinline__ cx<double> cpow_(cx<double> z, double y)
 #if FT_PREC == 0
 // ------------------------------------------------------------------ FP64 functions
 // The FP64 pipe takes 16 cycles of the whole SM per warp instruction (64x fewer lanes than
-// FP32), so the FP64 form costs what it issues there and integer work beside it is free.
-// Its functions are written for few FP64 instructions: table-driven after Tang (ACM TOMS
-// 15 (1989), 16 (1990); 18 (1992)) with the argument's exponent and table index taken by
-// integer operations, short polynomials (Taylor: the reduced arguments are below 0.013) and
-// textbook Newton steps from the approximate reciprocal.  Their results are within about an ulp
-// (log in two parts: 2^-62 absolute); arguments outside the stated ranges take the CUDA
-// library's function (out of line).  FP64 instructions: reciprocal 3, log 15, exp 12,
-// sincos 18, arg 17.  With them and the leaner algebra below the FP64 form issues half the
-// FP64 instructions per sample of the library's functions on the double box, a third on K4.
+// FP32) and bounds the FP64 form, with nine tenths of the issue slots idle.  Its powers,
+// exponentials, logarithms, sines and cosines are therefore evaluated in 64-bit fixed point
+// on the integer pipes (about 200 instructions each, where table-driven FP64 versions
+// issued 12 to 31 FP64 ones, several times their cost), table-driven after Tang (ACM TOMS
+// 15 (1989), 16 (1990), 17 (1991)) with Taylor polynomials, and assembled into doubles by
+// their bits.  Their error before the final rounding is below 2^-57, so results are within
+// 0.6 ulp (sines and cosines: 2^-58 absolute).  Reciprocals and arguments stay on the FP64
+// pipe (3 and 17 instructions).  Arguments outside the stated ranges take the CUDA library's
+// function (out of line).  Qn: a fixed-point number in units of 2^-n.
 static __device__ __forceinline__ int hi_word(double x) { return __double2hiint(x); }
 static __device__ __forceinline__ int exponent_of(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
 static __device__ __forceinline__ bool finite_(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
 static __device__ __forceinline__ double pow2_of(int e) { return __hiloint2double((1023 + e) << 20, 0); }
+static __device__ __forceinline__ bool normal_positive(double x) { return (u32)(hi_word(x) - 0x00100000) < 0x7fe00000u; }
+// the significand of a normal x, Q63 in [1, 2)
+static __device__ __forceinline__ u64 mantissa_of(double x) { return ((u64)__double_as_longlong(x) << 11) | (1ull << 63); }
+// w 2^e, w in Q63 with its top bit set, rounded to a double (e in the normal range)
+static __device__ __forceinline__ double round_q63(u64 w, int e)
+{
+    return __longlong_as_double((long long)(((u64)(1022 + e) << 52) + (w >> 11) + ((w >> 10) & 1ull)));
+}
+// v in Qq as a double
+static __device__ __forceinline__ double double_of(u64 v, int q)
+{
+    if (v == 0ull) return 0.0;
+    const int lz = __clzll((long long)v);
+    return round_q63(v << lz, 63 - lz - q);
+}
+// log2 of m 2^-52 in [1, 2): Q62 in [0, 1].  With i its top 8 fraction bits, r_i is 10 bits at
+// least 1024 / M, so that z = M r / 1024 - 1 is exact and in [0, 0.005)
+static __device__ __forceinline__ u64 log2_q62(u64 m)
+{
+    const ulonglong2 t = FT_LOG64[(m >> 44) & 255ull];   // r, -log2(r / 1024) in Q62
+    const u64 z = (m * t.x - (1ull << 62)) << 8;        // Q70
+    u64 h = (1ull << 63) / 7ull;                         // Q63
+    h = (1ull << 63) / 6ull - (__umul64hi(z, h) >> 6);
+    h = (1ull << 63) / 5ull - (__umul64hi(z, h) >> 6);
+    h = (1ull << 63) / 4ull - (__umul64hi(z, h) >> 6);
+    h = (1ull << 63) / 3ull - (__umul64hi(z, h) >> 6);
+    h = (1ull << 63) / 2ull - (__umul64hi(z, h) >> 6);
+    const u64 l = z - (__umul64hi(__umul64hi(z, z), h) >> 5);   // log1p z, Q70
+    const u64 f = t.y + (__umul64hi(l, FT_LOG2E_Q63) >> 7);
+    return f < (1ull << 62) ? f : (1ull << 62);
+}
+// 2^(f - n), f in Q64
+static __device__ __forceinline__ double exp2_q64(u64 f, int n)
+{
+    const u64 T = FT_EXP64[f >> 56];                     // 2^(j/256), Q63
+    const u64 w = __umul64hi(f << 8, FT_LN2_Q64);       // Q72, below ln2/256
+    u64 h = (1ull << 63) / 120ull;
+    h = (1ull << 63) / 24ull + (__umul64hi(w, h) >> 8);
+    h = (1ull << 63) / 6ull + (__umul64hi(w, h) >> 8);
+    h = (1ull << 63) / 2ull + (__umul64hi(w, h) >> 8);
+    h = (1ull << 63) + (__umul64hi(w, h) >> 8);
+    const u64 R = T + (__umul64hi(T, __umul64hi(w, h)) >> 7);
+    return round_q63(R, -n);
+}
+static __device__ __noinline__ double pow_slow(double x, double y) { return pow(x, y); }
+// (1 - u)^y, u = (x >> 11) 2^-53
+static __device__ __forceinline__ double pow_1mu(u64 x, double y)
+{
+    const u64 q = (~x & ~0x7ffull) + 0x800ull;   // (1 - u) 2^64, 0 for u = 0
+    if (q == 0ull) return 1.0;
+    const int lz = __clzll((long long)q), K = 1 + lz;
+    const u64 F = log2_q62((q << lz) >> 11);
+    // -log2(1 - u) = K - F, K in b bits: Q(64 - b)
+    const int b = 32 - __clz(K);
+    const u64 L = ((u64)K << (64 - b)) - ((F << 1) >> (b - 1));
+    const u64 P = __umul64hi(L, mantissa_of(y));
+    const int S = 63 - b - (exponent_of(y) - 1023);   // y log2 = P 2^-S
+    const int n = S < 64 ? (int)min(P >> (S & 63), 100000ull) : 0;
+    if (!normal_positive(y) || S < 1 || n > 1000) return pow_slow(1.0 - u01(x), y);
+    const u64 f = S < 64 ? P << (64 - S) : (S < 128 ? P >> (S - 64) : 0ull);   // S = 64: P
+    return exp2_q64(0ull - f, n + (f != 0ull));
+}
+// log2 x = k + f of a positive normal x, f in [0, 1] (a double), k an integer
+struct log2_parts {
+    int k;
+    double kd, f;
+};
+static __device__ __forceinline__ double small_int(int k)
+{
+    const double v = double_of((u64)(k < 0 ? -k : k), 0);
+    return k < 0 ? -v : v;
+}
+static __device__ __forceinline__ log2_parts log2_64(double x)
+{
+    log2_parts r;
+    r.k = (hi_word(x) >> 20) - 1023;
+    r.kd = small_int(r.k);
+    r.f = double_of(log2_q62((u64)__double_as_longlong(x) & 0xfffffffffffffull | (1ull << 52)), 62);
+    return r;
+}
+// x added to the fixed-point number i + f 2^-64 (|x| < 2^31)
+static __device__ __forceinline__ void fixed_add(double x, int& i, u64& f)
+{
+    const int e = exponent_of(x) - 1023;
+    const u64 m = mantissa_of(x);
+    int I = e >= 0 ? (int)(m >> ((63 - e) & 63)) : 0;
+    u64 F = e >= 0 ? (m << (e & 63)) << 1 : (e >= -64 ? m >> (-e - 1) : 0ull);
+    if (hi_word(x) < 0) {
+        I = -I - (F != 0ull);
+        F = 0ull - F;
+    }
+    f += F;
+    i += I + (f < F);
+}
+static __device__ __noinline__ double exp2_slow(double t) { return exp2(t); }
+// 2^(a (la.k + la.f) + b (lb.k + lb.f)): the products with their errors, summed in fixed point
+static __device__ __forceinline__ double power_product(double a, log2_parts la, double b, log2_parts lb)
+{
+    const double p = a * la.kd, q = b * lb.kd;
+    const double u = fma(a, la.f, fma(a, la.kd, -p)), v = fma(b, lb.f, fma(b, lb.kd, -q));
+    const int big = max(max(exponent_of(p), exponent_of(q)), max(exponent_of(u), exponent_of(v)));
+    if (big >= 1023 + 12) return exp2_slow((p + q) + (u + v));
+    int i = 0;
+    u64 f = 0ull;
+    fixed_add(p, i, f);
+    fixed_add(q, i, f);
+    fixed_add(u, i, f);
+    fixed_add(v, i, f);
+    if (i > 1000 || i < -1000) return exp2_slow((p + q) + (u + v));
+    return exp2_q64(f, -i);
+}
+static __device__ __noinline__ void sincos_slow(double x, double* s, double* c) { sincos(x, s, c); }
+// 256 steps per turn, 64 of them in the table
+static __device__ __forceinline__ void sincos_64(double x, double& sn, double& cs)
+{
+    if ((u32)(hi_word(x) & 0x7fffffff) > 0x40f86a00u) {   // |x| > 1e5
+        sincos_slow(x, &sn, &cs);
+        return;
+    }
+    // |x| 128/pi = m C 2^e, C in Q58 and 64 more bits
+    const int S = 57 - (exponent_of(x) - 1023);
+    const u64 m = mantissa_of(x), c0 = m * FT_STEPS_Q58;
+    const u64 lo = c0 + __umul64hi(m, FT_STEPS_LO);
+    const u64 hi = __umul64hi(m, FT_STEPS_Q58) + (lo < c0);
+    const u32 k = S < 64 ? (u32)(hi >> (S & 63)) : 0u;
+    const u64 f = S < 64 ? (hi << ((64 - S) & 63)) | (lo >> (S & 63)) : (S < 128 ? hi >> (S - 64) : 0ull);   // Q64
+    const u64 w = __umul64hi(f, FT_STEP_Q69), w2 = __umul64hi(w, w);   // Q69, Q74
+    u64 h = (1ull << 63) / 120ull - (__umul64hi(w2, (1ull << 63) / 5040ull) >> 10);
+    h = (1ull << 63) / 6ull - (__umul64hi(w2, h) >> 10);
+    const u64 s = __umul64hi(w, (1ull << 63) - (__umul64hi(w2, h) >> 10));   // sin w, Q68
+    h = (1ull << 63) / 720ull - (__umul64hi(w2, (1ull << 63) / 40320ull) >> 10);
+    h = (1ull << 63) / 24ull - (__umul64hi(w2, h) >> 10);
+    h = (1ull << 63) / 2ull - (__umul64hi(w2, h) >> 10);
+    const u64 v = __umul64hi(w2, h);   // 1 - cos w, Q73
+    const ulonglong2 T = FT_SC64[k & 63u];   // sin, cos of k pi/128, Q63
+    const u64 A = (T.x >> 1) + (__umul64hi(T.y, s) >> 5) - (__umul64hi(T.x, v) >> 10);
+    const u64 B0 = (T.y >> 1) - (__umul64hi(T.y, v) >> 10), B1 = __umul64hi(T.x, s) >> 5;
+    const double a = double_of(A, 62), b = double_of(B0 > B1 ? B0 - B1 : 0ull, 62);
+    const bool odd = (k >> 6) & 1u, up = (k >> 7) & 1u;   // quadrant
+    sn = odd ? b : a;
+    cs = odd ? a : b;
+    if (up != (hi_word(x) < 0)) sn = -sn;
+    if (odd != up) cs = -cs;
+}
 
 static __device__ __noinline__ double rcp_slow(double x) { return 1.0 / x; }
 static __device__ __forceinline__ double rcp64(double x)
@@ -295,84 +442,6 @@ static __device__ __forceinline__ double rcp64(double x)
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
     const double e = fma(-x, r, 1.0);
     return fma(r, fma(e, e, e), r);
-}
-
-struct dd {
-    double hi, lo;
-};
-static __device__ __forceinline__ dd dd_mk(double h, double l)
-{
-    dd r;
-    r.hi = h;
-    r.lo = l;
-    return r;
-}
-// log(2^k M), M in [1, 2) with i its top 7 fraction bits: r_i a 9-bit approximation of 1/M
-// there, so that z = M r_i - 1 is exact, |z| < 0.006; -log r_i in two parts, the first a
-// multiple of 2^-41 like that of ln 2, so that k ln2 - log r_i is exact in the first.  The
-// result's low part is not below the high one's last place (up to 2e-5): add them where one
-// number is wanted.
-static __device__ __forceinline__ dd log_parts(double M, int i, int k)
-{
-    const double kd = __hiloint2double(0x43300000, k ^ 0x80000000) - 4503601774854144.0;   // k
-    const double2 a = FT_LOG64[2 * i], b = FT_LOG64[2 * i + 1];   // r, hi; lo, -
-    const double z = fma(M, a.x, -1.0);
-    const double H = fma(kd, FT_LN2_HI, a.y);
-    const double z2 = z * z;
-    const double P = fma(
-        z, fma(z, fma(z, fma(z, fma(z, 1.0 / 7.0, -1.0 / 6.0), 1.0 / 5.0), -1.0 / 4.0), 1.0 / 3.0), -1.0 / 2.0);
-    const double lo = fma(z2, P, fma(kd, FT_LN2_LO, b.x));
-    const double s = H + z;
-    return dd_mk(s, (z - (s - H)) + lo);
-}
-// log(1 - u), u = (x >> 11) 2^-53
-static __device__ __forceinline__ dd log1m_64(u64 x)
-{
-    const u64 q = (~x & ~0x7ffull) + 0x800ull;   // (1 - u) 2^64, 0 for u = 0
-    if (q == 0ull) return dd_mk(0.0, 0.0);
-    const int lz = __clzll((long long)q);
-    const u64 mb = q << lz;
-    const double M = __longlong_as_double((long long)(((mb >> 11) & 0xfffffffffffffull) | 0x3ff0000000000000ull));
-    return log_parts(M, (int)((mb >> 56) & 127ull), -1 - lz);
-}
-// log x of a positive normal x
-static __device__ __forceinline__ bool normal_positive(double x) { return (u32)(hi_word(x) - 0x00100000) < 0x7fe00000u; }
-static __device__ __forceinline__ dd log_64(double x)
-{
-    const int h = hi_word(x);
-    return log_parts(__hiloint2double((h & 0xfffff) | 0x3ff00000, __double2loint(x)), (h >> 13) & 127, (h >> 20) - 1023);
-}
-static __device__ __noinline__ double exp_slow(double x) { return exp(x); }
-// e^(hi + lo), |lo| far below 1: 128 steps per octave, |r| < 0.0028
-static __device__ __forceinline__ double exp_64(double hi, double lo)
-{
-    if ((u32)(hi_word(hi) & 0x7fffffff) > 0x40858000u) return exp_slow(hi + lo);   // |hi| > 691
-    const double MAGIC = 6755399441055744.0;
-    const double t = fma(hi, FT_EXP_C, MAGIC), kd = t - MAGIC;
-    const int k = __double2loint(t);
-    const double r = fma(kd, -FT_EXP_L2, fma(kd, -FT_EXP_L1, hi)) + lo;
-    const double q = fma(r * r, fma(r, fma(r, fma(r, 1.0 / 120.0, 1.0 / 24.0), 1.0 / 6.0), 0.5), r);
-    const double2 T = FT_EXP64[k & 127];
-    const double v = T.x + fma(T.x, q, T.y);
-    return __hiloint2double(hi_word(v) + ((k >> 7) << 20), __double2loint(v));
-}
-static __device__ __noinline__ void sincos_slow(double x, double* s, double* c) { sincos(x, s, c); }
-// 256 steps per turn, |r| <= pi/256
-static __device__ __forceinline__ void sincos_64(double x, double& sn, double& cs)
-{
-    if ((u32)(hi_word(x) & 0x7fffffff) > 0x40f86a00u) {   // |x| > 1e5
-        sincos_slow(x, &sn, &cs);
-        return;
-    }
-    const double MAGIC = 6755399441055744.0;
-    const double t = fma(x, FT_SC_C, MAGIC), kd = t - MAGIC;
-    const double2 T = FT_SC64[__double2loint(t) & 255];   // sin, cos
-    const double r = fma(kd, -FT_SC_P2, fma(kd, -FT_SC_P1, x));
-    const double r2 = r * r;
-    const double s = fma(r2 * r, fma(r2, fma(r2, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), r);
-    const double c = r2 * fma(r2, fma(r2, -1.0 / 720.0, 1.0 / 24.0), -0.5);
-    sn = T.x + fma(T.y, s, T.x * c);
-    cs = T.y + fma(-T.x, s, T.y * c);
 }
 static __device__ __noinline__ double arg_slow(double y, double x) { return atan2(y, x); }
 // principal argument of re + i im: with x, y the larger and smaller modulus, c = i/128 the
@@ -412,18 +481,6 @@ static __device__ __forceinline__ cx<double> cinv_64(cx<double> z)
     const double m = rcp64(fma(z.re, z.re, z.im * z.im));
     return cmk(z.re * m, -z.im * m);
 }
-// t (hi + lo) of a two-part logarithm and a factor
-static __device__ __forceinline__ dd dd_times(double t, dd l)
-{
-    const double p = t * l.hi;
-    return dd_mk(p, fma(t, l.lo, fma(t, l.hi, -p)));
-}
-static __device__ __forceinline__ dd dd_plus(dd a, dd b)
-{
-    const double s = a.hi + b.hi, bb = s - a.hi;
-    return dd_mk(s, ((a.hi - (s - bb)) + (b.hi - bb)) + (a.lo + b.lo));
-}
-
 // ------------------------------------------------------------------ robust complex LU
 // Complete-pivoting LU of the complex reduced Laplacian (largest modulus, first in
 // column-major order), used when the static elimination reports pivot growth.
@@ -830,10 +887,7 @@ static __device__ __forceinline__ void draw_sector64(xo& g, const table_ref& t, 
         if (META_L(m) < META_L(meta)) F *= XX;
         meta = m;
         if (FT_RECORD) ord[j] = (unsigned char)e;
-        if (j < FT_E - 1) {
-            const dd l = dd_times(rinv, log1m_64(g.next()));
-            XX *= exp_64(l.hi, l.lo);
-        }
+        if (j < FT_E - 1) XX *= pow_1mu(g.next(), rinv);
     }
 }
 
@@ -882,9 +936,7 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
     // normalise so that psi_tr^(-D/2) (psi_tr/xi_tr)^W = 1 (srcs/feynman_integral.hpp:201-204)
     double scale;
     if (normal_positive(psi_tr) && normal_positive(Gv)) {
-        const dd l = dd_plus(dd_times(-0.5 * D, log_64(psi_tr)), dd_times(-W, log_64(Gv)));
-        const dd t = dd_times(prm[P_NORM], l);
-        scale = exp_64(t.hi, t.lo);
+        scale = power_product(prm[P_NORM_F], log2_64(psi_tr), prm[P_NORM_G], log2_64(Gv));
     } else {
         scale = scale_slow(psi_tr, Gv, D, W, prm[P_NORM]);
     }
@@ -966,20 +1018,18 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
         for (int j = 0; j < FT_K; j++) out[j] = cmk(R[j], 0.0);
         return ok;
     }
-    const dd lp = log_64(psi);
+    const log2_parts lp = log2_64(psi);
 #if FT_ONLY_PSI
-    const dd t = dd_times(-0.5 * D, lp);
-    const double v = IGtr * exp_64(t.hi, t.lo);
+    const double v = IGtr * power_product(-0.5 * D, lp, 0.0, lp);
     if (!finite_(v)) return false;
     out[0] = cmk(v, 0.0);
 #else
-    const dd lv = log_64(pxi);
-    const dd t = dd_plus(dd_times(-0.5 * D, lp), dd_times(-W, lv));
-    double v = IGtr * exp_64(t.hi, t.lo);
+    const log2_parts lv = log2_64(pxi);
+    double v = IGtr * power_product(-0.5 * D, lp, -W, lv);
     if (!finite_(v)) return false;
     out[0] = cmk(v, 0.0);
     if (FT_K > 1) {
-        const double ef = fma(-(double)FT_LOOPS, lv.hi + lv.lo, lp.hi + lp.lo);
+        const double ef = LN2_D * (small_int(lp.k - FT_LOOPS * lv.k) + fma(-(double)FT_LOOPS, lv.f, lp.f));
 #pragma unroll
         for (int j = 1; j < FT_K; j++) {
             v *= ef * (1.0 / (double)j);
@@ -1266,19 +1316,21 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
         detJ = (Xprod * pow2_of(-sum) * pow2_of(-sum)) * detJ;   // prod X / D^2
     }
     // cR = IGtr cPsi^(-D/2) cV^(-W) det J e^(i nu . theta)
-    cx<double> lp, lv, pw;
+    cx<double> ef, pw;   // log cPsi - L log cV, the powers
     const double np = fma(cPsi.re, cPsi.re, cPsi.im * cPsi.im), nv = fma(cV.re, cV.re, cV.im * cV.im);
     if (normal_positive(np) && normal_positive(nv)) {
-        const dd a2 = log_64(np), b2 = log_64(nv);
-        lp = cmk(0.5 * (a2.hi + a2.lo), arg_64(cPsi.re, cPsi.im));
-        lv = cmk(0.5 * (b2.hi + b2.lo), arg_64(cV.re, cV.im));
-        const dd t = dd_plus(dd_times(-0.25 * D, a2), dd_times(-0.5 * W, b2));
-        const double m = exp_64(t.hi, t.lo);
+        const log2_parts a2 = log2_64(np), b2 = log2_64(nv);
+        const double ap = arg_64(cPsi.re, cPsi.im), av = arg_64(cV.re, cV.im);
+        ef = cmk(0.5 * LN2_D * (small_int(a2.k - FT_LOOPS * b2.k) + fma(-(double)FT_LOOPS, b2.f, a2.f)),
+                 fma(-(double)FT_LOOPS, av, ap));
+        const double m = power_product(-0.25 * D, a2, -0.5 * W, b2);
         double sn, cs;
-        sincos_64(fma(-0.5 * D, lp.im, -W * lv.im), sn, cs);
+        sincos_64(fma(-0.5 * D, ap, -W * av), sn, cs);
         pw = cmk(m * cs, m * sn);
     } else {
+        cx<double> lp, lv;
         pw = powers_slow(cPsi, cV, D, W, lp, lv);
+        ef = cmk(lp.re - FT_LOOPS * lv.re, lp.im - FT_LOOPS * lv.im);
     }
     double sn, cs;
     sincos_64(xnu, sn, cs);
@@ -1286,7 +1338,6 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
     if (!finite_(cR.re) || !finite_(cR.im)) return false;
     out[0] = cR;
     if (FT_K > 1) {
-        const cx<double> ef = cmk(fma(-(double)FT_LOOPS, lv.re, lp.re), fma(-(double)FT_LOOPS, lv.im, lp.im));
 #pragma unroll
         for (int j = 1; j < FT_K; j++) {
             cR = cR * ((1.0 / (double)j) * ef);

@@ -212,6 +212,8 @@ void build_blocks(ft_plan& pl)
     pl.prm[3] = p.def_ref;
     pl.prm[4] = 1. / (p.D / 2. * p.loops + p.W);
     pl.prm[5] = p.Jr[(1ULL << E) - 1];
+    pl.prm[6] = -pl.prm[4] * (p.D / 2.);
+    pl.prm[7] = -pl.prm[4] * p.W;
     for (int e = 0; e < E; e++) {
         pl.prm[8 + e] = p.m2[e];
         pl.prm[8 + E + e] = p.nu[e];
