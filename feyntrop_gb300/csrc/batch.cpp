@@ -174,7 +174,7 @@ void build(ft_batch& b)
         ft_plan* pl = b.plans[i];
         if (!pl) throw std::invalid_argument("ft_batch_create: NULL plan");
         if (pl->device != b.device) throw std::invalid_argument("ft_batch_create: plans on different devices");
-        const ft::kernel_key k = pl->key(prec, 0);
+        const ft::kernel_key k = pl->key(prec, 0, 1);
         const std::string id = class_id(k);
         auto it = ids.find(id);
         if (it == ids.end()) {
@@ -194,11 +194,9 @@ void build(ft_batch& b)
     std::vector<ft::kernel_key> keys, keys64;
     for (ft_batch::group& g : b.groups) {
         g.key.rank = g.rank;
-        g.key.batch = 1;
         keys.push_back(g.key);
-        ft::kernel_key k64 = b.plans[g.members[0]]->key(0, 0);
+        ft::kernel_key k64 = b.plans[g.members[0]]->key(0, 0, 1);
         k64.rank = g.rank;
-        k64.batch = 1;
         keys64.push_back(k64);
     }
     {
@@ -217,7 +215,7 @@ void build(ft_batch& b)
         const ft::launch_shape tuned = ft::choose_shape(g.key);
         g.chunk = ft::chunk_override()
                       ? ft::chunk_override()
-                      : env_u64("FEYNTROP_GB300_BATCH_CHUNK", tuned.chunk ? tuned.chunk : (prec ? 128 : 16));
+                      : env_u64("FEYNTROP_GB300_BATCH_CHUNK", tuned.chunk ? tuned.chunk : ft::default_chunk(g.key));
         if (g.chunk < 1 || g.chunk >= (1ull << 18)) throw std::invalid_argument("batch chunk out of range");
         g.grid = (unsigned)(ds.sms * g.ks->blocks_per_sm);
         g.qgrid = prec ? (unsigned)(ds.sms * 2) : 0;

@@ -89,7 +89,7 @@ struct ft_plan {
     int forced_prec = 0;
     ft::launch_shape forced_shape;
 
-    ft::kernel_key key(int prec, int record) const
+    ft::kernel_key key(int prec, int record, int batch = 0) const
     {
         ft::kernel_key k;
         k.E = P.E;
@@ -101,6 +101,7 @@ struct ft_plan {
         k.mode = P.deformed() ? 1 : 0;
         k.only_psi = P.only_psi() ? 1 : 0;
         k.record = record;
+        k.batch = batch;
         k.ek = kek;
         k.el = kel;
         k.q0 = q0;

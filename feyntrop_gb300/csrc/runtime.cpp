@@ -680,14 +680,8 @@ int ft_precompile(const ft_problem* pb, int32_t precision, double* seconds)
         const bool batch = (precision & FT_PRECOMPILE_BATCH) != 0;
         std::vector<ft::kernel_key> keys;
         for (int bt = 0; bt <= (batch ? 1 : 0); bt++) {
-            ft::kernel_key k = pl.key(0, 0);
-            k.batch = bt;
-            keys.push_back(k);
-            if (prec == FT_PRECISION_MIXED) {
-                k = pl.key(1, 0);
-                k.batch = bt;
-                keys.push_back(k);
-            }
+            keys.push_back(pl.key(0, 0, bt));
+            if (prec == FT_PRECISION_MIXED) keys.push_back(pl.key(1, 0, bt));
         }
         ft::precompile_all(keys);
         if (seconds) *seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -850,10 +844,10 @@ int ft_autotune(ft_plan* pl, int32_t precision, uint64_t samples, ft_tune_result
             // per SM) to 255 (8 warps, no spills)
             // (four 128-thread blocks won one-integral trials by noise and ran the
             // persistent batch kernel 9 % slower: not a candidate)
-            add(256, 2, 29);
             add(512, 1, 29);
+            add(256, 2, 29);
             add(384, 1, 29);
-            add(384, 1, 21);
+            add(256, 2, 21);
             add(256, 2, 5);
             add(256, 1, 29);
         } else if (prec == 1) {
@@ -863,9 +857,12 @@ int ft_autotune(ft_plan* pl, int32_t precision, uint64_t samples, ft_tune_result
                 add(512, 1, var);
             }
         } else {
-            const int v = deformed ? 1 : 0;
-            for (int var : {v | 4, v})
-                for (int bm : {256, 128, 512}) add(bm, bm == 128 ? 2 : 1, var);
+            for (int var : {4, 0}) {
+                add(256, 1, var);
+                add(256, 2, var);
+                add(384, 1, var);
+                add(512, 1, var);
+            }
         }
         {
             // every candidate's kernels compiled concurrently before the timing
@@ -938,11 +935,11 @@ int ft_autotune(ft_plan* pl, int32_t precision, uint64_t samples, ft_tune_result
         // largest item leaves every SM four items
         double best_batch = -1, default_batch = -1;
         unsigned long long best_chunk = 0;
-        const unsigned long long default_chunk = prec ? 128ull : 16ull;
+        const unsigned long long default_chunk = ft::default_chunk(pl->key(prec, 0));
         const uint64_t bsamples =
             std::max<uint64_t>(tsamples, (uint64_t)dev_state().sms * (uint64_t)pl->key(prec, 0).block * 256ull * 4ull);
-        for (unsigned long long c : {16ull, 32ull, 64ull, 128ull, 256ull}) {
-            if (c == 16 && prec) continue;   // below the mixed default's range
+        for (unsigned long long c : {8ull, 16ull, 32ull, 64ull, 128ull, 256ull}) {
+            if (prec ? c < 32 : c > 64) continue;   // outside the precision's range
             ft::set_chunk_override(c);
             ft_batch* b = nullptr;
             int rc = ft_batch_create(&pl, 1, prec, &b);

@@ -82,25 +82,41 @@ std::string tune_class(const kernel_key& k)
 
 launch_shape default_shape(const kernel_key& k)
 {
-    // GB300 sweeps.  Mixed form: the per-sample barrier (variant bit 2) makes the warps of a
-    // block share their instruction fetches.  Undeformed (two samples per thread) 256 threads
-    // with up to 255 registers (five-loop cube, N = 5e7: 5.3 ms; 512 x 128 registers 5.4,
-    // 384 7.1).  Deformed: 16 warps of 128 registers per SM, with one out-of-line copy of the
-    // FP32 transcendentals, of the larger two-float routines and of the complex two-float
-    // product (bits 0, 3, 4): 3-loop ladder 1.35e9 samples/s (inlined 0.86e9), box-pentagon
-    // 1.73e9 (inlined 1.72e9, 12 warps of 168 registers 1.48e9), double box 2.62e9 (12 warps
-    // 2.77e9), one-loop box 5.8e9.  The FP64 form is FP64-pipe bound (256 x 1); the barrier
-    // keeps its warps from drifting apart too (cube +10 %, double box +1 %).
+    // GB300 sweeps.  The per-sample barrier (variant bit 2) makes the warps of a block share
+    // their instruction fetches.
+    // Mixed, undeformed (two samples per thread): 256 threads with up to 255 registers
+    // (five-loop cube, N = 5e7: 5.3 ms; 512 x 128 registers 5.4, 384 7.1).
+    // Mixed, deformed: 16 warps of 128 registers per SM, with one out-of-line copy of the FP32
+    // transcendentals, of the larger two-float routines and of the complex two-float product
+    // (bits 0, 3, 4).  One block of 512 keeps all of them together (samples/s against two
+    // blocks of 256: double box 3.00e9 / 2.73e9, six-edge one-loop 2.70e9 / 2.43e9, 3-loop
+    // ladder 1.36e9 / 1.28e9, box-pentagon 1.81e9 / 1.80e9; 12 warps of 168 registers 2.97e9
+    // on the double box, 1.17e9 on the ladder); in a batch, where a block also waits for
+    // its slowest warp at every item's end, two blocks are as fast or faster (24
+    // box-pentagon points 12.4 ms against 12.8).
+    // FP64 form, bound by the FP64 pipe: 12 to 16 warps per SM keep it busy (double box 3e6:
+    // 7.1 ms with 384 threads, 7.4 with 256; box-pentagon scan 3.4 against 4.5; cube 1.26 with
+    // 512 against 1.40), two blocks where the staged table leaves the room (up to E = 10; K4
+    // 3.13 ms, one block of 512 3.48).
     launch_shape s;
     if (k.prec == 1) {
-        s.block = 256;
-        s.minb = k.mode == 1 ? 2 : 1;
-    } else {
-        s.block = 256;
+        s.block = k.mode == 1 && !k.batch ? 512 : 256;
+        s.minb = k.mode == 1 && k.batch ? 2 : 1;
+    } else if (k.mode == 1) {
+        s.block = 384;
         s.minb = 1;
+    } else {
+        s.block = k.E > 10 ? 512 : 256;
+        s.minb = k.E > 10 ? 1 : 2;
     }
-    s.variant = (k.prec == 1 && k.mode == 1) ? 29 : (k.mode == 1 ? 5 : 4);
+    s.variant = (k.prec == 1 && k.mode == 1) ? 29 : 4;
     return s;
+}
+
+unsigned long long default_chunk(const kernel_key& k)
+{
+    if (k.prec == 1) return k.mode == 1 ? 32 : 128;
+    return k.mode == 1 ? 8 : 16;
 }
 
 // Shared memory of one block: the dynamic part (staged table, sums) plus the kernel
@@ -139,7 +155,16 @@ launch_shape choose_shape(const kernel_key& k)
         std::lock_guard<std::mutex> lock(g_mu);
         load_locked();
         auto it = g_table.find(tune_class(k));
-        if (it != g_table.end()) s = it->second;
+        if (it != g_table.end()) {
+            // a class whose default won its trials (one integral each) keeps the batch default too
+            kernel_key single = k;
+            single.batch = 0;
+            const launch_shape d = default_shape(single), &t = it->second;
+            if (k.batch && t.block == d.block && t.minb == d.minb && t.variant == d.variant)
+                s.chunk = t.chunk;
+            else
+                s = t;
+        }
     }
     if (const char* e = std::getenv("FEYNTROP_GB300_BLOCK")) s.block = std::atoi(e);
     if (const char* e = std::getenv("FEYNTROP_GB300_MINB")) s.minb = std::atoi(e);
