@@ -74,7 +74,7 @@ struct ft_batch {
         unsigned long long* d_mats = nullptr;        // stride matrices of the chunk
         unsigned long long* d_item_mats = nullptr;   // powers of the item stride, item_digits octal digits
         int item_digits = 0, want_digits = 0;
-        unsigned long long* d_state = nullptr;       // the integrals' start states
+        unsigned long long* d_state = nullptr;       // the integrals' start states (with the above in d_static)
         size_t item_cap = 0;
         double* d_parts = nullptr;
         unsigned long long* d_queue = nullptr;
@@ -91,9 +91,10 @@ struct ft_batch {
     std::vector<int> group_of, slot_of;     // per plan: class and position in it
     // run descriptors: [class headers][batch_inst records][item_prep records], copied in
     size_t desc_bytes = 0, hdr_bytes = 0, out_doubles = 0, qacc_words = 0;
-    unsigned char* h_desc = nullptr;
-    unsigned char* d_desc = nullptr;
-    double* d_out = nullptr;     // per integral 8K+8 sums
+    unsigned char* d_static = nullptr;   // every class's parameters, tables, stride matrices, start states
+    unsigned char* h_desc = nullptr;     // pinned; h_out and h_hdr_out follow it
+    unsigned char* d_desc = nullptr;     // d_out and d_qacc follow it
+    double* d_out = nullptr;   // per integral 8K+8 sums
     double* h_out = nullptr;
     class_header* h_hdr_out = nullptr;
     unsigned long long* d_qacc = nullptr;   // per integral the FP64 pass's exact accumulators (exact_words)
@@ -109,22 +110,15 @@ struct ft_batch {
     {
         if (exec) cudaGraphExecDestroy(exec);
         for (group& g : groups) {
-            cudaFree(g.d_prm);
-            cudaFree(g.d_tab);
-            cudaFree(g.d_mats);
             cudaFree(g.d_item_mats);
-            cudaFree(g.d_state);
             cudaFree(g.d_parts);
             cudaFree(g.d_queue);
             if (g.stream) cudaStreamDestroy(g.stream);
             if (g.done) cudaEventDestroy(g.done);
         }
         if (h_desc) cudaFreeHost(h_desc);
-        if (h_out) cudaFreeHost(h_out);
-        if (h_hdr_out) cudaFreeHost(h_hdr_out);
+        cudaFree(d_static);
         cudaFree(d_desc);
-        cudaFree(d_out);
-        cudaFree(d_qacc);
         if (stream) cudaStreamDestroy(stream);
         if (fork) cudaEventDestroy(fork);
         if (ev0) cudaEventDestroy(ev0);
@@ -204,7 +198,11 @@ void build(ft_batch& b)
         if (prec) all.insert(all.end(), keys64.begin(), keys64.end());
         ft::precompile_all(all);
     }
-    size_t hdr = 0, inst = 0, prep = 0;
+    size_t hdr = 0, inst = 0, prep = 0, total = 0;
+    // every class's parameter blocks and tables (copied in one go), then the room for its
+    // stride matrices and start states
+    std::vector<unsigned char> blob;
+    std::vector<std::vector<size_t>> off(b.groups.size());
     for (size_t gi = 0; gi < b.groups.size(); gi++) {
         ft_batch::group& g = b.groups[gi];
         const ft_plan& p0 = *b.plans[g.members[0]];
@@ -224,21 +222,16 @@ void build(ft_batch& b)
         const std::vector<double> blk0 = param_block(padded_params(p0, g.rank));
         g.prm_stride = align_up(blk0.size() * 8, 256);
         g.tab_stride = align_up(p0.tab.size(), 256);
-        std::vector<unsigned char> hp(g.prm_stride * nm, 0), ht(g.tab_stride * nm, 0);
+        const size_t o_prm = total, o_tab = o_prm + g.prm_stride * nm;
+        total = o_tab + g.tab_stride * nm;
+        blob.resize(total, 0);
         for (size_t m = 0; m < nm; m++) {
             const ft_plan& pl = *b.plans[g.members[m]];
             const std::vector<double> blk = param_block(padded_params(pl, g.rank));
-            std::memcpy(hp.data() + m * g.prm_stride, blk.data(), blk.size() * 8);
-            std::memcpy(ht.data() + m * g.tab_stride, pl.tab.data(), pl.tab.size());
+            std::memcpy(blob.data() + o_prm + m * g.prm_stride, blk.data(), blk.size() * 8);
+            std::memcpy(blob.data() + o_tab + m * g.tab_stride, pl.tab.data(), pl.tab.size());
         }
-        cu(cudaMalloc(&g.d_prm, hp.size()), "cudaMalloc(batch parameters)");
-        cu(cudaMalloc(&g.d_tab, ht.size()), "cudaMalloc(batch tables)");
-        cu(cudaMemcpy(g.d_prm, hp.data(), hp.size(), cudaMemcpyHostToDevice), "cudaMemcpy(batch parameters)");
-        cu(cudaMemcpy(g.d_tab, ht.data(), ht.size(), cudaMemcpyHostToDevice), "cudaMemcpy(batch tables)");
-        // stride matrices of the chunk for a block's threads (two octal digits of warps)
-        cu(cudaMalloc(&g.d_mats, ft::stride_words(2) * 8), "cudaMalloc(stride matrices)");
-        cu(cudaMalloc(&g.d_state, nm * 32), "cudaMalloc(batch start states)");
-        cu(ft::launch_stride_matrices(ds.tpow, g.chunk * g.draws, 2, g.d_mats, 0), "stride matrices");
+        off[gi] = {o_prm, o_tab};
         cu(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking), "cudaStreamCreate");
         cu(cudaEventCreateWithFlags(&g.done, cudaEventDisableTiming), "cudaEventCreate");
         g.off_hdr = hdr;
@@ -252,6 +245,23 @@ void build(ft_batch& b)
         g.off_qacc = b.qacc_words;
         b.qacc_words += nm * ft::exact_words(g.K);
     }
+    // stride matrices of the chunk for a block's threads (two octal digits of warps)
+    for (size_t gi = 0; gi < b.groups.size(); gi++) {
+        off[gi].push_back(total);
+        total += align_up(ft::stride_words(2) * 8, 256);
+        off[gi].push_back(total);
+        total += align_up(b.groups[gi].members.size() * 32, 256);
+    }
+    cu(cudaMalloc(&b.d_static, total), "cudaMalloc(batch data)");
+    cu(cudaMemcpy(b.d_static, blob.data(), blob.size(), cudaMemcpyHostToDevice), "cudaMemcpy(batch data)");
+    for (size_t gi = 0; gi < b.groups.size(); gi++) {
+        ft_batch::group& g = b.groups[gi];
+        g.d_prm = b.d_static + off[gi][0];
+        g.d_tab = b.d_static + off[gi][1];
+        g.d_mats = (unsigned long long*)(b.d_static + off[gi][2]);
+        g.d_state = (unsigned long long*)(b.d_static + off[gi][3]);
+        cu(ft::launch_stride_matrices(ds.tpow, g.chunk * g.draws, 2, g.d_mats, 0), "stride matrices");
+    }
     b.hdr_bytes = align_up(hdr, 64);
     const size_t inst_base = b.hdr_bytes, prep_base = inst_base + inst;
     for (ft_batch::group& g : b.groups) {
@@ -259,12 +269,13 @@ void build(ft_batch& b)
         g.off_prep += prep_base;
     }
     b.desc_bytes = prep_base + prep;
-    cu(cudaMallocHost(&b.h_desc, b.desc_bytes), "cudaMallocHost(batch descriptors)");
-    cu(cudaMalloc(&b.d_desc, b.desc_bytes), "cudaMalloc(batch descriptors)");
-    cu(cudaMallocHost(&b.h_out, b.out_doubles * 8), "cudaMallocHost(batch results)");
-    cu(cudaMallocHost(&b.h_hdr_out, b.hdr_bytes), "cudaMallocHost(batch counters)");
-    cu(cudaMalloc(&b.d_out, b.out_doubles * 8), "cudaMalloc(batch results)");
-    if (prec) cu(cudaMalloc(&b.d_qacc, b.qacc_words * 8), "cudaMalloc(batch FP64-pass sums)");
+    const size_t o_out = align_up(b.desc_bytes, 256), o_more = o_out + align_up(b.out_doubles * 8, 256);
+    cu(cudaMallocHost(&b.h_desc, o_more + b.hdr_bytes), "cudaMallocHost(batch descriptors and results)");
+    b.h_out = (double*)(b.h_desc + o_out);
+    b.h_hdr_out = (class_header*)(b.h_desc + o_more);
+    cu(cudaMalloc(&b.d_desc, o_more + (prec ? b.qacc_words * 8 : 0)), "cudaMalloc(batch descriptors and results)");
+    b.d_out = (double*)(b.d_desc + o_out);
+    if (prec) b.d_qacc = (unsigned long long*)(b.d_desc + o_more);
     std::memset(b.h_desc, 0, b.desc_bytes);
     // static parts of the instance records
     for (ft_batch::group& g : b.groups)

@@ -8,6 +8,8 @@
 #include <chrono>
 #include <cstdlib>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <sstream>
 #include <stdexcept>
 #include <string>
@@ -96,6 +98,23 @@ parsed parse_input(const std::string& text)
     return p;
 }
 
+// the current device's name (asked once per device)
+std::string device_name()
+{
+    static std::mutex mu;
+    static std::map<int, std::string> names;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = names.find(dev);
+    if (it == names.end()) {
+        cudaDeviceProp prop;
+        if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) return "a CUDA device";
+        it = names.emplace(dev, prop.name).first;
+    }
+    return it->second;
+}
+
 char* dup(const std::string& s)
 {
     char* c = (char*)std::malloc(s.size() + 1);
@@ -133,11 +152,7 @@ extern "C" int ft_run_json(const char* input_json, char** output, char** log)
         ft_plan_info info;
         ft_plan_get_info(plan, &info);
         for (int i = 0; i < info.num_log_lines; i++) lg << ft_plan_log_line(plan, i) << "\n";
-        int dev = 0;
-        cudaDeviceProp prop;
-        cudaGetDevice(&dev);
-        cudaGetDeviceProperties(&prop, dev);
-        lg << "Started integrating on " << prop.name << " ("
+        lg << "Started integrating on " << device_name() << " ("
            << (in.precision == FT_PRECISION_MIXED ? "mixed FP32/FP64" : "FP64") << ") and N = " << (double)in.N
            << " points.\n";
         const int K = in.K;

@@ -51,23 +51,16 @@ void fill_result(const ft::prepared& P, const std::vector<double>& acc, ft_resul
 
 }  // namespace ftrt
 
-struct ft_plan {
-    ft::prepared P;
-    // the kernels' vertex labels: vertices without external momentum first, the external
-    // ones last, the last of them the deleted (ground) vertex; kek/kel the edges in these
-    // labels and kP the scalar products; reduced vertices [0, q0) carry no momentum
-    std::vector<int> kek, kel;
-    std::vector<double> kP;
-    int q0 = 0;
-    std::vector<double> sigma, q, prm;
-    std::vector<unsigned char> tab;
-    int device = 0;
-    double* d_prm = nullptr;
-    unsigned char* d_tab = nullptr;
-    // scratch reused by launches
+// What a plan's runs need beside its data: a stream, events, pinned words, scratch.  Sets
+// are handed from plan to plan (acquire, release in runtime.cpp): making one takes 200 us
+// and freeing it 90, more than a small integration.
+struct run_scratch {
+    unsigned char *d_in = nullptr, *h_in = nullptr;   // parameter block and table: device, pinned staging
+    size_t in_cap = 0;
     double* d_parts = nullptr;
     size_t parts_cap = 0;
     double* h_final = nullptr;   // pinned, written by the last block of a launch
+    size_t final_cap = 0;
     unsigned long long* d_queue = nullptr;
     unsigned int* d_qcount = nullptr;   // hand-offs, finished blocks: both zero between launches
     size_t qcap = 0;
@@ -83,6 +76,33 @@ struct ft_plan {
     unsigned long long stride_clock = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+};
+
+namespace ftrt {
+// a set for the current device: an idle one, or a new one
+run_scratch acquire_scratch(int device);
+// back to the idle ones (at most 8 per device of at most 32 MB each, else freed); `dirty`: its
+// last run did not complete, so it is freed
+void release_scratch(int device, run_scratch& s, bool dirty);
+}  // namespace ftrt
+
+struct ft_plan : run_scratch {
+    ft::prepared P;
+    // the kernels' vertex labels: vertices without external momentum first, the external
+    // ones last, the last of them the deleted (ground) vertex; kek/kel the edges in these
+    // labels and kP the scalar products; reduced vertices [0, q0) carry no momentum
+    std::vector<int> kek, kel;
+    std::vector<double> kP;
+    int q0 = 0;
+    std::vector<double> sigma, q, prm;
+    std::vector<unsigned char> tab;
+    int device = 0;
+    double* d_prm = nullptr;   // in d_in
+    unsigned char* d_tab = nullptr;
+    size_t queue_entries = 0;  // hand-offs that this plan's mixed runs may queue
+    bool uploading = false;    // the copy to d_in may still be in flight on `stream`
+    bool running = false;      // a run was started and did not complete
+    bool detached = false;     // ft_integrate_noalloc ran: work of this plan may be in flight
     std::mutex mu;
     // a launch shape under measurement by the autotuner (for one precision)
     bool forced = false;
@@ -119,16 +139,15 @@ struct ft_plan {
 
     ~ft_plan()
     {
-        if (d_prm) cudaFree(d_prm);
-        if (d_tab) cudaFree(d_tab);
-        if (d_parts) cudaFree(d_parts);
-        if (h_final) cudaFreeHost(h_final);
-        if (d_queue) cudaFree(d_queue);
-        if (d_qcount) cudaFree(d_qcount);
-        for (stride_entry& e : strides)
-            if (e.d) cudaFree(e.d);
-        if (ev0) cudaEventDestroy(ev0);
-        if (ev1) cudaEventDestroy(ev1);
-        if (stream) cudaStreamDestroy(stream);
+        if (!stream) return;
+        if (uploading) cudaStreamSynchronize(stream);
+        if (detached) {   // on whichever stream
+            int cur = 0;
+            cudaGetDevice(&cur);
+            cudaSetDevice(device);
+            cudaDeviceSynchronize();
+            cudaSetDevice(cur);
+        }
+        ftrt::release_scratch(device, *this, running);
     }
 };

@@ -15,6 +15,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <sstream>
@@ -69,6 +70,77 @@ void require_device()
         cudaGetLastError();
         throw std::logic_error("no CUDA device: the feyntrop_gb300 sampling path runs on the GPU only");
     }
+}
+
+// idle scratch sets per device; never destroyed, so that a plan may outlive it at exit
+struct scratch_pool {
+    std::mutex mu;
+    std::map<int, std::vector<run_scratch>> idle;
+};
+static scratch_pool& idle_scratch()
+{
+    static scratch_pool* p = new scratch_pool;
+    return *p;
+}
+
+run_scratch acquire_scratch(int device)
+{
+    {
+        scratch_pool& pool = idle_scratch();
+        std::lock_guard<std::mutex> lock(pool.mu);
+        std::vector<run_scratch>& idle = pool.idle[device];
+        if (!idle.empty()) {
+            const run_scratch s = idle.back();
+            idle.pop_back();
+            return s;
+        }
+    }
+    run_scratch s;
+    try {
+        cu(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking), "cudaStreamCreate");
+        cu(cudaEventCreate(&s.ev0), "cudaEventCreate");
+        cu(cudaEventCreate(&s.ev1), "cudaEventCreate");
+        cu(cudaMalloc(&s.d_qcount, 16), "cudaMalloc(queue count)");
+        cu(cudaMemset(s.d_qcount, 0, 16), "cudaMemset(queue count)");
+    } catch (...) {
+        release_scratch(device, s, true);
+        throw;
+    }
+    return s;
+}
+
+void release_scratch(int device, run_scratch& s, bool dirty)
+{
+    if (s.qcap * 40 > (8u << 20)) {   // a long mixed run's hand-off queue
+        cudaFree(s.d_queue);
+        s.d_queue = nullptr;
+        s.qcap = 0;
+    }
+    size_t bytes = 2 * s.in_cap + s.parts_cap * 8 + s.final_cap * 8 + s.qcap * 40;
+    for (const run_scratch::stride_entry& e : s.strides)
+        if (e.d) bytes += ft::stride_words(e.cap) * 8;
+    if (!dirty && bytes <= (32u << 20)) {
+        scratch_pool& pool = idle_scratch();
+        std::lock_guard<std::mutex> lock(pool.mu);
+        std::vector<run_scratch>& idle = pool.idle[device];
+        if (idle.size() < 8) {
+            idle.push_back(s);
+            s = run_scratch();
+            return;
+        }
+    }
+    if (s.d_in) cudaFree(s.d_in);
+    if (s.h_in) cudaFreeHost(s.h_in);
+    if (s.d_parts) cudaFree(s.d_parts);
+    if (s.h_final) cudaFreeHost(s.h_final);
+    if (s.d_queue) cudaFree(s.d_queue);
+    if (s.d_qcount) cudaFree(s.d_qcount);
+    for (run_scratch::stride_entry& e : s.strides)
+        if (e.d) cudaFree(e.d);
+    if (s.ev0) cudaEventDestroy(s.ev0);
+    if (s.ev1) cudaEventDestroy(s.ev1);
+    if (s.stream) cudaStreamDestroy(s.stream);
+    s = run_scratch();
 }
 
 device_state& dev_state()
@@ -269,21 +341,44 @@ void build_blocks(ft_plan& pl)
 }
 
 // device copies and scratch of a plan, made on its first integration (a plan used only
-// through batches never allocates its own)
+// through batches never has its own)
 void upload(ft_plan& pl)
 {
     if (pl.d_prm) return;
+    if (!pl.stream) static_cast<run_scratch&>(pl) = acquire_scratch(pl.device);
     const std::vector<double> blk = param_block(pl.prm);
-    cu(cudaMalloc(&pl.d_prm, blk.size() * 8), "cudaMalloc(params)");
-    cu(cudaMalloc(&pl.d_tab, pl.tab.size()), "cudaMalloc(table)");
-    cu(cudaMemcpy(pl.d_prm, blk.data(), blk.size() * 8, cudaMemcpyHostToDevice), "cudaMemcpy(params)");
-    cu(cudaMemcpy(pl.d_tab, pl.tab.data(), pl.tab.size(), cudaMemcpyHostToDevice), "cudaMemcpy(table)");
-    cu(cudaStreamCreateWithFlags(&pl.stream, cudaStreamNonBlocking), "cudaStreamCreate");
-    cu(cudaEventCreate(&pl.ev0), "cudaEventCreate");
-    cu(cudaEventCreate(&pl.ev1), "cudaEventCreate");
-    cu(cudaMallocHost(&pl.h_final, pl.slots() * 8), "cudaMallocHost(final)");
-    cu(cudaMalloc(&pl.d_qcount, 16), "cudaMalloc(queue count)");
-    cu(cudaMemset(pl.d_qcount, 0, 16), "cudaMemset(queue count)");
+    const size_t off = (blk.size() * 8 + 255) & ~(size_t)255, bytes = off + pl.tab.size();
+    if (bytes > pl.in_cap) {
+        if (pl.d_in) cudaFree(pl.d_in);
+        if (pl.h_in) cudaFreeHost(pl.h_in);
+        pl.d_in = pl.h_in = nullptr;
+        pl.in_cap = 0;
+        const size_t cap = std::max<size_t>(bytes, 64 * 1024);
+        cu(cudaMalloc(&pl.d_in, cap), "cudaMalloc(parameters and table)");
+        cu(cudaMallocHost(&pl.h_in, cap), "cudaMallocHost(parameters and table)");
+        pl.in_cap = cap;
+    }
+    if ((size_t)pl.slots() > pl.final_cap) {
+        if (pl.h_final) cudaFreeHost(pl.h_final);
+        pl.h_final = nullptr;
+        pl.final_cap = 0;
+        cu(cudaMallocHost(&pl.h_final, pl.slots() * 8), "cudaMallocHost(final)");
+        pl.final_cap = pl.slots();
+    }
+    std::memcpy(pl.h_in, blk.data(), blk.size() * 8);
+    std::memcpy(pl.h_in + off, pl.tab.data(), pl.tab.size());
+    pl.uploading = true;
+    cu(cudaMemcpyAsync(pl.d_in, pl.h_in, bytes, cudaMemcpyHostToDevice, pl.stream), "cudaMemcpyAsync(parameters)");
+    pl.d_prm = (double*)pl.d_in;
+    pl.d_tab = pl.d_in + off;
+}
+
+// before work of the plan on stream st
+void order_after_upload(ft_plan& pl, cudaStream_t st)
+{
+    if (!pl.uploading || st == pl.stream) return;
+    cu(cudaStreamSynchronize(pl.stream), "upload");
+    pl.uploading = false;
 }
 
 void ensure_parts(ft_plan& pl, size_t nparts)
@@ -292,6 +387,7 @@ void ensure_parts(ft_plan& pl, size_t nparts)
     if (need <= pl.parts_cap) return;
     if (pl.d_parts) cudaFree(pl.d_parts);
     pl.d_parts = nullptr;
+    pl.parts_cap = 0;
     cu(cudaMalloc(&pl.d_parts, need * 8), "cudaMalloc(partial sums)");
     pl.parts_cap = need;
 }
@@ -301,6 +397,7 @@ void ensure_queue(ft_plan& pl, size_t entries)
     if (entries <= pl.qcap) return;
     if (pl.d_queue) cudaFree(pl.d_queue);
     pl.d_queue = nullptr;
+    pl.qcap = 0;
     cu(cudaMalloc(&pl.d_queue, entries * 5 * 8), "cudaMalloc(FP64 queue)");
     pl.qcap = entries;
 }
@@ -309,8 +406,8 @@ void ensure_queue(ft_plan& pl, size_t entries)
 const unsigned long long* stride_matrices(ft_plan& pl, unsigned long long S, int digits, cudaStream_t st, bool* made)
 {
     pl.stride_clock++;
-    ft_plan::stride_entry* victim = &pl.strides[0];
-    for (ft_plan::stride_entry& e : pl.strides) {
+    run_scratch::stride_entry* victim = &pl.strides[0];
+    for (run_scratch::stride_entry& e : pl.strides) {
         if (e.d && e.S == S && e.digits >= digits) {
             e.used = pl.stride_clock;
             *made = false;
@@ -400,6 +497,10 @@ run_out run(ft_plan& pl, const ft_run_options& o, cudaStream_t st, const records
     out.acc.assign(pl.slots(), 0.0);
     if (N == 0) return out;
 
+    order_after_upload(pl, st);
+    if (pl.running)   // the last run failed: its counters may not be back at zero
+        cu(cudaMemsetAsync(pl.d_qcount, 0, 16, st), "cudaMemsetAsync");
+    pl.running = true;
     bool made = false;
     int digits = ft::stride_digits(g.lanebits);
     const unsigned long long* mats = stride_matrices(pl, g.chunk * draws, digits, st, &made);
@@ -409,11 +510,12 @@ run_out run(ft_plan& pl, const ft_run_options& o, cudaStream_t st, const records
     if (prec) {
         size_t want = (size_t)std::min<unsigned long long>(N, N / 16 + 65536);
         ensure_queue(pl, want);
+        pl.queue_entries = std::max(pl.queue_entries, want);   // not qcap: a pooled queue may be longer
     }
     ft::xstate base = ft::advance(ft::seed_state(o.seed), o.first_sample * draws);
     cu(cudaEventRecord(pl.ev0, st), "cudaEventRecord");
     unsigned long long nsamples = N, chunk = g.chunk;
-    unsigned int qcap = (unsigned int)pl.qcap;
+    unsigned int qcap = (unsigned int)pl.queue_entries;
     unsigned long long* queue = pl.d_queue;
     unsigned int *qcount = pl.d_qcount, *ticket = pl.d_qcount + 1;
     double *parts = pl.d_parts, *final_out = pl.h_final, *none = nullptr;
@@ -445,12 +547,14 @@ run_out run(ft_plan& pl, const ft_run_options& o, cudaStream_t st, const records
     }
     cu(cudaEventRecord(pl.ev1, st), "cudaEventRecord");
     cu(cudaStreamSynchronize(st), "sampling");
+    pl.running = false;
+    if (st == pl.stream) pl.uploading = false;
     float ms = 0;
     cu(cudaEventElapsedTime(&ms, pl.ev0, pl.ev1), "cudaEventElapsedTime");
     out.kernel_ms = ms;
     out.acc.assign(pl.h_final, pl.h_final + pl.slots());
     const unsigned long long queued = (unsigned long long)out.acc[8 * pl.P.K + 2];
-    if (prec && queued > pl.qcap) {
+    if (prec && queued > qcap) {
         // more samples needed FP64 than the queue holds: redo the whole range in FP64
         ft_run_options o64 = o;
         o64.precision = FT_PRECISION_FP64;
@@ -783,6 +887,8 @@ int ft_integrate_noalloc(ft_plan* pl, const ft_run_options* o, double* d_slots)
         ft::noalloc_layout sc;
         cu(ft::noalloc_scratch(&sc), "cudaGetSymbolAddress(no-allocation scratch)");
         cudaStream_t st = o->stream ? (cudaStream_t)o->stream : pl->stream;
+        order_after_upload(*pl, st);
+        pl->detached = true;
         const unsigned long long draws = 2ULL * pl->P.E - 1;
         int digits = ft::stride_digits(g.lanebits);
         cu(ft::launch_stride_matrices(dev_state().tpow, g.chunk * draws, digits, sc.mats, st), "stride matrices");
