@@ -215,6 +215,22 @@ struct xo {
     }
 };
 
+static __device__ __forceinline__ void rewind(xo& g, int n)
+{
+    // n steps back: b = y ^ (b << 17) with y = b' ^ c' solved by substitution
+#pragma unroll 1
+    for (int i = 0; i < n; i++) {
+        const u64 d1 = rotl64(g.d, 19);
+        const u64 y = g.b ^ g.c;
+        const u64 b = y ^ (y << 17) ^ (y << 34) ^ (y << 51);
+        const u64 c1 = g.c ^ (b << 17);
+        g.a ^= d1;
+        g.b = b;
+        g.c = c1 ^ g.a;
+        g.d = d1 ^ b;
+    }
+}
+
 static __device__ __forceinline__ double u01(u64 x) { return (double)(x >> 11) * 0x1.0p-53; }
 
 template <class T>
@@ -924,13 +940,57 @@ static __device__ __noinline__ cx<double> powers_slow(cx<double> psi, cx<double>
     lv = clog_(v);
     return cpow_(psi, -D / 2.) * cpow_(v, -W);
 }
+// The derivatives by the reference's route of the sample drawn just before g, for an edge
+// whose ends float together.  Differences of the potentials' products cancel there to
+// eps / x_e^2: below x_e = 1e-8 the phases are rounding noise, and the last bit of X decides
+// them.  So the sample is drawn again with the general functions, which keeps the values
+// that the plain FP64 form gives: with X from pow_1mu a single sample of 3e6 moved double
+// box integrals by up to 5e-7 (6 of 40 kinematics by more than 1e-9), with this by 1e-12.
+static __device__ __noinline__ bool derivatives_slow(xo g, const unsigned char* gm, const double* prm,
+                                                     const double (*G)[FT_N], double* dphi, double (*H)[FT_E])
+{
+    bool cancel = false;
+    for (int e = 0; e < FT_E; e++) {
+        const int k = FT_EK[e], l = FT_EL[e];
+        if (k == FT_V - 1) continue;
+        const double big = G[k][k] + G[l][l], t = big - 2.0 * G[k][l];
+        cancel |= !(t > 1e-7 * big);
+    }
+    if (!cancel) return false;
+    const double* ri = (const double*)(gm + T_RI64);
+    const u32* meta = (const u32*)(gm + T_META);
+    double X[FT_E], Xi[FT_E];
+    double XX = 1.0, F = 1.0, Gv = 0.0;
+    u32 sub = FT_FULL;
+    rewind(g, 2 * FT_E - 1);
+#pragma unroll 1
+    for (int j = 0; j < FT_E; j++) {
+        const int e = exact_cut(g.next(), sub, gm);
+        const u32 m0 = meta[sub];
+        sub ^= 1u << e;
+        const u32 m = meta[sub];
+        if (META_MM(m0) && !META_MM(m)) Gv = XX;
+        X[e] = XX;
+        if (META_L(m) < META_L(m0)) F *= XX;
+        if (j < FT_E - 1) XX *= pow(1.0 - u01(g.next()), ri[sub]);
+    }
+    const double tgt = pow(F, -prm[P_D] / 2.) * pow(F / (Gv * F), prm[P_W]);
+    const double scale = pow(tgt, prm[P_NORM]);
+    for (int e = 0; e < FT_E; e++) {
+        X[e] *= scale;
+        Xi[e] = 1.0 / X[e];
+    }
+    robust_derivatives(X, Xi, prm, dphi, H);
+    return true;
+}
 #endif
 
 // X: unnormalised sector point, psi_tr and Gv = xi_tr / psi_tr there; returns R per eps
 // order, false when dropped.  `robust` reports that the complete-pivoting LU or the
-// reference's route to the derivatives was needed.
+// reference's route to the derivatives was needed.  g: the stream behind the sample's draws.
 static __device__ __forceinline__ bool integrand64(const double* prm, double* X, double psi_tr, double Gv,
-                                                   cx<double>* out, bool& robust)
+                                                   const xo& g, const unsigned char* gm, cx<double>* out,
+                                                   bool& robust)
 {
     const double D = prm[P_D], W = prm[P_W], IGtr = prm[P_IGTR];
     // normalise so that psi_tr^(-D/2) (psi_tr/xi_tr)^W = 1 (srcs/feynman_integral.hpp:201-204)
@@ -1136,11 +1196,11 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
             s = r == 0 ? sg[r] * hb[r][e] : fma(sg[r], hb[r][e], s);
         }
         const double t = wd(ke, le);
-        // an edge whose ends float together: its resistance difference cancels (t below about
-        // 1e-7 of the entries it comes from, by their exponents)
+        // an edge whose ends may float together: its resistance difference cancels (t below
+        // 2^-21 of the entries it comes from, by their exponents; derivatives_slow tests for 1e-7)
         if (ke != FT_V - 1) {
             const int big = max(exponent_of(G[ke][ke]), exponent_of(G[le][le]));
-            cancel |= hi_word(t) < 0 || exponent_of(t) < big - 23;
+            cancel |= hi_word(t) < 0 || exponent_of(t) < big - 20;
         }
         A[e][e] = s * (t - X[e]);
         theta[e] = fma(s * (X[e] * X[e]), pow2_of(-2 * ex[e] - 1), kappa * prm[P_M2 + e]);
@@ -1153,14 +1213,19 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
         }
     }
     if (cancel) {
-        double dphi[FT_E], H[FT_E][FT_E];
-        robust_derivatives(X, Xi, prm, dphi, H);
-        robust = true;
+        double dphi[FT_E], H[FT_E][FT_E], Gm[FT_N][FT_N];   // Gm: so that G stays in registers
 #pragma unroll
-        for (int e = 0; e < FT_E; e++) {
-            theta[e] = (dphi[e] + prm[P_M2 + e]) * kappa;
+        for (int k = 0; k < FT_N; k++)
 #pragma unroll
-            for (int f = e; f < FT_E; f++) A[e][f] = kappa * H[e][f] * pow2_of(ex[e]) * pow2_of(ex[f]);
+            for (int l = 0; l < FT_N; l++) Gm[k][l] = G[k][l];
+        if (derivatives_slow(g, gm, prm, Gm, dphi, H)) {
+            robust = true;
+#pragma unroll
+            for (int e = 0; e < FT_E; e++) {
+                theta[e] = (dphi[e] + prm[P_M2 + e]) * kappa;
+#pragma unroll
+                for (int f = e; f < FT_E; f++) A[e][f] = kappa * H[e][f] * pow2_of(ex[e]) * pow2_of(ex[f]);
+            }
         }
     }
     // deformation x -> x exp(i theta), theta = -lambda (d(phi/psi)/dx + m^2)
@@ -1570,22 +1635,6 @@ static __device__ FT_BIGFN df log1m_pair(u64 xa, u64 xb)
     const fv lo = fma_(kk, fv_of(1.428606765330187e-06f), make_float2(a.nl, b.nl)) +
                   fma_(kk, fv_of(5.497923e-14f), z.lo + tail);
     return fast_two_sum(t.hi, (t.lo + s.lo) + lo);
-}
-
-static __device__ __forceinline__ void rewind(xo& g, int n)
-{
-    // n steps back: b = y ^ (b << 17) with y = b' ^ c' solved by substitution
-#pragma unroll 1
-    for (int i = 0; i < n; i++) {
-        const u64 d1 = rotl64(g.d, 19);
-        const u64 y = g.b ^ g.c;
-        const u64 b = y ^ (y << 17) ^ (y << 34) ^ (y << 51);
-        const u64 c1 = g.c ^ (b << 17);
-        g.a ^= d1;
-        g.b = b;
-        g.c = c1 ^ g.a;
-        g.d = d1 ^ b;
-    }
 }
 
 // the draw of the step undecided by the thresholds, in FP64; g stands `back` draws behind it
@@ -3178,7 +3227,7 @@ static __device__ __forceinline__ void sample64(xo& g, const table_ref& tr, cons
     if (FT_RECORD)
         for (int e = 0; e < FT_E; e++) rec_X[i * FT_E + e] = X[e];
     bool rob = false;
-    const bool ok = integrand64(prm, X, F, Gv, R, rob);
+    const bool ok = integrand64(prm, X, F, Gv, g, FT_EXACT_TABLE(tr), R, rob);
     if (rob) {
         A.count(CNT_ROBUST, 1);
         flags |= REC_ROBUST;
@@ -3556,7 +3605,7 @@ extern "C" __global__ void __launch_bounds__(FT_BLOCK) ft_sample_queue_batch(
         unsigned char ord[FT_E];
         draw_sector64(g, tr, FT_EXACT_TABLE(tr), prm[P_JRFULL], X, F, Gv, ord);
         bool rob = false;
-        const bool ok = integrand64(prm, X, F, Gv, R, rob);
+        const bool ok = integrand64(prm, X, F, Gv, g, FT_EXACT_TABLE(tr), R, rob);
         u64* qa = qacc + (size_t)id * (4 * FT_K * FT_XA_DIGITS + 4);
         u64* cnt = qa + 4 * FT_K * FT_XA_DIGITS;
         if (rob) atomicAdd(cnt + 2, 1ull);
