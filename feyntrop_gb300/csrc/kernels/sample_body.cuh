@@ -2936,6 +2936,15 @@ struct accum {
     {
         if (n) atomicAdd(&s_count[c], (u64)n);
     }
+    // A warp's threads first: a 64-bit addition in shared memory is a compare-and-swap loop,
+    // and the block's 256 to 512 threads took 10 us of every launch and batch item in it.
+    __device__ __forceinline__ void add_owned(u64 owned)
+    {
+        const u32 lo = __reduce_add_sync(0xffffffffu, (u32)owned & 0xffffffu);
+        const u32 mid = __reduce_add_sync(0xffffffffu, (u32)(owned >> 24) & 0xffffffu);
+        const u32 hi = __reduce_add_sync(0xffffffffu, (u32)(owned >> 48));
+        if ((threadIdx.x & 31u) == 0) atomicAdd(&s_count[CNT_OWNED], (u64)lo + ((u64)mid << 24) + ((u64)hi << 48));
+    }
 
 #if FT_PREC == 0
     __device__ __forceinline__ double& S(int s) { return ((double*)base)[s * FT_BLOCK + threadIdx.x]; }
@@ -2984,7 +2993,7 @@ struct accum {
     // own threads took three times the FP64 additions).
     __device__ __forceinline__ void finish(double* dst, u64 owned)
     {
-        if (owned) atomicAdd(&s_count[CNT_OWNED], owned);
+        add_owned(owned);
         __syncthreads();
         const int lane = threadIdx.x & 31;
 #pragma unroll 1
@@ -3121,7 +3130,7 @@ struct accum {
     // block's sums go to dst[0 .. ACC_SLOTS)
     __device__ __forceinline__ void finish(double* dst, u64 owned)
     {
-        if (owned) atomicAdd(&s_count[CNT_OWNED], owned);
+        add_owned(owned);
         fold();
         __syncthreads();
         for (int s = threadIdx.x; s < ACC_NS; s += FT_BLOCK) {
