@@ -194,8 +194,12 @@ void build(ft_batch& b)
         keys64.push_back(k64);
     }
     {
-        std::vector<ft::kernel_key> all = keys;
-        if (prec) all.insert(all.end(), keys64.begin(), keys64.end());
+        // those not loaded yet: finding a kernel's file costs its generated source and a hash
+        std::vector<ft::kernel_key> all;
+        for (const ft::kernel_key& k : keys)
+            if (!ft::find_kernels(k)) all.push_back(k);
+        for (const ft::kernel_key& k : keys64)
+            if (prec && !ft::find_kernels(k)) all.push_back(k);
         ft::precompile_all(all);
     }
     size_t hdr = 0, inst = 0, prep = 0, total = 0;
