@@ -50,7 +50,7 @@ struct class_header {
     unsigned long long total_items;
     unsigned long long counter;   // next work item
     unsigned long long qcount;    // FP64 hand-offs (the kernel counts in the low 32 bits)
-    unsigned long long pad;
+    unsigned long long chunk;     // samples per thread of a work item (read by the FP64 form)
 };
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -64,7 +64,9 @@ struct ft_batch {
         const ft::kernel_set* k64 = nullptr;    // FP64 batch module (queue kernel), mixed only
         std::vector<int> members;               // indices into plans
         int K = 1, rank = 1, draws = 1;
-        unsigned long long chunk = 64;
+        unsigned long long chunk = 64;          // samples per thread of a work item
+        unsigned long long max_chunk = 0;       // FP64: at most; 0: chunk is fixed
+        unsigned long long mats_chunk = 0;      // chunk that d_mats and d_item_mats are for
         unsigned grid = 0, qgrid = 0;
         size_t prm_stride = 0, tab_stride = 0;  // bytes
         // offsets of this class's records in the run descriptors
@@ -74,6 +76,7 @@ struct ft_batch {
         unsigned long long* d_mats = nullptr;        // stride matrices of the chunk
         unsigned long long* d_item_mats = nullptr;   // powers of the item stride, item_digits octal digits
         int item_digits = 0, want_digits = 0;
+        int item_digits_set = 0;   // digits of d_item_mats computed for the present chunk
         unsigned long long* d_state = nullptr;       // the integrals' start states (with the above in d_static)
         size_t item_cap = 0;
         double* d_parts = nullptr;
@@ -219,6 +222,7 @@ void build(ft_batch& b)
                       ? ft::chunk_override()
                       : env_u64("FEYNTROP_GB300_BATCH_CHUNK", tuned.chunk ? tuned.chunk : ft::default_chunk(g.key));
         if (g.chunk < 1 || g.chunk >= (1ull << 18)) throw std::invalid_argument("batch chunk out of range");
+        if (prec == 0 && !ft::chunk_override() && !std::getenv("FEYNTROP_GB300_BATCH_CHUNK")) g.max_chunk = g.chunk;
         g.grid = (unsigned)(ds.sms * g.ks->blocks_per_sm);
         g.qgrid = prec ? (unsigned)(ds.sms * 2) : 0;
         // parameter blocks and tables of the class's integrals
@@ -264,7 +268,9 @@ void build(ft_batch& b)
         g.d_tab = b.d_static + off[gi][1];
         g.d_mats = (unsigned long long*)(b.d_static + off[gi][2]);
         g.d_state = (unsigned long long*)(b.d_static + off[gi][3]);
+        if (g.max_chunk) continue;   // FP64: when the run's chunk is known
         cu(ft::launch_stride_matrices(ds.tpow, g.chunk * g.draws, 2, g.d_mats, 0), "stride matrices");
+        g.mats_chunk = g.chunk;
     }
     b.hdr_bytes = align_up(hdr, 64);
     const size_t inst_base = b.hdr_bytes, prep_base = inst_base + inst;
@@ -373,13 +379,46 @@ void capture(ft_batch& b)
     b.captures++;
 }
 
+// Samples per thread of the FP64 form's work items: the chunk, an eighth of the largest or a
+// multiple of it, that ends first when every block takes the same number of items and an item
+// costs its samples and a start worth `start` of them.  Pentabox points, 12 of 1e4 to 3e5
+// samples (338 items of 8 for 152 blocks: three rounds, the last a fifth full): chunks of 1, 2,
+// 3, 4, 6, 8, 16 take 4.37, 3.98, 3.88, 4.18, 3.75, 4.82, 6.25 ms, 0.2 ms times this count.  A
+// function of the counts alone, so that equal runs add in equal order.
+unsigned long long run_chunk(const ft_batch& b, const ft_batch::group& g, const ft_run_options* opts)
+{
+    const double start = g.key.mode == 1 ? 0.2 : 1.0;
+    unsigned long long best = g.max_chunk;
+    double cost = 0;
+    for (unsigned long long k = 8; k >= 1; k--) {
+        const unsigned long long c = g.max_chunk * k / 8, per_item = (unsigned long long)g.ks->block * c;
+        if (c == 0) break;
+        unsigned long long items = 0;
+        for (int m : g.members) items += (opts[m].num_samples + per_item - 1) / per_item;
+        const double t = (double)((items + g.grid - 1) / g.grid) * ((double)c + start);
+        if (k == 8 || t < 0.97 * cost) {
+            best = c;
+            cost = t;
+        }
+    }
+    return best;
+}
+
 // grows the item and queue buffers to what the descriptors need; true when it did
 bool ensure_capacity(ft_batch& b, const std::vector<size_t>& qwant)
 {
     bool grew = false;
     for (size_t gi = 0; gi < b.groups.size(); gi++) {
         ft_batch::group& g = b.groups[gi];
-        const size_t items = std::max<size_t>(g.total_items, 1);
+        // at least 16 rounds' worth: fewer samples may mean more items (run_chunk)
+        const size_t items = std::max<size_t>(g.total_items, g.max_chunk ? 16 * (size_t)g.grid : 1);
+        if (g.mats_chunk != g.chunk) {
+            g.mats_chunk = 0;
+            g.item_digits_set = 0;
+            cu(ft::launch_stride_matrices(dev_state().tpow, g.chunk * g.draws, 2, g.d_mats, b.stream), "stride matrices");
+            cu(cudaStreamSynchronize(b.stream), "stride matrices");   // the graph may run on another stream
+            g.mats_chunk = g.chunk;
+        }
         if (items > g.item_cap) {
             const size_t cap = std::max(items, g.item_cap + g.item_cap / 4);
             cudaFree(g.d_parts);
@@ -392,15 +431,18 @@ bool ensure_capacity(ft_batch& b, const std::vector<size_t>& qwant)
         if (g.want_digits > g.item_digits) {
             cudaFree(g.d_item_mats);
             g.d_item_mats = nullptr;
-            g.item_digits = 0;
-            const size_t bytes = (size_t)g.want_digits * 7 * 1024 * 8;
-            cu(cudaMalloc(&g.d_item_mats, bytes), "cudaMalloc(item stride matrices)");
+            g.item_digits = g.item_digits_set = 0;
+            const int digits = std::max(g.want_digits, g.max_chunk ? 4 : 0);
+            cu(cudaMalloc(&g.d_item_mats, (size_t)digits * 7 * 1024 * 8), "cudaMalloc(item stride matrices)");
+            g.item_digits = digits;
+            grew = true;
+        }
+        if (g.item_digits_set < g.want_digits) {
             cu(ft::launch_digit_matrices(dev_state().tpow, (unsigned long long)g.ks->block * g.chunk * g.draws,
-                                         g.want_digits, g.d_item_mats, b.stream),
+                                         g.item_digits, g.d_item_mats, b.stream),
                "item stride matrices");
             cu(cudaStreamSynchronize(b.stream), "item stride matrices");   // the graph may run on another stream
-            g.item_digits = g.want_digits;
-            grew = true;
+            g.item_digits_set = g.item_digits;
         }
         if (b.precision && qwant[gi] > g.qcap) {
             const size_t cap = std::min<size_t>(std::max(qwant[gi], g.qcap + g.qcap / 4), 0xffffffffull);
@@ -452,6 +494,7 @@ int ft_batch_run(ft_batch* b, const ft_run_options* opts, ft_result* results)
         std::vector<size_t> qwant(b->groups.size(), 0);
         for (size_t gi = 0; gi < b->groups.size(); gi++) {
             ft_batch::group& g = b->groups[gi];
+            if (g.max_chunk) g.chunk = run_chunk(*b, g, opts);
             const unsigned long long per_item = (unsigned long long)g.ks->block * g.chunk;
             unsigned long long next = 0, most = 0;
             size_t q = 0;
@@ -484,6 +527,7 @@ int ft_batch_run(ft_batch* b, const ft_run_options* opts, ft_result* results)
             h->total_items = next;
             h->counter = 0;
             h->qcount = 0;
+            h->chunk = g.chunk;
             qwant[gi] = q;
         }
         cudaStream_t st = opts[0].stream ? (cudaStream_t)opts[0].stream : b->stream;

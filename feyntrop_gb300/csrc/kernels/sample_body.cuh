@@ -3560,6 +3560,9 @@ extern "C" __global__ void __launch_bounds__(FT_BLOCK, FT_MINB) ft_sample_batch(
     __shared__ __align__(16) double s_prm[PRM_WORDS];
     __shared__ int s_inst;
     int cur = -1;
+#if FT_PREC == 0
+    chunk = total_items[3];   // the run's, from the class's header: the launch's own is of the capture
+#endif
     for (;;) {
         if (threadIdx.x == 0) {
             const u64 it = atomicAdd(counter, 1ull);
