@@ -950,9 +950,9 @@ int ft_autotune(ft_plan* pl, int32_t precision, uint64_t samples, ft_tune_result
             // per SM) to 255 (8 warps, no spills)
             // (four 128-thread blocks won one-integral trials by noise and ran the
             // persistent batch kernel 9 % slower: not a candidate)
+            add(512, 1, 20);
             add(512, 1, 29);
             add(256, 2, 29);
-            add(384, 1, 29);
             add(256, 2, 21);
             add(256, 2, 5);
             add(256, 1, 29);

@@ -84,24 +84,24 @@ launch_shape default_shape(const kernel_key& k)
 {
     // GB300 sweeps.  The per-sample barrier (variant bit 2) makes the warps of a block share
     // their instruction fetches.
-    // Mixed, undeformed (two samples per thread): 256 threads with up to 255 registers
-    // (five-loop cube, N = 5e7: 5.3 ms; 512 x 128 registers 5.4, 384 7.1).
-    // Mixed, deformed: 16 warps of 128 registers per SM, with one out-of-line copy of the FP32
-    // transcendentals, of the larger two-float routines and of the complex two-float product
-    // (bits 0, 3, 4).  One block of 512 keeps all of them together (samples/s against two
-    // blocks of 256: double box 3.00e9 / 2.73e9, six-edge one-loop 2.70e9 / 2.43e9, 3-loop
-    // ladder 1.36e9 / 1.28e9, box-pentagon 1.81e9 / 1.80e9; 12 warps of 168 registers 2.97e9
-    // on the double box, 1.17e9 on the ladder); in a batch, where a block also waits for
-    // its slowest warp at every item's end, two blocks are as fast or faster (24
-    // box-pentagon points 12.4 ms against 12.8).
+    // Mixed, undeformed (two samples per thread): 16 warps of 128 registers in one block (1e9
+    // samples/s against 256 threads with up to 255 registers: K4 24.4 / 19.8, wheel 19.2 /
+    // 16.0, undeformed box-pentagon 18.0 / 15.1, 3-loop ladder 14.2 / 12.1, cube 10.05 / 9.66,
+    // triangle 43.8 / 44.8; two blocks of 256 3 to 6 % below the one).
+    // Mixed, deformed: 16 warps of 128 registers per SM.  Single integrals: one block, which
+    // keeps all of them together, with one out-of-line copy of the complex two-float product
+    // (bit 4; also of the FP32 transcendentals and the larger two-float routines, bits 0 and 3:
+    // double box 16.4 ms against 15.9, ladder 7.96 against 7.07; without any 18.3 and 8.6).
+    // Batches, where a block also waits for its slowest warp at every item's end: two blocks,
+    // with all three (24 box-pentagon points 12.2 ms, one block 12.5; bit 4 alone 12.35).
     // FP64 form, bound by the FP64 pipe: 12 to 16 warps per SM keep it busy (double box 3e6:
     // 7.1 ms with 384 threads, 7.4 with 256; box-pentagon scan 3.4 against 4.5; cube 1.26 with
     // 512 against 1.40), two blocks where the staged table leaves the room (up to E = 10; K4
     // 3.13 ms, one block of 512 3.48).
     launch_shape s;
     if (k.prec == 1) {
-        s.block = k.mode == 1 && !k.batch ? 512 : 256;
-        s.minb = k.mode == 1 && k.batch ? 2 : 1;
+        s.block = k.batch && k.mode == 1 ? 256 : 512;
+        s.minb = k.batch && k.mode == 1 ? 2 : 1;
     } else if (k.mode == 1) {
         s.block = 384;
         s.minb = 1;
@@ -109,7 +109,7 @@ launch_shape default_shape(const kernel_key& k)
         s.block = k.E > 10 ? 512 : 256;
         s.minb = k.E > 10 ? 1 : 2;
     }
-    s.variant = (k.prec == 1 && k.mode == 1) ? 29 : 4;
+    s.variant = k.prec == 1 && k.mode == 1 ? (k.batch ? 29 : 20) : 4;
     return s;
 }
 
