@@ -40,7 +40,8 @@ __global__ void __launch_bounds__(1024) ft_stride_matrices(const u64* __restrict
         n = (lanes ? 32ull : 1ull) * S * (u64)(b % 7 + 1) << (3 * (b / 7));
         dst = out + (lanes ? 131072 : 0) + (size_t)b * 1024;
     }
-    M[c * 4 + w] = (w == (c >> 6)) ? (1ull << (c & 63)) : 0ull;
+    // the identity, or the first factor: each word written once before the first barrier
+    if (n == 0) M[c * 4 + w] = (w == (c >> 6)) ? (1ull << (c & 63)) : 0ull;
     bool first = true;
     for (; n; n &= n - 1) {
         const u64* P = tpow + (size_t)(__ffsll((long long)n) - 1) * 1024;

@@ -21,9 +21,10 @@
 // Numerical design (the reference's algebra, restated for a GPU thread):
 //  * Sector draw (srcs/tropical_sampling.hpp:468-564): the cut scan compares running
 //    sums of Jr/r against u*Jr in FP64 in the reference's order, so the removal order
-//    is bit-identical.  The mixed form decides each comparison in FP32 with a
-//    rigorous error margin and repeats the scan in FP64 when a comparison falls
-//    inside the margin.  The mixed form keeps log X in a two-float sum.
+//    is bit-identical.  Where the table fits in shared memory (E <= 12) both forms compare
+//    the draw with 28-bit thresholds and repeat the step in FP64 when that does not
+//    decide; beyond, the mixed form scans in FP32 with a rigorous margin.  The mixed
+//    form keeps log X in a two-float sum; the FP64 form takes its powers in fixed point.
 //  * The deleted vertex of the reduced Laplacian is always the last one of the
 //    kernel's labels (the host numbers the vertices without external momentum first,
 //    so it is an external one).  Any choice gives the same psi, phi/psi and
@@ -41,9 +42,9 @@
 //    conductance form with a pivot-growth check (the FP64 form's failing samples take
 //    a complete-pivoting LU, srcs/feynman_integral.hpp:305; the mixed form runs this
 //    elimination and V in two-float and hands the rare failing samples to FP64), and
-//    the Jacobian determinant as det(I + i*lambda' X^1/2 H X^1/2) (similar to
-//    I + i*lambda' H X, srcs/feynman_integral.hpp:312), whose real part is the
-//    identity, so symmetric elimination without pivoting is stable.
+//    the Jacobian determinant det(I + i*lambda' H X) (srcs/feynman_integral.hpp:312) as
+//    that of D^2/X + i*lambda' D H D, D ~ X^1/2 powers of two: its real part is diagonal
+//    and at least 1, so symmetric elimination without pivoting is stable.
 //  * Updates on structural zeros of the eliminations (from each topology's fill
 //    pattern, generated by the host) and additions to zero are left out.
 
@@ -64,10 +65,10 @@ typedef unsigned int u32;
 // Code size: the per-topology kernel is straight-line code (every loop unrolled so
 // that the small matrices stay in registers), and the FP32 library functions carry
 // large slow paths.  FT_VARIANT bit 0 keeps one out-of-line copy of each FP32
-// transcendental, bit 1 does the same for the two-float primitives, so the code the
-// SM streams per sample fits the instruction caches better; bit 2 starts every sample
-// with a block-wide barrier, so that the block's warps walk the code together and
-// share its instruction fetches; bit 3 keeps one out-of-line copy of each larger
+// transcendental, so the code the SM streams per sample fits the instruction caches
+// better; bit 2 starts every sample with a block-wide barrier, so that the block's
+// warps walk the code together and share its instruction fetches;
+// bit 3 keeps one out-of-line copy of each larger
 // two-float routine (logarithm, exponential, e^(ix), complex inverse, argument), bit 4
 // of the complex two-float product and multiply-add.
 #ifndef FT_VARIANT
