@@ -498,6 +498,47 @@ static __device__ __forceinline__ cx<double> cinv_64(cx<double> z)
     const double m = rcp64(fma(z.re, z.re, z.im * z.im));
     return cmk(z.re * m, -z.im * m);
 }
+
+// The FP64 pass over hand-offs runs a handful of samples through code that no instruction cache
+// holds: its time is that of fetching it (150 us for one sample).  There the functions are
+// called (COLD), where the sampling kernels, whose warps share the code, inline them: 14
+// hand-offs of the 3-loop ladder (E = 10) took 0.6 ms more of its 7.9 ms inlined; with 7 and 8
+// edges no difference.
+static __device__ __noinline__ double pow_1mu_call(u64 x, double y) { return pow_1mu(x, y); }
+static __device__ __noinline__ log2_parts log2_call(double x) { return log2_64(x); }
+static __device__ __noinline__ double power_call(double a, log2_parts la, double b, log2_parts lb)
+{
+    return power_product(a, la, b, lb);
+}
+static __device__ __noinline__ double2 sincos_call(double x)
+{
+    double2 r;
+    sincos_64(x, r.x, r.y);
+    return r;
+}
+static __device__ __noinline__ double arg_call(double re, double im) { return arg_64(re, im); }
+static __device__ __noinline__ cx<double> cinv_call(cx<double> z) { return cinv_64(z); }
+template <bool COLD>
+struct fn64 {
+    static __device__ __forceinline__ double pow1mu(u64 x, double y) { return COLD ? pow_1mu_call(x, y) : pow_1mu(x, y); }
+    static __device__ __forceinline__ log2_parts log2(double x) { return COLD ? log2_call(x) : log2_64(x); }
+    static __device__ __forceinline__ double power(double a, log2_parts la, double b, log2_parts lb)
+    {
+        return COLD ? power_call(a, la, b, lb) : power_product(a, la, b, lb);
+    }
+    static __device__ __forceinline__ void sincos(double x, double& sn, double& cs)
+    {
+        if (COLD) {
+            const double2 r = sincos_call(x);
+            sn = r.x;
+            cs = r.y;
+        } else {
+            sincos_64(x, sn, cs);
+        }
+    }
+    static __device__ __forceinline__ double arg(double re, double im) { return COLD ? arg_call(re, im) : arg_64(re, im); }
+    static __device__ __forceinline__ cx<double> cinv(cx<double> z) { return COLD ? cinv_call(z) : cinv_64(z); }
+};
 // ------------------------------------------------------------------ robust complex LU
 // Complete-pivoting LU of the complex reduced Laplacian (largest modulus, first in
 // column-major order), used when the static elimination reports pivot growth.
@@ -859,6 +900,13 @@ static __device__ __forceinline__ int scan_cut(u64 x, u32 sub, const table_ref& 
 #endif
 
 #if FT_PREC == 0
+#if FT_CUT
+static __device__ __noinline__ int find_cut_call(u32 h, u32 sub, u32 meta, const table_ref& t, int n, bool& unsure)
+{
+    return find_cut(h, sub, meta, t, n, unsure);
+}
+#endif
+template <bool COLD>
 static __device__ __forceinline__ void draw_sector64(xo& g, const table_ref& t, const unsigned char* gm,
                                                      double Jr_full, double* X, double& F, double& Gv,
                                                      unsigned char* ord)
@@ -878,7 +926,8 @@ static __device__ __forceinline__ void draw_sector64(xo& g, const table_ref& t, 
         const u64 x = g.next();
 #if FT_CUT
         bool unsure = false;
-        int e = find_cut((u32)(x >> 32), sub, meta, t, FT_E - j, unsure);
+        int e = COLD ? find_cut_call((u32)(x >> 32), sub, meta, t, FT_E - j, unsure)
+                     : find_cut((u32)(x >> 32), sub, meta, t, FT_E - j, unsure);
         if (unsure) e = exact_cut(x, sub, gm);
         sub ^= 1u << e;
 #else
@@ -904,7 +953,7 @@ static __device__ __forceinline__ void draw_sector64(xo& g, const table_ref& t, 
         if (META_L(m) < META_L(meta)) F *= XX;
         meta = m;
         if (FT_RECORD) ord[j] = (unsigned char)e;
-        if (j < FT_E - 1) XX *= pow_1mu(g.next(), rinv);
+        if (j < FT_E - 1) XX *= fn64<COLD>::pow1mu(g.next(), rinv);
     }
 }
 
@@ -989,6 +1038,7 @@ static __device__ __noinline__ bool derivatives_slow(xo g, const unsigned char* 
 // X: unnormalised sector point, psi_tr and Gv = xi_tr / psi_tr there; returns R per eps
 // order, false when dropped.  `robust` reports that the complete-pivoting LU or the
 // reference's route to the derivatives was needed.  g: the stream behind the sample's draws.
+template <bool COLD>
 static __device__ __forceinline__ bool integrand64(const double* prm, double* X, double psi_tr, double Gv,
                                                    const xo& g, const unsigned char* gm, cx<double>* out,
                                                    bool& robust)
@@ -997,7 +1047,7 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
     // normalise so that psi_tr^(-D/2) (psi_tr/xi_tr)^W = 1 (srcs/feynman_integral.hpp:201-204)
     double scale;
     if (normal_positive(psi_tr) && normal_positive(Gv)) {
-        scale = power_product(prm[P_NORM_F], log2_64(psi_tr), prm[P_NORM_G], log2_64(Gv));
+        scale = fn64<COLD>::power(prm[P_NORM_F], fn64<COLD>::log2(psi_tr), prm[P_NORM_G], fn64<COLD>::log2(Gv));
     } else {
         scale = scale_slow(psi_tr, Gv, D, W, prm[P_NORM]);
     }
@@ -1079,14 +1129,14 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
         for (int j = 0; j < FT_K; j++) out[j] = cmk(R[j], 0.0);
         return ok;
     }
-    const log2_parts lp = log2_64(psi);
+    const log2_parts lp = fn64<COLD>::log2(psi);
 #if FT_ONLY_PSI
-    const double v = IGtr * power_product(-0.5 * D, lp, 0.0, lp);
+    const double v = IGtr * fn64<COLD>::power(-0.5 * D, lp, 0.0, lp);
     if (!finite_(v)) return false;
     out[0] = cmk(v, 0.0);
 #else
-    const log2_parts lv = log2_64(pxi);
-    double v = IGtr * power_product(-0.5 * D, lp, -W, lv);
+    const log2_parts lv = fn64<COLD>::log2(pxi);
+    double v = IGtr * fn64<COLD>::power(-0.5 * D, lp, -W, lv);
     if (!finite_(v)) return false;
     out[0] = cmk(v, 0.0);
     if (FT_K > 1) {
@@ -1237,7 +1287,7 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
 #pragma unroll
     for (int e = 0; e < FT_E; e++) {
         double sn, cs;
-        sincos_64(theta[e], sn, cs);
+        fn64<COLD>::sincos(theta[e], sn, cs);
         const cx<double> cX = cmk(X[e] * cs, X[e] * sn);
         cy[e] = cmk(Xi[e] * cs, -Xi[e] * sn);   // 1 / cX
         const double m2 = prm[P_M2 + e];
@@ -1279,7 +1329,7 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
             }
             growth &= expo(dk) > big - 26;   // a pivot above about 1e-8 of its row, by the exponents
             cdet = k == 0 ? dk : cdet * dk;
-            ci[k] = cinv_64(dk);
+            ci[k] = fn64<COLD>::cinv(dk);
 #pragma unroll
             for (int i = k + 1; i < FT_N; i++)
                 if (NZC(k, i)) ca[k][i] = c[k][i] * ci[k];
@@ -1357,7 +1407,7 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
             const cx<double> piv = J[k][k];
             detJ = k == 0 ? piv : detJ * piv;
             if (k == FT_E - 1) continue;
-            const cx<double> inv = cinv_64(piv);
+            const cx<double> inv = fn64<COLD>::cinv(piv);
 #pragma unroll
             for (int i = k + 1; i < FT_E; i++) {
                 // the first row's entries have no real part
@@ -1385,13 +1435,13 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
     cx<double> ef, pw;   // log cPsi - L log cV, the powers
     const double np = fma(cPsi.re, cPsi.re, cPsi.im * cPsi.im), nv = fma(cV.re, cV.re, cV.im * cV.im);
     if (normal_positive(np) && normal_positive(nv)) {
-        const log2_parts a2 = log2_64(np), b2 = log2_64(nv);
-        const double ap = arg_64(cPsi.re, cPsi.im), av = arg_64(cV.re, cV.im);
+        const log2_parts a2 = fn64<COLD>::log2(np), b2 = fn64<COLD>::log2(nv);
+        const double ap = fn64<COLD>::arg(cPsi.re, cPsi.im), av = fn64<COLD>::arg(cV.re, cV.im);
         ef = cmk(0.5 * LN2_D * (small_int(a2.k - FT_LOOPS * b2.k) + fma(-(double)FT_LOOPS, b2.f, a2.f)),
                  fma(-(double)FT_LOOPS, av, ap));
-        const double m = power_product(-0.25 * D, a2, -0.5 * W, b2);
+        const double m = fn64<COLD>::power(-0.25 * D, a2, -0.5 * W, b2);
         double sn, cs;
-        sincos_64(fma(-0.5 * D, ap, -W * av), sn, cs);
+        fn64<COLD>::sincos(fma(-0.5 * D, ap, -W * av), sn, cs);
         pw = cmk(m * cs, m * sn);
     } else {
         cx<double> lp, lv;
@@ -1399,7 +1449,7 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
         ef = cmk(lp.re - FT_LOOPS * lv.re, lp.im - FT_LOOPS * lv.im);
     }
     double sn, cs;
-    sincos_64(xnu, sn, cs);
+    fn64<COLD>::sincos(xnu, sn, cs);
     cx<double> cR = (IGtr * pw) * (detJ * cmk(cs, sn));
     if (!finite_(cR.re) || !finite_(cR.im)) return false;
     out[0] = cR;
@@ -3275,6 +3325,7 @@ static __device__ __forceinline__ void write_record(u64 i, const unsigned char* 
 
 #if FT_PREC == 0
 // one sample in FP64 from stream state g (advanced past the sample's 2E-1 draws)
+template <bool COLD>
 static __device__ __forceinline__ void sample64(xo& g, const table_ref& tr, const double* prm, u64 i, accum& A,
                                                 unsigned char flags, unsigned char* rec_order, double* rec_X,
                                                 double* rec_R, unsigned char* rec_flags)
@@ -3285,11 +3336,11 @@ static __device__ __forceinline__ void sample64(xo& g, const table_ref& tr, cons
     for (int j = 0; j < FT_K; j++) R[j] = cmk(0.0, 0.0);
     double X[FT_E];
     double F, Gv;
-    draw_sector64(g, tr, FT_EXACT_TABLE(tr), prm[P_JRFULL], X, F, Gv, ord);
+    draw_sector64<COLD>(g, tr, FT_EXACT_TABLE(tr), prm[P_JRFULL], X, F, Gv, ord);
     if (FT_RECORD)
         for (int e = 0; e < FT_E; e++) rec_X[i * FT_E + e] = X[e];
     bool rob = false;
-    const bool ok = integrand64(prm, X, F, Gv, g, FT_EXACT_TABLE(tr), R, rob);
+    const bool ok = integrand64<COLD>(prm, X, F, Gv, g, FT_EXACT_TABLE(tr), R, rob);
     if (rob) {
         A.count(CNT_ROBUST, 1);
         flags |= REC_ROBUST;
@@ -3349,7 +3400,7 @@ static __device__ __forceinline__ void sample_range(xo& g, const table_ref& tr, 
 #endif
         const u64 i = first + k;
         if (i >= last) continue;
-        sample64(g, tr, prm, i, A, 0, rec_order, rec_X, rec_R, rec_flags);
+        sample64<false>(g, tr, prm, i, A, 0, rec_order, rec_X, rec_R, rec_flags);
     }
 #else
     const float* pf = (const float*)(prm + P_SIZE);
@@ -3483,7 +3534,7 @@ extern "C" __global__ void __launch_bounds__(FT_BLOCK) ft_sample_queue(
             g.b = q[2];
             g.c = q[3];
             g.d = q[4];
-            sample64(g, tr, prm, q[0], A, REC_QUEUED, rec_order, rec_X, rec_R, rec_flags);
+            sample64<true>(g, tr, prm, q[0], A, REC_QUEUED, rec_order, rec_X, rec_R, rec_flags);
         }
         A.finish(acc_out + (size_t)(nparts + 1u + blockIdx.x) * ACC_SLOTS, owned);
     }
@@ -3668,9 +3719,9 @@ extern "C" __global__ void __launch_bounds__(FT_BLOCK) ft_sample_queue_batch(
         double X[FT_E];
         double F, Gv;
         unsigned char ord[FT_E];
-        draw_sector64(g, tr, FT_EXACT_TABLE(tr), prm[P_JRFULL], X, F, Gv, ord);
+        draw_sector64<true>(g, tr, FT_EXACT_TABLE(tr), prm[P_JRFULL], X, F, Gv, ord);
         bool rob = false;
-        const bool ok = integrand64(prm, X, F, Gv, g, FT_EXACT_TABLE(tr), R, rob);
+        const bool ok = integrand64<true>(prm, X, F, Gv, g, FT_EXACT_TABLE(tr), R, rob);
         u64* qa = qacc + (size_t)id * (4 * FT_K * FT_XA_DIGITS + 4);
         u64* cnt = qa + 4 * FT_K * FT_XA_DIGITS;
         if (rob) atomicAdd(cnt + 2, 1ull);
