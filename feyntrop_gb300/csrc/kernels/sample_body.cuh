@@ -385,6 +385,15 @@ static __device__ __forceinline__ log2_parts log2_64(double x)
     r.f = double_of(log2_q62((u64)__double_as_longlong(x) & 0xfffffffffffffull | (1ull << 52)), 62);
     return r;
 }
+// The logarithms (|log2| + 1) that the power of exponent a takes in fixed point: |a log2| is
+// at most 500, so that a product of two powers stays in range and none of its factors is
+// infinite or zero by itself.
+static __device__ __forceinline__ int log2_limit(double a)
+{
+    const int e = exponent_of(a) - 1022;   // |a| < 2^e
+    return e > 9 ? 0 : 500 >> max(e, 0);
+}
+static __device__ __forceinline__ bool in_reach(log2_parts l, int limit) { return abs(l.k) < limit; }
 // x added to the fixed-point number i + f 2^-64 (|x| < 2^31)
 static __device__ __forceinline__ void fixed_add(double x, int& i, u64& f)
 {
@@ -958,7 +967,7 @@ static __device__ __forceinline__ void draw_sector64(xo& g, const table_ref& t, 
 }
 
 // ------------------------------------------------------------------ integrand, FP64
-// powers of the undeformed integrand outside log_64's range, as the reference takes them
+// powers of the undeformed integrand out of the fixed-point ones' reach, as the reference takes them
 // (srcs/feynman_integral.hpp:246-262): out = R per eps order, false when dropped
 static __device__ __noinline__ bool undeformed_slow(double psi, double pxi, double D, double W, double IGtr, double* out)
 {
@@ -1046,10 +1055,15 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
     const double D = prm[P_D], W = prm[P_W], IGtr = prm[P_IGTR];
     // normalise so that psi_tr^(-D/2) (psi_tr/xi_tr)^W = 1 (srcs/feynman_integral.hpp:201-204)
     double scale;
-    if (normal_positive(psi_tr) && normal_positive(Gv)) {
-        scale = fn64<COLD>::power(prm[P_NORM_F], fn64<COLD>::log2(psi_tr), prm[P_NORM_G], fn64<COLD>::log2(Gv));
-    } else {
-        scale = scale_slow(psi_tr, Gv, D, W, prm[P_NORM]);
+    {
+        const log2_parts lf = fn64<COLD>::log2(psi_tr), lg = fn64<COLD>::log2(Gv);
+        if (normal_positive(psi_tr) && normal_positive(Gv) &&
+            in_reach(lf, min(log2_limit(0.5 * D), log2_limit(prm[P_NORM_F]))) &&
+            in_reach(lg, min(log2_limit(W), log2_limit(prm[P_NORM_G])))) {
+            scale = fn64<COLD>::power(prm[P_NORM_F], lf, prm[P_NORM_G], lg);
+        } else {
+            scale = scale_slow(psi_tr, Gv, D, W, prm[P_NORM]);
+        }
     }
     double Xi[FT_E];
     double Xprod = 1.0;
@@ -1122,20 +1136,20 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
 #pragma unroll
     for (int e = 0; e < FT_E; e++) pxi = fma(prm[P_M2 + e], X[e], pxi);
 #endif
-    double R[FT_K];
-    if (!normal_positive(psi) || !normal_positive(pxi)) {
+    const log2_parts lp = fn64<COLD>::log2(psi), lv = fn64<COLD>::log2(pxi);
+    if (!normal_positive(psi) || !normal_positive(pxi) || !in_reach(lp, log2_limit(0.5 * D)) ||
+        !in_reach(lv, log2_limit(W))) {
+        double R[FT_K];
         const bool ok = undeformed_slow(psi, pxi, D, W, IGtr, R);
 #pragma unroll
         for (int j = 0; j < FT_K; j++) out[j] = cmk(R[j], 0.0);
         return ok;
     }
-    const log2_parts lp = fn64<COLD>::log2(psi);
 #if FT_ONLY_PSI
-    const double v = IGtr * fn64<COLD>::power(-0.5 * D, lp, 0.0, lp);
+    const double v = IGtr * fn64<COLD>::power(-0.5 * D, lp, 0.0, lv);
     if (!finite_(v)) return false;
     out[0] = cmk(v, 0.0);
 #else
-    const log2_parts lv = fn64<COLD>::log2(pxi);
     double v = IGtr * fn64<COLD>::power(-0.5 * D, lp, -W, lv);
     if (!finite_(v)) return false;
     out[0] = cmk(v, 0.0);
@@ -1434,8 +1448,9 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
     // cR = IGtr cPsi^(-D/2) cV^(-W) det J e^(i nu . theta)
     cx<double> ef, pw;   // log cPsi - L log cV, the powers
     const double np = fma(cPsi.re, cPsi.re, cPsi.im * cPsi.im), nv = fma(cV.re, cV.re, cV.im * cV.im);
-    if (normal_positive(np) && normal_positive(nv)) {
-        const log2_parts a2 = fn64<COLD>::log2(np), b2 = fn64<COLD>::log2(nv);
+    const log2_parts a2 = fn64<COLD>::log2(np), b2 = fn64<COLD>::log2(nv);
+    if (normal_positive(np) && normal_positive(nv) && in_reach(a2, log2_limit(0.25 * D)) &&
+        in_reach(b2, log2_limit(0.5 * W))) {
         const double ap = fn64<COLD>::arg(cPsi.re, cPsi.im), av = fn64<COLD>::arg(cV.re, cV.im);
         ef = cmk(0.5 * LN2_D * (small_int(a2.k - FT_LOOPS * b2.k) + fma(-(double)FT_LOOPS, b2.f, a2.f)),
                  fma(-(double)FT_LOOPS, av, ap));
