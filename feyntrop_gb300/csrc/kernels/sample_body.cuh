@@ -297,10 +297,12 @@ static __device__ __forceinline__ cx<double> cpow_(cx<double> z, double y)
 // on the integer pipes (about 200 instructions each, where table-driven FP64 versions
 // issued 12 to 31 FP64 ones, several times their cost), table-driven after Tang (ACM TOMS
 // 15 (1989), 16 (1990), 17 (1991)) with Taylor polynomials, and assembled into doubles by
-// their bits.  Their error before the final rounding is below 2^-57, so results are within
-// 0.6 ulp (sines and cosines: 2^-58 absolute).  Reciprocals and arguments stay on the FP64
-// pipe (3 and 17 instructions).  Arguments outside the stated ranges take the CUDA library's
-// function (out of line).  Qn: a fixed-point number in units of 2^-n.
+// their bits.  A logarithm's error is below 2^-61 and is multiplied by the exponent, so the
+// fixed-point powers take exponents below 32 only (their error before the final rounding is
+// then below 2^-55: 0.75 ulp); sines and cosines are within 2^-58 absolute, the sine of a
+// small angle within 0.75 ulp.  Reciprocals and arguments stay on the FP64 pipe (3 and 17
+// instructions).  Arguments outside the stated ranges take the CUDA library's function (out of
+// line).  Qn: a fixed-point number in units of 2^-n.
 static __device__ __forceinline__ int hi_word(double x) { return __double2hiint(x); }
 static __device__ __forceinline__ int exponent_of(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
 static __device__ __forceinline__ bool finite_(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
@@ -350,80 +352,104 @@ static __device__ __forceinline__ double exp2_q64(u64 f, int n)
     return round_q63(R, -n);
 }
 static __device__ __noinline__ double pow_slow(double x, double y) { return pow(x, y); }
-// (1 - u)^y, u = (x >> 11) 2^-53
+// v 2^-64 of the signed 128-bit v, shifted by s in [-58, 6]: integer part i, fraction f in Q64
+static __device__ __forceinline__ void shift_fixed(long long hi, u64 lo, int s, int& i, u64& f)
+{
+    if (s >= 0) {
+        i = (int)(((u64)hi << s) | ((lo >> 1) >> (63 - s)));
+        f = lo << s;
+    } else {
+        i = (int)(hi >> -s);
+        f = (lo >> -s) | ((u64)hi << (64 + s));
+    }
+}
+// (1 - u)^y, u = (x >> 11) 2^-53, y in [2^-60, 32)
 static __device__ __forceinline__ double pow_1mu(u64 x, double y)
 {
     const u64 q = (~x & ~0x7ffull) + 0x800ull;   // (1 - u) 2^64, 0 for u = 0
     if (q == 0ull) return 1.0;
-    const int lz = __clzll((long long)q), K = 1 + lz;
-    const u64 F = log2_q62((q << lz) >> 11);
-    // -log2(1 - u) = K - F, K in b bits: Q(64 - b)
-    const int b = 32 - __clz(K);
-    const u64 L = ((u64)K << (64 - b)) - ((F << 1) >> (b - 1));
-    const u64 P = __umul64hi(L, mantissa_of(y));
-    const int S = 63 - b - (exponent_of(y) - 1023);   // y log2 = P 2^-S
-    const int n = S < 64 ? (int)min(P >> (S & 63), 100000ull) : 0;
-    if (!normal_positive(y) || S < 1 || n > 1000) return pow_slow(1.0 - u01(x), y);
-    const u64 f = S < 64 ? P << (64 - S) : (S < 128 ? P >> (S - 64) : 0ull);   // S = 64: P
+    const int ey = (hi_word(y) >> 20) - 1023;   // negative y: far below
+    if ((u32)(ey + 60) > 64u) return pow_slow(1.0 - u01(x), y);
+    const int lz = __clzll((long long)q);
+    // y (K - F), -log2(1 - u) = K - F: the product with K is exact, with F a Q62 one
+    const u64 F = log2_q62((q << lz) >> 11), m = mantissa_of(y);
+    const u64 k = (m >> 11) * (u64)(1 + lz), p = __umul64hi(m, F << 1), lo = (k << 10) - p;
+    int n;
+    u64 f;
+    shift_fixed((long long)((k >> 54) - ((k << 10) < p)), lo, ey + 2, n, f);
+    if (n > 1000) return pow_slow(1.0 - u01(x), y);
     return exp2_q64(0ull - f, n + (f != 0ull));
 }
-// log2 x = k + f of a positive normal x, f in [0, 1] (a double), k an integer
+// log2 x = k + f of a positive normal x, f in Q62 in [0, 1], k an integer
 struct log2_parts {
     int k;
-    double kd, f;
+    u64 f;
 };
-static __device__ __forceinline__ double small_int(int k)
-{
-    const double v = double_of((u64)(k < 0 ? -k : k), 0);
-    return k < 0 ? -v : v;
-}
 static __device__ __forceinline__ log2_parts log2_64(double x)
 {
     log2_parts r;
     r.k = (hi_word(x) >> 20) - 1023;
-    r.kd = small_int(r.k);
-    r.f = double_of(log2_q62((u64)__double_as_longlong(x) & 0xfffffffffffffull | (1ull << 52)), 62);
+    r.f = log2_q62((u64)__double_as_longlong(x) & 0xfffffffffffffull | (1ull << 52));
     return r;
 }
 // The logarithms (|log2| + 1) that the power of exponent a takes in fixed point: |a log2| is
 // at most 500, so that a product of two powers stays in range and none of its factors is
-// infinite or zero by itself.
+// infinite or zero by itself, and |a| is in [2^-60, 32) or 0.
 static __device__ __forceinline__ int log2_limit(double a)
 {
     const int e = exponent_of(a) - 1022;   // |a| < 2^e
-    return e > 9 ? 0 : 500 >> max(e, 0);
+    if (e == -1022) return 500;
+    return (u32)(e + 59) > 64u ? 0 : 500 >> max(e, 0);
 }
 static __device__ __forceinline__ bool in_reach(log2_parts l, int limit) { return abs(l.k) < limit; }
-// x added to the fixed-point number i + f 2^-64 (|x| < 2^31)
-static __device__ __forceinline__ void fixed_add(double x, int& i, u64& f)
+// i + f 2^-64 += a (l.k + l.f): the product with k is exact, with f a Q62 one
+static __device__ __forceinline__ void add_product(double a, log2_parts l, int& i, u64& f)
 {
-    const int e = exponent_of(x) - 1023;
-    const u64 m = mantissa_of(x);
-    int I = e >= 0 ? (int)(m >> ((63 - e) & 63)) : 0;
-    u64 F = e >= 0 ? (m << (e & 63)) << 1 : (e >= -64 ? m >> (-e - 1) : 0ull);
-    if (hi_word(x) < 0) {
-        I = -I - (F != 0ull);
-        F = 0ull - F;
+    const int ea = exponent_of(a) - 1023;
+    if (ea < -60) return;   // 0
+    const u64 m = mantissa_of(a), k = (m >> 11) * (u64)abs(l.k), p = __umul64hi(m, l.f << 1);
+    u64 lo = k << 10, hi = k >> 54;
+    if (l.k < 0) {
+        lo = 0ull - lo;
+        hi = ~hi + (lo == 0ull);
     }
+    lo += p;
+    hi += lo < p;
+    if (hi_word(a) < 0) {
+        lo = 0ull - lo;
+        hi = ~hi + (lo == 0ull);
+    }
+    int I;
+    u64 F;
+    shift_fixed((long long)hi, lo, ea + 2, I, F);
     f += F;
     i += I + (f < F);
 }
-static __device__ __noinline__ double exp2_slow(double t) { return exp2(t); }
-// 2^(a (la.k + la.f) + b (lb.k + lb.f)): the products with their errors, summed in fixed point
+// 2^(a (la.k + la.f) + b (lb.k + lb.f)), both in reach
 static __device__ __forceinline__ double power_product(double a, log2_parts la, double b, log2_parts lb)
 {
-    const double p = a * la.kd, q = b * lb.kd;
-    const double u = fma(a, la.f, fma(a, la.kd, -p)), v = fma(b, lb.f, fma(b, lb.kd, -q));
-    const int big = max(max(exponent_of(p), exponent_of(q)), max(exponent_of(u), exponent_of(v)));
-    if (big >= 1023 + 12) return exp2_slow((p + q) + (u + v));
     int i = 0;
     u64 f = 0ull;
-    fixed_add(p, i, f);
-    fixed_add(q, i, f);
-    fixed_add(u, i, f);
-    fixed_add(v, i, f);
-    if (i > 1000 || i < -1000) return exp2_slow((p + q) + (u + v));
+    add_product(a, la, i, f);
+    add_product(b, lb, i, f);
     return exp2_q64(f, -i);
+}
+// log2 x - L log2 y as a double, its error below 2^-61 (L + 1) before the rounding
+static __device__ __forceinline__ double log2_difference(log2_parts x, log2_parts y, int L)
+{
+    const int k = x.k - L * y.k;
+    const u64 p = y.f * (u64)L, d = x.f - p, add = (u64)(long long)k << 62;
+    u64 lo = d + add, hi = (u64)((long long)k >> 2) - __umul64hi(y.f, (u64)L) - (x.f < p) + (lo < add);
+    const bool neg = (long long)hi < 0;
+    if (neg) {
+        lo = 0ull - lo;
+        hi = ~hi + (lo == 0ull);
+    }
+    if ((hi | lo) == 0ull) return 0.0;
+    const int lz = hi ? __clzll((long long)hi) : 64 + __clzll((long long)lo);
+    const u64 w = lz >= 64 ? lo << (lz - 64) : (lz ? (hi << lz) | (lo >> (64 - lz)) : hi);
+    const double v = round_q63(w, 127 - lz - 62);
+    return neg ? -v : v;
 }
 static __device__ __noinline__ void sincos_slow(double x, double* s, double* c) { sincos(x, s, c); }
 // 256 steps per turn, 64 of them in the table
@@ -433,8 +459,14 @@ static __device__ __forceinline__ void sincos_64(double x, double& sn, double& c
         sincos_slow(x, &sn, &cs);
         return;
     }
+    const int ex = exponent_of(x) - 1023;
+    if (ex < -30) {   // x^2/6 below 2^-62
+        sn = x;
+        cs = 1.0;
+        return;
+    }
     // |x| 128/pi = m C 2^e, C in Q58 and 64 more bits
-    const int S = 57 - (exponent_of(x) - 1023);
+    const int S = 57 - ex;
     const u64 m = mantissa_of(x), c0 = m * FT_STEPS_Q58;
     const u64 lo = c0 + __umul64hi(m, FT_STEPS_LO);
     const u64 hi = __umul64hi(m, FT_STEPS_Q58) + (lo < c0);
@@ -443,7 +475,8 @@ static __device__ __forceinline__ void sincos_64(double x, double& sn, double& c
     const u64 w = __umul64hi(f, FT_STEP_Q69), w2 = __umul64hi(w, w);   // Q69, Q74
     u64 h = (1ull << 63) / 120ull - (__umul64hi(w2, (1ull << 63) / 5040ull) >> 10);
     h = (1ull << 63) / 6ull - (__umul64hi(w2, h) >> 10);
-    const u64 s = __umul64hi(w, (1ull << 63) - (__umul64hi(w2, h) >> 10));   // sin w, Q68
+    const u64 ratio = (1ull << 63) - (__umul64hi(w2, h) >> 10);   // sin w / w, Q63
+    const u64 s = __umul64hi(w, ratio);                            // sin w, Q68
     h = (1ull << 63) / 720ull - (__umul64hi(w2, (1ull << 63) / 40320ull) >> 10);
     h = (1ull << 63) / 24ull - (__umul64hi(w2, h) >> 10);
     h = (1ull << 63) / 2ull - (__umul64hi(w2, h) >> 10);
@@ -451,7 +484,9 @@ static __device__ __forceinline__ void sincos_64(double x, double& sn, double& c
     const ulonglong2 T = FT_SC64[k & 63u];   // sin, cos of k pi/128, Q63
     const u64 A = (T.x >> 1) + (__umul64hi(T.y, s) >> 5) - (__umul64hi(T.x, v) >> 10);
     const u64 B0 = (T.y >> 1) - (__umul64hi(T.y, v) >> 10), B1 = __umul64hi(T.x, s) >> 5;
-    const double a = double_of(A, 62), b = double_of(B0 > B1 ? B0 - B1 : 0ull, 62);
+    // in the first step |x| itself times sin w / w, which keeps the relative accuracy
+    const double a = double_of(k ? A : __umul64hi(m, ratio), k ? 62 : 62 - ex);
+    const double b = double_of(B0 > B1 ? B0 - B1 : 0ull, 62);
     const bool odd = (k >> 6) & 1u, up = (k >> 7) & 1u;   // quadrant
     sn = odd ? b : a;
     cs = odd ? a : b;
@@ -1154,7 +1189,7 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
     if (!finite_(v)) return false;
     out[0] = cmk(v, 0.0);
     if (FT_K > 1) {
-        const double ef = LN2_D * (small_int(lp.k - FT_LOOPS * lv.k) + fma(-(double)FT_LOOPS, lv.f, lp.f));
+        const double ef = LN2_D * log2_difference(lp, lv, FT_LOOPS);
 #pragma unroll
         for (int j = 1; j < FT_K; j++) {
             v *= ef * (1.0 / (double)j);
@@ -1452,8 +1487,7 @@ static __device__ __forceinline__ bool integrand64(const double* prm, double* X,
     if (normal_positive(np) && normal_positive(nv) && in_reach(a2, log2_limit(0.25 * D)) &&
         in_reach(b2, log2_limit(0.5 * W))) {
         const double ap = fn64<COLD>::arg(cPsi.re, cPsi.im), av = fn64<COLD>::arg(cV.re, cV.im);
-        ef = cmk(0.5 * LN2_D * (small_int(a2.k - FT_LOOPS * b2.k) + fma(-(double)FT_LOOPS, b2.f, a2.f)),
-                 fma(-(double)FT_LOOPS, av, ap));
+        ef = cmk(0.5 * LN2_D * log2_difference(a2, b2, FT_LOOPS), fma(-(double)FT_LOOPS, av, ap));
         const double m = fn64<COLD>::power(-0.25 * D, a2, -0.5 * W, b2);
         double sn, cs;
         fn64<COLD>::sincos(fma(-0.5 * D, ap, -W * av), sn, cs);
