@@ -192,7 +192,7 @@ void build(ft_batch& b)
     for (ft_batch::group& g : b.groups) {
         g.key.rank = g.rank;
         keys.push_back(g.key);
-        ft::kernel_key k64 = b.plans[g.members[0]]->key(0, 0, 1);
+        ft::kernel_key k64 = b.plans[g.members[0]]->key(0, 0, 1, 1);
         k64.rank = g.rank;
         keys64.push_back(k64);
     }
@@ -201,8 +201,12 @@ void build(ft_batch& b)
         std::vector<ft::kernel_key> all;
         for (const ft::kernel_key& k : keys)
             if (!ft::find_kernels(k)) all.push_back(k);
-        for (const ft::kernel_key& k : keys64)
-            if (prec && !ft::find_kernels(k)) all.push_back(k);
+        for (ft::kernel_key k : keys64) {
+            if (!prec || ft::find_kernels(k)) continue;
+            all.push_back(k);
+            k.part = 0;   // the class's FP64 batches
+            if (!ft::find_kernels(k)) all.push_back(k);
+        }
         ft::precompile_all(all);
     }
     size_t hdr = 0, inst = 0, prep = 0, total = 0;

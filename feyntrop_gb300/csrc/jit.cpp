@@ -205,6 +205,7 @@ std::string kernel_source(const kernel_key& k)
     s << "#define FT_BLOCK " << k.block << "\n#define FT_TABLE_GLOBAL " << k.table_global << "\n";
     s << "#define FT_MINB " << k.minb << "\n#define FT_VARIANT " << k.variant << "\n";
     s << "#define FT_BATCH " << k.batch << "\n#define FT_XA_DIGITS " << kExactDigits << "\n";
+    s << "#define FT_PART " << k.part << "\n";
     s << "#define FT_SCRATCH " << k.scratch << "\n";
     s << "#define FT_Q0 " << k.q0 << "\n";
     s << "__device__ constexpr int FT_EK[" << k.E << "] = {";
@@ -428,7 +429,7 @@ static std::string key_string(const kernel_key& k)
     std::ostringstream s;
     s << k.E << "," << k.V << "," << k.K << "," << k.loops << "," << k.rank << "," << k.prec << "," << k.mode << ","
       << k.only_psi << "," << k.record << "," << k.block << "," << k.table_global << "," << k.minb << "," << k.variant
-      << "," << k.batch << "," << k.q0 << "," << k.scratch;
+      << "," << k.batch << "," << k.q0 << "," << k.scratch << "," << k.part;
     for (int e = 0; e < k.E; e++) s << ";" << k.ek[e] << "-" << k.el[e];
     return s.str();
 }
@@ -470,23 +471,17 @@ const kernel_set& get_kernels(const kernel_key& key)
     check(drv().ModuleLoadData(&ks.module, cubin.data()), "cuModuleLoadData");
     const char* sname = key.batch ? "ft_sample_batch" : "ft_sample";
     const char* qname = key.batch ? "ft_sample_queue_batch" : "ft_sample_queue";
-    check(drv().ModuleGetFunction(&ks.sample, ks.module, sname), "cuModuleGetFunction(sampling kernel)");
-    if (key.prec == 0) check(drv().ModuleGetFunction(&ks.queue, ks.module, qname), "cuModuleGetFunction(queue)");
+    CUfunction& f = key.part ? ks.queue : ks.sample;
+    check(drv().ModuleGetFunction(&f, ks.module, key.part ? qname : sname), "cuModuleGetFunction");
     ks.smem = table_smem_bytes(key);
-    CUfunction fs[2] = {ks.sample, ks.queue};
-    for (CUfunction f : fs) {
-        if (!f) continue;
-        check(drv().FuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)ks.smem),
-              "cuFuncSetAttribute(smem)");
-    }
-    check(drv().FuncGetAttribute(&ks.regs, CU_FUNC_ATTRIBUTE_NUM_REGS, ks.sample), "cuFuncGetAttribute");
-    check(drv().FuncGetAttribute(&ks.local_bytes, CU_FUNC_ATTRIBUTE_LOCAL_SIZE_BYTES, ks.sample), "cuFuncGetAttribute");
-    check(drv().OccupancyMaxActiveBlocksPerMultiprocessor(&ks.blocks_per_sm, ks.sample, ks.block, ks.smem),
+    check(drv().FuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)ks.smem),
+          "cuFuncSetAttribute(smem)");
+    check(drv().FuncGetAttribute(&ks.regs, CU_FUNC_ATTRIBUTE_NUM_REGS, f), "cuFuncGetAttribute");
+    check(drv().FuncGetAttribute(&ks.local_bytes, CU_FUNC_ATTRIBUTE_LOCAL_SIZE_BYTES, f), "cuFuncGetAttribute");
+    check(drv().OccupancyMaxActiveBlocksPerMultiprocessor(key.part ? &ks.queue_blocks_per_sm : &ks.blocks_per_sm, f,
+                                                          ks.block, ks.smem),
           "cuOccupancyMaxActiveBlocksPerMultiprocessor");
-    if (ks.queue)
-        check(drv().OccupancyMaxActiveBlocksPerMultiprocessor(&ks.queue_blocks_per_sm, ks.queue, ks.block, ks.smem),
-              "cuOccupancyMaxActiveBlocksPerMultiprocessor");
-    if (ks.blocks_per_sm < 1) throw std::runtime_error("sampling kernel does not fit on an SM");
+    if (!key.part && ks.blocks_per_sm < 1) throw std::runtime_error("sampling kernel does not fit on an SM");
     return loaded.emplace(k, ks).first->second;
 }
 

@@ -25,6 +25,7 @@ struct kernel_key {
     int minb = 1;           // minimum resident blocks per SM asked of the register allocator
     int variant = 0;        // code-size options of the kernel body (FT_VARIANT)
     int batch = 0;          // 1: the batch kernels (many integrals of the topology per launch)
+    int part = 0;           // 0: the sampling kernel, 1: the FP64 pass over hand-offs (FP64 keys only)
     int scratch = 0;        // mixed: what the threads' shared-memory scratch holds (FT_SCRATCH of the kernel body)
     int q0 = 0;             // reduced vertices [0, q0) carry no external momentum (zero rows of P~)
     std::vector<int> ek, el;   // endpoints in the kernel's vertex labels, ek > el
@@ -37,8 +38,8 @@ inline bool staged_table(int E) { return E <= 12; }
 
 struct kernel_set {
     CUmodule module = nullptr;
-    CUfunction sample = nullptr;   // ft_sample (ft_sample_batch in batch modules)
-    CUfunction queue = nullptr;    // ft_sample_queue / ft_sample_queue_batch (FP64 modules only)
+    CUfunction sample = nullptr;   // ft_sample, ft_sample_batch (part 0)
+    CUfunction queue = nullptr;    // ft_sample_queue, ft_sample_queue_batch (part 1)
     int block = 128;
     int variant = 0;               // FT_VARIANT of the module
     unsigned smem = 0;             // dynamic shared memory per block

@@ -58,6 +58,14 @@
 #ifndef FT_BATCH
 #define FT_BATCH 0
 #endif
+// The sampling kernel (0) and the FP64 pass over hand-offs (1, FP64 form) are modules of their
+// own: each holds the straight-line code of a sample.  In one module an FP64 class took 1.3 s
+// (triangle), 6.9 (double box) and 10.8 (3-loop ladder) to compile on 8 host cores; the sampling
+// kernel alone 0.8, 4.3 and 7.3.  Mixed classes compile theirs and the two FP64 modules side by
+// side: double box 6.2 -> 4.2 s, ladder 12.4 -> 6.8.
+#ifndef FT_PART
+#define FT_PART 0
+#endif
 
 typedef unsigned long long u64;
 typedef unsigned int u32;
@@ -3519,6 +3527,7 @@ static __device__ __forceinline__ void sample_range(xo& g, const table_ref& tr, 
 }
 
 #if !FT_BATCH
+#if !FT_PART
 // ------------------------------------------------------------------ single-integral kernels
 // Thread t of the launch owns samples [t*chunk, min(nsamples, (t+1)*chunk)) counted
 // from the launch's first sample, whose stream state is (s0 .. s3).  Block b writes its
@@ -3554,7 +3563,7 @@ extern "C" __global__ void __launch_bounds__(FT_BLOCK, FT_MINB) ft_sample(
     if (final_out && last_block(ticket)) sum_parts(acc_out, gridDim.x, final_out);
 }
 
-#if FT_PREC == 0
+#elif FT_PREC == 0
 // FP64 pass over the samples a mixed launch queued (grid-stride over the entries).  The
 // blocks with entries add their sums after the nparts of the sampling launch in acc_out.
 // Meanwhile the last blocks add those parts (a unit of the sums each, one warp: the FP64
@@ -3649,6 +3658,7 @@ static __device__ __forceinline__ int find_instance(const batch_inst* __restrict
 // the same as floats, then the two-float quadruples)
 #define PRM_WORDS (P_PAIR + 2 * P_SIZE)
 
+#if !FT_PART
 extern "C" __global__ void __launch_bounds__(FT_BLOCK, FT_MINB) ft_sample_batch(
     const batch_inst* __restrict__ inst, int ninst, const u64* __restrict__ total_items,
     const u64* __restrict__ inst_state, const u64* __restrict__ item_mats, const u64* __restrict__ mats, u64 chunk,
@@ -3711,7 +3721,7 @@ extern "C" __global__ void __launch_bounds__(FT_BLOCK, FT_MINB) ft_sample_batch(
     }
 }
 
-#if FT_PREC == 0
+#elif FT_PREC == 0
 // Exact, order-independent sum of doubles: digit j of an accumulator (a signed 64-bit
 // counter) weighs 2^(32 j - 1074); v = m 2^(p - 1074) with its integer significand m
 // (53 bits) enters as the three 32-bit digits of m 2^(p mod 32) at digit p / 32, so

@@ -109,7 +109,7 @@ struct ft_plan : run_scratch {
     int forced_prec = 0;
     ft::launch_shape forced_shape;
 
-    ft::kernel_key key(int prec, int record, int batch = 0) const
+    ft::kernel_key key(int prec, int record, int batch = 0, int part = 0) const
     {
         ft::kernel_key k;
         k.E = P.E;
@@ -122,6 +122,7 @@ struct ft_plan : run_scratch {
         k.only_psi = P.only_psi() ? 1 : 0;
         k.record = record;
         k.batch = batch;
+        k.part = part;
         k.ek = kek;
         k.el = kel;
         k.q0 = q0;

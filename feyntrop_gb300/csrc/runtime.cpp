@@ -487,9 +487,13 @@ run_out run(ft_plan& pl, const ft_run_options& o, cudaStream_t st, const records
 {
     const int prec = o.precision == FT_PRECISION_MIXED ? 1 : 0;
     const int record = rec ? 1 : 0;
-    if (prec && !ft::find_kernels(pl.key(prec, record))) ft::precompile_all({pl.key(prec, record), pl.key(0, record)});
+    if (prec && !ft::find_kernels(pl.key(prec, record))) {
+        // with the FP64 sampling kernel, for a run that hands over more than its queue holds
+        ft::precompile_all({pl.key(prec, record), pl.key(0, record), pl.key(0, record, 0, 1)});
+        ft::get_kernels(pl.key(0, record));
+    }
     const ft::kernel_set& ks = ft::get_kernels(pl.key(prec, record));
-    const ft::kernel_set* k64 = prec ? &ft::get_kernels(pl.key(0, record)) : nullptr;
+    const ft::kernel_set* k64 = prec ? &ft::get_kernels(pl.key(0, record, 0, 1)) : nullptr;
     const unsigned long long N = o.num_samples;
     const launch_geometry g = geometry(ks, N);
     const unsigned long long draws = 2ULL * pl.P.E - 1;
@@ -785,7 +789,9 @@ int ft_precompile(const ft_problem* pb, int32_t precision, double* seconds)
         std::vector<ft::kernel_key> keys;
         for (int bt = 0; bt <= (batch ? 1 : 0); bt++) {
             keys.push_back(pl.key(0, 0, bt));
-            if (prec == FT_PRECISION_MIXED) keys.push_back(pl.key(1, 0, bt));
+            if (prec != FT_PRECISION_MIXED) continue;
+            keys.push_back(pl.key(1, 0, bt));
+            keys.push_back(pl.key(0, 0, bt, 1));
         }
         ft::precompile_all(keys);
         if (seconds) *seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -870,7 +876,7 @@ int ft_integrate_noalloc(ft_plan* pl, const ft_run_options* o, double* d_slots)
         if (pl->slots() > NOALLOC_MAX_SLOTS)
             throw std::invalid_argument("ft_integrate_noalloc: more than 16 eps orders exceed the static scratch");
         const ft::kernel_set* ks = ft::find_kernels(pl->key(prec, 0));
-        const ft::kernel_set* k64 = prec ? ft::find_kernels(pl->key(0, 0)) : nullptr;
+        const ft::kernel_set* k64 = prec ? ft::find_kernels(pl->key(0, 0, 0, 1)) : nullptr;
         if (!ks || (prec && !k64) || !pl->d_prm)
             throw std::invalid_argument(
                 "ft_integrate_noalloc: this plan's kernels are not loaded; call ft_integrate once with the same "
@@ -978,7 +984,10 @@ int ft_autotune(ft_plan* pl, int32_t precision, uint64_t samples, ft_tune_result
                 ft::apply_shape(k, c);
                 keys.push_back(k);
             }
-            if (prec == 1) keys.push_back(pl->key(0, 0));
+            if (prec == 1) {
+                keys.push_back(pl->key(0, 0));
+                keys.push_back(pl->key(0, 0, 0, 1));
+            }
             ft::precompile_all(keys);
         }
         // trials long enough for the steady state: at least 256 samples per thread of a
