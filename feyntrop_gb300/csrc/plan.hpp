@@ -26,7 +26,9 @@ struct cuda_error : std::runtime_error {
 
 inline void cu(cudaError_t e, const char* what)
 {
-    if (e != cudaSuccess) throw cuda_error(std::string(what) + ": " + cudaGetErrorString(e));
+    if (e == cudaSuccess) return;
+    cudaGetLastError();   // reported here, not again by the next launch's check
+    throw cuda_error(std::string(what) + ": " + cudaGetErrorString(e));
 }
 
 // status code of the exception in flight (sets g_error)
