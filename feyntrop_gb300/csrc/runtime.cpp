@@ -502,8 +502,13 @@ run_out run(ft_plan& pl, const ft_run_options& o, cudaStream_t st, const records
     if (N == 0) return out;
 
     order_after_upload(pl, st);
-    if (pl.running)   // the last run failed: its counters may not be back at zero
+    if (pl.running) {
+        // the last run failed: its work may be in flight on another stream, its stride
+        // matrices unwritten, its counters not back at zero
+        cu(cudaDeviceSynchronize(), "after a failed run");
+        for (run_scratch::stride_entry& e : pl.strides) e.digits = -1;
         cu(cudaMemsetAsync(pl.d_qcount, 0, 16, st), "cudaMemsetAsync");
+    }
     pl.running = true;
     bool made = false;
     int digits = ft::stride_digits(g.lanebits);

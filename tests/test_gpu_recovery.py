@@ -25,3 +25,19 @@ def test_a_refused_allocation_fails_one_run_only():
     b.close()
     p.close()
     fresh.close()
+
+
+def test_a_run_after_a_failed_one_on_another_stream():
+    """The failed run has launched its stride matrices and stopped before the sampling kernel; the next
+    ones, on other streams, with its stride and others, give a fresh plan's values."""
+    import torch
+    p, fresh = ft.Plan(workloads.double_box()), ft.Plan(workloads.double_box())
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    for n, s in ((70_001, 0), (500, 1), (2_000_003, 2), (70_001, 1)):
+        with pytest.raises(ft.FeyntropError):
+            p.integrate(10**13, seed=1, precision=ft.MIXED, stream=streams[(s + 1) % 3].cuda_stream)
+        got = p.integrate(n, seed=2, precision=ft.MIXED, stream=streams[s].cuda_stream)
+        want = fresh.integrate(n, seed=2, precision=ft.MIXED)
+        assert got["moments"] == want["moments"] and got["kept"] == want["kept"]
+    p.close()
+    fresh.close()
