@@ -37,7 +37,7 @@ EXPORTED = ["ft_plan_create", "ft_plan_destroy", "ft_plan_get_info", "ft_plan_lo
             "ft_integrate_batch", "ft_finalize_moments", "ft_sample_records", "ft_run_json", "ft_free",
             "ft_precompile", "ft_last_error", "ft_version", "ft_subgraph_table", "ft_device_peaks", "ft_integrate_noalloc",
             "ft_batch_create", "ft_batch_destroy", "ft_batch_run", "ft_batch_get_info", "ft_plans_create",
-            "ft_autotune"]
+            "ft_autotune", "ft_release_scratch"]
 PRECOMPILE_BATCH = 0x100
 
 
@@ -254,6 +254,12 @@ class Plan:
         opts = RunOptions(int(count), int(seed), int(first_sample), int(precision), None)
         _check(lib().ft_sample_records(self.h, ctypes.byref(opts), _ptr(order), _ptr(X), _ptr(R), _ptr(flags)))
         return {"order": order.astype(np.int32), "X": X, "R": R[..., 0] + 1j * R[..., 1], "flags": flags}
+
+
+def release_scratch():
+    """Gives the device memory that closed plans left for later ones (up to 8 sets per device,
+    a few MB each for ordinary runs) back to the driver."""
+    lib().ft_release_scratch()
 
 
 def create_plans(inputs, skip_failed=False):

@@ -264,7 +264,7 @@ void build(ft_batch& b)
         off[gi].push_back(total);
         total += align_up(b.groups[gi].members.size() * 32, 256);
     }
-    cu(cudaMalloc(&b.d_static, total), "cudaMalloc(batch data)");
+    device_alloc((void**)&b.d_static, total, "cudaMalloc(batch data)");
     cu(cudaMemcpy(b.d_static, blob.data(), blob.size(), cudaMemcpyHostToDevice), "cudaMemcpy(batch data)");
     for (size_t gi = 0; gi < b.groups.size(); gi++) {
         ft_batch::group& g = b.groups[gi];
@@ -287,7 +287,7 @@ void build(ft_batch& b)
     cu(cudaMallocHost(&b.h_desc, o_more + b.hdr_bytes), "cudaMallocHost(batch descriptors and results)");
     b.h_out = (double*)(b.h_desc + o_out);
     b.h_hdr_out = (class_header*)(b.h_desc + o_more);
-    cu(cudaMalloc(&b.d_desc, o_more + (prec ? b.qacc_words * 8 : 0)), "cudaMalloc(batch descriptors and results)");
+    device_alloc((void**)&b.d_desc, o_more + (prec ? b.qacc_words * 8 : 0), "cudaMalloc(batch descriptors and results)");
     b.d_out = (double*)(b.d_desc + o_out);
     if (prec) b.d_qacc = (unsigned long long*)(b.d_desc + o_more);
     std::memset(b.h_desc, 0, b.desc_bytes);
@@ -428,7 +428,7 @@ bool ensure_capacity(ft_batch& b, const std::vector<size_t>& qwant)
             cudaFree(g.d_parts);
             g.d_parts = nullptr;
             g.item_cap = 0;
-            cu(cudaMalloc(&g.d_parts, cap * (8 * g.K + 8) * 8), "cudaMalloc(batch item sums)");
+            device_alloc((void**)&g.d_parts, cap * (8 * g.K + 8) * 8, "cudaMalloc(batch item sums)");
             g.item_cap = cap;
             grew = true;
         }
@@ -437,7 +437,7 @@ bool ensure_capacity(ft_batch& b, const std::vector<size_t>& qwant)
             g.d_item_mats = nullptr;
             g.item_digits = g.item_digits_set = 0;
             const int digits = std::max(g.want_digits, g.max_chunk ? 4 : 0);
-            cu(cudaMalloc(&g.d_item_mats, (size_t)digits * 7 * 1024 * 8), "cudaMalloc(item stride matrices)");
+            device_alloc((void**)&g.d_item_mats, (size_t)digits * 7 * 1024 * 8, "cudaMalloc(item stride matrices)");
             g.item_digits = digits;
             grew = true;
         }
@@ -453,7 +453,7 @@ bool ensure_capacity(ft_batch& b, const std::vector<size_t>& qwant)
             cudaFree(g.d_queue);
             g.d_queue = nullptr;
             g.qcap = 0;
-            cu(cudaMalloc(&g.d_queue, cap * 5 * 8), "cudaMalloc(batch FP64 queue)");
+            device_alloc((void**)&g.d_queue, cap * 5 * 8, "cudaMalloc(batch FP64 queue)");
             g.qcap = cap;
             grew = true;
         }

@@ -86,6 +86,10 @@ run_scratch acquire_scratch(int device);
 // back to the idle ones (at most 8 per device of at most 32 MB each, else freed); `dirty`: its
 // last run did not complete, so it is freed
 void release_scratch(int device, run_scratch& s, bool dirty);
+// frees the idle sets of every device
+void free_idle_scratch();
+// cudaMalloc; where the device has no room, once more without the idle sets
+void device_alloc(void** p, size_t bytes, const char* what);
 }  // namespace ftrt
 
 struct ft_plan : run_scratch {

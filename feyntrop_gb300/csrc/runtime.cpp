@@ -83,6 +83,45 @@ static scratch_pool& idle_scratch()
     return *p;
 }
 
+static void free_scratch(run_scratch& s)
+{
+    if (s.d_in) cudaFree(s.d_in);
+    if (s.h_in) cudaFreeHost(s.h_in);
+    if (s.d_parts) cudaFree(s.d_parts);
+    if (s.h_final) cudaFreeHost(s.h_final);
+    if (s.d_queue) cudaFree(s.d_queue);
+    if (s.d_qcount) cudaFree(s.d_qcount);
+    for (run_scratch::stride_entry& e : s.strides)
+        if (e.d) cudaFree(e.d);
+    if (s.ev0) cudaEventDestroy(s.ev0);
+    if (s.ev1) cudaEventDestroy(s.ev1);
+    if (s.stream) cudaStreamDestroy(s.stream);
+    s = run_scratch();
+}
+
+void free_idle_scratch()
+{
+    std::map<int, std::vector<run_scratch>> sets;
+    {
+        scratch_pool& pool = idle_scratch();
+        std::lock_guard<std::mutex> lock(pool.mu);
+        sets.swap(pool.idle);
+    }
+    for (auto& d : sets)
+        for (run_scratch& s : d.second) free_scratch(s);
+}
+
+void device_alloc(void** p, size_t bytes, const char* what)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        free_idle_scratch();
+        e = cudaMalloc(p, bytes);
+    }
+    cu(e, what);
+}
+
 run_scratch acquire_scratch(int device)
 {
     {
@@ -100,7 +139,7 @@ run_scratch acquire_scratch(int device)
         cu(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking), "cudaStreamCreate");
         cu(cudaEventCreate(&s.ev0), "cudaEventCreate");
         cu(cudaEventCreate(&s.ev1), "cudaEventCreate");
-        cu(cudaMalloc(&s.d_qcount, 16), "cudaMalloc(queue count)");
+        device_alloc((void**)&s.d_qcount, 16, "cudaMalloc(queue count)");
         cu(cudaMemset(s.d_qcount, 0, 16), "cudaMemset(queue count)");
     } catch (...) {
         release_scratch(device, s, true);
@@ -129,18 +168,7 @@ void release_scratch(int device, run_scratch& s, bool dirty)
             return;
         }
     }
-    if (s.d_in) cudaFree(s.d_in);
-    if (s.h_in) cudaFreeHost(s.h_in);
-    if (s.d_parts) cudaFree(s.d_parts);
-    if (s.h_final) cudaFreeHost(s.h_final);
-    if (s.d_queue) cudaFree(s.d_queue);
-    if (s.d_qcount) cudaFree(s.d_qcount);
-    for (run_scratch::stride_entry& e : s.strides)
-        if (e.d) cudaFree(e.d);
-    if (s.ev0) cudaEventDestroy(s.ev0);
-    if (s.ev1) cudaEventDestroy(s.ev1);
-    if (s.stream) cudaStreamDestroy(s.stream);
-    s = run_scratch();
+    free_scratch(s);
 }
 
 device_state& dev_state()
@@ -354,7 +382,7 @@ void upload(ft_plan& pl)
         pl.d_in = pl.h_in = nullptr;
         pl.in_cap = 0;
         const size_t cap = std::max<size_t>(bytes, 64 * 1024);
-        cu(cudaMalloc(&pl.d_in, cap), "cudaMalloc(parameters and table)");
+        device_alloc((void**)&pl.d_in, cap, "cudaMalloc(parameters and table)");
         cu(cudaMallocHost(&pl.h_in, cap), "cudaMallocHost(parameters and table)");
         pl.in_cap = cap;
     }
@@ -388,7 +416,7 @@ void ensure_parts(ft_plan& pl, size_t nparts)
     if (pl.d_parts) cudaFree(pl.d_parts);
     pl.d_parts = nullptr;
     pl.parts_cap = 0;
-    cu(cudaMalloc(&pl.d_parts, need * 8), "cudaMalloc(partial sums)");
+    device_alloc((void**)&pl.d_parts, need * 8, "cudaMalloc(partial sums)");
     pl.parts_cap = need;
 }
 
@@ -398,7 +426,7 @@ void ensure_queue(ft_plan& pl, size_t entries)
     if (pl.d_queue) cudaFree(pl.d_queue);
     pl.d_queue = nullptr;
     pl.qcap = 0;
-    cu(cudaMalloc(&pl.d_queue, entries * 5 * 8), "cudaMalloc(FP64 queue)");
+    device_alloc((void**)&pl.d_queue, entries * 5 * 8, "cudaMalloc(FP64 queue)");
     pl.qcap = entries;
 }
 
@@ -420,7 +448,7 @@ const unsigned long long* stride_matrices(ft_plan& pl, unsigned long long S, int
         if (victim->d) cudaFree(victim->d);
         victim->d = nullptr;
         victim->cap = -1;
-        cu(cudaMalloc(&victim->d, ft::stride_words(digits) * 8), "cudaMalloc(stride matrices)");
+        device_alloc((void**)&victim->d, ft::stride_words(digits) * 8, "cudaMalloc(stride matrices)");
         victim->cap = digits;
     }
     cu(ft::launch_stride_matrices(dev_state().tpow, S, digits, victim->d, st), "stride matrices");
@@ -751,6 +779,8 @@ int ft_plans_create(const ft_problem* problems, int32_t count, ft_plan** out, in
 }
 
 void ft_plan_destroy(ft_plan* p) { delete p; }
+
+void ft_release_scratch(void) { free_idle_scratch(); }
 
 int ft_plan_get_info(const ft_plan* pl, ft_plan_info* info)
 {
@@ -1121,10 +1151,10 @@ int ft_sample_records(ft_plan* pl, const ft_run_options* o, uint8_t* order, doub
         upload(*pl);
         const size_t N = o->num_samples, E = pl->P.E, K = pl->P.K;
         records d;
-        cu(cudaMalloc(&d.order, N * E + 1), "cudaMalloc(records)");
-        cu(cudaMalloc(&d.X, N * E * 8 + 8), "cudaMalloc(records)");
-        cu(cudaMalloc(&d.R, N * K * 16 + 16), "cudaMalloc(records)");
-        cu(cudaMalloc(&d.flags, N + 1), "cudaMalloc(records)");
+        device_alloc((void**)&d.order, N * E + 1, "cudaMalloc(records)");
+        device_alloc((void**)&d.X, N * E * 8 + 8, "cudaMalloc(records)");
+        device_alloc((void**)&d.R, N * K * 16 + 16, "cudaMalloc(records)");
+        device_alloc((void**)&d.flags, N + 1, "cudaMalloc(records)");
         cu(cudaMemset(d.flags, 0, N + 1), "cudaMemset");
         run(*pl, *o, pl->stream, &d);
         if (order) cu(cudaMemcpy(order, d.order, N * E, cudaMemcpyDeviceToHost), "cudaMemcpy");

@@ -57,6 +57,12 @@ typedef struct {
 int ft_plan_create(const ft_problem* problem, ft_plan** out);
 void ft_plan_destroy(ft_plan* plan);
 
+/* Destroyed plans leave their streams and scratch to later ones: up to 8 sets per device,
+ * a few MB each for ordinary runs and at most 32.  This gives the idle sets back to the
+ * driver (no counterpart in the reference).  The library does so itself when a device
+ * allocation of its own fails. */
+void ft_release_scratch(void);
+
 /* ft_plan_create for many problems at once on all host threads (kinematic scans,
  * batches; the reference prepares one input per process, srcs/feyntrop.cpp:143-158).  out[i] is NULL where problem i failed; status[i] (may be NULL) holds each
  * problem's code.  Returns FT_OK, or the code of the first failure (its message, with
