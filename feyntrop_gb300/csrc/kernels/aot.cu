@@ -26,7 +26,8 @@ namespace {
 __global__ void __launch_bounds__(1024) ft_stride_matrices(const u64* __restrict__ tpow, u64 S, int lanes,
                                                            u64* __restrict__ out)
 {
-    __shared__ u64 A[1024], M[1024];
+    __shared__ __align__(16) u64 A[1024];   // read in 16-byte words
+    __shared__ u64 M[1024];
     __shared__ ulonglong2 part[4][256][2];
     const int w = threadIdx.x >> 8, c = threadIdx.x & 255;
     int b = (int)blockIdx.x;
