@@ -385,10 +385,20 @@ void capture(ft_batch& b)
 
 // Samples per thread of the FP64 form's work items: the chunk, an eighth of the largest or a
 // multiple of it, that ends first when every block takes the same number of items and an item
-// costs its samples and a start worth `start` of them.  Pentabox points, 12 of 1e4 to 3e5
-// samples (338 items of 8 for 152 blocks: three rounds, the last a fifth full): chunks of 1, 2,
-// 3, 4, 6, 8, 16 take 4.37, 3.98, 3.88, 4.18, 3.75, 4.82, 6.25 ms, 0.2 ms times this count.  A
-// function of the counts alone, so that equal runs add in equal order.
+// costs its samples and a start worth `start` of them.  Kernel ms of one batch with fixed
+// chunks, and what this rule takes:
+//   chunk                              1      2      4      6      8     12     16     rule
+//   12 box-pentagons, 1e4 to 3e5     3.77   3.54   3.80   3.41   4.48   4.47   5.92   3.41
+//   12 K4, 1e4 to 3e5                0.681  0.471  0.409  0.410  0.410  0.526  0.398  0.354 (14)
+//   24 K4, 1e5 to 3e6               13.16   8.44   6.97   6.49   6.30   6.00   5.88   5.88
+//   12 triangles, 1e4 to 3e5         0.581  0.385  0.315  0.312  0.275  0.349  0.250  0.225 (14)
+//   12 cubes, 1e5 to 1e6             4.69   3.67   3.21   3.12   2.97   3.10   2.83   2.83
+//   20 of every kind, 1e4 to 1e5     1.88   1.61   1.88   1.90   2.02   3.00   3.97   1.70
+//   20 of every kind, 1e5 to 1e6    17.39  15.66  15.16  14.73  15.12  14.25  15.26  14.74
+// (the classes of a batch share the SMs; each counts the whole grid here).  A function of the
+// counts alone, so that equal runs add in equal order; beside integrals of other counts the low
+// words of an integral's sums may differ, its values did not (1440 in 120 runs).  Where a run's
+// chunk is not the last one's, its matrices take 0.1 ms more.
 unsigned long long run_chunk(const ft_batch& b, const ft_batch::group& g, const ft_run_options* opts)
 {
     const double start = g.key.mode == 1 ? 0.2 : 1.0;

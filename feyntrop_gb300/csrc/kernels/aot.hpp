@@ -36,7 +36,7 @@ inline unsigned long long exact_words(int K) { return 4ull * (unsigned long long
 
 // Limits of the no-allocation path (ft_integrate_noalloc): per-block partial moments
 // for up to 2048 blocks of up to 136 slots (16 eps orders), 65536 FP64 hand-off
-// entries, stride matrices for up to 2^24 threads.  About 7 MB per device.
+// entries, stride matrices for up to 2^24 threads.  6.3 MB per device.
 #define NOALLOC_MAX_BLOCKS 2048
 #define NOALLOC_MAX_SLOTS 136
 #define NOALLOC_PART_DOUBLES ((NOALLOC_MAX_BLOCKS + 1) * NOALLOC_MAX_SLOTS)   // one for the sampling launch's sum

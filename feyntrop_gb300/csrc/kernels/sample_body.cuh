@@ -133,7 +133,6 @@ static __device__ constexpr bool first_in_slot(int e)
     return true;
 }
 #define FT_FULL ((1u << FT_E) - 1u)
-#define FT_NPAIR (FT_E * (FT_E - 1) / 2)
 
 // ------------------------------------------------------------------ parameter block
 // doubles: 0 D, 1 W, 2 IGtr, 3 def_ref, 4 norm = 1/(D/2*L+W), 5 Jr(full), 6 -norm D/2, 7 -norm W,
@@ -280,15 +279,9 @@ static __device__ __forceinline__ cx<T> crecip(cx<T> z)
     return cmk(r * id, -i * id);
 }
 static __device__ __forceinline__ double cabs_(cx<double> z) { return hypot(z.re, z.im); }
-// principal logarithm, exp, real power (the reference's std::log / std::pow on
+// principal logarithm and real power (the reference's std::log / std::pow on
 // complex<double>, srcs/feynman_integral.hpp:310,327,354)
 static __device__ __forceinline__ cx<double> clog_(cx<double> z) { return cmk(log(hypot(z.re, z.im)), atan2(z.im, z.re)); }
-static __device__ __forceinline__ cx<double> cexp_(cx<double> z)
-{
-    double s, c, m = exp(z.re);
-    sincos(z.im, &s, &c);
-    return cmk(m * c, m * s);
-}
 static __device__ __forceinline__ cx<double> cpow_(cx<double> z, double y)
 {
     double lr = log(hypot(z.re, z.im)), th = atan2(z.im, z.re);
@@ -876,8 +869,6 @@ __shared__ const unsigned char* s_batch_tab;
 // sample in the lane's chunk (the other four hold the sample's stream state)
 #define BQ_ITEM_SHIFT 28
 #define BQ_LANE_SHIFT 18
-#define BQ_OFF_MASK ((1ull << BQ_LANE_SHIFT) - 1ull)
-#define BQ_LANE_MASK 1023ull
 #else
 #define TABLE_GM(t) ((t).gm)
 #define FT_EXACT_TABLE(t) ((t).gm)
@@ -1565,13 +1556,6 @@ static __device__ __forceinline__ V rcp_newton(V x)
 {
     const V r = rcp_fast(x);
     return fma_(r, fma_(x, -r, all_of<V>(1.0f)), r);
-}
-// x^(-1/2): the approximate instruction and one Newton step
-static __device__ __forceinline__ float rsqrt_newton(float x)
-{
-    float r;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return fmaf(0.5f * r, fmaf(x * r, -r, 1.0f), r);
 }
 
 // Two-float numbers hi + lo (about 48 significant bits) from error-free transformations
@@ -2784,17 +2768,6 @@ static __device__ __forceinline__ bool integrand_one(const float4* pp, const flo
 #endif
 
 // ------------------------------------------------------------------ accumulation
-// double-double sum of two (hi, lo) pairs
-static __device__ __forceinline__ void dd_add(double& ah, double& al, double bh, double bl)
-{
-    double s = ah + bh;
-    double bb = s - ah;
-    double err = (ah - (s - bb)) + (bh - bb);
-    err += al + bl;
-    ah = s + err;
-    al = err - (ah - s);
-}
-
 // stream state from 4 words (16-byte aligned)
 static __device__ __forceinline__ xo load_state(const u64* __restrict__ s)
 {

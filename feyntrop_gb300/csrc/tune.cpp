@@ -86,18 +86,23 @@ launch_shape default_shape(const kernel_key& k)
     // their instruction fetches.
     // Mixed, undeformed (two samples per thread): 16 warps of 128 registers in one block (1e9
     // samples/s against 256 threads with up to 255 registers: K4 24.4 / 19.8, wheel 19.2 /
-    // 16.0, undeformed box-pentagon 18.0 / 15.1, 3-loop ladder 14.2 / 12.1, cube 10.05 / 9.66,
-    // triangle 43.8 / 44.8; two blocks of 256 3 to 6 % below the one).
+    // 16.0, undeformed box-pentagon 18.0 / 15.1, 3-loop ladder 14.2 / 12.1, triangle 43.8 / 44.8;
+    // two blocks of 256 3 to 6 % below the one).  The cube's table leaves one block of 256 threads
+    // whatever is asked for (apply_shape): 10.05 held to 128 registers, 9.66 with up to 255.
     // Mixed, deformed: 16 warps of 128 registers per SM.  Single integrals: one block, which
     // keeps all of them together, with one out-of-line copy of the complex two-float product
     // (bit 4; also of the FP32 transcendentals and the larger two-float routines, bits 0 and 3:
     // double box 16.4 ms against 15.9, ladder 7.96 against 7.07; without any 18.3 and 8.6).
     // Batches, where a block also waits for its slowest warp at every item's end: two blocks,
     // with all three (24 box-pentagon points 12.2 ms, one block 12.5; bit 4 alone 12.35).
-    // FP64 form, bound by the FP64 pipe: 12 to 16 warps per SM keep it busy (double box 3e6:
-    // 7.1 ms with 384 threads, 7.4 with 256; box-pentagon scan 3.4 against 4.5; cube 1.26 with
-    // 512 against 1.40), two blocks where the staged table leaves the room (up to E = 10; K4
-    // 3.13 ms, one block of 512 3.48).
+    // FP64 form, bound by the FP64 pipe: 12 to 16 warps per SM keep it busy.  Deformed, ms with
+    // 256, 384 and 512 threads: double box, 3e6 samples, 7.4, 7.1; 12 box-pentagon points of 1e4
+    // to 3e5 3.70, 3.41, 3.47; 4-loop ladder (E = 13), 6e6, 51.4, 47.4, 47.4; 5-loop (E = 16),
+    // 3e6, 39.9, 39.1, 37.6 (the spills that fewer registers add cost less than the warps give).
+    // Undeformed with 256 x 2, 256, 384 and 512: 24 K4 points of 1e5 to 3e6 5.87, 7.96, 7.30,
+    // 7.13; 24 triangles 3.53, 5.08, 4.70, 4.54; where the table leaves no room for two blocks
+    // (above E = 10), 12 cubes of 1e5 to 1e6 3.35, 3.34, 2.96, 2.85; 4-loop ladder, 1e7, 13.28,
+    // 11.45, 10.54 (256, 384, 512).
     launch_shape s;
     if (k.prec == 1) {
         s.block = k.batch && k.mode == 1 ? 256 : 512;
@@ -138,10 +143,14 @@ void apply_shape(kernel_key& k, const launch_shape& s)
     k.block = s.block;
     k.minb = s.minb;
     k.variant = s.variant;
-    // as much of the deformed integrand's scratch in shared memory as fits
+    // as much of the deformed integrand's scratch in shared memory as fits beside minb blocks.
+    // Not raised again for a block that is halved below: what its table and sums leave serves the
+    // spilled frames as L1 (a cube above threshold, E = 12, 1e7 samples: 13.0 ms with 3 eps orders,
+    // 14.1 with the angles in shared memory; in a batch 14.2 and 16.8).
     k.scratch = k.prec == 1 && k.mode == 1 ? 2 : 0;
     while (k.scratch > 0 && block_smem_bytes(k) * (unsigned)k.minb > kSmemLimit) k.scratch--;
-    // keep the warps per SM while halving the block until the shared memory fits
+    // keep the warps per SM while halving the block until the shared memory fits (with a staged
+    // table of E = 12 only one block does: minb then only bounds the registers)
     while (k.block > 64 && block_smem_bytes(k) > kSmemLimit) {
         k.block /= 2;
         k.minb = k.minb * 2 > 32 ? 32 : k.minb * 2;

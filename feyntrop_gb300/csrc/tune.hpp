@@ -27,10 +27,12 @@ launch_shape choose_shape(const kernel_key& k);
 // default shape (no table, no environment)
 launch_shape default_shape(const kernel_key& k);
 
-// default samples per thread of a batch's work items: items of about a millisecond, so that a
-// batch of a few items per block does not wait for the last ones (24 box-pentagon points of
-// 1e5 to 3e6 samples: 12.4 ms with 32, 15.5 with 128, 13.6 with 8, whose start and sums
-// show; 12 FP64 points 3.4 with 8, 3.4 with 16)
+// default samples per thread of a batch's work items (FP64: the most that a run takes, run_chunk
+// of batch.cpp): items of about a millisecond, so that a batch of a few items per block does not
+// wait for the last ones (24 mixed box-pentagon points of 1e5 to 3e6 samples: 12.4 ms with 32,
+// 15.5 with 128, 13.6 with 8, whose start and sums show; FP64, 8, 16 and 24: a batch of 20 of every
+// kind, 1e5 to 1e6, 15.1, 15.3, 16.2; 24 K4 points of 1e5 to 3e6 6.30, 5.88, 5.76, and longer items
+// only balance worse: 12 of 1e4 to 3e5 0.41, 0.40, 0.57)
 unsigned long long default_chunk(const kernel_key& k);
 
 // record a tuned shape for the class of k (in memory and in the table file)

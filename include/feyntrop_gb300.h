@@ -167,7 +167,7 @@ int ft_batch_get_info(const ft_batch* batch, ft_batch_info* info);
  * (hi, lo), sum f^2 (hi, lo); then kept, dropped, samples handed to the FP64 pass
  * (all of them, also those beyond the queue), exact sector steps, complete-pivoting
  * factorisations.
- * Scratch is one static device array per GPU (about 7 MB, held until exit): at most
+ * Scratch is one static device array per GPU (6.3 MB, held until exit): at most
  * 2048 blocks, 16 eps orders and 65536 samples handed to the FP64 pass per call; the
  * hand-offs beyond 65536 are not evaluated, which slot 8K+2 > 65536 (equivalently
  * kept + dropped < N) reports.  The plan's kernels must already be
