@@ -57,8 +57,10 @@ void fill_result(const ft::prepared& P, const std::vector<double>& acc, ft_resul
 // are handed from plan to plan (acquire, release in runtime.cpp): making one takes 200 us
 // and freeing it 90, more than a small integration.
 struct run_scratch {
-    unsigned char *d_in = nullptr, *h_in = nullptr;   // parameter block and table: device, pinned staging
+    // parameter block and table: device, pinned staging (NULL above kStagedBytes)
+    unsigned char *d_in = nullptr, *h_in = nullptr;
     size_t in_cap = 0;
+    static constexpr size_t kStagedBytes = 12u << 20;
     double* d_parts = nullptr;
     size_t parts_cap = 0;
     double* h_final = nullptr;   // pinned, written by the last block of a launch

@@ -155,7 +155,7 @@ void release_scratch(int device, run_scratch& s, bool dirty)
         s.d_queue = nullptr;
         s.qcap = 0;
     }
-    size_t bytes = 2 * s.in_cap + s.parts_cap * 8 + s.final_cap * 8 + s.qcap * 40;
+    size_t bytes = (s.h_in ? 2 : 1) * s.in_cap + s.parts_cap * 8 + s.final_cap * 8 + s.qcap * 40;
     for (const run_scratch::stride_entry& e : s.strides)
         if (e.d) bytes += ft::stride_words(e.cap) * 8;
     if (!dirty && bytes <= (32u << 20)) {
@@ -376,14 +376,19 @@ void upload(ft_plan& pl)
     if (!pl.stream) static_cast<run_scratch&>(pl) = acquire_scratch(pl.device);
     const std::vector<double> blk = param_block(pl.prm);
     const size_t off = (blk.size() * 8 + 255) & ~(size_t)255, bytes = off + pl.tab.size();
-    if (bytes > pl.in_cap) {
+    // up to 12 MB (E = 18) through pinned staging, which the next plans of the set use again.  Larger
+    // tables go from the plan's own memory: pinning as much again, for sets too large to be kept,
+    // cost more than it saved (E = 19, 23 MB: first integration of a plan 2.3 -> 0.45 ms, closing it
+    // 0.61 -> 0.004, as its set now fits the 32 MB)
+    const bool staged = bytes <= pl.kStagedBytes;
+    if (bytes > pl.in_cap || (staged && !pl.h_in)) {
         if (pl.d_in) cudaFree(pl.d_in);
         if (pl.h_in) cudaFreeHost(pl.h_in);
         pl.d_in = pl.h_in = nullptr;
         pl.in_cap = 0;
         const size_t cap = std::max<size_t>(bytes, 64 * 1024);
         device_alloc((void**)&pl.d_in, cap, "cudaMalloc(parameters and table)");
-        cu(cudaMallocHost(&pl.h_in, cap), "cudaMallocHost(parameters and table)");
+        if (staged) cu(cudaMallocHost(&pl.h_in, cap), "cudaMallocHost(parameters and table)");
         pl.in_cap = cap;
     }
     if ((size_t)pl.slots() > pl.final_cap) {
@@ -393,10 +398,17 @@ void upload(ft_plan& pl)
         cu(cudaMallocHost(&pl.h_final, pl.slots() * 8), "cudaMallocHost(final)");
         pl.final_cap = pl.slots();
     }
-    std::memcpy(pl.h_in, blk.data(), blk.size() * 8);
-    std::memcpy(pl.h_in + off, pl.tab.data(), pl.tab.size());
     pl.uploading = true;
-    cu(cudaMemcpyAsync(pl.d_in, pl.h_in, bytes, cudaMemcpyHostToDevice, pl.stream), "cudaMemcpyAsync(parameters)");
+    if (staged) {
+        std::memcpy(pl.h_in, blk.data(), blk.size() * 8);
+        std::memcpy(pl.h_in + off, pl.tab.data(), pl.tab.size());
+        cu(cudaMemcpyAsync(pl.d_in, pl.h_in, bytes, cudaMemcpyHostToDevice, pl.stream), "cudaMemcpyAsync(parameters)");
+    } else {   // pageable: read before the calls return
+        cu(cudaMemcpyAsync(pl.d_in, blk.data(), blk.size() * 8, cudaMemcpyHostToDevice, pl.stream),
+           "cudaMemcpyAsync(parameters)");
+        cu(cudaMemcpyAsync(pl.d_in + off, pl.tab.data(), pl.tab.size(), cudaMemcpyHostToDevice, pl.stream),
+           "cudaMemcpyAsync(table)");
+    }
     pl.d_prm = (double*)pl.d_in;
     pl.d_tab = pl.d_in + off;
 }
