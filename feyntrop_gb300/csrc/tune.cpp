@@ -1,5 +1,6 @@
 #include "tune.hpp"
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <fstream>
@@ -140,7 +141,7 @@ static unsigned block_smem_bytes(const kernel_key& k)
 
 void apply_shape(kernel_key& k, const launch_shape& s)
 {
-    k.block = s.block;
+    k.block = std::max(32, s.block & ~31);   // whole warps: their collective operations name all lanes
     k.minb = s.minb;
     k.variant = s.variant;
     // as much of the deformed integrand's scratch in shared memory as fits beside minb blocks.
@@ -151,8 +152,9 @@ void apply_shape(kernel_key& k, const launch_shape& s)
     while (k.scratch > 0 && block_smem_bytes(k) * (unsigned)k.minb > kSmemLimit) k.scratch--;
     // keep the warps per SM while halving the block until the shared memory fits (with a staged
     // table of E = 12 only one block does: minb then only bounds the registers)
-    while (k.block > 64 && block_smem_bytes(k) > kSmemLimit) {
-        k.block /= 2;
+    // (many eps orders: 12 edges and 14 orders halve the FP64 form's 384 threads three times)
+    while (k.block > 32 && block_smem_bytes(k) > kSmemLimit) {
+        k.block = (k.block / 2 + 31) & ~31;
         k.minb = k.minb * 2 > 32 ? 32 : k.minb * 2;
     }
 }
